@@ -264,6 +264,7 @@ void nb6_lib_opened();             // gpunb_open_ / irr_simd_open_
 void nb6_lib_closed();             // their closes: the pool stops with the last
 int nb6_check_dev_status();        // read (and clear) after a stream sync
 void nb6_status_fetch(cudaStream_t st);  // enqueue the status copy before that sync
+int *nb6_status_post();            // or: the pinned word for the call's last kernel to write
 bool nb6_uva();                    // device reads/writes pinned host memory in place
 int nb6_num_sms();
 

@@ -1086,27 +1086,21 @@ NB6_DEV void add_partial(const float4 *p, double *v) {
 // Second half of a finalize row (one warp, one i): reduce the lanes' FP64
 // sums, write outf, reset the neighbour counter, and write the list row
 // sorted ascending (warp bitonic sort in shared memory) or -nnb on overflow.
+// Host calls have the rows written straight into pinned host memory, where a
+// store costs a bus transaction of its own unless the warp's lanes write one
+// run: the eight doubles leave as one 64-byte store and the list row (its
+// stride ls a multiple of 32 ints there) as whole 128-byte lines, count
+// included (a call of 531 bodies 217 -> 198 us, one of 7 bodies 61 -> 52 us).
 NB6_DEV void finalize_row(int i, int lane, double *v, int *__restrict__ nbcnt,
-                          const int *__restrict__ nbbuf, int lcap, int cap, int W, int *sb,
+                          const int *__restrict__ nbbuf, int lcap, int cap, int ls, int *sb,
                           double *__restrict__ outf, int *__restrict__ outl, const MlpArgs &mlp,
                           const __nv_bfloat16 *sw) {
 #pragma unroll
     for (int c = 0; c < 7; ++c) v[c] = warp_sum_d(v[c]);
-    if (lane == 0) {
-        double *o = outf + (size_t)i * 8;
-        o[0] = v[0] * 0.125;
-        o[1] = v[1] * 0.125;
-        o[2] = v[2] * 0.125;
-        o[3] = v[3] * 0.125;
-        o[4] = v[4] * 0.125;
-        o[5] = v[5] * 0.125;
-        o[6] = v[6] * 0.5;
-        o[7] = 0.0;
-    }
-
     const int n = nbcnt[i];
     __syncwarp();
     if (lane == 0) nbcnt[i] = 0;
+    double o = 0.0;   // lane c < 8 holds value c of the row
     if (mlp.on) {
         // learned radius proposal from this call's own results (out slot 7)
         float fe[MLP_IN];
@@ -1114,9 +1108,13 @@ NB6_DEV void finalize_row(int i, int lane, double *v, int *__restrict__ nbcnt,
         mlp_features((double)n, mlp.h2[i], ax * ax + ay * ay + az * az, mlp.dtr[i], fe);
         MlpAct act;
         const float out = mlp_forward_warp(sw, mlp.norm, fe, lane, act);
-        if (lane == 0) outf[(size_t)i * 8 + 7] = (double)(out * mlp.norm[2 * MLP_IN + 1] + mlp.norm[2 * MLP_IN]);
+        o = (double)(out * mlp.norm[2 * MLP_IN + 1] + mlp.norm[2 * MLP_IN]);
     }
-    int *row = outl + (size_t)i * W;
+#pragma unroll
+    for (int c = 0; c < 7; ++c)
+        if (lane == c) o = v[c] * (c < 6 ? 0.125 : 0.5);
+    if (lane < 8) outf[(size_t)i * 8 + lane] = o;
+    int *row = outl + (size_t)i * ls;
     if (n > cap) {
         if (lane == 0) row[0] = -n;
         return;
@@ -1142,8 +1140,13 @@ NB6_DEV void finalize_row(int i, int lane, double *v, int *__restrict__ nbcnt,
             __syncwarp();
         }
     }
-    if (lane == 0) row[0] = n;
-    for (int k = lane; k < n; k += 32) row[1 + k] = sb[k];
+    for (int k = lane; k <= n; k += 32) row[k] = k == 0 ? n : sb[k - 1];
+}
+
+// The device status word into the pinned copy the host reads after the
+// call's synchronize (hstatus null: the caller fetches it itself).
+NB6_DEV void post_status(const int *status, int *hstatus) {
+    if (hstatus && blockIdx.x == 0 && threadIdx.x == 0) *hstatus = *status;
 }
 
 // One warp per i: FP64 sum over slices in a fixed order, then the neighbour
@@ -1153,8 +1156,9 @@ NB6_DEV void finalize_row(int i, int lane, double *v, int *__restrict__ nbcnt,
 __global__ void __launch_bounds__(FIN_WARPS * 32)
     regf_finalize(const float4 *__restrict__ part, int nslices, int ni, int ni_pad,
                   int *__restrict__ nbcnt, const int *__restrict__ nbbuf, int lcap,
-                  int cap, int W, int pmax, double *__restrict__ outf,
-                  int *__restrict__ outl, const MlpArgs mlp) {
+                  int cap, int ls, int pmax, double *__restrict__ outf,
+                  int *__restrict__ outl, const int *status, int *hstatus, const MlpArgs mlp) {
+    post_status(status, hstatus);
     extern __shared__ __align__(16) int sbuf[];
     __nv_bfloat16 *sw = reinterpret_cast<__nv_bfloat16 *>(sbuf + FIN_WARPS * pmax);
     if (mlp.on) {
@@ -1167,7 +1171,7 @@ __global__ void __launch_bounds__(FIN_WARPS * 32)
     if (i >= ni) return;
     double v[7] = {0, 0, 0, 0, 0, 0, 0};
     for (int sl = lane; sl < nslices; sl += 32) add_partial(part + ((size_t)sl * ni_pad + i) * 4, v);
-    finalize_row(i, lane, v, nbcnt, nbbuf, lcap, cap, W, sbuf + warp * pmax, outf, outl, mlp, sw);
+    finalize_row(i, lane, v, nbcnt, nbbuf, lcap, cap, ls, sbuf + warp * pmax, outf, outl, mlp, sw);
 }
 
 // ----------------------------------------------------------------------------
@@ -1242,8 +1246,10 @@ __global__ void __launch_bounds__(JPAR_NT)
 
 __global__ void __launch_bounds__(FIN_WARPS * 32)
     regf_finalize_seg(const float4 *__restrict__ part, const int2 *__restrict__ pinfo, int ni,
-                      int *__restrict__ nbcnt, const int *__restrict__ nbbuf, int lcap, int cap, int W,
-                      int pmax, double *__restrict__ outf, int *__restrict__ outl, const MlpArgs mlp) {
+                      int *__restrict__ nbcnt, const int *__restrict__ nbbuf, int lcap, int cap, int ls,
+                      int pmax, double *__restrict__ outf, int *__restrict__ outl, const int *status,
+                      int *hstatus, const MlpArgs mlp) {
+    post_status(status, hstatus);
     extern __shared__ __align__(16) int sbuf[];
     __nv_bfloat16 *sw = reinterpret_cast<__nv_bfloat16 *>(sbuf + FIN_WARPS * pmax);
     if (mlp.on) {
@@ -1257,7 +1263,7 @@ __global__ void __launch_bounds__(FIN_WARPS * 32)
     const int2 pi = pinfo[i];
     double v[7] = {0, 0, 0, 0, 0, 0, 0};
     for (int q = lane; q < pi.y; q += 32) add_partial(part + ((size_t)pi.x + q) * 4, v);
-    finalize_row(i, lane, v, nbcnt, nbbuf, lcap, cap, W, sbuf + warp * pmax, outf, outl, mlp, sw);
+    finalize_row(i, lane, v, nbcnt, nbbuf, lcap, cap, ls, sbuf + warp * pmax, outf, outl, mlp, sw);
 }
 
 // FP64 (m, x, v) -> SoA float4 tiles; padding slots are massless and far.
@@ -1767,6 +1773,8 @@ struct RegLaunch {
     Plan plan;
     RegArgs a;
     int ni = 0, W = 1, cap = 0, pmax = 32, fblocks = 1;
+    int ls = 1;                  // stride of the list rows regf_finalize writes
+    int *hstatus = nullptr;      // where it posts the status word (direct calls)
     size_t smem = 0;
     bool mf = false;
     MlpArgs mlp{};
@@ -1781,22 +1789,29 @@ struct RegLaunch {
     bool direct = false;
 };
 
+// Row stride of a list of W ints in the pinned staging: whole 128-byte lines,
+// so that a row's lines are written by one store each (finalize_row).
+static int host_row_stride(int W) { return (W + 31) / 32 * 32; }
+
 // Arguments of regf_finalize, addressable for a kernel node.
 struct FinArgs {
     const float4 *part;
     int nslices, ni, ni_pad;
     int *nbcnt;
     const int *nbbuf;
-    int lcap, cap, W, pmax;
+    int lcap, cap, ls, pmax;
     double *outf;
     int *outl;
+    const int *status;
+    int *hstatus;
     MlpArgs mlp;
-    void *p[13];
+    void *p[15];
     explicit FinArgs(const RegLaunch &L)
         : part(L.a.part), nslices(L.plan.nslices), ni(L.ni), ni_pad(L.a.ni_pad), nbcnt(L.a.nbcnt),
-          nbbuf(L.a.nbbuf), lcap(L.a.lcap), cap(L.cap), W(L.W), pmax(L.pmax), outf(L.outf),
-          outl(L.outl), mlp(L.mlp) {
-        void *q[13] = {&part, &nslices, &ni, &ni_pad, &nbcnt, &nbbuf, &lcap, &cap, &W, &pmax, &outf, &outl, &mlp};
+          nbbuf(L.a.nbbuf), lcap(L.a.lcap), cap(L.cap), ls(L.ls), pmax(L.pmax), outf(L.outf),
+          outl(L.outl), status(L.a.status), hstatus(L.hstatus), mlp(L.mlp) {
+        void *q[15] = {&part, &nslices, &ni,   &ni_pad, &nbcnt,  &nbbuf,   &lcap, &cap,
+                       &ls,   &pmax,    &outf, &outl,   &status, &hstatus, &mlp};
         memcpy(p, q, sizeof(q));
     }
 };
@@ -2008,11 +2023,13 @@ static void regf_prepare(int ni, const double *d_h2, const double *d_dtr, const 
         NB6_CUDA_CHECK(cudaFuncSetAttribute(regf_finalize, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                             (int)smem));
     L.mlp = mlp;
+    L.direct = L.hin != nullptr && nb6_uva();
+    L.ls = L.direct ? host_row_stride(W) : W;
+    L.hstatus = L.direct ? nb6_status_post() : nullptr;
     if (L.hin) {
         R.houtf.reserve((size_t)ni * 8);
-        R.houtl.reserve((size_t)ni * W);
+        R.houtl.reserve((size_t)ni * L.ls);
     }
-    L.direct = L.hin != nullptr && nb6_uva();
     L.outf = L.direct ? R.houtf.ptr : R.outf.ptr;
     L.outl = L.direct ? R.houtl.ptr : R.outl.ptr;
     L.plan = plan;
@@ -2046,8 +2063,8 @@ static void regf_eager(const RegLaunch &L, cudaStream_t st) {
     NB6_CUDA_CHECK(cudaGetLastError());
     NB6_CUDA_CHECK(cudaEventRecord(R.ev1, st));
     regf_finalize<<<L.fblocks, FIN_WARPS * 32, L.smem, st>>>(
-        L.a.part, L.plan.nslices, L.ni, L.a.ni_pad, R.nbcnt.ptr, R.nbbuf.ptr, L.a.lcap, L.cap, L.W,
-        L.pmax, L.outf, L.outl, L.mlp);
+        L.a.part, L.plan.nslices, L.ni, L.a.ni_pad, R.nbcnt.ptr, R.nbbuf.ptr, L.a.lcap, L.cap, L.ls,
+        L.pmax, L.outf, L.outl, L.a.status, L.hstatus, L.mlp);
     NB6_CUDA_CHECK(cudaGetLastError());
     if (L.hin && !L.direct) regf_copy_out(L, st);
     R.nbcnt_dirty = false;
@@ -2531,12 +2548,10 @@ void gpunb_regf_(int *ni_, double *h2, double *dtr, double (*xi)[3], double (*vi
     L.hin = h;
     L.in_bytes = sizeof(double) * nin;
     regf_prepare(ni, d, d + ni, d + 2 * (size_t)ni, d + 5 * (size_t)ni, lmax, nnbmax, *m_flag, st, L);
-    const int W = L.W;
     regf_submit(L, st);
-    nb6_status_fetch(st);
+    if (!L.direct) nb6_status_fetch(st);
     if (ni >= POOL_MIN_NI) nb6_copy_pool().arm();   // the helpers spin while the GPU works
     NB6_CUDA_CHECK(cudaStreamSynchronize(st));
-    NB6_CUDA_CHECK(cudaEventElapsedTime(&R.last_kernel_ms, R.ev0, R.ev1));
     const double wt = nb6_wtime();
     R.time_grav += wt;
     R.time_reduce -= wt;
@@ -2545,7 +2560,7 @@ void gpunb_regf_(int *ni_, double *h2, double *dtr, double (*xi)[3], double (*vi
         return;
     }
 
-    unpack_results(ni, W, lmax, acc, jrk, pot, list);
+    unpack_results(ni, L.ls, lmax, acc, jrk, pot, list);
     R.time_reduce += nb6_wtime();
     if (R.selfcheck > 0)
         selfcheck_rows(ni, h2, dtr, xi, vi, acc, jrk, pot, list, lmax, nnbmax, *m_flag);
@@ -2628,7 +2643,6 @@ void nb6_regf_seg_(int *ni_, int *iseg, double *h2, double *dtr, double (*xi)[3]
                                        cudaMemcpyDeviceToHost, st));
         nb6_status_fetch(st);
         NB6_CUDA_CHECK(cudaStreamSynchronize(st));
-        NB6_CUDA_CHECK(cudaEventElapsedTime(&R.last_kernel_ms, R.ev0, R.ev1));
         const double wt2 = nb6_wtime();
         R.time_grav += wt2;
         R.time_reduce -= wt2;
@@ -2717,7 +2731,7 @@ void nb6_regf_seg_(int *ni_, int *iseg, double *h2, double *dtr, double (*xi)[3]
     R.outf.reserve((size_t)ni * 8);
     R.outl.reserve((size_t)ni * W);
     R.houtf.reserve((size_t)ni * 8);
-    R.houtl.reserve((size_t)ni * W);
+    R.houtl.reserve((size_t)ni * host_row_stride(W));
     if (!R.ev0) {
         NB6_CUDA_CHECK(cudaEventCreate(&R.ev0));
         NB6_CUDA_CHECK(cudaEventCreate(&R.ev1));
@@ -2774,9 +2788,11 @@ void nb6_regf_seg_(int *ni_, int *iseg, double *h2, double *dtr, double (*xi)[3]
     // finalize writes the pinned host staging in place, unless a device
     // kernel consumes the results (regular_seg_on_device)
     const bool direct = nb6_uva() && !g_seg_keep_device;
+    const int ls = direct ? host_row_stride(W) : W;
     regf_finalize_seg<<<(ni + FIN_WARPS - 1) / FIN_WARPS, FIN_WARPS * 32, smem, st>>>(
-        R.part.ptr, d_pinfo, ni, R.nbcnt.ptr, R.nbbuf.ptr, a.lcap, cap, W, pmax,
-        direct ? R.houtf.ptr : R.outf.ptr, direct ? R.houtl.ptr : R.outl.ptr, mlp);
+        R.part.ptr, d_pinfo, ni, R.nbcnt.ptr, R.nbbuf.ptr, a.lcap, cap, ls, pmax,
+        direct ? R.houtf.ptr : R.outf.ptr, direct ? R.houtl.ptr : R.outl.ptr, a.status,
+        direct ? nb6_status_post() : nullptr, mlp);
     NB6_CUDA_CHECK(cudaGetLastError());
     if (g_seg_keep_device) {
         R.time_grav += nb6_wtime();
@@ -2787,10 +2803,9 @@ void nb6_regf_seg_(int *ni_, int *iseg, double *h2, double *dtr, double (*xi)[3]
                                        st));
         NB6_CUDA_CHECK(cudaMemcpyAsync(R.houtl.ptr, R.outl.ptr, sizeof(int) * (size_t)W * ni,
                                        cudaMemcpyDeviceToHost, st));
+        nb6_status_fetch(st);
     }
-    nb6_status_fetch(st);
     NB6_CUDA_CHECK(cudaStreamSynchronize(st));
-    NB6_CUDA_CHECK(cudaEventElapsedTime(&R.last_kernel_ms, R.ev0, R.ev1));
     const double wt2 = nb6_wtime();
     R.time_grav += wt2;
     R.time_reduce -= wt2;
@@ -2798,7 +2813,7 @@ void nb6_regf_seg_(int *ni_, int *iseg, double *h2, double *dtr, double (*xi)[3]
         R.nbcnt_dirty = true;
         return;
     }
-    unpack_results(ni, W, lmax, acc, jrk, pot, list);
+    unpack_results(ni, ls, lmax, acc, jrk, pot, list);
     R.time_reduce += nb6_wtime();
 }
 

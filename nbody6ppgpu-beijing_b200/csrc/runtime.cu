@@ -114,6 +114,13 @@ void nb6_status_fetch(cudaStream_t st) {
     g_status_fetched = true;
 }
 
+// The pinned word itself, for a kernel that posts the status word as its last
+// act in place of that copy.
+int *nb6_status_post() {
+    g_status_fetched = true;
+    return g_status_host;
+}
+
 // Read (and clear) the device status word; call after a stream sync.
 int nb6_check_dev_status() {
     int st = 0;
