@@ -4,14 +4,16 @@
 //
 // The j set (m, x) is copied once per call into device buffers that persist
 // across calls (the reference allocates and frees per call,
-// gpupot.gpu.cu:72-79,107-108), split into hi/lo SoA float4 tiles, and
-// streamed through a 4-stage bulk-copy ring exactly like the regular kernel.
-// Each thread holds NI i-particles; pair math is FP32 on hi/lo differences
-// with rsqrt + one Newton step, FP32 partial sums fold into double-single
-// accumulators per 128-j tile, slices are summed in FP64 in a fixed order.
+// gpupot.gpu.cu:72-79,107-108), split into hi/lo FP32 rows laid out tile by
+// tile, and streamed through a 4-stage ring of bulk copies, one per 128-j
+// tile.  Each thread holds NI i-particles; pair math is packed FP32 (two j per
+// f32x2 instruction) on hi/lo differences with rsqrt + one Newton step, FP32
+// partial sums fold into double-single accumulators per tile, slices are
+// summed in FP64 in a fixed order.  Large calls order the bodies in space
+// first, so that most tiles are far from a whole warp's i-particles and take
+// a shorter loop (pot_kernel).
 #include "nb6_common.cuh"
-
-#include <cub/device/device_radix_sort.cuh>
+#include "spatial.cuh"
 
 #include <algorithm>
 #include <string.h>
@@ -23,586 +25,459 @@ constexpr int NSTAGE = 4;
 constexpr int NT = 128;
 constexpr unsigned long long WAIT_NS = 2000000000ull;
 
+// Rows of one 128-body tile, JT floats each: xh, yh, zh, m, xl, yl, zl and,
+// for an ordered set, xr, yr, zr (positions relative to the tile's box
+// centre).  A tile is one contiguous block, so one bulk copy brings it in.
+constexpr int ROWS_HL = 7, ROWS_ORD = 10;
+
+// The call whose pairs number at least POT_ORDER_PAIRS, against a set of at
+// least POT_ORDER_MIN bodies, orders the set: the order costs about 80 us at
+// 131,071 bodies, and a far pair takes half the time of a near one.  (32,767 of
+// 131,071 bodies, 4.3e9 pairs: 3,017 us as a scalar loop over the unordered
+// set, 1,480 us ordered and packed, the order included.)
+constexpr int POT_ORDER_MIN = 32768;
+constexpr double POT_ORDER_PAIRS = 1.0e9;
+
 struct PotArgs {
-    const float4 *__restrict__ posH;  // (xH, yH, zH, m)
-    const float4 *__restrict__ posL;  // (xL, yL, zL, 0)
+    const float *__restrict__ tiles;  // [ntile][rows][JT]
+    const float4 *__restrict__ tbox;  // ordered: per tile (centre, 0), (half extents, 0)
+    const double *__restrict__ x;     // FP64 positions [n][3], caller's order
+    const int *__restrict__ idx;      // i-particle of slot k; null: body i0 + k
     int ntile, nslices;
     int i0, ni;                       // absolute first i (0-based), count
-    float2 *__restrict__ part;        // [nslices][ni] (hi, lo)
+    float2 *__restrict__ part;        // [nslices][ni] (hi, lo) over slots
     int *status;
 };
-
-template <int NI>
-__global__ void __launch_bounds__(NT) pot_kernel(const PotArgs a) {
-    __shared__ __align__(128) float4 sj[NSTAGE][2][JT];
-    __shared__ __align__(8) uint64_t bar[NSTAGE];
-    const int tid = threadIdx.x;
-    const int slice = blockIdx.y;
-    const int t_begin = (int)(((long long)slice * a.ntile) / a.nslices);
-    const int t_end = (int)(((long long)(slice + 1) * a.ntile) / a.nslices);
-    const int nt = t_end - t_begin;
-
-    float xh[NI], yh[NI], zh[NI], xl[NI], yl[NI], zl[NI];
-    float ph[NI], pl[NI], ps[NI];
-    int ii[NI];
-#pragma unroll
-    for (int k = 0; k < NI; ++k) {
-        const int i = blockIdx.x * (NT * NI) + k * NT + tid;
-        ii[k] = i;
-        ph[k] = pl[k] = ps[k] = 0.f;
-        if (i < a.ni) {
-            const float4 h = a.posH[a.i0 + i];
-            const float4 l = a.posL[a.i0 + i];
-            xh[k] = h.x; yh[k] = h.y; zh[k] = h.z;
-            xl[k] = l.x; yl[k] = l.y; zl[k] = l.z;
-        } else {
-            xh[k] = yh[k] = zh[k] = xl[k] = yl[k] = zl[k] = 0.f;
-        }
-    }
-    if (tid == 0) {
-#pragma unroll
-        for (int st = 0; st < NSTAGE; ++st) mbar_init(&bar[st], 1);
-        fence_mbar_init();
-    }
-    __syncthreads();
-    auto issue = [&](int st, int tile) {
-        const size_t off = (size_t)tile * JT;
-        mbar_arrive_expect_tx(&bar[st], 2u * JT * sizeof(float4));
-        bulk_g2s(sj[st][0], a.posH + off, JT * sizeof(float4), &bar[st]);
-        bulk_g2s(sj[st][1], a.posL + off, JT * sizeof(float4), &bar[st]);
-    };
-    if (tid == 0)
-        for (int st = 0; st < NSTAGE && st < nt; ++st) issue(st, t_begin + st);
-
-    for (int t = 0; t < nt; ++t) {
-        const int st = t % NSTAGE;
-        const bool ok = mbar_wait_timed(&bar[st], (uint32_t)((t / NSTAGE) & 1), WAIT_NS);
-        if (__syncthreads_or(!ok)) {
-            if (tid == 0) {
-                set_status(a.status, NB6_ERR_WAIT_TIMEOUT);
-                const int issued = min(nt, NSTAGE + max(t - 1, 0));
-                for (int u = t; u < issued; ++u)
-                    mbar_wait_timed(&bar[u % NSTAGE], (uint32_t)((u / NSTAGE) & 1), WAIT_NS / 8);
-            }
-            return;
-        }
-        if (tid == 0 && t >= 1 && t - 1 + NSTAGE < nt) issue((t - 1) % NSTAGE, t_begin + t - 1 + NSTAGE);
-        const float4 *A = sj[st][0];
-        const float4 *B = sj[st][1];
-#pragma unroll 8
-        for (int q = 0; q < JT; ++q) {
-            const float4 h = A[q];
-            const float4 l = B[q];
-#pragma unroll
-            for (int k = 0; k < NI; ++k) {
-                const float dx = (h.x - xh[k]) + (l.x - xl[k]);
-                const float dy = (h.y - yh[k]) + (l.y - yl[k]);
-                const float dz = (h.z - zh[k]) + (l.z - zl[k]);
-                const float r2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
-                float y = rsqrt2_nr(r2);          // 2/r
-                y = (r2 > 0.f) ? y : 0.f;         // gpupot.gpu.cu:52 skips r2 == 0
-                ps[k] = fmaf(h.w, y, ps[k]);
-            }
-        }
-#pragma unroll
-        for (int k = 0; k < NI; ++k) {
-            ds_fold(ph[k], pl[k], ps[k]);
-            ps[k] = 0.f;
-        }
-    }
-#pragma unroll
-    for (int k = 0; k < NI; ++k)
-        if (ii[k] < a.ni) a.part[(size_t)slice * a.ni + ii[k]] = make_float2(ph[k], pl[k]);
-}
-
-__global__ void pot_finalize(const float2 *__restrict__ part, int nslices, int ni,
-                             double *__restrict__ out) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= ni) return;
-    double s = 0.0;
-    for (int sl = 0; sl < nslices; ++sl) {
-        const float2 p = part[(size_t)sl * ni + i];
-        s += (double)p.x + (double)p.y;
-    }
-    out[i] = 0.5 * s;  // undo the 2/r scaling of rsqrt2_nr
-}
-
-__global__ void pot_pack(int n, int npad, const double *__restrict__ m,
-                         const double *__restrict__ x, float4 *__restrict__ posH,
-                         float4 *__restrict__ posL, int *status) {
-    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < npad; j += gridDim.x * blockDim.x) {
-        if (j < n) {
-            const double x0 = x[3 * j], x1 = x[3 * j + 1], x2 = x[3 * j + 2], mj = m[j];
-            if (x0 != x0 || x1 != x1 || x2 != x2 || mj != mj) set_status(status, NB6_ERR_NAN_INPUT);
-            float4 h, l;
-            split_hl(x0, h.x, l.x);
-            split_hl(x1, h.y, l.y);
-            split_hl(x2, h.z, l.z);
-            h.w = (float)mj;
-            l.w = 0.f;
-            posH[j] = h;
-            posL[j] = l;
-        } else {
-            posH[j] = make_float4(1.0e15f, 1.0e15f, 1.0e15f, 0.f);
-            posL[j] = make_float4(0.f, 0.f, 0.f, 0.f);
-        }
-    }
-}
-
-// ----------------------------------------------------------------------------
-// Ordered path (the whole set, n >= POT_ORDER_MIN): the bodies in Morton
-// order with one bounding box per 128-body tile, as the regular force orders
-// its j set.  A (warp, tile) whose box is at least one half extent away
-// from every lane's i takes the packed far loop: differences from
-// tile-relative coordinates fl32(x_j - c) (stored) and fl32(x_i - c)
-// (formed in FP64 per tile), one FP32 add each instead of three, within 4
-// FP32 ulps of the FP64-formed difference (|x_j - c| <= h <= r), and two j
-// per f32x2 instruction.  Other tiles take the hi/lo loop above.  Results
-// are written back in the caller's order.
-// ----------------------------------------------------------------------------
-constexpr int POT_ORDER_MIN = 32768;
 
 NB6_DEV float2 pair2(float v) { return make_float2(v, v); }
+NB6_DEV float2 lo2(const float4 &v) { return make_float2(v.x, v.y); }
+NB6_DEV float2 hi2(const float4 &v) { return make_float2(v.z, v.w); }
+NB6_DEV float4 ld4(const float *p) { return *reinterpret_cast<const float4 *>(p); }
 
-__global__ void pot_extent(int n, const double *__restrict__ x, unsigned *__restrict__ ext) {
-    unsigned mn[3] = {0xffffffffu, 0xffffffffu, 0xffffffffu}, mx[3] = {0u, 0u, 0u};
-    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x)
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            const unsigned o = f2ord((float)x[3 * (size_t)j + k]);
-            mn[k] = min(mn[k], o);
-            mx[k] = max(mx[k], o);
-        }
-#pragma unroll
-    for (int k = 0; k < 3; ++k)
-        for (int o = 16; o > 0; o >>= 1) {
-            mn[k] = min(mn[k], __shfl_xor_sync(0xffffffffu, mn[k], o));
-            mx[k] = max(mx[k], __shfl_xor_sync(0xffffffffu, mx[k], o));
-        }
-    if ((threadIdx.x & 31) == 0)
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            atomicMin(&ext[k], mn[k]);
-            atomicMax(&ext[3 + k], mx[k]);
-        }
+NB6_DEV float2 rsqrt_approx2(float2 r2) {
+    float2 y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y.x) : "f"(r2.x));
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y.y) : "f"(r2.y));
+    return y;
 }
 
-__global__ void pot_keys(int n, const double *__restrict__ x, const unsigned *__restrict__ ext,
-                         unsigned *__restrict__ keys, int *__restrict__ vals) {
-    float lo[3], sc[3];
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        lo[k] = ord2f(ext[k]);
-        const float w = ord2f(ext[3 + k]) - lo[k];
-        sc[k] = w > 0.f ? 1023.99f / w : 0.f;
-    }
-    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
-        unsigned key = 0;
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            const float f = ((float)x[3 * (size_t)j + k] - lo[k]) * sc[k];
-            key |= spread10((unsigned)fminf(fmaxf(f, 0.f), 1023.f)) << k;
-        }
-        keys[j] = key;
-        vals[j] = j;
-    }
+// sum -2 m / r over two j's into acc (lane = j parity), hi/lo differences
+NB6_DEV void near_pair(float2 xh, float2 yh, float2 zh, float2 m, float2 xl, float2 yl, float2 zl, float2 nxh,
+                       float2 nyh, float2 nzh, float2 nxl, float2 nyl, float2 nzl, float2 &acc) {
+    const float2 dx = __fadd2_rn(__fadd2_rn(xh, nxh), __fadd2_rn(xl, nxl));
+    const float2 dy = __fadd2_rn(__fadd2_rn(yh, nyh), __fadd2_rn(yl, nyl));
+    const float2 dz = __fadd2_rn(__fadd2_rn(zh, nzh), __fadd2_rn(zl, nzl));
+    const float2 r2 = __ffma2_rn(dz, dz, __ffma2_rn(dy, dy, __fmul2_rn(dx, dx)));
+    const float2 y0 = rsqrt_approx2(r2);
+    const float2 nb = __ffma2_rn(__fmul2_rn(r2, y0), y0, pair2(-3.0f));  // -(3 - r2 y0^2)
+    float2 ny = __fmul2_rn(y0, nb);                                      // -2/r
+    ny.x = r2.x > 0.f ? ny.x : 0.f;  // gpupot.gpu.cu:52 skips r2 == 0
+    ny.y = r2.y > 0.f ? ny.y : 0.f;
+    acc = __ffma2_rn(m, ny, acc);
 }
 
-// Ordered hi/lo layout (+ mass) and FP64 positions; padding slots massless
-// and far away.
-__global__ void pot_permute(int n, int npad, const int *__restrict__ perm, const double *__restrict__ m,
-                            const double *__restrict__ x, float4 *__restrict__ posH, float4 *__restrict__ posL,
-                            double *__restrict__ xs) {
-    for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < npad; s += gridDim.x * blockDim.x) {
-        if (s < n) {
-            const int j = perm[s];
-            const double x0 = x[3 * (size_t)j], x1 = x[3 * (size_t)j + 1], x2 = x[3 * (size_t)j + 2];
-            float4 h, l;
-            split_hl(x0, h.x, l.x);
-            split_hl(x1, h.y, l.y);
-            split_hl(x2, h.z, l.z);
-            h.w = (float)m[j];
-            l.w = 0.f;
-            posH[s] = h;
-            posL[s] = l;
-            xs[3 * (size_t)s] = x0;
-            xs[3 * (size_t)s + 1] = x1;
-            xs[3 * (size_t)s + 2] = x2;
-        } else {
-            posH[s] = make_float4(1.0e15f, 1.0e15f, 1.0e15f, 0.f);
-            posL[s] = make_float4(0.f, 0.f, 0.f, 0.f);
-            xs[3 * (size_t)s] = xs[3 * (size_t)s + 1] = xs[3 * (size_t)s + 2] = 1.0e15;
-        }
-    }
+// sum m / r over two j's of a far tile: tile-relative differences, and 1/r
+// straight from rsqrt.approx: every term of the sum is positive, so its
+// relative error bound carries over to the sum unamplified (no Newton step
+// needed, unlike the cancelling force sums).
+NB6_DEV void far_pair(float2 xr, float2 yr, float2 zr, float2 m, float2 nxr, float2 nyr, float2 nzr, float2 &acc) {
+    const float2 dx = __fadd2_rn(xr, nxr);
+    const float2 dy = __fadd2_rn(yr, nyr);
+    const float2 dz = __fadd2_rn(zr, nzr);
+    const float2 r2 = __ffma2_rn(dz, dz, __ffma2_rn(dy, dy, __fmul2_rn(dx, dx)));
+    acc = __ffma2_rn(m, rsqrt_approx2(r2), acc);
 }
 
-// One warp per tile: box of the hi positions of its real bodies (centre
-// rounded to nearest, half extents rounded up).
-__global__ void pot_boxes(int n, int ntile, const float4 *__restrict__ posH, float4 *__restrict__ tbox) {
-    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    if (warp >= ntile) return;
-    double mn[3] = {1e300, 1e300, 1e300}, mx[3] = {-1e300, -1e300, -1e300};
-    for (int q = lane; q < JT; q += 32) {
-        const int k = warp * JT + q;
-        if (k >= n) break;
-        const float4 p = posH[k];
-        const double c[3] = {p.x, p.y, p.z};
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-            mn[d] = fmin(mn[d], c[d]);
-            mx[d] = fmax(mx[d], c[d]);
-        }
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-            mn[d] = fmin(mn[d], __shfl_xor_sync(0xffffffffu, mn[d], o));
-            mx[d] = fmax(mx[d], __shfl_xor_sync(0xffffffffu, mx[d], o));
-        }
-    if (lane == 0) {
-        tbox[2 * warp] = make_float4(__double2float_rn(0.5 * (mn[0] + mx[0])), __double2float_rn(0.5 * (mn[1] + mx[1])),
-                                     __double2float_rn(0.5 * (mn[2] + mx[2])), 0.f);
-        tbox[2 * warp + 1] = make_float4(__double2float_ru(0.5 * (mx[0] - mn[0])), __double2float_ru(0.5 * (mx[1] - mn[1])),
-                                         __double2float_ru(0.5 * (mx[2] - mn[2])), 0.f);
-    }
-}
-
-// Tile-relative positions and masses, component-major rows (xr, yr, zr, m)
-// of npad floats each.
-__global__ void pot_rel(int npad, const double *__restrict__ xs, const float4 *__restrict__ posH,
-                        const float4 *__restrict__ tbox, float *__restrict__ rel) {
-    for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < npad; s += gridDim.x * blockDim.x) {
-        const float4 c = tbox[2 * (s / JT)];
-        rel[s] = __double2float_rn(xs[3 * (size_t)s] - (double)c.x);
-        rel[(size_t)npad + s] = __double2float_rn(xs[3 * (size_t)s + 1] - (double)c.y);
-        rel[2 * (size_t)npad + s] = __double2float_rn(xs[3 * (size_t)s + 2] - (double)c.z);
-        rel[3 * (size_t)npad + s] = posH[s].w;
-    }
-}
-
-struct PotOrdArgs {
-    const float4 *__restrict__ posH;  // ordered (xH, yH, zH, m)
-    const float4 *__restrict__ posL;  // ordered (xL, yL, zL, 0)
-    const float *__restrict__ rel;    // ordered rows xr, yr, zr, m (4 x npad)
-    const double *__restrict__ xs;    // ordered FP64 positions
-    const float4 *__restrict__ tbox;  // per tile: (centre, 0), (half extents, 0)
-    size_t npad;
-    int n, ntile, nslices;
-    float2 *__restrict__ part;        // [nslices][n] over ordered slots
-    int *status;
-};
-
-__global__ void __launch_bounds__(NT) pot_kernel_ord(const PotOrdArgs a) {
-    __shared__ __align__(128) float4 sh[NSTAGE][2][JT];
-    __shared__ __align__(128) float sr[NSTAGE][4][JT];
-    __shared__ __align__(8) uint64_t bar[NSTAGE];
+// One CTA: NT * NI i-particles against the tiles slice, slice + nslices, ...
+// (the near tiles of a compact group of i are dealt out among the slices).
+//
+// ORD (bodies in Morton order with one bounding box per tile): a (warp, tile)
+// whose box is at least one half extent away from every lane's i takes the
+// far loop: differences from tile-relative coordinates fl32(x_j - c) (stored)
+// and fl32(x_i - c) (formed in FP64 per tile), one FP32 add each instead of
+// three, within 4 FP32 ulps of the FP64-formed difference (|x_j - c| <= h
+// <= r).  Other tiles take the hi/lo loop.
+//
+// What bounds it: a far pair costs 7 FMA-pipe lane operations and one MUFU
+// rsqrt, i.e. 1.75 and 2 cycles of an SM per warp and j, so the MUFU rate
+// (16 lanes per cycle) is the floor.  One shared-memory load of 16 bytes per
+// lane costs two cycles as well, and the loop needs one per j: with one i per
+// thread the load path was 70% busy and the MUFU 64%.  Two i per thread
+// (NI = 2, 96 registers, five CTAs per SM) share each load.  Warps release a
+// stage on its own "empty" barrier, so they drift apart instead of meeting at
+// a CTA barrier per tile.  249,036 bodies of a King cluster: 20.8 ms before
+// (64% of the MUFU floor), 18.0 ms with one i per thread, 17.3 ms with two.
+template <int NI, bool ORD>
+__global__ void __launch_bounds__(NT, NI == 2 ? 5 : 8) pot_kernel(const PotArgs a) {
+    constexpr int ROWS = ORD ? ROWS_ORD : ROWS_HL;
+    constexpr uint32_t TILE_BYTES = ROWS * JT * sizeof(float);
+    __shared__ __align__(128) float sj[NSTAGE][ROWS][JT];
+    __shared__ __align__(8) uint64_t bar[NSTAGE], ebar[NSTAGE];
     const int tid = threadIdx.x, lane = tid & 31;
     const int slice = blockIdx.y;
-    // tiles of this slice: every nslices-th (the near tiles of a compact
-    // group of i are dealt out among the slices)
     const int nt = slice < a.ntile ? (a.ntile - slice + a.nslices - 1) / a.nslices : 0;
-    const int s = blockIdx.x * NT + tid;
-    const bool on = s < a.n;
-    float xh = 0.f, yh = 0.f, zh = 0.f, xl = 0.f, yl = 0.f, zl = 0.f;
-    double xd = 0.0, yd = 0.0, zd = 0.0;
-    if (on) {
-        const float4 h = a.posH[s], l = a.posL[s];
-        xh = h.x; yh = h.y; zh = h.z;
-        xl = l.x; yl = l.y; zl = l.z;
-        xd = a.xs[3 * (size_t)s];
-        yd = a.xs[3 * (size_t)s + 1];
-        zd = a.xs[3 * (size_t)s + 2];
+
+    double xd[NI], yd[NI], zd[NI];
+    float ph[NI], pl[NI];
+    bool on[NI];
+#pragma unroll
+    for (int k = 0; k < NI; ++k) {
+        const int s = blockIdx.x * (NT * NI) + k * NT + tid;
+        on[k] = s < a.ni;
+        xd[k] = yd[k] = zd[k] = 0.0;
+        ph[k] = pl[k] = 0.f;
+        if (on[k]) {
+            const double *p = a.x + 3 * (size_t)(a.idx ? a.idx[s] : a.i0 + s);
+            xd[k] = p[0];
+            yd[k] = p[1];
+            zd[k] = p[2];
+        }
     }
-    float ph = 0.f, pl = 0.f;
     if (tid == 0) {
 #pragma unroll
-        for (int st = 0; st < NSTAGE; ++st) mbar_init(&bar[st], 1);
+        for (int st = 0; st < NSTAGE; ++st) {
+            mbar_init(&bar[st], 1);
+            mbar_init(&ebar[st], NT / 32);
+        }
         fence_mbar_init();
     }
     __syncthreads();
-    auto issue = [&](int st, int tile) {
-        const size_t off = (size_t)tile * JT;
-        mbar_arrive_expect_tx(&bar[st], 2u * JT * sizeof(float4) + 4u * JT * sizeof(float));
-        bulk_g2s(sh[st][0], a.posH + off, JT * sizeof(float4), &bar[st]);
-        bulk_g2s(sh[st][1], a.posL + off, JT * sizeof(float4), &bar[st]);
-#pragma unroll
-        for (int c = 0; c < 4; ++c) bulk_g2s(sr[st][c], a.rel + (size_t)c * a.npad + off, JT * sizeof(float), &bar[st]);
+    auto issue = [&](int t) {
+        const int st = t % NSTAGE;
+        mbar_arrive_expect_tx(&bar[st], TILE_BYTES);
+        bulk_g2s(sj[st], a.tiles + (size_t)(slice + t * a.nslices) * (ROWS * JT), TILE_BYTES, &bar[st]);
     };
+    int issued = 0;  // thread 0 only
     if (tid == 0)
-        for (int st = 0; st < NSTAGE && st < nt; ++st) issue(st, slice + st * a.nslices);
+        for (; issued < min(nt, NSTAGE); ++issued) issue(issued);
 
     for (int t = 0; t < nt; ++t) {
         const int st = t % NSTAGE;
-        const bool ok = mbar_wait_timed(&bar[st], (uint32_t)((t / NSTAGE) & 1), WAIT_NS);
-        if (__syncthreads_or(!ok)) {
-            if (tid == 0) {
-                set_status(a.status, NB6_ERR_WAIT_TIMEOUT);
-                const int issued = min(nt, NSTAGE + max(t - 1, 0));
+        const uint32_t par = (uint32_t)((t / NSTAGE) & 1);
+        if (!__all_sync(0xffffffffu, mbar_wait_timed(&bar[st], par, WAIT_NS))) {
+            set_status(a.status, NB6_ERR_WAIT_TIMEOUT);
+            if (tid == 0)  // drain copies still in flight before the CTA's smem goes away
                 for (int u = t; u < issued; ++u)
                     mbar_wait_timed(&bar[u % NSTAGE], (uint32_t)((u / NSTAGE) & 1), WAIT_NS / 8);
-            }
             return;
         }
-        if (tid == 0 && t >= 1 && t - 1 + NSTAGE < nt) issue((t - 1) % NSTAGE, slice + (t - 1 + NSTAGE) * a.nslices);
-        const int tile = slice + t * a.nslices;
-        const float4 bc = __ldg(&a.tbox[2 * tile]), bh = __ldg(&a.tbox[2 * tile + 1]);
-        // far: the box at least one half extent from this lane's i (with a
-        // margin for the FP32 test); padding lanes are far
-        const float ex = fmaxf(fabsf(xh - bc.x) - bh.x, 0.f);
-        const float ey = fmaxf(fabsf(yh - bc.y) - bh.y, 0.f);
-        const float ez = fmaxf(fabsf(zh - bc.z) - bh.z, 0.f);
-        const float hm = fmaxf(fmaxf(bh.x, bh.y), bh.z);
-        const bool far = __all_sync(0xffffffffu, !on || ex * ex + ey * ey + ez * ez > 1.01f * hm * hm);
-        float p;
-        if (far) {
-            const float2 nxr = pair2(-__double2float_rn(xd - (double)bc.x));
-            const float2 nyr = pair2(-__double2float_rn(yd - (double)bc.y));
-            const float2 nzr = pair2(-__double2float_rn(zd - (double)bc.z));
-            float2 acc = make_float2(0.f, 0.f);  // sum m / r, lane = j parity
-#pragma unroll 4
-            for (int q = 0; q < JT; q += 4) {
-                const float4 X = *reinterpret_cast<const float4 *>(&sr[st][0][q]);
-                const float4 Y = *reinterpret_cast<const float4 *>(&sr[st][1][q]);
-                const float4 Z = *reinterpret_cast<const float4 *>(&sr[st][2][q]);
-                const float4 M = *reinterpret_cast<const float4 *>(&sr[st][3][q]);
+        const float(*S)[JT] = sj[st];
+        bool far = false;
+        float4 bc;
+        if constexpr (ORD) {
+            const int tile = slice + t * a.nslices;
+            bc = __ldg(&a.tbox[2 * tile]);
+            const float4 bh = __ldg(&a.tbox[2 * tile + 1]);
+            // far: the box at least one half extent from this thread's i
+            // (with a margin for the FP32 test); padding slots are far
+            const float hm = fmaxf(fmaxf(bh.x, bh.y), bh.z);
+            bool f = true;
 #pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    const float2 xr = h ? make_float2(X.z, X.w) : make_float2(X.x, X.y);
-                    const float2 yr = h ? make_float2(Y.z, Y.w) : make_float2(Y.x, Y.y);
-                    const float2 zr = h ? make_float2(Z.z, Z.w) : make_float2(Z.x, Z.y);
-                    const float2 mm = h ? make_float2(M.z, M.w) : make_float2(M.x, M.y);
-                    const float2 dx = __fadd2_rn(xr, nxr);
-                    const float2 dy = __fadd2_rn(yr, nyr);
-                    const float2 dz = __fadd2_rn(zr, nzr);
-                    const float2 r2 = __ffma2_rn(dz, dz, __ffma2_rn(dy, dy, __fmul2_rn(dx, dx)));
-                    // 1/r straight from rsqrt.approx: every term of the
-                    // sum is positive, so its relative error bound carries
-                    // over to the sum unamplified (no Newton step needed,
-                    // unlike the cancelling force sums)
-                    float2 y0;
-                    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y0.x) : "f"(r2.x));
-                    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y0.y) : "f"(r2.y));
-                    acc = __ffma2_rn(mm, y0, acc);
+            for (int k = 0; k < NI; ++k) {
+                const float ex = fmaxf(fabsf((float)xd[k] - bc.x) - bh.x, 0.f);
+                const float ey = fmaxf(fabsf((float)yd[k] - bc.y) - bh.y, 0.f);
+                const float ez = fmaxf(fabsf((float)zd[k] - bc.z) - bh.z, 0.f);
+                f = f && (!on[k] || ex * ex + ey * ey + ez * ez > 1.01f * hm * hm);
+            }
+            far = __all_sync(0xffffffffu, f);
+        }
+        float2 acc[NI];
+#pragma unroll
+        for (int k = 0; k < NI; ++k) acc[k] = make_float2(0.f, 0.f);
+        if (ORD && far) {
+            float2 nx[NI], ny[NI], nz[NI];
+#pragma unroll
+            for (int k = 0; k < NI; ++k) {
+                nx[k] = pair2(-__double2float_rn(xd[k] - (double)bc.x));
+                ny[k] = pair2(-__double2float_rn(yd[k] - (double)bc.y));
+                nz[k] = pair2(-__double2float_rn(zd[k] - (double)bc.z));
+            }
+#pragma unroll 8
+            for (int q = 0; q < JT; q += 4) {
+                const float4 M = ld4(&S[3][q]), X = ld4(&S[ROWS - 3][q]), Y = ld4(&S[ROWS - 2][q]),
+                             Z = ld4(&S[ROWS - 1][q]);
+#pragma unroll
+                for (int k = 0; k < NI; ++k) {
+                    far_pair(lo2(X), lo2(Y), lo2(Z), lo2(M), nx[k], ny[k], nz[k], acc[k]);
+                    far_pair(hi2(X), hi2(Y), hi2(Z), hi2(M), nx[k], ny[k], nz[k], acc[k]);
                 }
             }
-            p = 2.0f * (acc.x + acc.y);  // the 2/r units of the hi/lo loop
         } else {
-            const float4 *A = sh[st][0];
-            const float4 *B = sh[st][1];
-            float ps = 0.f;
-#pragma unroll 8
-            for (int q = 0; q < JT; ++q) {
-                const float4 h = A[q];
-                const float4 l = B[q];
-                const float dx = (h.x - xh) + (l.x - xl);
-                const float dy = (h.y - yh) + (l.y - yl);
-                const float dz = (h.z - zh) + (l.z - zl);
-                const float r2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
-                float y = rsqrt2_nr(r2);          // 2/r
-                y = (r2 > 0.f) ? y : 0.f;         // gpupot.gpu.cu:52 skips r2 == 0
-                ps = fmaf(h.w, y, ps);
+            float2 nxh[NI], nyh[NI], nzh[NI], nxl[NI], nyl[NI], nzl[NI];
+#pragma unroll
+            for (int k = 0; k < NI; ++k) {
+                float h, l;
+                split_hl(xd[k], h, l);
+                nxh[k] = pair2(-h);
+                nxl[k] = pair2(-l);
+                split_hl(yd[k], h, l);
+                nyh[k] = pair2(-h);
+                nyl[k] = pair2(-l);
+                split_hl(zd[k], h, l);
+                nzh[k] = pair2(-h);
+                nzl[k] = pair2(-l);
             }
-            p = ps;
+#pragma unroll 4
+            for (int q = 0; q < JT; q += 4) {
+                const float4 XH = ld4(&S[0][q]), YH = ld4(&S[1][q]), ZH = ld4(&S[2][q]), M = ld4(&S[3][q]),
+                             XL = ld4(&S[4][q]), YL = ld4(&S[5][q]), ZL = ld4(&S[6][q]);
+#pragma unroll
+                for (int k = 0; k < NI; ++k) {
+                    near_pair(lo2(XH), lo2(YH), lo2(ZH), lo2(M), lo2(XL), lo2(YL), lo2(ZL), nxh[k], nyh[k], nzh[k],
+                              nxl[k], nyl[k], nzl[k], acc[k]);
+                    near_pair(hi2(XH), hi2(YH), hi2(ZH), hi2(M), hi2(XL), hi2(YL), hi2(ZL), nxh[k], nyh[k], nzh[k],
+                              nxl[k], nyl[k], nzl[k], acc[k]);
+                }
+            }
         }
-        ds_fold(ph, pl, p);
-        (void)lane;
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&ebar[st]);
+        if (tid == 0 && issued < nt) {
+            // once every warp has released tile t, refill its stage
+            if (!mbar_wait_timed(&ebar[st], par, WAIT_NS)) {
+                set_status(a.status, NB6_ERR_WAIT_TIMEOUT);
+                for (int u = t + 1; u < issued; ++u)
+                    mbar_wait_timed(&bar[u % NSTAGE], (uint32_t)((u / NSTAGE) & 1), WAIT_NS / 8);
+                return;
+            }
+            issue(issued);
+            ++issued;
+        }
+        const float f = far ? 1.0f : -0.5f;
+#pragma unroll
+        for (int k = 0; k < NI; ++k) ds_fold(ph[k], pl[k], f * (acc[k].x + acc[k].y));
     }
-    if (on) a.part[(size_t)slice * a.n + s] = make_float2(ph, pl);
+#pragma unroll
+    for (int k = 0; k < NI; ++k) {
+        const int s = blockIdx.x * (NT * NI) + k * NT + tid;
+        if (on[k]) a.part[(size_t)slice * a.ni + s] = make_float2(ph[k], pl[k]);
+    }
 }
 
-// Sum of the slices of ordered slot s, written to the caller's index perm[s].
-__global__ void pot_finalize_ord(const float2 *__restrict__ part, int nslices, int n, const int *__restrict__ perm,
-                                 double *__restrict__ out) {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= n) return;
+// Sum of the slices of slot k, in order, to out[idx[k] - i0] (the caller's
+// index) or out[k].  hstatus: see nb6_status_post.
+__global__ void pot_finalize(const float2 *__restrict__ part, int nslices, int i0, int ni,
+                             const int *__restrict__ idx, double *__restrict__ out, const int *status,
+                             int *hstatus) {
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (hstatus && k == 0) *hstatus = *status;
+    if (k >= ni) return;
     double v = 0.0;
+#pragma unroll 8
     for (int sl = 0; sl < nslices; ++sl) {
-        const float2 p = part[(size_t)sl * n + s];
+        const float2 p = __ldg(part + (size_t)sl * ni + k);
         v += (double)p.x + (double)p.y;
     }
-    out[perm[s]] = 0.5 * v;
+    out[idx ? idx[k] - i0 : k] = v;
+}
+
+// One CTA per tile: its rows of the tile layout, from the bodies in the
+// caller's order (ROWS_HL) or, with perm, in Morton order, with the tile's
+// box (of the hi positions of its real bodies: centre rounded to nearest,
+// half extents rounded up) and the tile-relative rows.  Padding slots are
+// massless and far away.
+template <bool ORD>
+__global__ void __launch_bounds__(JT) pot_tiles(int n, const int *__restrict__ perm, const double *__restrict__ m,
+                                                const double *__restrict__ x, float *__restrict__ tiles,
+                                                float4 *__restrict__ tbox, int *status) {
+    constexpr int ROWS = ORD ? ROWS_ORD : ROWS_HL;
+    const int t = threadIdx.x, s = blockIdx.x * JT + t;
+    double c[3] = {1.0e15, 1.0e15, 1.0e15}, mj = 0.0;
+    if (s < n) {
+        const size_t j = ORD ? perm[s] : s;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) c[k] = x[3 * j + k];
+        mj = m[j];
+        if (c[0] != c[0] || c[1] != c[1] || c[2] != c[2] || mj != mj) set_status(status, NB6_ERR_NAN_INPUT);
+    }
+    float *o = tiles + (size_t)blockIdx.x * (ROWS * JT) + t;
+    float h[3], l[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        split_hl(c[k], h[k], l[k]);
+        o[k * JT] = h[k];
+        o[(4 + k) * JT] = l[k];
+    }
+    o[3 * JT] = (float)mj;
+    if constexpr (ORD) {
+        __shared__ unsigned smn[JT / 32][3], smx[JT / 32][3];
+        __shared__ float sc[3];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            const unsigned u = f2ord(h[k]);
+            const unsigned mn = __reduce_min_sync(0xffffffffu, s < n ? u : 0xffffffffu);
+            const unsigned mx = __reduce_max_sync(0xffffffffu, s < n ? u : 0u);
+            if ((t & 31) == 0) {
+                smn[t >> 5][k] = mn;
+                smx[t >> 5][k] = mx;
+            }
+        }
+        __syncthreads();
+        if (t < 3) {
+            unsigned a = smn[0][t], b = smx[0][t];
+            for (int w = 1; w < JT / 32; ++w) {
+                a = min(a, smn[w][t]);
+                b = max(b, smx[w][t]);
+            }
+            const double lo = ord2f(a), hi = ord2f(b);
+            sc[t] = __double2float_rn(0.5 * (lo + hi));
+            float *bx = reinterpret_cast<float *>(tbox + 2 * blockIdx.x);
+            bx[t] = sc[t];
+            bx[4 + t] = __double2float_ru(0.5 * (hi - lo));
+            if (t == 0) bx[3] = bx[7] = 0.f;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < 3; ++k) o[(7 + k) * JT] = __double2float_rn(c[k] - (double)sc[k]);
+    }
+}
+
+// The bodies [i0, i0+ni) of an ordered set, in that order: idx[k] = the k-th
+// slot's body, among the slots whose body is in the range.  Two launches:
+// counts per CTA, then each CTA adds up the counts before its own and packs
+// its slots.
+constexpr int SEL_NT = 1024;
+__global__ void __launch_bounds__(SEL_NT) pot_select_count(int n, const int *__restrict__ perm, int i0, int ni,
+                                                           int *__restrict__ count) {
+    const int s = blockIdx.x * SEL_NT + threadIdx.x;
+    const int c = __syncthreads_count(s < n && (unsigned)(perm[s] - i0) < (unsigned)ni);
+    if (threadIdx.x == 0) count[blockIdx.x] = c;
+}
+
+__global__ void __launch_bounds__(SEL_NT) pot_select(int n, const int *__restrict__ perm, int i0, int ni,
+                                                     const int *__restrict__ count, int *__restrict__ idx) {
+    __shared__ int wsum[SEL_NT / 32];
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    const int s = blockIdx.x * SEL_NT + t;
+    const int body = s < n ? perm[s] : -1;
+    const bool in = s < n && (unsigned)(body - i0) < (unsigned)ni;
+    const unsigned b = __ballot_sync(0xffffffffu, in);
+    int before = 0;
+    for (int q = t; q < (int)blockIdx.x; q += SEL_NT) before += count[q];
+    // this warp's share of the counts before the CTA, plus its own slots
+    const int share = __reduce_add_sync(0xffffffffu, before);
+    __shared__ int base[SEL_NT / 32];
+    if (lane == 0) {
+        base[warp] = share;
+        wsum[warp] = __popc(b);
+    }
+    __syncthreads();
+    int off = 0;
+    for (int w = 0; w < SEL_NT / 32; ++w) off += base[w] + (w < warp ? wsum[w] : 0);
+    if (in) idx[off + __popc(b & ((1u << lane) - 1u))] = body;
 }
 
 struct PotState {
     DevBuf<double> m, x, out;
-    DevBuf<float4> posH, posL;
+    DevBuf<float> tiles;
+    DevBuf<float4> tbox;
     DevBuf<float2> part;
+    DevBuf<int> count, idx;
     HostBuf<double> hout;
+    SpatialOrder order;
     int n = 0, ntile = 0;
+    const double *dm = nullptr, *dx = nullptr;  // the uploaded m, x of the call
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     float last_ms = 0.f;
-    // ordered set (whole-set calls with n >= POT_ORDER_MIN)
-    const double *dm = nullptr, *dx = nullptr;  // the uploaded m, x of the call
-    DevBuf<float4> posH_s, posL_s, tbox;
-    DevBuf<float> rel;
-    DevBuf<double> xs;
-    DevBuf<unsigned> keys_in, keys_out, ext;
-    DevBuf<int> vals_in, perm;
-    DevBuf<char> sort_tmp;
 };
 PotState P;
 
-// Build the ordered set of the uploaded bodies (P.dm, P.dx, P.n).
-void pot_order(cudaStream_t st) {
-    const int n = P.n;
-    const size_t npad = (size_t)P.ntile * JT;
-    P.keys_in.reserve(n);
-    P.keys_out.reserve(n);
-    P.vals_in.reserve(n);
-    P.perm.reserve(n);
-    P.ext.reserve(6);
-    P.posH_s.reserve(npad);
-    P.posL_s.reserve(npad);
-    P.xs.reserve(3 * npad);
-    P.rel.reserve(4 * npad);
-    P.tbox.reserve(2 * (size_t)P.ntile);
-    const unsigned init[6] = {0xffffffffu, 0xffffffffu, 0xffffffffu, 0u, 0u, 0u};
-    NB6_CUDA_CHECK(cudaMemcpyAsync(P.ext.ptr, init, sizeof(init), cudaMemcpyHostToDevice, st));
-    const int blocks = std::max(1, std::min((n + 255) / 256, nb6_num_sms() * 8));
-    pot_extent<<<blocks, 256, 0, st>>>(n, P.dx, P.ext.ptr);
-    pot_keys<<<blocks, 256, 0, st>>>(n, P.dx, P.ext.ptr, P.keys_in.ptr, P.vals_in.ptr);
-    NB6_CUDA_CHECK(cudaGetLastError());
-    size_t tmp = 0;
-    NB6_CUDA_CHECK(cub::DeviceRadixSort::SortPairs(nullptr, tmp, P.keys_in.ptr, P.keys_out.ptr, P.vals_in.ptr,
-                                                   P.perm.ptr, n, 0, 30, st));
-    P.sort_tmp.reserve(tmp + 16);
-    NB6_CUDA_CHECK(cub::DeviceRadixSort::SortPairs(P.sort_tmp.ptr, tmp, P.keys_in.ptr, P.keys_out.ptr,
-                                                   P.vals_in.ptr, P.perm.ptr, n, 0, 30, st));
-    const int pblocks = (int)std::min<size_t>((npad + 255) / 256, (size_t)nb6_num_sms() * 8);
-    pot_permute<<<pblocks, 256, 0, st>>>(n, (int)npad, P.perm.ptr, P.dm, P.dx, P.posH_s.ptr, P.posL_s.ptr, P.xs.ptr);
-    pot_boxes<<<(P.ntile * 32 + 255) / 256, 256, 0, st>>>(n, P.ntile, P.posH_s.ptr, P.tbox.ptr);
-    pot_rel<<<pblocks, 256, 0, st>>>((int)npad, P.xs.ptr, P.posH_s.ptr, P.tbox.ptr, P.rel.ptr);
-    NB6_CUDA_CHECK(cudaGetLastError());
-}
-
-int pot_ord_occ() {
-    static int occ = -1;
-    if (occ < 0) {
-        NB6_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, pot_kernel_ord, NT, 0));
-        if (occ < 1) occ = 1;
-    }
-    return occ;
-}
-
-// Potential of every body, ordered path; result in P.out (caller's order).
-void pot_device_ord(cudaStream_t st) {
-    const int n = P.n;
-    const int nitile = (n + NT - 1) / NT;
-    int nslices = std::max(1, nb6_num_sms() * pot_ord_occ() / nitile);
-    nslices = std::min(nslices, P.ntile);
-    P.part.reserve((size_t)nslices * n);
-    P.out.reserve(n);
-    PotOrdArgs a;
-    a.posH = P.posH_s.ptr;
-    a.posL = P.posL_s.ptr;
-    a.rel = P.rel.ptr;
-    a.xs = P.xs.ptr;
-    a.tbox = P.tbox.ptr;
-    a.npad = (size_t)P.ntile * JT;
-    a.n = n;
-    a.ntile = P.ntile;
-    a.nslices = nslices;
-    a.part = P.part.ptr;
-    a.status = nb6_dev_status();
-    pot_kernel_ord<<<dim3(nitile, nslices), NT, 0, st>>>(a);
-    NB6_CUDA_CHECK(cudaGetLastError());
-    pot_finalize_ord<<<(n + 255) / 256, 256, 0, st>>>(P.part.ptr, nslices, n, P.perm.ptr, P.out.ptr);
-    NB6_CUDA_CHECK(cudaGetLastError());
-}
-
-template <int NI> int pot_occ() {
-    static int occ = -1;
-    if (occ < 0) {
-        NB6_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, pot_kernel<NI>, NT, 0));
-        if (occ < 1) occ = 1;
-    }
-    return occ;
-}
-
-// The whole set of a large call takes the ordered path (NB6_POT_ORDER=0:
-// never).
-bool pot_ordered(int i0, int ni) {
+// Whether a call orders its set (NB6_POT_ORDER=0: never).
+bool pot_ordered(int ni) {
     static const int ordered = [] {
         const char *e = getenv("NB6_POT_ORDER");
         return (e && atoi(e) == 0) ? 0 : 1;
     }();
-    return ordered && i0 == 0 && ni == P.n && P.n >= POT_ORDER_MIN;
+    return ordered && P.n >= POT_ORDER_MIN && (double)P.n * ni >= POT_ORDER_PAIRS;
 }
 
-// Potential of i in [i0, i0+ni) against the packed j set; result in P.out.
-// The whole set of a large call takes the ordered path (built by
-// pot_prepare).
-void pot_device(int i0, int ni, cudaStream_t st) {
-    if (pot_ordered(i0, ni)) {
-        pot_device_ord(st);
-        return;
-    }
-    int NI = 1;
-    for (int c : {4, 2, 1}) {
-        const int tile = NT * c;
-        const int nit = (ni + tile - 1) / tile;
-        if ((double)ni / ((double)nit * tile) >= 0.9 || c == 1) {
-            NI = c;
-            break;
-        }
-    }
-    const int tile = NT * NI;
-    const int nitile = (ni + tile - 1) / tile;
-    const int occ = NI == 4 ? pot_occ<4>() : NI == 2 ? pot_occ<2>() : pot_occ<1>();
-    int nslices = std::max(1, nb6_num_sms() * occ / nitile);
-    nslices = std::min(nslices, P.ntile);
-    P.part.reserve((size_t)nslices * ni);
-    P.out.reserve(ni);
-    PotArgs a;
-    a.posH = P.posH.ptr;
-    a.posL = P.posL.ptr;
+template <int NI, bool ORD> int pot_occ() {
+    static const int occ = [] {
+        int o = 0;
+        NB6_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, pot_kernel<NI, ORD>, NT, 0));
+        return std::max(o, 1);
+    }();
+    return occ;
+}
+
+// Slices per i-tile.  A call that fills the GPU is cut into about six waves
+// of CTAs, so that the last one leaves little idle, each of at least 16 tiles
+// (its set-up costs about half a tile); a small one into one wave.
+template <int NI, bool ORD> void pot_launch(PotArgs &a, cudaStream_t st) {
+    const int nitile = (a.ni + NT * NI - 1) / (NT * NI);
+    const int slots = nb6_num_sms() * pot_occ<NI, ORD>();
+    const int one_wave = std::max(1, slots / nitile), six_waves = (6 * slots + nitile - 1) / nitile;
+    a.nslices = std::min(std::max(one_wave, std::min(six_waves, a.ntile / 16)), a.ntile);
+    P.part.reserve((size_t)a.nslices * a.ni);
+    a.part = P.part.ptr;
+    pot_kernel<NI, ORD><<<dim3(nitile, a.nslices), NT, 0, st>>>(a);
+    NB6_CUDA_CHECK(cudaGetLastError());
+}
+
+// Potential of i in [i0, i0+ni) of the uploaded bodies (P.dm, P.dx, P.n).
+// The result goes to hout (pinned, with the status word posted) when the
+// call writes it in the caller's order, else to P.out; returns whether it
+// went to hout.
+bool pot_compute(int i0, int ni, double *hout, cudaStream_t st) {
+    const int n = P.n;
+    PotArgs a{};
+    a.x = P.dx;
     a.ntile = P.ntile;
-    a.nslices = nslices;
     a.i0 = i0;
     a.ni = ni;
-    a.part = P.part.ptr;
     a.status = nb6_dev_status();
-    dim3 grid(nitile, nslices);
-    if (NI == 4) pot_kernel<4><<<grid, NT, 0, st>>>(a);
-    else if (NI == 2) pot_kernel<2><<<grid, NT, 0, st>>>(a);
-    else pot_kernel<1><<<grid, NT, 0, st>>>(a);
+    const bool ord = pot_ordered(ni);
+    P.tiles.reserve((size_t)P.ntile * (ord ? ROWS_ORD : ROWS_HL) * JT);
+    a.tiles = P.tiles.ptr;
+    if (ord) {
+        P.order.build(n, P.dx, st);
+        P.tbox.reserve(2 * (size_t)P.ntile);
+        pot_tiles<true><<<P.ntile, JT, 0, st>>>(n, P.order.perm.ptr, P.dm, P.dx, P.tiles.ptr, P.tbox.ptr, a.status);
+        NB6_CUDA_CHECK(cudaGetLastError());
+        a.tbox = P.tbox.ptr;
+        a.idx = P.order.perm.ptr;
+        if (ni < n) {
+            const int sb = (n + SEL_NT - 1) / SEL_NT;
+            P.count.reserve(sb);
+            P.idx.reserve(ni);
+            pot_select_count<<<sb, SEL_NT, 0, st>>>(n, P.order.perm.ptr, i0, ni, P.count.ptr);
+            pot_select<<<sb, SEL_NT, 0, st>>>(n, P.order.perm.ptr, i0, ni, P.count.ptr, P.idx.ptr);
+            NB6_CUDA_CHECK(cudaGetLastError());
+            a.idx = P.idx.ptr;
+        }
+    } else {
+        pot_tiles<false><<<P.ntile, JT, 0, st>>>(n, nullptr, P.dm, P.dx, P.tiles.ptr, nullptr, a.status);
+        NB6_CUDA_CHECK(cudaGetLastError());
+    }
+    // two i per thread once that still leaves a tile of i for every SM
+    const bool two = ni >= 2 * NT * nb6_num_sms() / 8;
+    if (ord) two ? pot_launch<2, true>(a, st) : pot_launch<1, true>(a, st);
+    else two ? pot_launch<2, false>(a, st) : pot_launch<1, false>(a, st);
+    // ordered results are scattered eight bytes at a time: into device memory
+    const bool direct = hout && !ord;
+    P.out.reserve(ni);
+    pot_finalize<<<(ni + 127) / 128, 128, 0, st>>>(P.part.ptr, a.nslices, i0, ni, a.idx,
+                                                   direct ? hout : P.out.ptr, a.status,
+                                                   direct ? nb6_status_post() : nullptr);
     NB6_CUDA_CHECK(cudaGetLastError());
-    pot_finalize<<<(ni + 255) / 256, 256, 0, st>>>(P.part.ptr, nslices, ni, P.out.ptr);
-    NB6_CUDA_CHECK(cudaGetLastError());
+    return direct;
 }
 
 // The bodies of a call on the device (copied from the host when they are
-// there); pot_prepare then packs (and orders) them.
+// there).
 void pot_upload(int n, const double *m, const double *x, cudaStream_t st, bool from_host) {
     P.n = n;
     P.ntile = std::max(1, (n + JT - 1) / JT);
-    const size_t npad = (size_t)P.ntile * JT;
-    const double *dm = m, *dx = x;
+    P.dm = m;
+    P.dx = x;
     if (from_host) {
-        P.m.reserve(npad);
-        P.x.reserve(3 * npad);
-        if (n > 0) {
-            NB6_CUDA_CHECK(cudaMemcpyAsync(P.m.ptr, m, sizeof(double) * n, cudaMemcpyHostToDevice, st));
-            NB6_CUDA_CHECK(cudaMemcpyAsync(P.x.ptr, x, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, st));
-        }
-        dm = P.m.ptr;
-        dx = P.x.ptr;
+        P.m.reserve(n);
+        P.x.reserve(3 * (size_t)n);
+        NB6_CUDA_CHECK(cudaMemcpyAsync(P.m.ptr, m, sizeof(double) * n, cudaMemcpyHostToDevice, st));
+        NB6_CUDA_CHECK(cudaMemcpyAsync(P.x.ptr, x, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, st));
+        P.dm = P.m.ptr;
+        P.dx = P.x.ptr;
     }
-    P.dm = dm;
-    P.dx = dx;
-}
-
-void pot_prepare(int i0, int ni, cudaStream_t st) {
-    const int n = P.n;
-    const size_t npad = (size_t)P.ntile * JT;
-    const double *dm = P.dm, *dx = P.dx;
-    P.posH.reserve(npad);
-    P.posL.reserve(npad);
-    const int blocks = (int)std::min<size_t>((npad + 255) / 256, (size_t)nb6_num_sms() * 8);
-    pot_pack<<<blocks, 256, 0, st>>>(n, (int)npad, dm, dx, P.posH.ptr, P.posL.ptr, nb6_dev_status());
-    NB6_CUDA_CHECK(cudaGetLastError());
-    if (pot_ordered(i0, ni)) pot_order(st);
 }
 
 }  // namespace
@@ -623,15 +498,16 @@ void gpupot_(int *irank, int *istart, int *ni_, int *n_, double *m, double (*x)[
         NB6_CUDA_CHECK(cudaEventCreate(&P.ev0));
         NB6_CUDA_CHECK(cudaEventCreate(&P.ev1));
     }
+    P.hout.reserve(ni);
     pot_upload(n, m, &x[0][0], st, true);
     NB6_CUDA_CHECK(cudaEventRecord(P.ev0, st));
-    pot_prepare(i0, ni, st);
-    pot_device(i0, ni, st);
+    const bool direct = pot_compute(i0, ni, nb6_uva() ? P.hout.ptr : nullptr, st);
     NB6_CUDA_CHECK(cudaEventRecord(P.ev1, st));
-    P.hout.reserve(ni);
-    NB6_CUDA_CHECK(cudaMemcpyAsync(P.hout.ptr, P.out.ptr, sizeof(double) * ni, cudaMemcpyDeviceToHost, st));
+    if (!direct) {
+        NB6_CUDA_CHECK(cudaMemcpyAsync(P.hout.ptr, P.out.ptr, sizeof(double) * ni, cudaMemcpyDeviceToHost, st));
+        nb6_status_fetch(st);
+    }
     NB6_CUDA_CHECK(cudaStreamSynchronize(st));
-    NB6_CUDA_CHECK(cudaEventElapsedTime(&P.last_ms, P.ev0, P.ev1));
     if (nb6_check_dev_status() != 0) return;
     memcpy(pot, P.hout.ptr, sizeof(double) * ni);
     if (getenv("NB6_VERBOSE"))
@@ -652,8 +528,7 @@ void nb6_pot_device_(int *istart, int *ni, int *n, const double *d_m, const doub
     }
     pot_upload(*n, d_m, d_x, st, false);
     NB6_CUDA_CHECK(cudaEventRecord(P.ev0, st));
-    pot_prepare(*istart - 1, *ni, st);
-    pot_device(*istart - 1, *ni, st);
+    pot_compute(*istart - 1, *ni, nullptr, st);
     NB6_CUDA_CHECK(cudaEventRecord(P.ev1, st));
     *d_out = P.out.ptr;
 }

@@ -1,0 +1,31 @@
+"""The force kernels at the sizes where their tiles, ranges and queues can go
+wrong, against the FP64 oracle.  Tolerances: the per-particle bounds of the
+other parity tests (acceleration and potential 1e-6, jerk 1e-5 relative), which
+the FP32 pair math on hi/lo differences with double-single sums meets at any
+size; neighbour lists identical."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from parity import rel_err_vec
+
+pytestmark = pytest.mark.gpu
+
+
+# tile of 128 bodies, i-tile of 128 (256 once ni >= 4736), order from 1e9 pairs
+@pytest.mark.parametrize("n,i0,ni", [(127, 0, 127), (257, 129, 128), (4736, 0, 4736), (5001, 265, 4735),
+                                     (33000, 0, 30304), (33000, 2696, 30304), (40007, 14997, 25010),
+                                     (65537, 65537 - 15361, 15361), (40960, 0, 40960)])
+def test_potential_ranges(nb6, orc, n, i0, ni):
+    """Ranges of the set on both sides of the rule that orders it, at its
+    start, inside and at its end, whole and ragged tiles."""
+    from nb6b200 import ics
+    cl = ics.plummer(n, seed=n + i0, imf=True)
+    x = cl.pos.copy()
+    x[i0] = x[(i0 + 1) % n]                       # a coincident pair
+    p = nb6.gpupot(cl.mass, x, istart=i0 + 1, ni=ni)
+    sel = np.unique(np.concatenate([[0, ni - 1], np.random.default_rng(n).integers(0, ni, 300)]))
+    po = np.array([orc.pot(cl.mass, x, i0 + 1 + int(k), 1)[0] for k in sel])
+    assert np.all(p > 0)
+    assert rel_err_vec(p[sel], po).max() <= 1e-6
