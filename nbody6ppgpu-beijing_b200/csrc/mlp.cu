@@ -7,12 +7,13 @@
 // NNBOPT neighbours at its next regular step (estimated from the count that
 // step found, nnb ~ RS^3).  Loss: mean squared error in standardised units.
 //
-//   mlp_grad_kernel   one warp per sample: bf16-weight forward pass, FP32
-//                     backward pass; per-warp gradient buffers in shared
-//                     memory, summed per CTA in a fixed order;
-//   mlp_reduce        CTA partials summed in block order (deterministic);
-//   mlp_adam          Adam step on the FP32 master copy, then the bf16 copy
-//                     that every forward pass reads.
+//   mlp_grad_kernel   32 samples per CTA and round, one warp each: bf16-weight
+//                     forward pass, FP32 backward pass to the layers' inputs;
+//                     then every thread sums its own parameters' gradients
+//                     over the samples, in a fixed order;
+//   mlp_reduce        CTA partials summed in block order (deterministic), and
+//                     in training the Adam step on the FP32 master copy and
+//                     the bf16 copy that every forward pass reads.
 //
 // The model is small (4,609 parameters, ~4.5 kFLOP per sample), so the
 // passes run on the FP32 pipes: a batch of 1024 samples is ~10 MFLOP, far
@@ -26,10 +27,17 @@
 
 namespace {
 
-constexpr int GW = 4;  // warps per CTA, gradient kernel
-constexpr int MLP_SMEM_W2T = MLP_H * MLP_H * 2;  // transposed W2 (bf16) for the backward pass
-constexpr size_t GRAD_SMEM = (size_t)MLP_SMEM_BYTES + MLP_SMEM_W2T + (size_t)GW * MLP_NPARAM * sizeof(float) +
-                             GW * sizeof(float);
+// Gradient kernel: GW sample streams per CTA, GK samples of each per round,
+// a warp for each of the GW * GK samples.
+constexpr int GW = 4, GK = 8, GS = GW * GK;
+constexpr int W2S = MLP_H + 8;  // row stride of W2 in shared memory (bf16): 16-byte reads of 8 lanes miss no bank
+// What one sample hands from its warp to the gradient sums.
+struct MlpSample {
+    float h1[MLP_H], dz1[MLP_H], h2[MLP_H], dz2[MLP_H];
+    float xn[MLP_IN], d, err2, pad;
+};
+static_assert(sizeof(MlpSample) % 16 == 0, "float4 reads of the sample rows");
+constexpr size_t GRAD_SMEM = (size_t)MLP_SMEM_BYTES + 2 * (size_t)MLP_H * W2S * 2 + GS * sizeof(MlpSample);
 
 struct MlpState {
     bool have = false;      // parameters set or trained
@@ -47,111 +55,203 @@ __global__ void mlp_to_bf16(const float *__restrict__ w32, __nv_bfloat16 *__rest
         w16[k] = __float2bfloat16_rn(k < MLP_NPARAM ? w32[k] : 0.0f);
 }
 
+// Eight bf16 weights (one 16-byte read) times eight inputs, in index order.
+NB6_DEV float fma8(const __nv_bfloat16 *w, const float *in, float z) {
+    const uint4 p = *reinterpret_cast<const uint4 *>(w);
+    const float4 a = *reinterpret_cast<const float4 *>(in), b = *reinterpret_cast<const float4 *>(in + 4);
+    const unsigned q[4] = {p.x, p.y, p.z, p.w};
+    const float v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+        z = fmaf(__uint_as_float(q[c] << 16), v[2 * c], z);
+        z = fmaf(__uint_as_float(q[c] & 0xffff0000u), v[2 * c + 1], z);
+    }
+    return z;
+}
+
 // Gradient of sum_s (out_s - y_s)^2 / n over the samples [off, off + cnt)
 // of the (optionally permuted) set; per-CTA partials into part[block][.],
 // squared-error partials into part_loss[block].
-__global__ void __launch_bounds__(GW * 32)
+//
+// Sample q = (block GW + w) + k (blocks GW) is the k-th of stream w of its
+// block.  A parameter's gradient is summed over k within a stream, then over
+// the streams, so the sums do not depend on how many samples run at a time.
+// Eight samples of each stream are in flight (a warp each): with one warp per
+// stream the kernel was a chain of eight samples' forward and backward passes
+// and of 8,192 read-modify-writes each of a gradient buffer in shared memory
+// (45 us for 1,024 samples; an epoch of 32,768 samples in batches of 1,024
+// 2,070 us, now 1,037 us).  The layers read eight weights per 16-byte load,
+// W2 along its rows (backward) and, from a transposed copy, along its columns
+// (forward).
+__global__ void __launch_bounds__(GS * 32)
     mlp_grad_kernel(int cnt, int off, float inv_n, const float *__restrict__ x, const float *__restrict__ y,
                     const int *__restrict__ perm, const __nv_bfloat16 *__restrict__ w16,
                     const float *__restrict__ norm, float *__restrict__ part, float *__restrict__ part_loss) {
     extern __shared__ __align__(16) unsigned char smem[];
     __nv_bfloat16 *sw = reinterpret_cast<__nv_bfloat16 *>(smem);
-    __nv_bfloat16 *w2t = reinterpret_cast<__nv_bfloat16 *>(smem + MLP_SMEM_BYTES);
-    float *gbuf = reinterpret_cast<float *>(smem + MLP_SMEM_BYTES + MLP_SMEM_W2T);
-    float *lbuf = gbuf + (size_t)GW * MLP_NPARAM;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    __nv_bfloat16 *w2 = sw + MLP_SMEM_BYTES / 2;   // w2[k][r] = W2[k][r]
+    __nv_bfloat16 *w2t = w2 + MLP_H * W2S;         // w2t[r][k] = W2[k][r]
+    MlpSample *smp = reinterpret_cast<MlpSample *>(w2t + MLP_H * W2S);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     mlp_load(sw, w16);
-    for (int k = threadIdx.x; k < MLP_H * MLP_H; k += blockDim.x) {
-        const int kin = k / MLP_H, r = k % MLP_H;  // W2[kin][r] -> w2t[r][kin]
-        w2t[r * MLP_H + kin] = w16[MLP_OFF_W2 + k];
+    for (int q = tid; q < MLP_H * MLP_H; q += GS * 32) {
+        const int k = q / MLP_H, r = q % MLP_H;
+        const __nv_bfloat16 v = w16[MLP_OFF_W2 + q];
+        w2[k * W2S + r] = v;
+        w2t[r * W2S + k] = v;
     }
-    float *g = gbuf + (size_t)warp * MLP_NPARAM;
-    for (int k = lane; k < MLP_NPARAM; k += 32) g[k] = 0.0f;
     __syncthreads();
-    float lsum = 0.0f;
+    // this thread's parameters: W2[gk][gr .. gr+3], and one of the others
+    const int gk = tid >> 4, gr = (tid & 15) * 4;
+    float g2[GW][4], g1[GW];
+#pragma unroll
+    for (int w = 0; w < GW; ++w) g1[w] = g2[w][0] = g2[w][1] = g2[w][2] = g2[w][3] = 0.0f;
+    float lsum[GW] = {0.0f, 0.0f, 0.0f, 0.0f};
     const float ymean = norm[2 * MLP_IN], yinv = 1.0f / norm[2 * MLP_IN + 1];
-    for (int q = blockIdx.x * GW + warp; q < cnt; q += gridDim.x * GW) {
-        const int s = perm ? perm[off + q] : off + q;
-        float f[MLP_IN];
+    const int sw_w = warp % GW, sw_k = warp / GW;
+    MlpSample &S = smp[warp];
+    const int stride = gridDim.x * GW;
+    for (int base = 0; base < cnt; base += GK * stride) {
+        // forward and backward pass of this warp's sample
+        const int q = base + sw_k * stride + blockIdx.x * GW + sw_w;
+        if (q < cnt) {
+            const int s = perm ? perm[off + q] : off + q;
+            float xn[MLP_IN];
 #pragma unroll
-        for (int k = 0; k < MLP_IN; ++k) f[k] = x[(size_t)s * MLP_IN + k];
-        MlpAct a;
-        const float out = mlp_forward_warp(sw, norm, f, lane, a);
-        const float err = out - (y[s] - ymean) * yinv;
-        lsum += err * err;
-        const float d = 2.0f * err * inv_n;
-        if (lane == 0) g[MLP_OFF_B3] += d;
-        float dz2[2];
+            for (int k = 0; k < MLP_IN; ++k) xn[k] = (x[(size_t)s * MLP_IN + k] - norm[k]) * norm[MLP_IN + k];
+            float z1[2], z2[2];
 #pragma unroll
-        for (int u = 0; u < 2; ++u) {
-            const int r = lane + 32 * u;
-            g[MLP_OFF_W3 + r] += d * a.h2[u];
-            dz2[u] = d * bf(sw, MLP_OFF_W3 + r) * mlp_dsilu(a.z2[u]);
-            g[MLP_OFF_B2 + r] += dz2[u];
+            for (int u = 0; u < 2; ++u) {
+                const int r = lane + 32 * u;
+                float z = bf(sw, MLP_OFF_B1 + r);
+#pragma unroll
+                for (int k = 0; k < MLP_IN; ++k) z = fmaf(bf(sw, MLP_OFF_W1 + k * MLP_H + r), xn[k], z);
+                z1[u] = z;
+                S.h1[r] = mlp_silu(z);
+            }
+            __syncwarp();
+#pragma unroll
+            for (int u = 0; u < 2; ++u) z2[u] = bf(sw, MLP_OFF_B2 + lane + 32 * u);
+#pragma unroll
+            for (int k = 0; k < MLP_H; k += 8)
+#pragma unroll
+                for (int u = 0; u < 2; ++u) z2[u] = fma8(w2t + (lane + 32 * u) * W2S + k, S.h1 + k, z2[u]);
+            const float h2[2] = {mlp_silu(z2[0]), mlp_silu(z2[1])};
+            float o = bf(sw, MLP_OFF_W3 + lane) * h2[0] + bf(sw, MLP_OFF_W3 + lane + 32) * h2[1];
+#pragma unroll
+            for (int t = 16; t > 0; t >>= 1) o += __shfl_xor_sync(0xffffffffu, o, t);
+            const float out = o + bf(sw, MLP_OFF_B3);
+            const float err = out - (y[s] - ymean) * yinv;
+            const float d = 2.0f * err * inv_n;
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const int r = lane + 32 * u;
+                S.h2[r] = h2[u];
+                S.dz2[r] = d * bf(sw, MLP_OFF_W3 + r) * mlp_dsilu(z2[u]);
+            }
+            __syncwarp();
+            float dh1[2] = {0.0f, 0.0f};
+#pragma unroll
+            for (int k = 0; k < MLP_H; k += 8)
+#pragma unroll
+                for (int u = 0; u < 2; ++u) dh1[u] = fma8(w2 + (lane + 32 * u) * W2S + k, S.dz2 + k, dh1[u]);
+#pragma unroll
+            for (int u = 0; u < 2; ++u) S.dz1[lane + 32 * u] = dh1[u] * mlp_dsilu(z1[u]);
+            if (lane == 0) {
+#pragma unroll
+                for (int k = 0; k < MLP_IN; ++k) S.xn[k] = xn[k];
+                S.d = d;
+                S.err2 = err;
+            }
+        } else {   // no sample: every product below is zero
+            for (int k = lane; k < (int)(sizeof(MlpSample) / 4); k += 32) reinterpret_cast<float *>(&S)[k] = 0.0f;
         }
-        float dh1[2] = {0.0f, 0.0f};
-#pragma unroll 8
-        for (int k = 0; k < MLP_H; ++k) {
-            const float hk = __shfl_sync(0xffffffffu, a.h1[k >> 5], k & 31);
-            const float dk = __shfl_sync(0xffffffffu, dz2[k >> 5], k & 31);
-            // dW2[k][r] for the lane's r; dh1 for the lane's k' via W2[k'][k] = w2t[k][k']
-            g[MLP_OFF_W2 + k * MLP_H + lane] += dz2[0] * hk;
-            g[MLP_OFF_W2 + k * MLP_H + lane + 32] += dz2[1] * hk;
-            dh1[0] = fmaf(__bfloat162float(w2t[k * MLP_H + lane]), dk, dh1[0]);
-            dh1[1] = fmaf(__bfloat162float(w2t[k * MLP_H + lane + 32]), dk, dh1[1]);
-        }
+        __syncthreads();
 #pragma unroll
-        for (int u = 0; u < 2; ++u) {
-            const int r = lane + 32 * u;
-            const float dz1 = dh1[u] * mlp_dsilu(a.z1[u]);
-            g[MLP_OFF_B1 + r] += dz1;
+        for (int w = 0; w < GW; ++w)
+#pragma unroll 4
+            for (int k = 0; k < GK; ++k) {
+                const MlpSample &T = smp[k * GW + w];
+                const float h = T.h1[gk];
+                const float4 z = *reinterpret_cast<const float4 *>(&T.dz2[gr]);
+                g2[w][0] = fmaf(z.x, h, g2[w][0]);
+                g2[w][1] = fmaf(z.y, h, g2[w][1]);
+                g2[w][2] = fmaf(z.z, h, g2[w][2]);
+                g2[w][3] = fmaf(z.w, h, g2[w][3]);
+            }
+        // the other parameters, by thread: W1, B1, B2, W3, B3 and the loss
 #pragma unroll
-            for (int k = 0; k < MLP_IN; ++k) g[MLP_OFF_W1 + k * MLP_H + r] += dz1 * a.xn[k];
-        }
+        for (int w = 0; w < GW; ++w)
+            for (int k = 0; k < GK; ++k) {
+                const MlpSample &T = smp[k * GW + w];
+                if (tid < MLP_IN * MLP_H) g1[w] = fmaf(T.dz1[tid % MLP_H], T.xn[tid / MLP_H], g1[w]);
+                else if (tid < MLP_OFF_W2) g1[w] += T.dz1[tid % MLP_H];
+                else if (tid < MLP_OFF_W2 + MLP_H) g1[w] += T.dz2[tid % MLP_H];
+                else if (tid < MLP_OFF_W2 + 2 * MLP_H) g1[w] = fmaf(T.d, T.h2[tid % MLP_H], g1[w]);
+                else if (tid == MLP_OFF_W2 + 2 * MLP_H) {
+                    g1[w] += T.d;
+                    lsum[w] = fmaf(T.err2, T.err2, lsum[w]);
+                }
+            }
+        __syncthreads();
     }
-    if (lane == 0) lbuf[warp] = lsum;
-    __syncthreads();
     float *p = part + (size_t)blockIdx.x * MLP_NPARAM;
-    for (int k = threadIdx.x; k < MLP_NPARAM; k += blockDim.x) {
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
         float acc = 0.0f;
 #pragma unroll
-        for (int w = 0; w < GW; ++w) acc += gbuf[(size_t)w * MLP_NPARAM + k];
-        p[k] = acc;
+        for (int w = 0; w < GW; ++w) acc += g2[w][c];
+        p[MLP_OFF_W2 + gk * MLP_H + gr + c] = acc;
     }
-    if (threadIdx.x == 0) {
-        float l = 0.0f;
-        for (int w = 0; w < GW; ++w) l += lbuf[w];
-        part_loss[blockIdx.x] = l;
+    if (tid <= MLP_OFF_W2 + 2 * MLP_H) {
+        float acc = 0.0f, l = 0.0f;
+#pragma unroll
+        for (int w = 0; w < GW; ++w) {
+            acc += g1[w];
+            l += lsum[w];
+        }
+        p[tid < MLP_OFF_W2 ? tid : tid + MLP_H * MLP_H] = acc;
+        if (tid == MLP_OFF_W2 + 2 * MLP_H) part_loss[blockIdx.x] = l;
     }
 }
+
+// The Adam step of one training batch.
+struct AdamArgs {
+    float *w, *m1, *m2;
+    __nv_bfloat16 *w16;
+    float lr, b1, b2, eps, bc1, bc2;
+};
 
 // grad[k] = sum over blocks in block order; loss[0] += sum of squared errors.
-__global__ void mlp_reduce(int nb, const float *__restrict__ part, const float *__restrict__ part_loss,
-                           float *__restrict__ grad, float *__restrict__ loss) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+// ADAM: then the step on parameter k and its bf16 copy, which the next
+// batch's forward pass reads, in the same launch.
+constexpr int RED_NT = 64;
+template <bool ADAM>
+__global__ void __launch_bounds__(RED_NT)
+    mlp_reduce(int nb, const float *__restrict__ part, const float *__restrict__ part_loss,
+               float *__restrict__ grad, float *__restrict__ loss, const AdamArgs ad) {
+    const int k = blockIdx.x * RED_NT + threadIdx.x;
     if (k < MLP_NPARAM) {
-        float acc = 0.0f;
-        for (int b = 0; b < nb; ++b) acc += part[(size_t)b * MLP_NPARAM + k];
-        grad[k] = acc;
-    }
-    if (k == 0) {
+        float g = 0.0f;
+#pragma unroll 16
+        for (int b = 0; b < nb; ++b) g += __ldg(part + (size_t)b * MLP_NPARAM + k);
+        if (ADAM) {
+            const float a = ad.b1 * ad.m1[k] + (1.0f - ad.b1) * g;
+            const float b = ad.b2 * ad.m2[k] + (1.0f - ad.b2) * g * g;
+            ad.m1[k] = a;
+            ad.m2[k] = b;
+            const float w = ad.w[k] - ad.lr * (a / ad.bc1) / (sqrtf(b / ad.bc2) + ad.eps);
+            ad.w[k] = w;
+            ad.w16[k] = __float2bfloat16_rn(w);
+        } else {
+            grad[k] = g;
+        }
+    } else if (k == MLP_NPARAM) {
         float l = 0.0f;
-        for (int b = 0; b < nb; ++b) l += part_loss[b];
+#pragma unroll 16
+        for (int b = 0; b < nb; ++b) l += __ldg(part_loss + b);
         loss[0] += l;
     }
-}
-
-__global__ void mlp_adam(float *__restrict__ w, float *__restrict__ m1, float *__restrict__ m2,
-                         const float *__restrict__ g, float lr, float b1, float b2, float eps, float bc1,
-                         float bc2) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= MLP_NPARAM) return;
-    const float gk = g[k];
-    const float a = b1 * m1[k] + (1.0f - b1) * gk;
-    const float b = b2 * m2[k] + (1.0f - b2) * gk * gk;
-    m1[k] = a;
-    m2[k] = b;
-    w[k] -= lr * (a / bc1) / (sqrtf(b / bc2) + eps);
 }
 
 __global__ void __launch_bounds__(128)
@@ -216,17 +316,20 @@ void mlp_upload_samples(int n, const float *x, const float *y) {
     }
 }
 
-int grad_blocks(int cnt) { return std::max(1, std::min((cnt + GW * 8 - 1) / (GW * 8), nb6_num_sms() * 2)); }
+int grad_blocks(int cnt) { return std::max(1, std::min((cnt + GS - 1) / GS, nb6_num_sms() * 2)); }
 
-// One gradient over samples [off, off+cnt) of the uploaded set into M.grad.
-void mlp_grad_launch(int cnt, int off, const int *perm, cudaStream_t st) {
+// One gradient over samples [off, off+cnt) of the uploaded set: into M.grad,
+// or through the Adam step `adam` into the parameters.
+void mlp_grad_launch(int cnt, int off, const int *perm, const AdamArgs *adam, cudaStream_t st) {
     const int nb = grad_blocks(cnt);
     M.part.reserve((size_t)nb * (MLP_NPARAM + 1));
     float *part_loss = M.part.ptr + (size_t)nb * MLP_NPARAM;
-    mlp_grad_kernel<<<nb, GW * 32, GRAD_SMEM, st>>>(cnt, off, 1.0f / (float)cnt, M.dx.ptr, M.dy.ptr, perm,
+    mlp_grad_kernel<<<nb, GS * 32, GRAD_SMEM, st>>>(cnt, off, 1.0f / (float)cnt, M.dx.ptr, M.dy.ptr, perm,
                                                     M.w16.ptr, M.norm.ptr, M.part.ptr, part_loss);
     NB6_CUDA_CHECK(cudaGetLastError());
-    mlp_reduce<<<(MLP_NPARAM + 255) / 256, 256, 0, st>>>(nb, M.part.ptr, part_loss, M.grad.ptr, M.loss.ptr);
+    constexpr int rb = MLP_NPARAM / RED_NT + 1;   // every parameter, and the loss
+    if (adam) mlp_reduce<true><<<rb, RED_NT, 0, st>>>(nb, M.part.ptr, part_loss, nullptr, M.loss.ptr, *adam);
+    else mlp_reduce<false><<<rb, RED_NT, 0, st>>>(nb, M.part.ptr, part_loss, M.grad.ptr, M.loss.ptr, AdamArgs{});
     NB6_CUDA_CHECK(cudaGetLastError());
 }
 
@@ -302,7 +405,7 @@ void nb6_mlp_grad_(int *n, const float *x, const float *y, float *grad, float *l
     mlp_upload_samples(*n, x, y);
     cudaStream_t st = nb6_stream();
     NB6_CUDA_CHECK(cudaMemsetAsync(M.loss.ptr, 0, sizeof(float), st));
-    mlp_grad_launch(*n, 0, nullptr, st);
+    mlp_grad_launch(*n, 0, nullptr, nullptr, st);
     NB6_CUDA_CHECK(cudaStreamSynchronize(st));
     NB6_CUDA_CHECK(cudaMemcpy(grad, M.grad.ptr, sizeof(float) * MLP_NPARAM, cudaMemcpyDeviceToHost));
     float l = 0.0f;
@@ -325,14 +428,16 @@ void nb6_mlp_train_(int *n_, const float *x, const float *y, int *epochs, int *b
     }
     // moments of the inputs and the target
     float *nm = M.host.data() + MLP_NPARAM;
-    for (int k = 0; k <= MLP_IN; ++k) {
-        double s1 = 0.0, s2 = 0.0;
-        for (int q = 0; q < n; ++q) {
+    // (one pass over the samples: the twelve sums are independent chains)
+    double s1[MLP_IN + 1] = {}, s2[MLP_IN + 1] = {};
+    for (int q = 0; q < n; ++q)
+        for (int k = 0; k <= MLP_IN; ++k) {
             const double v = k < MLP_IN ? x[(size_t)q * MLP_IN + k] : y[q];
-            s1 += v;
-            s2 += v * v;
+            s1[k] += v;
+            s2[k] += v * v;
         }
-        const double mean = s1 / n, var = std::max(s2 / n - mean * mean, 1e-12);
+    for (int k = 0; k <= MLP_IN; ++k) {
+        const double mean = s1[k] / n, var = std::max(s2[k] / n - mean * mean, 1e-12);
         if (k < MLP_IN) {
             nm[k] = (float)mean;
             nm[MLP_IN + k] = (float)(1.0 / std::sqrt(var));
@@ -355,15 +460,11 @@ void nb6_mlp_train_(int *n_, const float *x, const float *y, int *epochs, int *b
         NB6_CUDA_CHECK(cudaMemcpyAsync(M.perm.ptr, perm.data(), sizeof(int) * n, cudaMemcpyHostToDevice, st));
         NB6_CUDA_CHECK(cudaMemsetAsync(M.loss.ptr, 0, sizeof(float), st));
         for (int off = 0; off + B <= n; off += B) {
-            mlp_grad_launch(B, off, M.perm.ptr, st);
             M.adam_t++;
             const float bc1 = 1.0f - std::pow(b1, (float)M.adam_t);
             const float bc2 = 1.0f - std::pow(b2, (float)M.adam_t);
-            mlp_adam<<<(MLP_NPARAM + 255) / 256, 256, 0, st>>>(M.w32.ptr, M.m1.ptr, M.m2.ptr, M.grad.ptr, *lr,
-                                                               b1, b2, eps, bc1, bc2);
-            NB6_CUDA_CHECK(cudaGetLastError());
-            mlp_to_bf16<<<(MLP_SMEM_BYTES / 2 + 255) / 256, 256, 0, st>>>(M.w32.ptr, M.w16.ptr);
-            NB6_CUDA_CHECK(cudaGetLastError());
+            const AdamArgs ad{M.w32.ptr, M.m1.ptr, M.m2.ptr, M.w16.ptr, *lr, b1, b2, eps, bc1, bc2};
+            mlp_grad_launch(B, off, M.perm.ptr, &ad, st);
         }
         float l = 0.0f;
         NB6_CUDA_CHECK(cudaStreamSynchronize(st));

@@ -29,3 +29,24 @@ def test_potential_ranges(nb6, orc, n, i0, ni):
     po = np.array([orc.pot(cl.mass, x, i0 + 1 + int(k), 1)[0] for k in sel])
     assert np.all(p > 0)
     assert rel_err_vec(p[sel], po).max() <= 1e-6
+
+
+# 32 samples per CTA and round; 296 CTAs, so a second round from 9,473 samples
+@pytest.mark.parametrize("n", [31, 32, 33, 1000, 9472, 9473, 20011])
+def test_mlp_gradient_sample_counts(n):
+    """The gradient's sample streams at full and ragged rounds against the
+    FP64 oracle: within 2e-5 of its norm (FP32 sums over the batch)."""
+    import mlp_oracle as M
+    from nb6b200 import mlp
+    rng = np.random.default_rng(n)
+    model = np.zeros(M.NPARAM + M.NNORM, dtype=np.float32)
+    model[:M.NPARAM] = rng.normal(size=M.NPARAM) * 0.15
+    model[M.NPARAM + M.IN:M.NPARAM + 2 * M.IN] = 1.0
+    model[-1] = 0.5
+    mlp.set_model(model)
+    x = rng.normal(size=(n, 5)).astype(np.float32)
+    y = rng.normal(size=n).astype(np.float32)
+    g, loss = mlp.grad(x, y)
+    gr, lr = M.grad(model, x, y)
+    assert abs(loss - lr) <= 1e-5 * lr
+    assert np.linalg.norm(g - gr) <= 2e-5 * np.linalg.norm(gr)
