@@ -167,8 +167,9 @@ NB6_DEV bool reg_pair(const IPart &ip, const float4 &a, const float4 &b, const f
 // or, if it is not one, add its contribution (which the hot loop masked).
 // Operation order matches the FP64 rule of regint.f:41-65 with the strict
 // "<" of gpunb.velocity.cu:188,236; no FMA contraction.
+// Returns whether a contribution was added.
 template <bool MFLAG>
-NB6_DEV void reg_exact(const RegArgs &a, int i, int jslot, Sums &s, int joff = 0) {
+NB6_DEV bool reg_exact(const RegArgs &a, int i, int jslot, Sums &s, int joff = 0) {
     const int j = a.perm ? a.perm[jslot] : jslot;  // the caller's index of the body in this slot
     const double xi0 = a.ix[3 * i], xi1 = a.ix[3 * i + 1], xi2 = a.ix[3 * i + 2];
     const double vi0 = a.iv[3 * i], vi1 = a.iv[3 * i + 1], vi2 = a.iv[3 * i + 2];
@@ -192,6 +193,7 @@ NB6_DEV void reg_exact(const RegArgs &a, int i, int jslot, Sums &s, int joff = 0
         if (rmin < crit) {
             const int pos = atomicAdd(&a.nbcnt[i], 1);
             if (pos < a.lcap) a.nbbuf[(size_t)i * a.lcap + pos] = j - joff;
+            return false;
         } else {
             // inside the slack band but not a neighbour: add it here
             const double rinv2 = 1.0 / r2;
@@ -207,6 +209,7 @@ NB6_DEV void reg_exact(const RegArgs &a, int i, int jslot, Sums &s, int joff = 0
             s.jx += (float)(8.0 * mr3 * (dvx + al * dx));
             s.jy += (float)(8.0 * mr3 * (dvy + al * dy));
             s.jz += (float)(8.0 * mr3 * (dvz + al * dz));
+            return true;
         }
     }
 }
@@ -537,20 +540,6 @@ NB6_DEV unsigned pair_x2d(const IP2 &ip, double xi, double yi, double zi, double
     return (c0 ? 1u : 0u) | (c1 ? 2u : 0u);
 }
 
-// Rare path: the candidates of one 32-j group, as recorded bit by bit by the
-// hot loop, each decided exactly in FP64.
-template <bool MFLAG>
-NB6_DEV Sums reg_flush_mask(const RegArgs &a, int i, unsigned mask, int jbase, Sums s) {
-    while (mask) {
-        const int b = __ffs(mask) - 1;
-        mask &= mask - 1;
-        const int j = jbase + b;
-        if (j >= a.nj) continue;  // padding slots are never neighbours
-        reg_exact<MFLAG>(a, i, j, s);
-    }
-    return s;
-}
-
 // One tile into a stage of NB6_NCOMP float rows.  FP32 layout: the ten float
 // components.  FP64 layout: x, y, z as doubles in row pairs (0,1) (2,3) (4,5),
 // then m, vx, vy, vz in rows 6..9 -- the same 10*JT*4 bytes.
@@ -588,6 +577,13 @@ __global__ void __launch_bounds__(NT, X2_MINB / NI) regf_x2_kernel(const RegArgs
     // double-single accumulators, touched once per tile: kept in shared
     // memory (thread-private slots) to free registers for the pair math
     __shared__ float2 dsum[NI][7][NT];
+    // Each warp's queue of neighbour candidates (j slot, owner lane + 32 k)
+    // awaiting the exact FP64 decision.  They are decided 32 at a time, one
+    // per lane: deciding them where they arise held the whole warp through
+    // the memory round trips of every lane that had one (1,024 of 65,536
+    // bodies: 179 us, now 120 us).  Fewer than 32 wait between pushes and a
+    // push adds at most 32.
+    __shared__ int2 cq[NT / 32][64];
 
     const int tid = threadIdx.x, lane = tid & 31;
     const int slice = blockIdx.y;
@@ -663,6 +659,46 @@ __global__ void __launch_bounds__(NT, X2_MINB / NI) regf_x2_kernel(const RegArgs
             issue_tile_soa<F64DX>(a, sj[st], &bar[st], t_begin + st * t_step);
         issued = min(nt, NSTAGE);
     }
+
+    int2 *const wq = cq[tid >> 5];
+    int qn = 0;  // queued candidates of this warp (warp-uniform)
+    // Decide the last c <= 32 queued candidates, one per lane.  A slot inside
+    // the slack band that is no neighbour returns its contribution to the
+    // lane that owns the i-particle; the order is the queue's, which the data
+    // fix, so results are deterministic.
+    auto drain = [&](int c) {
+        const int2 e = lane < c ? wq[qn - c + lane] : make_int2(0, 0);
+        __syncwarp();
+        qn -= c;
+        int i = __shfl_sync(0xffffffffu, ii[0], e.y & 31);
+#pragma unroll
+        for (int k = 1; k < NI; ++k) {
+            const int ik = __shfl_sync(0xffffffffu, ii[k], e.y & 31);
+            if ((e.y >> 5) == k) i = ik;
+        }
+        Sums x;
+        zero(x);
+        const bool add = lane < c && reg_exact<MFLAG>(a, i, e.x, x);
+        for (unsigned m = __ballot_sync(0xffffffffu, add); m; m &= m - 1) {
+            const int src = __ffs(m) - 1;
+            const int o = __shfl_sync(0xffffffffu, e.y, src);
+            const float v[7] = {__shfl_sync(0xffffffffu, x.ax, src), __shfl_sync(0xffffffffu, x.ay, src),
+                                __shfl_sync(0xffffffffu, x.az, src), __shfl_sync(0xffffffffu, x.jx, src),
+                                __shfl_sync(0xffffffffu, x.jy, src), __shfl_sync(0xffffffffu, x.jz, src),
+                                __shfl_sync(0xffffffffu, x.po, src)};
+#pragma unroll
+            for (int k = 0; k < NI; ++k)
+                if (o == lane + 32 * k) {
+                    fx[k].ax += v[0];
+                    fx[k].ay += v[1];
+                    fx[k].az += v[2];
+                    fx[k].jx += v[3];
+                    fx[k].jy += v[4];
+                    fx[k].jz += v[5];
+                    fx[k].po += v[6];
+                }
+        }
+    };
 
     for (int t = 0; t < nt; ++t) {
         const int st = t % NSTAGE;
@@ -790,9 +826,20 @@ __global__ void __launch_bounds__(NT, X2_MINB / NI) regf_x2_kernel(const RegArgs
                     cnt[k] |= (c01 | (c23 << 2)) << u;
                 }
             }
+            const int j0 = jt0 + g * 32;
+            // padding slots are never neighbours
+            const unsigned real = j0 + 32 <= a.nj ? 0xffffffffu : j0 < a.nj ? (1u << (a.nj - j0)) - 1u : 0u;
 #pragma unroll
-            for (int k = 0; k < NI; ++k)
-                if (cnt[k]) fx[k] = reg_flush_mask<MFLAG>(a, ii[k], cnt[k], jt0 + g * 32, fx[k]);
+            for (int k = 0; k < NI; ++k) {
+                unsigned c = cnt[k] & real, has;
+                while ((has = __ballot_sync(0xffffffffu, c != 0u)) != 0u) {
+                    if (c) wq[qn + __popc(has & ((1u << lane) - 1u))] = make_int2(j0 + __ffs(c) - 1, lane + 32 * k);
+                    c &= c - 1u;
+                    qn += __popc(has);
+                    __syncwarp();
+                    if (qn >= 32) drain(32);
+                }
+            }
         }
         __syncwarp();
         if (lane == 0) mbar_arrive(&ebar[st]);
@@ -825,19 +872,24 @@ __global__ void __launch_bounds__(NT, X2_MINB / NI) regf_x2_kernel(const RegArgs
             zero(fx[k]);
         }
     }
+    if (qn > 0) drain(qn);
 
 #pragma unroll
     for (int k = 0; k < NI; ++k) {
         const int i = ii[k];
         if (i < a.ni) {
+            const float p[7] = {fx[k].ax, fx[k].ay, fx[k].az, fx[k].jx, fx[k].jy, fx[k].jz, fx[k].po};
             float2 d[7];
 #pragma unroll
-            for (int c = 0; c < 7; ++c) d[c] = dsum[k][c][tid];
-            float4 *p = a.part + ((size_t)slice * a.ni_pad + i) * 4;
-            p[0] = make_float4(d[0].x, d[0].y, d[1].x, d[1].y);
-            p[1] = make_float4(d[2].x, d[2].y, d[3].x, d[3].y);
-            p[2] = make_float4(d[4].x, d[4].y, d[5].x, d[5].y);
-            p[3] = make_float4(d[6].x, d[6].y, 0.f, 0.f);
+            for (int c = 0; c < 7; ++c) {
+                d[c] = dsum[k][c][tid];
+                ds_fold(d[c].x, d[c].y, p[c]);   // what the last drain returned
+            }
+            float4 *o = a.part + ((size_t)slice * a.ni_pad + i) * 4;
+            o[0] = make_float4(d[0].x, d[0].y, d[1].x, d[1].y);
+            o[1] = make_float4(d[2].x, d[2].y, d[3].x, d[3].y);
+            o[2] = make_float4(d[4].x, d[4].y, d[5].x, d[5].y);
+            o[3] = make_float4(d[6].x, d[6].y, 0.f, 0.f);
         }
     }
 }
@@ -1421,7 +1473,13 @@ int occupancy(int variant, bool mf) {
     return c;
 }
 
-// Geometry of one variant: enough CTAs for one full wave.
+// Geometry of one variant.  The tile kernels are cut into X2_WAVES waves of
+// CTAs, as long as a CTA keeps X2_MIN_TILES tiles (its set-up costs one or
+// two): the near tiles, with their candidates, fall to the i-tiles in the
+// dense parts, and with one wave the SMs that had none of those idled at the
+// end (1,024 of 996,147 King bodies: one wave 1,131 us, three 1,069, six
+// 1,062, twelve 1,076).  The j-parallel kernels get one wave.
+constexpr int X2_WAVES = 6, X2_MIN_TILES = 8;
 Plan make_plan(int variant, int ni, int nj, int ntile, bool mf, int forced_slices) {
     Plan p;
     p.variant = variant;
@@ -1429,8 +1487,9 @@ Plan make_plan(int variant, int ni, int nj, int ntile, bool mf, int forced_slice
     if (variant > 0) {
         const int tile = NT * i_per_thread(variant);
         p.igrid = (ni + tile - 1) / tile;
-        p.nslices = std::max(1, target / p.igrid);
-        p.nslices = std::min(p.nslices, ntile);
+        const int waves = std::max(1, std::min(X2_WAVES * target / p.igrid, ntile / X2_MIN_TILES));
+        p.nslices = std::min(std::max(target / p.igrid, waves), ntile);
+        p.nslices = std::max(p.nslices, 1);
     } else {
         const int ib = -variant;
         p.igrid = (ni + ib - 1) / ib;

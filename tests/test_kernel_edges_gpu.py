@@ -50,3 +50,65 @@ def test_mlp_gradient_sample_counts(n):
     gr, lr = M.grad(model, x, y)
     assert abs(loss - lr) <= 1e-5 * lr
     assert np.linalg.norm(g - gr) <= 2e-5 * np.linalg.norm(gr)
+
+
+def _shells(n, seed):
+    """n bodies, of which the first 40 sit at the centre of dense shells: most
+    pairs of theirs lie within 1% of their radius, inside and outside."""
+    rng = np.random.default_rng(seed)
+    x = rng.normal(size=(n, 3))
+    v = 0.3 * rng.normal(size=(n, 3))
+    m = rng.uniform(0.5, 1.5, n) / n
+    x[:40] *= 0.02
+    u = rng.normal(size=(n - 40, 3))
+    u /= np.sqrt((u * u).sum(1))[:, None]
+    x[40:] = u * (0.5 * (1.0 + 0.02 * rng.uniform(-1, 1, n - 40)))[:, None]
+    return m, x, v
+
+
+@pytest.mark.parametrize("variant", [11, 12, 13, -1, -2, -4, -8])
+@pytest.mark.parametrize("n", [200, 257, 1291])
+def test_candidate_queue_band_and_overflow(nb6, orc, variant, n):
+    """Candidate queues that fill on nearly every pair: bodies whose pairs
+    crowd the slack band about the radius (candidates that are no neighbours
+    give their force back), rows that list every body, rows that overflow,
+    and a ragged last tile whose padding is within reach."""
+    m, x, v = _shells(n, n)
+    ni = 67
+    h2 = np.full(ni, 0.25)
+    h2[41:45] = 100.0              # every body a neighbour
+    h2[45:47] = 1.0e31             # and the padding slots within reach
+    h2[47:50] = 0.0                # no neighbour at all
+    dtr = np.zeros(ni)
+    dtr[50:] = 2.0 ** -6
+    cap = 1300 if n < 1000 else 400
+    raw = nb6.lib
+    raw.nb6_regf_tune_(C.byref(C.c_int(variant)), C.byref(C.c_int(0)))
+    try:
+        nb6.gpunb_open(n, 0)
+        nb6.gpunb_send(m, x, v)
+        for mf in (0, 1):
+            hh = h2 * n if mf else h2
+            acc, jrk, pot, lst = nb6.gpunb_regf(hh, dtr, x[:ni], v[:ni], cap + 1, cap, mf)
+            oa, oj, op, ol = orc.regf(m, x, v, hh, dtr, x[:ni], v[:ni], cap + 1, cap, mf)
+            np.testing.assert_array_equal(lst[:, 0], ol[:, 0])
+            for r in range(ni):
+                k = max(int(ol[r, 0]), 0)
+                np.testing.assert_array_equal(lst[r, 1:1 + k], ol[r, 1:1 + k])
+            # FP32 sums of n terms against the sum of their sizes
+            j = np.arange(n)
+            for r in range(ni):
+                d = x - x[r]
+                r2 = (d * d).sum(1)
+                use = (r2 > 0) & ~np.isin(j, ol[r, 1:1 + max(int(ol[r, 0]), 0)])
+                if ol[r, 0] < 0:
+                    continue
+                if np.isnan(oa[r]).any():   # radius zero: the body acts on itself
+                    assert h2[r] == 0.0 and np.isnan(acc[r]).any()
+                    continue
+                size = (m[use] / r2[use]).sum()
+                assert np.abs(acc[r] - oa[r]).max() <= 1e-6 * size
+                assert abs(pot[r] - op[r]) <= 1e-6 * abs(op[r]) + 1e-300
+    finally:
+        raw.nb6_regf_tune_(C.byref(C.c_int(0)), C.byref(C.c_int(0)))
+        nb6.gpunb_close()
