@@ -909,12 +909,16 @@ constexpr int JPAR_NT = 256;
 // lanes, negated as pair_x2 takes them).  Padding particles (k >= nvalid)
 // have h2 = 0: never a candidate, results unused.
 template <int IB> struct JparI {
+    static constexpr int V = 7 * IB;           // sums of a CTA's i-particles
+    static constexpr int CH = V < 28 ? V : 28; // of which this many are transposed at a time
     float4 sip[IB][3];
     IP2 sip2[IB > 1 ? IB / 2 : 1];
-    // packed loop: each warp's queue of neighbour candidates (j << 3 | k)
-    // awaiting the exact FP64 decision; fewer than 32 wait between j
-    // iterations, and one iteration adds at most 32 IB
-    unsigned queue[IB > 1 ? JPAR_NT / 32 : 1][IB > 1 ? 32 + 32 * IB : 1];
+    // each warp's queue of neighbour candidates (j << 3 | k) awaiting the
+    // exact FP64 decision; fewer than 32 wait between pushes, and a push adds
+    // at most 32
+    unsigned queue[JPAR_NT / 32][64];
+    float tr[JPAR_NT / 32][CH][33];            // transposition of the lanes' sums
+    double red[JPAR_NT / 32][V];
 };
 
 template <int IB, bool X2>
@@ -947,100 +951,123 @@ NB6_DEV void jpar_stage_i(const RegArgs &a, JparI<IB> &S, int i0, int nvalid) {
 // the IB staged i-particles, results into s[k] (scaled as reg_pair keeps
 // them).  X2 (IB >= 2): two i-particles per f32x2 instruction (pair_x2 on
 // IP2 pairs, the j operands duplicated into both lanes; pair_x2 is reg_pair
-// operation for operation).  Neighbour candidates of the packed loop wait
-// in a per-warp queue and are decided 32 at a time, one per lane: in a small
-// cluster a sizeable share of all pairs are neighbours, and deciding them
-// where they arise would hold the whole warp for every lane that has one.
-// Any lane may decide any queued pair: its contribution joins that lane's
-// partial sum of particle k, which the CTA reduction adds up with the rest.
-// The order is fixed by the data, so results are deterministic; they differ
-// from the scalar loop's (X2 false) in the order of those sums.
+// operation for operation).  Neighbour candidates wait in a per-warp queue
+// and are decided 32 at a time, one per lane: in a small cluster a sizeable
+// share of all pairs are neighbours, and deciding them where they arise would
+// hold the whole warp for every lane that has one.  Any lane may decide any
+// queued pair: its contribution joins that lane's partial sum of particle k,
+// which the CTA reduction adds up with the rest.  The order is fixed by the
+// data, so results are deterministic; they differ from the scalar loop's (X2
+// false) in the order of those sums.
+//
+// Each thread loads its next j before the arithmetic of the current one: at
+// 16 warps per SM (the sums of four i take 100 registers) the L2 round trip
+// was the top stall.  With the ballot-ranked pushes and the transposing
+// reduction (jpar_reduce): 37 i of 500,009 bodies 70 -> 56 us, 531 of 16,384
+// 41 -> 32 us, the 64-cluster work list of regf_seg_kernel 299 -> 245 us.
 template <int IB, bool MFLAG, bool X2>
-NB6_DEV void jpar_loop(const RegArgs &a, const JparI<IB> &S, int j_begin, int j_end, int i0, int nvalid,
+NB6_DEV void jpar_loop(const RegArgs &a, JparI<IB> &S, int j_begin, int j_end, int i0, int nvalid,
                        int jbase, Sums *s) {
-    if constexpr (X2 && IB > 1) {
-        constexpr int NP = IB / 2;
+    if constexpr (X2 || IB == 1) {
+        constexpr int NP = IB > 1 ? IB / 2 : 1;
         S2 acc[NP];
 #pragma unroll
         for (int p = 0; p < NP; ++p) zero2(acc[p]);
+        zero(s[0]);
+        IPart ip1;
+        if constexpr (IB == 1) {
+            const float4 p = S.sip[0][0], q = S.sip[0][1], r = S.sip[0][2];
+            ip1.xh = p.x; ip1.yh = p.y; ip1.zh = p.z; ip1.h2c = p.w;
+            ip1.xl = q.x; ip1.yl = q.y; ip1.zl = q.z; ip1.dt = q.w;
+            ip1.vx = r.x; ip1.vy = r.y; ip1.vz = r.z;
+        }
         const int lane = threadIdx.x & 31;
-        unsigned *qw = const_cast<unsigned *>(S.queue[threadIdx.x >> 5]);
+        unsigned *qw = S.queue[threadIdx.x >> 5];
         int qn = 0;  // queued candidates of this warp (warp-uniform)
-        // decide queued entry e on this lane: its exact contribution (or its
-        // neighbour record) into lane k & 1 of acc[k / 2]
-        auto decide = [&](unsigned e) {
+        // decide the last c <= 32 queued candidates, one per lane: a
+        // neighbour's record, or its exact contribution into lane k & 1 of
+        // acc[k / 2]
+        auto drain = [&](int c) {
+            const unsigned e = lane < c ? qw[qn - c + lane] : 0u;
+            __syncwarp();
+            qn -= c;
+            if (lane >= c) return;
             const int k = (int)(e & 7u), jj = (int)(e >> 3);
             Sums t;
             zero(t);
-            reg_exact<MFLAG>(a, i0 + k, jj, t, jbase);
+            if (!reg_exact<MFLAG>(a, i0 + k, jj, t, jbase)) return;
+            if constexpr (IB == 1) {
+                s[0].ax += t.ax; s[0].ay += t.ay; s[0].az += t.az;
+                s[0].jx += t.jx; s[0].jy += t.jy; s[0].jz += t.jz; s[0].po += t.po;
+            } else {
 #pragma unroll
-            for (int kk = 0; kk < IB; ++kk) {
-                if (kk != k) continue;
-                S2 &q = acc[kk >> 1];
-                if (kk & 1) {
-                    q.ax.y -= t.ax; q.ay.y -= t.ay; q.az.y -= t.az;
-                    q.jx.y -= t.jx; q.jy.y -= t.jy; q.jz.y -= t.jz; q.po.y -= t.po;
-                } else {
-                    q.ax.x -= t.ax; q.ay.x -= t.ay; q.az.x -= t.az;
-                    q.jx.x -= t.jx; q.jy.x -= t.jy; q.jz.x -= t.jz; q.po.x -= t.po;
+                for (int kk = 0; kk < IB; ++kk) {
+                    if (kk != k) continue;
+                    S2 &q = acc[kk >> 1];
+                    if (kk & 1) {
+                        q.ax.y -= t.ax; q.ay.y -= t.ay; q.az.y -= t.az;
+                        q.jx.y -= t.jx; q.jy.y -= t.jy; q.jz.y -= t.jz; q.po.y -= t.po;
+                    } else {
+                        q.ax.x -= t.ax; q.ay.x -= t.ay; q.az.x -= t.az;
+                        q.jx.x -= t.jx; q.jy.x -= t.jy; q.jz.x -= t.jz; q.po.x -= t.po;
+                    }
                 }
             }
         };
-        const int j_stop = j_begin + (int)((j_end - j_begin + JPAR_NT - 1) / JPAR_NT) * JPAR_NT;
-        for (int j = j_begin + lane + (int)(threadIdx.x & ~31u); j < j_stop; j += JPAR_NT) {
-            // every lane of the warp takes every iteration (the queue is the
-            // warp's); lanes past j_end compute nothing
+        int j = j_begin + (int)threadIdx.x;
+        float4 na = make_float4(0.f, 0.f, 0.f, 0.f), nb = na, nc = na;
+        if (j < j_end) {
+            na = __ldg(a.posH + j);
+            nb = __ldg(a.posL + j);
+            nc = __ldg(a.vel + j);
+        }
+        // every lane of the warp takes every iteration (the queue is the
+        // warp's); lanes past j_end compute nothing
+        for (int left = j_end - j_begin; left > 0; left -= JPAR_NT, j += JPAR_NT) {
+            const float4 pa = na, pb = nb, pc = nc;
+            if (j + JPAR_NT < j_end) {
+                na = __ldg(a.posH + j + JPAR_NT);
+                nb = __ldg(a.posL + j + JPAR_NT);
+                nc = __ldg(a.vel + j + JPAR_NT);
+            }
             unsigned cm = 0u;
             if (j < j_end) {
-                const float4 pa = __ldg(a.posH + j);
-                const float4 pb = __ldg(a.posL + j);
-                const float4 pc = __ldg(a.vel + j);
+                if constexpr (IB == 1) {
+                    cm = reg_pair<MFLAG>(ip1, pa, pb, pc, s[0]) ? 1u : 0u;
+                } else {
 #pragma unroll
-                for (int p = 0; p < NP; ++p) {
-                    const IP2 ip = S.sip2[p];
-                    cm |= pair_x2<MFLAG>(ip, dup2(pa.x), dup2(pa.y), dup2(pa.z), dup2(pa.w), dup2(pb.x),
-                                         dup2(pb.y), dup2(pb.z), dup2(pc.x), dup2(pc.y), dup2(pc.z), acc[p])
-                          << (2 * p);
+                    for (int p = 0; p < NP; ++p) {
+                        const IP2 ip = S.sip2[p];
+                        cm |= pair_x2<MFLAG>(ip, dup2(pa.x), dup2(pa.y), dup2(pa.z), dup2(pa.w), dup2(pb.x),
+                                             dup2(pb.y), dup2(pb.z), dup2(pc.x), dup2(pc.y), dup2(pc.z), acc[p])
+                              << (2 * p);
+                    }
                 }
             }
-            if (__any_sync(0xffffffffu, cm != 0u)) {
-                // append this lane's candidates after those of the lanes below
-                const int c = __popc(cm);
-                int pre = c;
-#pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const int t = __shfl_up_sync(0xffffffffu, pre, o);
-                    if (lane >= o) pre += t;
-                }
-                const int tot = __shfl_sync(0xffffffffu, pre, 31);
-                int w = qn + pre - c;
-                for (unsigned m = cm; m; m &= m - 1) qw[w++] = ((unsigned)j << 3) | (unsigned)(__ffs(m) - 1);
+            // push the candidates, one per lane and round
+            unsigned has;
+            while ((has = __ballot_sync(0xffffffffu, cm != 0u)) != 0u) {
+                if (cm) qw[qn + __popc(has & ((1u << lane) - 1u))] = ((unsigned)j << 3) | (unsigned)(__ffs(cm) - 1);
+                cm &= cm - 1u;
+                qn += __popc(has);
                 __syncwarp();
-                qn += tot;
-                while (qn >= 32) {  // warp-uniform
-                    const unsigned e = qw[qn - 32 + lane];
-                    __syncwarp();
-                    qn -= 32;
-                    decide(e);
-                }
+                if (qn >= 32) drain(32);
             }
         }
-        if (qn > 0) {
-            const unsigned e = lane < qn ? qw[lane] : 0u;
-            __syncwarp();
-            if (lane < qn) decide(e);
-        }
+        if (qn > 0) drain(qn);
+        if constexpr (IB > 1) {
 #pragma unroll
-        for (int k = 0; k < IB; ++k) {
-            const S2 &q = acc[k >> 1];
-            const bool hi = k & 1;
-            s[k].ax = -(hi ? q.ax.y : q.ax.x);
-            s[k].ay = -(hi ? q.ay.y : q.ay.x);
-            s[k].az = -(hi ? q.az.y : q.az.x);
-            s[k].jx = -(hi ? q.jx.y : q.jx.x);
-            s[k].jy = -(hi ? q.jy.y : q.jy.x);
-            s[k].jz = -(hi ? q.jz.y : q.jz.x);
-            s[k].po = -(hi ? q.po.y : q.po.x);
+            for (int k = 0; k < IB; ++k) {
+                const S2 &q = acc[k >> 1];
+                const bool hi = k & 1;
+                s[k].ax = -(hi ? q.ax.y : q.ax.x);
+                s[k].ay = -(hi ? q.ay.y : q.ay.x);
+                s[k].az = -(hi ? q.az.y : q.az.x);
+                s[k].jx = -(hi ? q.jx.y : q.jx.x);
+                s[k].jy = -(hi ? q.jy.y : q.jy.x);
+                s[k].jz = -(hi ? q.jz.y : q.jz.x);
+                s[k].po = -(hi ? q.po.y : q.po.x);
+            }
         }
     } else {
 #pragma unroll
@@ -1073,11 +1100,46 @@ NB6_DEV void jpar_loop(const RegArgs &a, const JparI<IB> &S, int j_begin, int j_
     }
 }
 
-template <int IB, bool MFLAG, bool X2 = false>
-__global__ void __launch_bounds__(JPAR_NT) regf_jpar_kernel(const RegArgs a) {
-    __shared__ __align__(16) JparI<IB> S;
-    __shared__ double red[JPAR_NT / 32][IB][7];
+// The CTA's sums of its IB i-particles in FP64, as (hi, lo) pairs into the
+// partial rows part[4 row(k)] of its first nvalid particles.  Each warp
+// transposes its lanes' sums through shared memory, so that a lane adds up
+// one sum's 32 terms: a shuffle tree for each of the 28 sums of IB = 4 took
+// 420 instructions, a fifth of a 4,600-pair work item.
+template <int IB, class Row>
+NB6_DEV void jpar_reduce(JparI<IB> &S, const Sums *s, float4 *__restrict__ part, int nvalid, Row row) {
+    constexpr int V = JparI<IB>::V, CH = JparI<IB>::CH;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+#pragma unroll
+    for (int base = 0; base < V; base += CH) {
+#pragma unroll
+        for (int r = 0; r < CH; ++r) {
+            const Sums &q = s[(base + r) / 7];
+            const float v[7] = {q.ax, q.ay, q.az, q.jx, q.jy, q.jz, q.po};
+            S.tr[warp][r][lane] = v[(base + r) % 7];
+        }
+        __syncwarp();
+        if (lane < CH) {
+            double w[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+            for (int l = 0; l < 32; ++l) w[l & 3] += (double)S.tr[warp][lane][l];
+            S.red[warp][base + lane] = (w[0] + w[1]) + (w[2] + w[3]);
+        }
+        __syncwarp();
+    }
+    __syncthreads();
+    if (tid < V && tid / 7 < nvalid) {
+        double w = 0.0;
+#pragma unroll
+        for (int q = 0; q < JPAR_NT / 32; ++q) w += S.red[q][tid];
+        const float hi = (float)w;
+        reinterpret_cast<float2 *>(part + 4 * row(tid / 7))[tid % 7] = make_float2(hi, (float)(w - (double)hi));
+    }
+}
+
+// (IB = 8 keeps 56 sums: one CTA per SM.)
+template <int IB, bool MFLAG, bool X2 = false>
+__global__ void __launch_bounds__(JPAR_NT, IB <= 4 ? 2 : 1) regf_jpar_kernel(const RegArgs a) {
+    __shared__ __align__(16) JparI<IB> S;
     const int i0 = blockIdx.x * IB;
     jpar_stage_i<IB, X2>(a, S, i0, a.ni - i0);
     __syncthreads();
@@ -1085,42 +1147,7 @@ __global__ void __launch_bounds__(JPAR_NT) regf_jpar_kernel(const RegArgs a) {
     const int j_end = (int)(((long long)(blockIdx.y + 1) * a.nj) / a.nslices);
     Sums s[IB];
     jpar_loop<IB, MFLAG, X2>(a, S, j_begin, j_end, i0, a.ni - i0, 0, s);
-    // CTA reduction in FP64: warp shuffles, then across warps in shared memory
-#pragma unroll
-    for (int k = 0; k < IB; ++k) {
-        double v[7] = {s[k].ax, s[k].ay, s[k].az, s[k].jx, s[k].jy, s[k].jz, s[k].po};
-#pragma unroll
-        for (int c = 0; c < 7; ++c) {
-            const double w = warp_sum_d(v[c]);
-            if (lane == 0) red[warp][k][c] = w;
-        }
-    }
-    __syncthreads();
-    if (tid < IB * 7) {
-        const int k = tid / 7, c = tid % 7;
-        double w = 0.0;
-#pragma unroll
-        for (int q = 0; q < JPAR_NT / 32; ++q) w += red[q][k][c];
-        red[0][k][c] = w;
-    }
-    __syncthreads();
-    if (tid < IB) {
-        const int i = i0 + tid;
-        if (i < a.ni) {
-            float hv[7], lv[7];
-#pragma unroll
-            for (int c = 0; c < 7; ++c) {
-                const double w = red[0][tid][c];
-                hv[c] = (float)w;
-                lv[c] = (float)(w - (double)hv[c]);
-            }
-            float4 *p = a.part + ((size_t)blockIdx.y * a.ni_pad + i) * 4;
-            p[0] = make_float4(hv[0], lv[0], hv[1], lv[1]);
-            p[1] = make_float4(hv[2], lv[2], hv[3], lv[3]);
-            p[2] = make_float4(hv[4], lv[4], hv[5], lv[5]);
-            p[3] = make_float4(hv[6], lv[6], 0.f, 0.f);
-        }
-    }
+    jpar_reduce<IB>(S, s, a.part, a.ni - i0, [&](int k) { return (size_t)blockIdx.y * a.ni_pad + i0 + k; });
 }
 
 // Accumulate one (hi, lo) slice partial into FP64 sums.
@@ -1246,12 +1273,10 @@ struct SegItem {
 };
 
 template <int IB, bool MFLAG, bool X2 = false>
-__global__ void __launch_bounds__(JPAR_NT)
+__global__ void __launch_bounds__(JPAR_NT, 2)
     regf_seg_kernel(const RegArgs a, const SegItem *__restrict__ items, const int *__restrict__ nitems_p,
                     const int2 *__restrict__ pinfo) {
     __shared__ __align__(16) JparI<IB> S;
-    __shared__ double red[JPAR_NT / 32][IB][7];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int nitems = *nitems_p;
     for (int w = blockIdx.x; w < nitems; w += gridDim.x) {
         const SegItem it = items[w];
@@ -1260,39 +1285,7 @@ __global__ void __launch_bounds__(JPAR_NT)
         __syncthreads();
         Sums s[IB];
         jpar_loop<IB, MFLAG, X2>(a, S, it.j0, it.j1, it.i0, it.ni, it.jbase, s);
-#pragma unroll
-        for (int k = 0; k < IB; ++k) {
-            double v[7] = {s[k].ax, s[k].ay, s[k].az, s[k].jx, s[k].jy, s[k].jz, s[k].po};
-#pragma unroll
-            for (int c = 0; c < 7; ++c) {
-                const double wsum = warp_sum_d(v[c]);
-                if (lane == 0) red[warp][k][c] = wsum;
-            }
-        }
-        __syncthreads();
-        if (tid < IB * 7) {
-            const int k = tid / 7, c = tid % 7;
-            double wsum = 0.0;
-#pragma unroll
-            for (int q = 0; q < JPAR_NT / 32; ++q) wsum += red[q][k][c];
-            red[0][k][c] = wsum;
-        }
-        __syncthreads();
-        if (tid < it.ni && tid < IB) {
-            const int i = it.i0 + tid;
-            float hv[7], lv[7];
-#pragma unroll
-            for (int c = 0; c < 7; ++c) {
-                const double wsum = red[0][tid][c];
-                hv[c] = (float)wsum;
-                lv[c] = (float)(wsum - (double)hv[c]);
-            }
-            float4 *p = a.part + ((size_t)pinfo[i].x + it.q) * 4;
-            p[0] = make_float4(hv[0], lv[0], hv[1], lv[1]);
-            p[1] = make_float4(hv[2], lv[2], hv[3], lv[3]);
-            p[2] = make_float4(hv[4], lv[4], hv[5], lv[5]);
-            p[3] = make_float4(hv[6], lv[6], 0.f, 0.f);
-        }
+        jpar_reduce<IB>(S, s, a.part, it.ni, [&](int k) { return (size_t)pinfo[it.i0 + k].x + it.q; });
     }
 }
 
@@ -1478,7 +1471,7 @@ int occupancy(int variant, bool mf) {
 // two): the near tiles, with their candidates, fall to the i-tiles in the
 // dense parts, and with one wave the SMs that had none of those idled at the
 // end (1,024 of 996,147 King bodies: one wave 1,131 us, three 1,069, six
-// 1,062, twelve 1,076).  The j-parallel kernels get one wave.
+// 1,062, twelve 1,076).
 constexpr int X2_WAVES = 6, X2_MIN_TILES = 8;
 Plan make_plan(int variant, int ni, int nj, int ntile, bool mf, int forced_slices) {
     Plan p;
@@ -1491,11 +1484,22 @@ Plan make_plan(int variant, int ni, int nj, int ntile, bool mf, int forced_slice
         p.nslices = std::min(std::max(target / p.igrid, waves), ntile);
         p.nslices = std::max(p.nslices, 1);
     } else {
+        // the j range of each i-group cut so that the launch is short: w
+        // waves of CTAs, each of nj / (256 slices) steps and about four
+        // steps' worth of set-up and reduction
         const int ib = -variant;
         p.igrid = (ni + ib - 1) / ib;
-        // at least 4 j per thread so the per-CTA set-up and reduction amortise
-        const int maxsl = std::max(1, nj / (JPAR_NT * 4));
-        p.nslices = std::max(1, std::min(target / p.igrid, maxsl));
+        const double steps = std::max(1.0, (double)nj / JPAR_NT);
+        double best = 1e300;
+        for (int w = 1; w <= 8; ++w) {
+            const int sl = (int)std::max(1.0, std::min((double)((long long)w * target / p.igrid), steps));
+            const int waves = (int)(((long long)p.igrid * sl + target - 1) / target);
+            const double cost = waves * (std::ceil(steps / sl) + 4.0);
+            if (cost < best) {
+                best = cost;
+                p.nslices = sl;
+            }
+        }
     }
     if (forced_slices > 0) p.nslices = variant > 0 ? std::min(forced_slices, ntile) : forced_slices;
     p.nslices = std::max(p.nslices, 1);
