@@ -1162,9 +1162,57 @@ NB6_DEV void add_partial(const float4 *p, double *v) {
     v[6] += (double)q3.x + (double)q3.y;
 }
 
+// One list row of n <= 32 R ids: sorted ascending by a bitonic network over
+// R registers per lane (id r * 32 + lane in register r), exchanges below 32
+// through shuffles and the others within a lane, then written with the count
+// in front as whole 32-entry lines.  The network in shared memory that longer
+// rows take costs 12 instructions and a warp barrier per exchange: 531 rows of
+// up to 400 ids spent 40 us of a 180 us call in it.
+constexpr int ROW_REGS = 16;
+template <int R>
+NB6_DEV void write_sorted_row(int *__restrict__ row, const int *__restrict__ src, int n, int lane) {
+    int key[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) key[r] = r * 32 + lane < n ? src[r * 32 + lane] : INT_MAX;
+#pragma unroll
+    for (int kk = 2; kk <= 32 * R; kk <<= 1) {
+#pragma unroll
+        for (int jj = kk >> 1; jj > 0; jj >>= 1) {
+            if (jj >= 32) {
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                    const int q = r ^ (jj / 32);
+                    if (q <= r) continue;
+                    const int lo = min(key[r], key[q]), hi = max(key[r], key[q]);
+                    const bool up = ((r * 32) & kk) == 0;
+                    key[r] = up ? lo : hi;
+                    key[q] = up ? hi : lo;
+                }
+            } else {
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                    const int other = __shfl_xor_sync(0xffffffffu, key[r], jj);
+                    const bool up = ((r * 32 + lane) & kk) == 0;
+                    key[r] = up == ((lane & jj) == 0) ? min(key[r], other) : max(key[r], other);
+                }
+            }
+        }
+    }
+    int before = n;   // what stands in front of this register's first id
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const int up = __shfl_up_sync(0xffffffffu, key[r], 1);
+        const int last = __shfl_sync(0xffffffffu, key[r], 31);
+        if (r * 32 + lane <= n) row[r * 32 + lane] = lane == 0 ? before : up;
+        before = last;
+    }
+    if (n == 32 * R && lane == 0) row[n] = before;
+}
+
 // Second half of a finalize row (one warp, one i): reduce the lanes' FP64
 // sums, write outf, reset the neighbour counter, and write the list row
-// sorted ascending (warp bitonic sort in shared memory) or -nnb on overflow.
+// sorted ascending (sb: shared memory for rows beyond 32 ROW_REGS ids) or
+// -nnb on overflow.
 // Host calls have the rows written straight into pinned host memory, where a
 // store costs a bus transaction of its own unless the warp's lanes write one
 // run: the eight doubles leave as one 64-byte store and the list row (its
@@ -1198,28 +1246,35 @@ NB6_DEV void finalize_row(int i, int lane, double *v, int *__restrict__ nbcnt,
         if (lane == 0) row[0] = -n;
         return;
     }
-    int P = 32;
-    while (P < n) P <<= 1;
     const int *src = nbbuf + (size_t)i * lcap;
-    for (int k = lane; k < P; k += 32) sb[k] = (k < n) ? src[k] : INT_MAX;
-    __syncwarp();
-    for (int kk = 2; kk <= P; kk <<= 1) {
-        for (int jj = kk >> 1; jj > 0; jj >>= 1) {
-            for (int x = lane; x < P; x += 32) {
-                const int y = x ^ jj;
-                if (y > x) {
-                    const int p0 = sb[x], p1 = sb[y];
-                    const bool up = (x & kk) == 0;
-                    if ((p0 > p1) == up) {
-                        sb[x] = p1;
-                        sb[y] = p0;
+    if (n <= 32) write_sorted_row<1>(row, src, n, lane);
+    else if (n <= 64) write_sorted_row<2>(row, src, n, lane);
+    else if (n <= 128) write_sorted_row<4>(row, src, n, lane);
+    else if (n <= 256) write_sorted_row<8>(row, src, n, lane);
+    else if (n <= 32 * ROW_REGS) write_sorted_row<ROW_REGS>(row, src, n, lane);
+    else {
+        int P = 32;
+        while (P < n) P <<= 1;
+        for (int k = lane; k < P; k += 32) sb[k] = (k < n) ? src[k] : INT_MAX;
+        __syncwarp();
+        for (int kk = 2; kk <= P; kk <<= 1) {
+            for (int jj = kk >> 1; jj > 0; jj >>= 1) {
+                for (int x = lane; x < P; x += 32) {
+                    const int y = x ^ jj;
+                    if (y > x) {
+                        const int p0 = sb[x], p1 = sb[y];
+                        const bool up = (x & kk) == 0;
+                        if ((p0 > p1) == up) {
+                            sb[x] = p1;
+                            sb[y] = p0;
+                        }
                     }
                 }
+                __syncwarp();
             }
-            __syncwarp();
         }
+        for (int k = lane; k <= n; k += 32) row[k] = k == 0 ? n : sb[k - 1];
     }
-    for (int k = lane; k <= n; k += 32) row[k] = k == 0 ? n : sb[k - 1];
 }
 
 // The device status word into the pinned copy the host reads after the
@@ -1852,6 +1907,14 @@ struct RegLaunch {
     bool direct = false;
 };
 
+// Shared-memory words per warp that rows of up to cap ids need to be sorted.
+static int sort_words(int cap) {
+    if (cap <= 32 * ROW_REGS) return 0;
+    int p = 64 * ROW_REGS;
+    while (p < cap) p <<= 1;
+    return p;
+}
+
 // Row stride of a list of W ints in the pinned staging: whole 128-byte lines,
 // so that a row's lines are written by one store each (finalize_row).
 static int host_row_stride(int W) { return (W + 31) / 32 * 32; }
@@ -2078,8 +2141,7 @@ static void regf_prepare(int ni, const double *d_h2, const double *d_dtr, const 
     R.last_geometry[1] = plan.igrid;
     R.last_geometry[2] = plan.nslices;
 
-    int pmax = 32;
-    while (pmax < cap) pmax <<= 1;
+    const int pmax = sort_words(cap);
     const MlpArgs mlp = nb6_mlp_args(d_h2, d_dtr);
     const size_t smem = (size_t)FIN_WARPS * pmax * sizeof(int) + (mlp.on ? MLP_SMEM_BYTES : 0);
     if (smem > 48 * 1024)
@@ -2841,8 +2903,7 @@ void nb6_regf_seg_(int *ni_, int *iseg, double *h2, double *dtr, double (*xi)[3]
     R.last_geometry[0] = -ib;
     R.last_geometry[1] = std::min(nitems, grid_max);
     R.last_geometry[2] = nitems;
-    int pmax = 32;
-    while (pmax < cap) pmax <<= 1;
+    const int pmax = sort_words(cap);
     const MlpArgs mlp = nb6_mlp_args(a.ih2, a.idtr);
     const size_t smem = (size_t)FIN_WARPS * pmax * sizeof(int) + (mlp.on ? MLP_SMEM_BYTES : 0);
     if (smem > 48 * 1024)

@@ -112,3 +112,37 @@ def test_candidate_queue_band_and_overflow(nb6, orc, variant, n):
     finally:
         raw.nb6_regf_tune_(C.byref(C.c_int(0)), C.byref(C.c_int(0)))
         nb6.gpunb_close()
+
+
+@pytest.mark.parametrize("cap", [31, 400, 512, 700])
+def test_list_rows_at_register_widths(nb6, orc, cap):
+    """List rows whose count falls on either side of the widths the sort
+    takes in registers (32 .. 512 ids) and in shared memory, with and without
+    room in the row; the caller's row past the count is left alone."""
+    n = 1100
+    rng = np.random.default_rng(cap)
+    m = np.full(n, 1.0 / n)
+    x = np.zeros((n, 3))
+    x[:, 0] = rng.permutation(n)          # body at rank k: k neighbours within k + 1/2 of the first
+    v = np.zeros((n, 3))
+    at0 = int(np.argmin(x[:, 0]))
+    counts = np.array([1, 2, 30, 31, 32, 33, 63, 64, 65, 127, 128, 129, 255, 256, 257, 399, 400, 401, 511, 512,
+                       513, 699, 700, 701, 1100])
+    h2 = (counts - 0.5) ** 2
+    ni = len(counts)
+    xi, vi, dtr = np.repeat(x[at0:at0 + 1], ni, 0), np.zeros((ni, 3)), np.zeros(ni)
+    nb6.gpunb_open(n, 0)
+    try:
+        nb6.gpunb_send(m, x, v)
+        acc, jrk, pot, lst = nb6.gpunb_regf(h2, dtr, xi, vi, cap + 1, cap, 0)
+    finally:
+        nb6.gpunb_close()
+    order = np.argsort(x[:, 0])
+    for r, c in enumerate(counts):
+        if c > cap:
+            assert lst[r, 0] == -c
+            assert np.all(lst[r, 1:] == 0)
+        else:
+            assert lst[r, 0] == c
+            np.testing.assert_array_equal(lst[r, 1:1 + c], np.sort(order[:c]))
+            assert np.all(lst[r, 1 + c:] == 0)
