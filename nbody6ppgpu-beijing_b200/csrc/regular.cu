@@ -1436,7 +1436,7 @@ struct RegState {
     struct Graph {
         cudaGraph_t g = nullptr;
         cudaGraphExec_t x = nullptr;
-        cudaGraphNode_t h2d = nullptr, kmain = nullptr, kfin = nullptr, d2hf = nullptr, d2hl = nullptr;
+        cudaGraphNode_t kstage = nullptr, kmain = nullptr, kfin = nullptr;
     } graph[2];
     int use_graphs = -1;               // -1 = read NB6_GRAPHS on first use
     long long graph_builds = 0, graph_launches = 0;
@@ -1752,11 +1752,14 @@ __global__ void jset_rel(int npad, int ntile, const double *__restrict__ compd, 
 }
 
 // Spatial order of the active set of one call (ni <= ISORT_MAX): Morton keys
-// on the j set's grid, bitonic sort of (key, index) in one CTA.
-constexpr int ISORT_MAX = 4096;
-__global__ void __launch_bounds__(1024) iset_order(int ni, const double *__restrict__ ix,
-                                                   const unsigned *__restrict__ ext, int *__restrict__ iperm) {
-    __shared__ unsigned long long kv[ISORT_MAX];
+// on the j set's grid, bitonic sort of (key, index) in one CTA, element
+// r * STAGE_NT + tid in register r: exchanges below 32 go through shuffles,
+// those of STAGE_NT and more stay within a thread, the others through shared
+// memory.
+constexpr int ISORT_MAX = 4096, STAGE_NT = 1024;
+template <int E>
+NB6_DEV void order_active(int ni, const double *__restrict__ ix, const unsigned *__restrict__ ext,
+                          int *__restrict__ iperm, unsigned long long *kv) {
     float lo[3], sc[3];
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
@@ -1764,10 +1767,12 @@ __global__ void __launch_bounds__(1024) iset_order(int ni, const double *__restr
         const float w = ord2f(ext[3 + k]) - lo[k];
         sc[k] = w > 0.f ? 1023.99f / w : 0.f;
     }
-    int P = 1;
-    while (P < ni) P <<= 1;
-    for (int s = threadIdx.x; s < P; s += blockDim.x) {
-        unsigned long long v = ~0ull;  // padding sorts last
+    const int tid = threadIdx.x;
+    unsigned long long v[E];
+#pragma unroll
+    for (int r = 0; r < E; ++r) {
+        const int s = r * STAGE_NT + tid;
+        v[r] = ~0ull;  // padding sorts last
         if (s < ni) {
             unsigned key = 0;
 #pragma unroll
@@ -1776,26 +1781,74 @@ __global__ void __launch_bounds__(1024) iset_order(int ni, const double *__restr
                 const unsigned c = q <= 0.f ? 0u : (q >= 1023.f ? 1023u : (unsigned)q);
                 key |= spread10(c) << k;
             }
-            v = ((unsigned long long)key << 32) | (unsigned)s;
+            v[r] = ((unsigned long long)key << 32) | (unsigned)s;
         }
-        kv[s] = v;
     }
-    __syncthreads();
+    int P = 32;
+    while (P < ni) P <<= 1;
     for (int kk = 2; kk <= P; kk <<= 1)
         for (int jj = kk >> 1; jj > 0; jj >>= 1) {
-            for (int x = threadIdx.x; x < P; x += blockDim.x) {
-                const int y = x ^ jj;
-                if (y > x) {
-                    const unsigned long long p0 = kv[x], p1 = kv[y];
-                    if ((p0 > p1) == ((x & kk) == 0)) {
-                        kv[x] = p1;
-                        kv[y] = p0;
+            if (jj >= STAGE_NT) {
+#pragma unroll
+                for (int r = 0; r < E; ++r)
+#pragma unroll
+                    for (int q = r + 1; q < E; ++q) {
+                        if ((r ^ q) * STAGE_NT != jj) continue;
+                        const bool up = ((r * STAGE_NT) & kk) == 0;
+                        if ((v[r] > v[q]) == up) {
+                            const unsigned long long t = v[r];
+                            v[r] = v[q];
+                            v[q] = t;
+                        }
                     }
-                }
+                continue;
             }
-            __syncthreads();
+            unsigned long long o[E];
+            if (jj < 32) {
+#pragma unroll
+                for (int r = 0; r < E; ++r) o[r] = __shfl_xor_sync(0xffffffffu, v[r], jj);
+            } else {
+#pragma unroll
+                for (int r = 0; r < E; ++r) kv[r * STAGE_NT + tid] = v[r];
+                __syncthreads();
+#pragma unroll
+                for (int r = 0; r < E; ++r) o[r] = kv[r * STAGE_NT + (tid ^ jj)];
+                __syncthreads();
+            }
+#pragma unroll
+            for (int r = 0; r < E; ++r) {
+                const bool up = ((r * STAGE_NT + tid) & kk) == 0;
+                v[r] = up == ((tid & jj) == 0) ? min(v[r], o[r]) : max(v[r], o[r]);
+            }
         }
-    for (int s = threadIdx.x; s < ni; s += blockDim.x) iperm[s] = (int)(kv[s] & 0xffffffffu);
+#pragma unroll
+    for (int r = 0; r < E; ++r) {
+        const int s = r * STAGE_NT + tid;
+        if (s < ni) iperm[s] = (int)(v[r] & 0xffffffffu);
+    }
+}
+
+// First launch of a call: CTA 0 orders the active set when `order` is set,
+// and the CTAs after it copy a host call's i data [h2 | dtr | x | v] from
+// pinned memory (src) to the device, where the kernels read it.  CTA 0 takes
+// its positions from src too, so the two run side by side: in place of an
+// upload, an ordering launch that waited for it and the call's own upload
+// (18 us per call of 1,024 bodies, now 6).
+__global__ void __launch_bounds__(STAGE_NT)
+    regf_stage(int ni, int order, const double *__restrict__ src, double *__restrict__ dst,
+               const double *__restrict__ ix, const unsigned *__restrict__ ext, int *__restrict__ iperm) {
+    __shared__ unsigned long long kv[ISORT_MAX];
+    if ((int)blockIdx.x < order) {
+        const double *x = src ? src + 2 * (size_t)ni : ix;
+        if (ni <= STAGE_NT) order_active<1>(ni, x, ext, iperm, kv);
+        else if (ni <= 2 * STAGE_NT) order_active<2>(ni, x, ext, iperm, kv);
+        else order_active<4>(ni, x, ext, iperm, kv);
+        return;
+    }
+    const double2 *s = reinterpret_cast<const double2 *>(src);
+    double2 *d = reinterpret_cast<double2 *>(dst);
+    const size_t n = 4 * (size_t)ni, step = (size_t)(gridDim.x - order) * STAGE_NT;
+    for (size_t k = (size_t)(blockIdx.x - order) * STAGE_NT + threadIdx.x; k < n; k += step) d[k] = s[k];
 }
 
 }  // namespace
@@ -1896,9 +1949,12 @@ struct RegLaunch {
     size_t smem = 0;
     bool mf = false;
     MlpArgs mlp{};
-    // host staging (graph node of kind 1)
+    // host staging of the i data (host calls) and the ordering of the active
+    // set: regf_stage
     const double *hin = nullptr;
     size_t in_bytes = 0;
+    int order = 0;
+    const double *ix = nullptr;
     // where regf_finalize writes: the device buffers, or (host calls under
     // unified addressing) the pinned host staging itself, so only the used
     // part of each list row crosses the bus and no copy-back is needed
@@ -1954,6 +2010,33 @@ static bool nbcnt_reserve(int ni, cudaStream_t st) {
     if (R.nbcnt.ptr == before && R.nbcnt.cap == cap_before) return false;
     NB6_CUDA_CHECK(cudaMemsetAsync(R.nbcnt.ptr, 0, sizeof(int) * R.nbcnt.cap, st));
     return true;
+}
+
+// Arguments of regf_stage, addressable for a kernel node.
+struct StageArgs {
+    int ni, order;
+    const double *src;
+    double *dst;
+    const double *ix;
+    const unsigned *ext;
+    int *iperm, grid;
+    void *p[7];
+    explicit StageArgs(const RegLaunch &L)
+        : ni(L.ni), order(L.order), src(L.direct ? L.hin : nullptr), dst(R.iin.ptr), ix(L.ix), ext(R.ext.ptr),
+          iperm(R.iperm.ptr), grid(order + (src ? (int)std::min<size_t>((4 * (size_t)ni + STAGE_NT - 1) / STAGE_NT, 64) : 0)) {
+        void *q[7] = {&ni, &order, &src, &dst, &ix, &ext, &iperm};
+        memcpy(p, q, sizeof(q));
+    }
+};
+
+// i data and order of a call as plain launches (without unified addressing
+// the host's data come by an upload).
+static void regf_stage_launch(const RegLaunch &L, cudaStream_t st) {
+    if (L.hin && !L.direct)
+        NB6_CUDA_CHECK(cudaMemcpyAsync(R.iin.ptr, L.hin, L.in_bytes, cudaMemcpyHostToDevice, st));
+    StageArgs g(L);
+    if (g.grid == 0) return;
+    NB6_CUDA_CHECK(cudaLaunchKernel((const void *)regf_stage, dim3(g.grid), dim3(STAGE_NT), g.p, 0, st));
 }
 
 static void regf_prepare(int ni, const double *d_h2, const double *d_dtr, const double *d_x,
@@ -2033,14 +2116,12 @@ static void regf_prepare(int ni, const double *d_h2, const double *d_dtr, const 
     }();
     if (i_order && a.tbox && ni > NT && ni <= ISORT_MAX) {
         R.iperm.reserve(ni);
-        // the order reads this call's i positions: a host call's staging
-        // must be on the device first (the submission copies it again)
-        if (L.hin)
-            NB6_CUDA_CHECK(cudaMemcpyAsync(R.iin.ptr, L.hin, L.in_bytes, cudaMemcpyHostToDevice, st));
-        iset_order<<<1, 1024, 0, st>>>(ni, d_x, R.ext.ptr, R.iperm.ptr);
-        NB6_CUDA_CHECK(cudaGetLastError());
         a.iperm = R.iperm.ptr;
+        L.order = 1;
     }
+    L.ix = d_x;
+    L.ni = ni;
+    L.direct = L.hin != nullptr && nb6_uva();
     a.npad = R.npad;
     a.jm = R.jm.ptr;
     a.jx = R.jx.ptr;
@@ -2069,9 +2150,7 @@ static void regf_prepare(int ni, const double *d_h2, const double *d_dtr, const 
         NB6_CUDA_CHECK(cudaEventCreate(&R.tev1));
     }
     if (tune_now) {
-        // the trials read the i data: stage it first when the call brings it
-        if (L.hin)
-            NB6_CUDA_CHECK(cudaMemcpyAsync(R.iin.ptr, L.hin, L.in_bytes, cudaMemcpyHostToDevice, st));
+        regf_stage_launch(L, st);   // the trials read the i data and its order
         // time each candidate three times and keep its best (after one
         // warm-up launch whose time is not compared); when the warm-up took
         // 2 ms or more, once: the noise of so long a launch is well inside
@@ -2136,6 +2215,7 @@ static void regf_prepare(int ni, const double *d_h2, const double *d_dtr, const 
         a.tbox = nullptr;
         a.iperm = nullptr;
         a.comprel = nullptr;
+        L.order = 0;
     }
     R.last_geometry[0] = plan.variant;
     R.last_geometry[1] = plan.igrid;
@@ -2148,7 +2228,6 @@ static void regf_prepare(int ni, const double *d_h2, const double *d_dtr, const 
         NB6_CUDA_CHECK(cudaFuncSetAttribute(regf_finalize, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                             (int)smem));
     L.mlp = mlp;
-    L.direct = L.hin != nullptr && nb6_uva();
     L.ls = L.direct ? host_row_stride(W) : W;
     L.hstatus = L.direct ? nb6_status_post() : nullptr;
     if (L.hin) {
@@ -2159,7 +2238,6 @@ static void regf_prepare(int ni, const double *d_h2, const double *d_dtr, const 
     L.outl = L.direct ? R.houtl.ptr : R.outl.ptr;
     L.plan = plan;
     L.a = a;
-    L.ni = ni;
     L.W = W;
     L.cap = cap;
     L.pmax = pmax;
@@ -2177,8 +2255,7 @@ static void regf_copy_out(const RegLaunch &L, cudaStream_t st) {
 }
 
 static void regf_eager(const RegLaunch &L, cudaStream_t st) {
-    if (L.hin)
-        NB6_CUDA_CHECK(cudaMemcpyAsync(R.iin.ptr, L.hin, L.in_bytes, cudaMemcpyHostToDevice, st));
+    regf_stage_launch(L, st);
     NB6_CUDA_CHECK(cudaMemsetAsync(R.nbcnt.ptr, 0, sizeof(int) * (R.nbcnt_dirty ? R.nbcnt.cap : (size_t)L.ni), st));
     // kernel-only timing of the main force kernel (read by
     // nb6_regf_last_kernel_ms_ after the stream has drained)
@@ -2220,6 +2297,16 @@ static cudaKernelNodeParams fin_node(const RegLaunch &L, FinArgs &f) {
         if ((call) != cudaSuccess) return false; \
     } while (0)
 
+static cudaKernelNodeParams stage_node(StageArgs &g) {
+    cudaKernelNodeParams k{};
+    k.func = (void *)regf_stage;
+    k.gridDim = dim3(g.grid);
+    k.blockDim = dim3(STAGE_NT);
+    k.sharedMemBytes = 0;
+    k.kernelParams = g.p;
+    return k;
+}
+
 static bool graph_build(RegState::Graph &G, const RegLaunch &L) {
     const bool io = L.hin != nullptr;
     NB6_GRAPH_TRY(cudaGraphCreate(&G.g, 0));
@@ -2227,9 +2314,10 @@ static bool graph_build(RegState::Graph &G, const RegLaunch &L) {
     auto deps = [&]() { return prev ? &prev : (cudaGraphNode_t *)nullptr; };
     auto ndeps = [&]() { return (size_t)(prev ? 1 : 0); };
     if (io) {
-        NB6_GRAPH_TRY(cudaGraphAddMemcpyNode1D(&G.h2d, G.g, deps(), ndeps(), R.iin.ptr, L.hin, L.in_bytes,
-                                               cudaMemcpyHostToDevice));
-        prev = G.h2d;
+        StageArgs g(L);
+        const cudaKernelNodeParams ks = stage_node(g);
+        NB6_GRAPH_TRY(cudaGraphAddKernelNode(&G.kstage, G.g, deps(), ndeps(), &ks));
+        prev = G.kstage;
     }
     NB6_GRAPH_TRY(cudaGraphAddEventRecordNode(&n, G.g, deps(), ndeps(), R.ev0));
     prev = n;
@@ -2243,14 +2331,6 @@ static bool graph_build(RegState::Graph &G, const RegLaunch &L) {
     FinArgs f(L);
     const cudaKernelNodeParams kf = fin_node(L, f);
     NB6_GRAPH_TRY(cudaGraphAddKernelNode(&G.kfin, G.g, deps(), ndeps(), &kf));
-    prev = G.kfin;
-    if (io && !L.direct) {
-        NB6_GRAPH_TRY(cudaGraphAddMemcpyNode1D(&G.d2hf, G.g, deps(), ndeps(), R.houtf.ptr, R.outf.ptr,
-                                               sizeof(double) * 8 * L.ni, cudaMemcpyDeviceToHost));
-        prev = G.d2hf;
-        NB6_GRAPH_TRY(cudaGraphAddMemcpyNode1D(&G.d2hl, G.g, deps(), ndeps(), R.houtl.ptr, R.outl.ptr,
-                                               sizeof(int) * (size_t)L.W * L.ni, cudaMemcpyDeviceToHost));
-    }
     NB6_GRAPH_TRY(cudaGraphInstantiate(&G.x, G.g, 0));
     R.graph_builds++;
     return true;
@@ -2258,9 +2338,11 @@ static bool graph_build(RegState::Graph &G, const RegLaunch &L) {
 
 static bool graph_update(RegState::Graph &G, const RegLaunch &L) {
     const bool io = L.hin != nullptr;
-    if (io)
-        NB6_GRAPH_TRY(cudaGraphExecMemcpyNodeSetParams1D(G.x, G.h2d, R.iin.ptr, L.hin, L.in_bytes,
-                                                         cudaMemcpyHostToDevice));
+    if (io) {
+        StageArgs g(L);
+        const cudaKernelNodeParams ks = stage_node(g);
+        NB6_GRAPH_TRY(cudaGraphExecKernelNodeSetParams(G.x, G.kstage, &ks));
+    }
     RegArgs a = L.a;
     void *margs[1] = {&a};
     const cudaKernelNodeParams km = main_node(L, margs);
@@ -2268,13 +2350,6 @@ static bool graph_update(RegState::Graph &G, const RegLaunch &L) {
     FinArgs f(L);
     const cudaKernelNodeParams kf = fin_node(L, f);
     NB6_GRAPH_TRY(cudaGraphExecKernelNodeSetParams(G.x, G.kfin, &kf));
-    if (io && !L.direct) {
-        NB6_GRAPH_TRY(cudaGraphExecMemcpyNodeSetParams1D(G.x, G.d2hf, R.houtf.ptr, R.outf.ptr,
-                                                         sizeof(double) * 8 * L.ni, cudaMemcpyDeviceToHost));
-        NB6_GRAPH_TRY(cudaGraphExecMemcpyNodeSetParams1D(G.x, G.d2hl, R.houtl.ptr, R.outl.ptr,
-                                                         sizeof(int) * (size_t)L.W * L.ni,
-                                                         cudaMemcpyDeviceToHost));
-    }
     return true;
 }
 #undef NB6_GRAPH_TRY
@@ -2296,10 +2371,12 @@ static void regf_submit(const RegLaunch &L, cudaStream_t st) {
         const char *e = getenv("NB6_GRAPHS");
         R.use_graphs = (e && atoi(e) == 0) ? 0 : 1;
     }
-    if (!R.use_graphs) {
+    // (a host call without unified addressing: launches and copies)
+    if (!R.use_graphs || (L.hin && !L.direct)) {
         regf_eager(L, st);
         return;
     }
+    if (!L.hin) regf_stage_launch(L, st);
     RegState::Graph &G = R.graph[L.hin ? 1 : 0];
     bool ok = G.x ? graph_update(G, L) : graph_build(G, L);
     if (ok) {
