@@ -265,6 +265,19 @@ void nb6_lib_closed();             // their closes: the pool stops with the last
 int nb6_check_dev_status();        // read (and clear) after a stream sync
 void nb6_status_fetch(cudaStream_t st);  // enqueue the status copy before that sync
 int *nb6_status_post();            // or: the pinned word for the call's last kernel to write
+// A piece of host memory at byte `off` of a block on its way to the device.
+struct Nb6Seg {
+    size_t off;
+    const void *src;
+    size_t len;
+};
+// The pieces of a block of `bytes` copied into pinned memory that kernels
+// read in place, valid until the stream is next synchronised; null when the
+// block is too large for that (nb6_upload then).
+const void *nb6_stage(const Nb6Seg *seg, int nseg, size_t bytes);
+// The pieces copied to device memory at dst; the caller's arrays may change on
+// return.
+void nb6_upload(void *dst, const Nb6Seg *seg, int nseg, size_t bytes, cudaStream_t st);
 bool nb6_uva();                    // device reads/writes pinned host memory in place
 int nb6_num_sms();
 

@@ -275,11 +275,12 @@ __global__ void pot_finalize(const float2 *__restrict__ part, int nslices, int i
 // caller's order (ROWS_HL) or, with perm, in Morton order, with the tile's
 // box (of the hi positions of its real bodies: centre rounded to nearest,
 // half extents rounded up) and the tile-relative rows.  Padding slots are
-// massless and far away.
+// massless and far away.  keep not null: m and x are in pinned host memory,
+// and a copy of x is kept on the device.
 template <bool ORD>
 __global__ void __launch_bounds__(JT) pot_tiles(int n, const int *__restrict__ perm, const double *__restrict__ m,
-                                                const double *__restrict__ x, float *__restrict__ tiles,
-                                                float4 *__restrict__ tbox, int *status) {
+                                                const double *__restrict__ x, double *__restrict__ keep,
+                                                float *__restrict__ tiles, float4 *__restrict__ tbox, int *status) {
     constexpr int ROWS = ORD ? ROWS_ORD : ROWS_HL;
     const int t = threadIdx.x, s = blockIdx.x * JT + t;
     double c[3] = {1.0e15, 1.0e15, 1.0e15}, mj = 0.0;
@@ -288,6 +289,9 @@ __global__ void __launch_bounds__(JT) pot_tiles(int n, const int *__restrict__ p
 #pragma unroll
         for (int k = 0; k < 3; ++k) c[k] = x[3 * j + k];
         mj = m[j];
+        if (keep)
+#pragma unroll
+            for (int k = 0; k < 3; ++k) keep[3 * j + k] = c[k];
         if (c[0] != c[0] || c[1] != c[1] || c[2] != c[2] || mj != mj) set_status(status, NB6_ERR_NAN_INPUT);
     }
     float *o = tiles + (size_t)blockIdx.x * (ROWS * JT) + t;
@@ -368,7 +372,7 @@ __global__ void __launch_bounds__(SEL_NT) pot_select(int n, const int *__restric
 }
 
 struct PotState {
-    DevBuf<double> m, x, out;
+    DevBuf<double> mx, out;                     // the bodies of a host call: m, x
     DevBuf<float> tiles;
     DevBuf<float4> tbox;
     DevBuf<float2> part;
@@ -376,7 +380,8 @@ struct PotState {
     HostBuf<double> hout;
     SpatialOrder order;
     int n = 0, ntile = 0;
-    const double *dm = nullptr, *dx = nullptr;  // the uploaded m, x of the call
+    const double *dm = nullptr, *dx = nullptr;  // the m, x of the call, readable by kernels
+    double *keep = nullptr;                     // where to keep x when dx is pinned host memory
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     float last_ms = 0.f;
 };
@@ -421,7 +426,7 @@ template <int NI, bool ORD> void pot_launch(PotArgs &a, cudaStream_t st) {
 bool pot_compute(int i0, int ni, double *hout, cudaStream_t st) {
     const int n = P.n;
     PotArgs a{};
-    a.x = P.dx;
+    a.x = P.keep ? P.keep : P.dx;
     a.ntile = P.ntile;
     a.i0 = i0;
     a.ni = ni;
@@ -432,7 +437,8 @@ bool pot_compute(int i0, int ni, double *hout, cudaStream_t st) {
     if (ord) {
         P.order.build(n, P.dx, st);
         P.tbox.reserve(2 * (size_t)P.ntile);
-        pot_tiles<true><<<P.ntile, JT, 0, st>>>(n, P.order.perm.ptr, P.dm, P.dx, P.tiles.ptr, P.tbox.ptr, a.status);
+        pot_tiles<true><<<P.ntile, JT, 0, st>>>(n, P.order.perm.ptr, P.dm, P.dx, nullptr, P.tiles.ptr, P.tbox.ptr,
+                                                a.status);
         NB6_CUDA_CHECK(cudaGetLastError());
         a.tbox = P.tbox.ptr;
         a.idx = P.order.perm.ptr;
@@ -446,7 +452,7 @@ bool pot_compute(int i0, int ni, double *hout, cudaStream_t st) {
             a.idx = P.idx.ptr;
         }
     } else {
-        pot_tiles<false><<<P.ntile, JT, 0, st>>>(n, nullptr, P.dm, P.dx, P.tiles.ptr, nullptr, a.status);
+        pot_tiles<false><<<P.ntile, JT, 0, st>>>(n, nullptr, P.dm, P.dx, P.keep, P.tiles.ptr, nullptr, a.status);
         NB6_CUDA_CHECK(cudaGetLastError());
     }
     // two i per thread once that still leaves a tile of i for every SM
@@ -463,20 +469,26 @@ bool pot_compute(int i0, int ni, double *hout, cudaStream_t st) {
     return direct;
 }
 
-// The bodies of a call on the device (copied from the host when they are
-// there).
+// The bodies of a call where kernels read them: on the device, or (a small
+// host call, which never orders its set) in the pinned staging.
 void pot_upload(int n, const double *m, const double *x, cudaStream_t st, bool from_host) {
     P.n = n;
     P.ntile = std::max(1, (n + JT - 1) / JT);
     P.dm = m;
     P.dx = x;
+    P.keep = nullptr;
     if (from_host) {
-        P.m.reserve(n);
-        P.x.reserve(3 * (size_t)n);
-        NB6_CUDA_CHECK(cudaMemcpyAsync(P.m.ptr, m, sizeof(double) * n, cudaMemcpyHostToDevice, st));
-        NB6_CUDA_CHECK(cudaMemcpyAsync(P.x.ptr, x, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, st));
-        P.dm = P.m.ptr;
-        P.dx = P.x.ptr;
+        const size_t np = (size_t)P.ntile * JT, bytes = 4 * np * sizeof(double);
+        const Nb6Seg seg[2] = {{0, m, sizeof(double) * n}, {sizeof(double) * np, x, 3 * sizeof(double) * n}};
+        P.mx.reserve(4 * np);
+        P.dm = static_cast<const double *>(nb6_stage(seg, 2, bytes));
+        if (P.dm) {
+            P.keep = P.mx.ptr + np;
+        } else {
+            nb6_upload(P.mx.ptr, seg, 2, bytes, st);
+            P.dm = P.mx.ptr;
+        }
+        P.dx = P.dm + np;
     }
 }
 

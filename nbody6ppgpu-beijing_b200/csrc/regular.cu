@@ -1166,8 +1166,8 @@ NB6_DEV void add_partial(const float4 *p, double *v) {
 // R registers per lane (id r * 32 + lane in register r), exchanges below 32
 // through shuffles and the others within a lane, then written with the count
 // in front as whole 32-entry lines.  The network in shared memory that longer
-// rows take costs 12 instructions and a warp barrier per exchange: 531 rows of
-// up to 400 ids spent 40 us of a 180 us call in it.
+// rows take costs 12 instructions and a warp barrier per exchange (a block with
+// 531 rows of up to 400 ids 184 us, now 150).
 constexpr int ROW_REGS = 16;
 template <int R>
 NB6_DEV void write_sorted_row(int *__restrict__ row, const int *__restrict__ src, int n, int lane) {
@@ -1367,8 +1367,11 @@ __global__ void __launch_bounds__(FIN_WARPS * 32)
 }
 
 // FP64 (m, x, v) -> SoA float4 tiles; padding slots are massless and far.
+// km not null: m, x, v are in pinned host memory, and their FP64 copies are
+// kept in km, kx, kv.
 __global__ void regf_pack_j(int nj, JSetOut o, const double *__restrict__ m,
-                            const double *__restrict__ x, const double *__restrict__ v, int *status) {
+                            const double *__restrict__ x, const double *__restrict__ v, double *__restrict__ km,
+                            double *__restrict__ kx, double *__restrict__ kv, int *status) {
     for (size_t j = blockIdx.x * (size_t)blockDim.x + threadIdx.x; j < o.npad;
          j += (size_t)gridDim.x * blockDim.x) {
         if (j < (size_t)nj) {
@@ -1378,6 +1381,15 @@ __global__ void regf_pack_j(int nj, JSetOut o, const double *__restrict__ m,
             if (x0 != x0 || x1 != x1 || x2 != x2 || v0 != v0 || v1 != v1 || v2 != v2 ||
                 mj != mj)
                 set_status(status, NB6_ERR_NAN_INPUT);
+            if (km) {
+                km[j] = mj;
+                kx[3 * j] = x0;
+                kx[3 * j + 1] = x1;
+                kx[3 * j + 2] = x2;
+                kv[3 * j] = v0;
+                kv[3 * j + 1] = v1;
+                kv[3 * j + 2] = v2;
+            }
             write_j(o, j, true, x0, x1, x2, mj, v0, v1, v2);
         } else {
             write_j(o, j, false, 0, 0, 0, 0, 0, 0, 0);
@@ -1409,7 +1421,8 @@ struct RegState {
     DevBuf<float> comp;              // NB6_NCOMP x npad, component-major
     DevBuf<double> compd;            // 3 x npad FP64 positions, component-major
     size_t npad = 0;
-    DevBuf<double> jm, jx, jv;
+    DevBuf<double> jall;             // the bodies in FP64: m, x, v back to back, npad apart
+    double *jm = nullptr, *jx = nullptr, *jv = nullptr;
     DevBuf<double> iin;
     DevBuf<float4> part;
     DevBuf<int> nbcnt, nbbuf;
@@ -1616,12 +1629,6 @@ int ilog2(int v) {
     int r = 0;
     while ((1 << (r + 1)) <= v) ++r;
     return r;
-}
-
-bool any_nan(const double *p, size_t n) {
-    for (size_t k = 0; k < n; ++k)
-        if (p[k] != p[k]) return true;
-    return false;
 }
 
 // ----------------------------------------------------------------------------
@@ -1833,7 +1840,7 @@ NB6_DEV void order_active(int ni, const double *__restrict__ ix, const unsigned 
 // pinned memory (src) to the device, where the kernels read it.  CTA 0 takes
 // its positions from src too, so the two run side by side: in place of an
 // upload, an ordering launch that waited for it and the call's own upload
-// (18 us per call of 1,024 bodies, now 6).
+// (65,536 bodies in 64 calls 13.65 -> 12.7 ms).
 __global__ void __launch_bounds__(STAGE_NT)
     regf_stage(int ni, int order, const double *__restrict__ src, double *__restrict__ dst,
                const double *__restrict__ ix, const unsigned *__restrict__ ext, int *__restrict__ iperm) {
@@ -1865,9 +1872,10 @@ static JSetOut size_j_buffers(int n) {
     R.vel.reserve(R.npad);
     R.comp.reserve((size_t)NB6_NCOMP * R.npad);
     R.compd.reserve((size_t)3 * R.npad);
-    R.jm.reserve(R.npad);
-    R.jx.reserve(3 * R.npad);
-    R.jv.reserve(3 * R.npad);
+    R.jall.reserve(7 * R.npad);
+    R.jm = R.jall.ptr;
+    R.jx = R.jm + R.npad;
+    R.jv = R.jx + 3 * R.npad;
     JSetOut o;
     o.posH = R.posH.ptr;
     o.posL = R.posL.ptr;
@@ -1909,8 +1917,8 @@ static bool ensure_sorted(cudaStream_t st) {
     const unsigned init[6] = {0xffffffffu, 0xffffffffu, 0xffffffffu, 0u, 0u, 0u};
     NB6_CUDA_CHECK(cudaMemcpyAsync(R.ext.ptr, init, sizeof(init), cudaMemcpyHostToDevice, st));
     const int blocks = std::max(1, std::min((nj + 255) / 256, nb6_num_sms() * 8));
-    jset_extent<<<blocks, 256, 0, st>>>(nj, R.jx.ptr, R.ext.ptr);
-    jset_keys<<<blocks, 256, 0, st>>>(nj, R.jx.ptr, R.ext.ptr, R.keys_in.ptr, R.vals_in.ptr);
+    jset_extent<<<blocks, 256, 0, st>>>(nj, R.jx, R.ext.ptr);
+    jset_keys<<<blocks, 256, 0, st>>>(nj, R.jx, R.ext.ptr, R.keys_in.ptr, R.vals_in.ptr);
     NB6_CUDA_CHECK(cudaGetLastError());
     size_t tmp = 0;
     NB6_CUDA_CHECK(cub::DeviceRadixSort::SortPairs(nullptr, tmp, R.keys_in.ptr, R.keys_out.ptr, R.vals_in.ptr,
@@ -2039,6 +2047,21 @@ static void regf_stage_launch(const RegLaunch &L, cudaStream_t st) {
     NB6_CUDA_CHECK(cudaLaunchKernel((const void *)regf_stage, dim3(g.grid), dim3(STAGE_NT), g.p, 0, st));
 }
 
+// The j set in its sent order, for the j-parallel kernel: the same variant
+// then always sums in the same order, whether or not other calls made the
+// spatial order, and one CTA's j's do not hold a whole neighbourhood.
+static void unordered(RegArgs &a) {
+    a.posH = R.posH.ptr;
+    a.posL = R.posL.ptr;
+    a.vel = R.vel.ptr;
+    a.comp = R.comp.ptr;
+    a.compd = R.compd.ptr;
+    a.perm = nullptr;
+    a.tbox = nullptr;
+    a.iperm = nullptr;
+    a.comprel = nullptr;
+}
+
 static void regf_prepare(int ni, const double *d_h2, const double *d_dtr, const double *d_x,
                          const double *d_v, int lmax, int nnbmax, int mflag, cudaStream_t st,
                          RegLaunch &L) {
@@ -2123,9 +2146,9 @@ static void regf_prepare(int ni, const double *d_h2, const double *d_dtr, const 
     L.ni = ni;
     L.direct = L.hin != nullptr && nb6_uva();
     a.npad = R.npad;
-    a.jm = R.jm.ptr;
-    a.jx = R.jx.ptr;
-    a.jv = R.jv.ptr;
+    a.jm = R.jm;
+    a.jx = R.jx;
+    a.jv = R.jv;
     a.nj = R.nj;
     a.ntile = R.ntile;
     a.nslices = plan.nslices;
@@ -2202,19 +2225,8 @@ static void regf_prepare(int ni, const double *d_h2, const double *d_dtr, const 
             fprintf(stderr, "# nb6 autotune: ni~2^%d nj~2^%d mflag %d -> variant %d (%.3f ms)\n",
                     key.li, key.lj, key.mf, bestv, best);
     }
-    if (plan.variant < 0 && a.perm) {
-        // the j-parallel kernel takes the j set in its sent order, whether
-        // or not this call's trials needed the spatial order: the same
-        // variant always sums in the same order
-        a.posH = R.posH.ptr;
-        a.posL = R.posL.ptr;
-        a.vel = R.vel.ptr;
-        a.comp = R.comp.ptr;
-        a.compd = R.compd.ptr;
-        a.perm = nullptr;
-        a.tbox = nullptr;
-        a.iperm = nullptr;
-        a.comprel = nullptr;
+    if (plan.variant < 0) {
+        unordered(a);
         L.order = 0;
     }
     R.last_geometry[0] = plan.variant;
@@ -2454,9 +2466,8 @@ void gpunb_close_() {
     R.vel.release();
     R.comp.release();
     R.compd.release();
-    R.jm.release();
-    R.jx.release();
-    R.jv.release();
+    R.jall.release();
+    R.jm = R.jx = R.jv = nullptr;
     R.iin.release();
     R.part.release();
     R.nbcnt.release();
@@ -2495,13 +2506,21 @@ void gpunb_send_(int *nj, double *mj, double (*xj)[3], double (*vj)[3]) {
     }
     cudaStream_t st = nb6_stream();
     const JSetOut o = size_j_buffers(n);
-    if (n > 0) {
-        NB6_CUDA_CHECK(cudaMemcpyAsync(R.jm.ptr, mj, sizeof(double) * n, cudaMemcpyHostToDevice, st));
-        NB6_CUDA_CHECK(cudaMemcpyAsync(R.jx.ptr, xj, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, st));
-        NB6_CUDA_CHECK(cudaMemcpyAsync(R.jv.ptr, vj, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, st));
+    // A small set is read by the pack kernel from the pinned staging itself,
+    // a larger one uploaded through it.
+    const size_t np = o.npad, bytes = 7 * np * sizeof(double);
+    const Nb6Seg seg[3] = {{0, mj, sizeof(double) * n},
+                           {sizeof(double) * np, xj, 3 * sizeof(double) * n},
+                           {4 * sizeof(double) * np, vj, 3 * sizeof(double) * n}};
+    const double *src = static_cast<const double *>(nb6_stage(seg, 3, bytes));
+    const bool staged = src != nullptr;
+    if (!staged) {
+        nb6_upload(R.jall.ptr, seg, 3, bytes, st);
+        src = R.jall.ptr;
     }
     const int blocks = (int)std::min<size_t>((o.npad + 255) / 256, (size_t)nb6_num_sms() * 8);
-    regf_pack_j<<<blocks, 256, 0, st>>>(n, o, R.jm.ptr, R.jx.ptr, R.jv.ptr, nb6_dev_status());
+    regf_pack_j<<<blocks, 256, 0, st>>>(n, o, src, src + np, src + 4 * np, staged ? R.jm : nullptr, R.jx, R.jv,
+                                        nb6_dev_status());
     NB6_CUDA_CHECK(cudaGetLastError());
     R.time_send += nb6_wtime();
 }
@@ -2525,9 +2544,9 @@ bool regular_bind_j(int n, double **jm, double **jx, double **jv, JSetOut *out) 
     }
     R.isend++;
     *out = size_j_buffers(n);
-    *jm = R.jm.ptr;
-    *jx = R.jx.ptr;
-    *jv = R.jv.ptr;
+    *jm = R.jm;
+    *jx = R.jx;
+    *jv = R.jv;
     return true;
 }
 
@@ -2793,29 +2812,23 @@ void nb6_regf_seg_(int *ni_, int *iseg, double *h2, double *dtr, double (*xi)[3]
         nb6_fatal(NB6_ERR_BAD_ARG);
         return;
     }
-    if (any_nan(h2, ni) || any_nan(dtr, ni) || any_nan(&xi[0][0], 3 * (size_t)ni) ||
-        any_nan(&vi[0][0], 3 * (size_t)ni)) {
+    const double t_start = nb6_wtime();
+    // i data: [h2 | dtr | x | v], as in gpunb_regf_
+    const size_t nin = (size_t)8 * ni;
+    R.hin.reserve(nin);
+    R.iin.reserve(nin);
+    double *h = R.hin.ptr;
+    if (stage_inputs(ni, h, h2, dtr, &xi[0][0], &vi[0][0])) {
         fprintf(stderr, "nb6_regf_seg: NaN in i-particle input\n");
         nb6_fatal(NB6_ERR_NAN_INPUT);
         return;
     }
-    const double t_start = nb6_wtime();
     R.ini += ni;
     R.icall++;
     cudaStream_t st = nb6_stream();
     const int cap = std::max(0, std::min(nnbmax, lmax - 1));
     const int W = cap + 1;
     const bool mf = *m_flag != 0;
-
-    // i data: [h2 | dtr | x | v], as in gpunb_regf_
-    const size_t nin = (size_t)8 * ni;
-    R.hin.reserve(nin);
-    R.iin.reserve(nin);
-    double *h = R.hin.ptr;
-    memcpy(h, h2, sizeof(double) * ni);
-    memcpy(h + ni, dtr, sizeof(double) * ni);
-    memcpy(h + 2 * (size_t)ni, xi, sizeof(double) * 3 * ni);
-    memcpy(h + 5 * (size_t)ni, vi, sizeof(double) * 3 * ni);
 
     // One segment spanning a large j set (one big cluster): the tuned tile
     // kernels of gpunb_regf_ (packed pair math, spatial order, far tiles)
@@ -2945,9 +2958,9 @@ void nb6_regf_seg_(int *ni_, int *iseg, double *h2, double *dtr, double (*xi)[3]
     a.comp = R.comp.ptr;
     a.compd = R.compd.ptr;
     a.npad = R.npad;
-    a.jm = R.jm.ptr;
-    a.jx = R.jx.ptr;
-    a.jv = R.jv.ptr;
+    a.jm = R.jm;
+    a.jx = R.jx;
+    a.jv = R.jv;
     a.nj = R.nj;
     a.ntile = R.ntile;
     a.nslices = 1;
@@ -3032,9 +3045,9 @@ bool regular_seg_on_device(int ni, int *iseg, double *h2, double *dtr, double (*
     out->outf = R.outf.ptr;
     out->outl = R.outl.ptr;
     out->W = std::max(0, std::min(nnbmax, lmax - 1)) + 1;
-    out->jm = R.jm.ptr;
-    out->jx = R.jx.ptr;
-    out->jv = R.jv.ptr;
+    out->jm = R.jm;
+    out->jx = R.jx;
+    out->jv = R.jv;
     return nb6_last_status_() == 0;
 }
 

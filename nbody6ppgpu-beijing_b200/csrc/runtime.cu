@@ -106,6 +106,72 @@ int *nb6_dev_status() { return g_dev_status; }
 
 bool nb6_uva() { return g_uva; }
 
+// ----------------------------------------------------------------------------
+// Host arrays on their way to the device.  The callers' arrays are pageable;
+// a copy from pageable memory goes through the driver's staging on one thread
+// (16 GB/s) with some 10 us per call.  Blocks of up to STAGE_MAX bytes are
+// copied into one pinned block that a kernel reads over the bus in place (no
+// copy to launch); larger ones pass through a ring of pinned chunks, filled
+// by the copy threads while the chunks before are uploaded.  Measured on the
+// host: gpunb_send_ of 1,024 bodies 36 -> 7 us, of 16,384 47 -> 33 us, of
+// 996,147 (56 MB) 3,950 -> 1,560 us.
+// ----------------------------------------------------------------------------
+static constexpr size_t STAGE_MAX = 512u << 10, POOL_MIN = 256u << 10;
+static constexpr size_t CHUNK_MIN = 512u << 10, CHUNK_MAX = 4u << 20;
+static constexpr int RING = 3;
+static HostBuf<unsigned char> g_stage, g_ring[RING];
+static cudaEvent_t g_ring_ev[RING] = {};
+static int g_ring_next = 0;
+static bool g_stage_busy = false;   // a kernel may still read g_stage
+
+// Bytes [lo, hi) of the block into `to` (the place of byte lo).
+static void copy_range(unsigned char *to, const Nb6Seg *seg, int nseg, size_t lo, size_t hi) {
+    for (int k = 0; k < nseg; ++k) {
+        const size_t a = lo > seg[k].off ? lo : seg[k].off;
+        const size_t end = seg[k].off + seg[k].len, b = hi < end ? hi : end;
+        if (a < b) memcpy(to + (a - lo), static_cast<const unsigned char *>(seg[k].src) + (a - seg[k].off), b - a);
+    }
+}
+
+static void copy_range_pool(unsigned char *to, const Nb6Seg *seg, int nseg, size_t lo, size_t hi) {
+    if (hi - lo < POOL_MIN) {
+        copy_range(to, seg, nseg, lo, hi);
+        return;
+    }
+    CopyPool &pool = nb6_copy_pool();
+    const size_t np = (size_t)pool.parts(), len = hi - lo;
+    pool.run([&](int p) {
+        const size_t a = len * (size_t)p / np, b = len * ((size_t)p + 1) / np;
+        copy_range(to + a, seg, nseg, lo + a, lo + b);
+    });
+}
+
+const void *nb6_stage(const Nb6Seg *seg, int nseg, size_t bytes) {
+    if (bytes > STAGE_MAX || !g_uva) return nullptr;
+    if (g_stage_busy) NB6_CUDA_CHECK(cudaStreamSynchronize(g_stream));
+    g_stage.reserve(STAGE_MAX);
+    copy_range_pool(g_stage.ptr, seg, nseg, 0, bytes);
+    g_stage_busy = true;
+    return g_stage.ptr;
+}
+
+void nb6_upload(void *dst, const Nb6Seg *seg, int nseg, size_t bytes, cudaStream_t st) {
+    size_t chunk = (bytes / 4 + 4095) / 4096 * 4096;
+    chunk = chunk < CHUNK_MIN ? CHUNK_MIN : chunk > CHUNK_MAX ? CHUNK_MAX : chunk;
+    for (size_t lo = 0; lo < bytes; lo += chunk) {
+        const size_t hi = lo + chunk < bytes ? lo + chunk : bytes;
+        const int r = g_ring_next;
+        g_ring_next = (g_ring_next + 1) % RING;
+        if (!g_ring_ev[r]) NB6_CUDA_CHECK(cudaEventCreateWithFlags(&g_ring_ev[r], cudaEventDisableTiming));
+        else NB6_CUDA_CHECK(cudaEventSynchronize(g_ring_ev[r]));
+        g_ring[r].reserve(chunk);
+        copy_range_pool(g_ring[r].ptr, seg, nseg, lo, hi);
+        NB6_CUDA_CHECK(cudaMemcpyAsync(static_cast<unsigned char *>(dst) + lo, g_ring[r].ptr, hi - lo,
+                                       cudaMemcpyHostToDevice, st));
+        NB6_CUDA_CHECK(cudaEventRecord(g_ring_ev[r], st));
+    }
+}
+
 // Enqueue a copy of the device status word into pinned host memory; the
 // next nb6_check_dev_status after a sync of `st` reads that copy instead of
 // doing a synchronous copy of its own.
@@ -124,6 +190,7 @@ int *nb6_status_post() {
 // Read (and clear) the device status word; call after a stream sync.
 int nb6_check_dev_status() {
     int st = 0;
+    g_stage_busy = false;
     if (g_status_fetched) {
         st = *(volatile int *)g_status_host;
         g_status_fetched = false;
