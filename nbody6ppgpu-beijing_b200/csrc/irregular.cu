@@ -315,57 +315,122 @@ __global__ void __launch_bounds__(PS_NT) irr_predict_set(int n, double ti, const
     }
 }
 
-NB6_DEV void load_pv(const Pv *__restrict__ p, double *x, double *v, double &m) {
-    const double2 *q = reinterpret_cast<const double2 *>(p);
-    const double2 a = __ldg(q), b = __ldg(q + 1), c = __ldg(q + 2), d = __ldg(q + 3);
-    x[0] = a.x;
-    x[1] = a.y;
-    x[2] = b.x;
-    m = b.y;
-    v[0] = c.x;
-    v[1] = c.y;
-    v[2] = d.x;
+// 16 bytes global -> shared through L2, and the waits for them.
+NB6_DEV void copy16_async(double2 *dst, const double2 *src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
 }
+NB6_DEV void copy_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+NB6_DEV void copy_wait_all_but_one() { asm volatile("cp.async.wait_group 1;" ::: "memory"); }
 
-// irr_force_warp without a pair table, over the predicted set: the same
-// pair terms in the same order per lane, so the same bits.
-NB6_DEV void irr_force_warp_pv(int i, int lane, const Pv *__restrict__ pv, const int *__restrict__ lists, int ls,
-                               int nmax, double *a, double *jd, int &nnbid) {
-    double xi[3], vi[3], mi;
-    load_pv(pv + i, xi, vi, mi);
+// irr_force_warp without a pair table, for the calls over many bodies: the
+// neighbours' records (or, PV, their bodies of the predicted set) are brought
+// into shared memory by the warp together, 8 (4) lanes to a record, two rounds
+// of 32 neighbours in flight, and each lane then reads its own.  A lane that
+// gathers a record by itself makes each of its seven 16-byte loads touch 32
+// lines across the warp, and the L1 looks up one line per cycle: those lookups
+// bounded the walk (32,768 lists of 50 of 131,072 bodies: 80 us, now 64; what
+// remains is the L2's traffic, 210 MB of records).  Pieces are stored
+// XOR-swizzled, as in irr_predict_set.  The pair terms are irr_force_warp's, in
+// its order per lane, so the bits are the same.
+template <bool PV>
+NB6_DEV void irr_force_coop(int i, int lane, double ti, const double2 *__restrict__ set,
+                            const int *__restrict__ lists, int ls, int nmax, double2 *sm, double *a, double *jd,
+                            int &nnbid, int &nnb_out) {
+    constexpr int NP = PV ? 4 : 8, USED = PV ? 4 : 7;   // pieces per record, and those with data
     const int *row = lists + (size_t)i * ls;
     const int nnb = row[0];
+    int jn0 = 1 + lane < ls ? row[1 + lane] : -1;
+    int jn1 = 33 + lane < ls ? row[33 + lane] : -1;
+    auto swz = [](int q) { return PV ? (q >> 1) & 3 : q & 7; };
+    auto body = [&](const double2 *p, int sw, double *x, double *v, double &m) {
+        const double2 p0 = p[0 ^ sw], p1 = p[1 ^ sw], p2 = p[2 ^ sw], p3 = p[3 ^ sw];
+        if (PV) {
+            x[0] = p0.x; x[1] = p0.y; x[2] = p1.x; m = p1.y;
+            v[0] = p2.x; v[1] = p2.y; v[2] = p3.x;
+            return;
+        }
+        const double2 p4 = p[4 ^ sw], p5 = p[5 ^ sw], p6 = p[6 ^ sw];
+        Rec r;   // the piece order of load_rec
+        r.x[0] = p0.x; r.x[1] = p0.y; r.x[2] = p1.x;
+        r.v[0] = p1.y; r.v[1] = p2.x; r.v[2] = p2.y;
+        r.f[0] = p3.x; r.f[1] = p3.y; r.f[2] = p4.x;
+        r.fd[0] = p4.y; r.fd[1] = p5.x; r.fd[2] = p5.y;
+        r.m = p6.x; r.t0 = p6.y;
+        predict(r, ti, x, v);
+        m = r.m;
+    };
+    // start the copies of one round: lane l's neighbour j (-1: none) into
+    // record slot l of buffer b
+    auto gather = [&](int b, int j) {
+#pragma unroll
+        for (int s = 0; s < NP; ++s) {
+            const int q = s * (32 / NP) + lane / NP, piece = lane % NP;
+            const int id = __shfl_sync(0xffffffffu, j, q);
+            if (id >= 0 && piece < USED)
+                copy16_async(sm + (b * 32 + q) * NP + (piece ^ swz(q)), set + (size_t)id * NP + piece);
+        }
+    };
+    // (ids are checked at set_list time)
+    auto entry = [&](int l, int j) { return l < nnb && j >= 0 && j < nmax ? j : -1; };
+    int j0 = entry(lane, jn0), j1 = entry(32 + lane, jn1);
+    gather(0, j0);
+    copy_commit();
+    if (nnb > 32) gather(1, j1);
+    copy_commit();
+    double xi[3], vi[3], mi;
+    body(set + (size_t)i * NP, 0, xi, vi, mi);
     double ax = 0, ay = 0, az = 0, jx = 0, jy = 0, jz = 0;
     double rmin = 1.0e300;
     int jmin = 0x7fffffff;
-    auto add = [&](const double *xj, const double *vj, double m, int j) {
-        const double dxd = xj[0] - xi[0], dyd = xj[1] - xi[1], dzd = xj[2] - xi[2];
-        const double r2d = dxd * dxd + dyd * dyd + dzd * dzd;
-        if (r2d < rmin || (r2d == rmin && j < jmin)) {
-            rmin = r2d;
-            jmin = j;
+    for (int base = 0; base < nnb; base += 32) {
+        const int l2 = base + 64 + lane;
+        const int jn = l2 < nnb && 1 + l2 < ls ? row[1 + l2] : -1;
+        copy_wait_all_but_one();
+        __syncwarp();
+        const int b = (base >> 5) & 1;
+        if (j0 >= 0) {
+            double xj[3], vj[3], m;
+            body(sm + (b * 32 + lane) * NP, swz(lane), xj, vj, m);
+            const double dxd = xj[0] - xi[0], dyd = xj[1] - xi[1], dzd = xj[2] - xi[2];
+            const double r2d = dxd * dxd + dyd * dyd + dzd * dzd;
+            if (r2d < rmin || (r2d == rmin && j0 < jmin)) {
+                rmin = r2d;
+                jmin = j0;
+            }
+            const double dvx = vj[0] - vi[0], dvy = vj[1] - vi[1], dvz = vj[2] - vi[2];
+            const double rinv = rsqrt(r2d);
+            const double rinv2 = rinv * rinv;
+            const double mr3 = m * rinv * rinv2;
+            const double al = -3.0 * (dxd * dvx + dyd * dvy + dzd * dvz) * rinv2;
+            ax += mr3 * dxd;
+            ay += mr3 * dyd;
+            az += mr3 * dzd;
+            jx += mr3 * (dvx + al * dxd);
+            jy += mr3 * (dvy + al * dyd);
+            jz += mr3 * (dvz + al * dzd);
         }
-        const double dvx = vj[0] - vi[0], dvy = vj[1] - vi[1], dvz = vj[2] - vi[2];
-        const double rinv = rsqrt(r2d);
-        const double rinv2 = rinv * rinv;
-        const double mr3 = m * rinv * rinv2;
-        const double al = -3.0 * (dxd * dvx + dyd * dvy + dzd * dvz) * rinv2;
-        ax += mr3 * dxd;
-        ay += mr3 * dyd;
-        az += mr3 * dzd;
-        jx += mr3 * (dvx + al * dxd);
-        jy += mr3 * (dvy + al * dyd);
-        jz += mr3 * (dvz + al * dzd);
-    };
-    for (int l = lane; l < nnb; l += 32) {
-        const int j = row[1 + l];
-        if (j < 0 || j >= nmax) continue;   // ids are checked at set_list time
-        double xj[3], vj[3], m;
-        load_pv(pv + j, xj, vj, m);
-        add(xj, vj, m, j);
+        __syncwarp();
+        j0 = j1;
+        j1 = entry(l2, jn);
+        if (base + 64 < nnb) gather(b, j1);
+        copy_commit();
     }
     irr_warp_finish(ax, ay, az, jx, jy, jz, rmin, jmin, nnb, a, jd, nnbid);
+    nnb_out = max(nnb, 0);
 }
+
+// The active addresses (1-based) of a launch: in device-readable memory, or,
+// NA > 0, in the launch's own arguments -- a small call then has no trip over
+// the bus at the head of every walk.
+template <int NA> struct ActiveAddr {
+    int v[NA];
+    NB6_DEV int operator[](int k) const { return v[k]; }
+};
+template <> struct ActiveAddr<0> {
+    const int *__restrict__ p;
+    NB6_DEV int operator[](int k) const { return p[k]; }
+};
+constexpr int IRR_INLINE = 256;
 
 // out row k = (ax, ay, az, jx, jy, jz, nnbid, 0) (the correctors' rows),
 // or, with out null, the caller's layout in fv: acc[ni][3] | jrk[ni][3]
@@ -373,46 +438,42 @@ NB6_DEV void irr_force_warp_pv(int i, int lane, const Pv *__restrict__ pv, const
 // block copies into the caller's arrays.
 // KS: with the pair table (a separate instance: the corrections double the
 // registers of the plain walk).  PV (no pair table): the walk over the
-// predicted set pv instead of the records.
-template <bool KS, bool PV = false>
+// predicted set instead of the records.  hstatus: see nb6_status_post.
+template <bool KS, bool PV, int NA>
 __global__ void __launch_bounds__(IRR_WARPS * 32)
-    irr_kernel(int ni, const int *__restrict__ addr, double ti, const Rec *__restrict__ rec,
+    irr_kernel(int ni, const __grid_constant__ ActiveAddr<NA> addr, double ti, const Rec *__restrict__ rec,
                const Pv *__restrict__ pv, const int *__restrict__ lists, int ls, int nmax, KsArgs ks,
-               double *__restrict__ out, double *__restrict__ fv) {
+               double *__restrict__ out, double *__restrict__ fv, const int *status, int *hstatus) {
     static_assert(!(KS && PV), "the predicted-set walk has no pair table");
+    __shared__ __align__(128) double2 sm[KS ? 1 : IRR_WARPS][KS ? 1 : 64 * (PV ? 4 : 8)];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int k = blockIdx.x * IRR_WARPS + warp;
+    if (hstatus && k == 0 && lane == 0) *hstatus = *status;
     if (k >= ni) return;
+    const int i = addr[k] - 1;
     double a[3], jd[3];
-    int id;
-    if (PV)
-        irr_force_warp_pv(addr[k] - 1, lane, pv, lists, ls, nmax, a, jd, id);
-    else
-        irr_force_warp<KS>(addr[k] - 1, lane, ti, rec, lists, ls, nmax, ks, a, jd, id);
-    if (lane == 0 && !out) {
-        // the caller's layout, in the blocks of the output staging:
-        // acc[ni][3] | jrk[ni][3] (doubles) | nnbid[ni] | nnb[ni] (ints)
-        double *oa = fv;
-        int *oi = reinterpret_cast<int *>(oa + 6 * (size_t)ni);
-        oa[3 * (size_t)k] = a[0];
-        oa[3 * (size_t)k + 1] = a[1];
-        oa[3 * (size_t)k + 2] = a[2];
-        oa[3 * (size_t)ni + 3 * (size_t)k] = jd[0];
-        oa[3 * (size_t)ni + 3 * (size_t)k + 1] = jd[1];
-        oa[3 * (size_t)ni + 3 * (size_t)k + 2] = jd[2];
-        oi[k] = id;
-        oi[ni + k] = max(lists[(size_t)(addr[k] - 1) * ls], 0);
+    int id, nnb = 0;
+    if (KS) {
+        irr_force_warp<KS>(i, lane, ti, rec, lists, ls, nmax, ks, a, jd, id);
+        nnb = max(lists[(size_t)i * ls], 0);
+    } else {
+        irr_force_coop<PV>(i, lane, ti, reinterpret_cast<const double2 *>(PV ? (const void *)pv : (const void *)rec),
+                           lists, ls, nmax, sm[KS ? 0 : warp], a, jd, id, nnb);
     }
-    if (lane == 0 && out) {
-        double *o = out + (size_t)k * 8;
-        o[0] = a[0];
-        o[1] = a[1];
-        o[2] = a[2];
-        o[3] = jd[0];
-        o[4] = jd[1];
-        o[5] = jd[2];
-        o[6] = (double)id;
-        o[7] = 0.0;
+    // the row by its lanes: value c in lane c
+    double w = a[0];
+    if (lane == 1) w = a[1];
+    if (lane == 2) w = a[2];
+    if (lane == 3) w = jd[0];
+    if (lane == 4) w = jd[1];
+    if (lane == 5) w = jd[2];
+    if (out) {
+        if (lane < 8) out[(size_t)k * 8 + lane] = lane < 6 ? w : lane == 6 ? (double)id : 0.0;
+    } else {
+        int *oi = reinterpret_cast<int *>(fv + 6 * (size_t)ni);
+        if (lane < 6) fv[(lane < 3 ? 0 : 3 * (size_t)ni - 3) + 3 * (size_t)k + lane] = w;
+        else if (lane == 6) oi[k] = id;
+        else if (lane == 7) oi[ni + k] = nnb;
     }
 }
 
@@ -1539,14 +1600,19 @@ KsArgs ks_args() {
 // a B200 (lists of 64 in a Plummer N = 262,144) the call took 7% less time
 // at 4 entries per body set, 16% less at 16, the same at 2 and 9% more at
 // 1.
-const Pv *irr_predicted_set(int ni, double ti, cudaStream_t st) {
+bool irr_wants_predicted_set(int ni) {
     if (I.pv_mode < 0) {
         const char *e = getenv("NB6_IRR_PV");
         I.pv_mode = e ? atoi(e) : 1;
     }
+    const double n = I.addr_hi;
+    if (I.ks_npair > 0 || I.pv_mode == 0 || n <= 0) return false;
+    return I.pv_mode != 1 || (double)ni * (double)I.nnb_total >= 4.0 * n * n;
+}
+
+const Pv *irr_predicted_set(int ni, double ti, cudaStream_t st) {
+    if (!irr_wants_predicted_set(ni)) return nullptr;
     const int n = I.addr_hi;
-    if (I.ks_npair > 0 || I.pv_mode == 0 || n <= 0) return nullptr;
-    if (I.pv_mode == 1 && (double)ni * (double)I.nnb_total < 4.0 * (double)n * (double)n) return nullptr;
     if (!I.pv_zeroed) {
         // every address the lists or the active set can name (< nmax) has a
         // body; those never set keep the zeros that predict() makes of
@@ -1562,17 +1628,31 @@ const Pv *irr_predicted_set(int ni, double ti, cudaStream_t st) {
 // out: rows of 8 doubles; or, out null, the caller's layout in fv.  pv: the
 // call's predicted set (irr_predicted_set), null for the record walk.
 void launch_irr_kernel(int ni, const int *daddr, double ti, double *out, cudaStream_t st, double *fv = nullptr,
-                       const Pv *pv = nullptr) {
+                       const Pv *pv = nullptr, int *hstatus = nullptr) {
     const KsArgs ks = ks_args();
     const dim3 grid((ni + IRR_WARPS - 1) / IRR_WARPS), block(IRR_WARPS * 32);
     const Rec *rec = I.rec.ptr;
-    const int *lists = I.lists.ptr;
+    const int *lists = I.lists.ptr, *status = nb6_dev_status();
+    const ActiveAddr<0> ad{daddr};
     if (ks.slot)
-        irr_kernel<true><<<grid, block, 0, st>>>(ni, daddr, ti, rec, nullptr, lists, I.lmax, I.nmax, ks, out, fv);
+        irr_kernel<true, false, 0><<<grid, block, 0, st>>>(ni, ad, ti, rec, nullptr, lists, I.lmax, I.nmax, ks, out,
+                                                           fv, status, hstatus);
     else if (pv)
-        irr_kernel<false, true><<<grid, block, 0, st>>>(ni, daddr, ti, rec, pv, lists, I.lmax, I.nmax, ks, out, fv);
+        irr_kernel<false, true, 0><<<grid, block, 0, st>>>(ni, ad, ti, rec, pv, lists, I.lmax, I.nmax, ks, out, fv,
+                                                           status, hstatus);
     else
-        irr_kernel<false><<<grid, block, 0, st>>>(ni, daddr, ti, rec, nullptr, lists, I.lmax, I.nmax, ks, out, fv);
+        irr_kernel<false, false, 0><<<grid, block, 0, st>>>(ni, ad, ti, rec, nullptr, lists, I.lmax, I.nmax, ks, out,
+                                                            fv, status, hstatus);
+}
+
+// The record walk of ni <= IRR_INLINE bodies, their addresses (host memory)
+// passed with the launch.
+void launch_irr_inline(int ni, const int *addr, double ti, cudaStream_t st, double *fv, int *hstatus) {
+    ActiveAddr<IRR_INLINE> ad;
+    memcpy(ad.v, addr, sizeof(int) * ni);
+    irr_kernel<false, false, IRR_INLINE><<<(ni + IRR_WARPS - 1) / IRR_WARPS, IRR_WARPS * 32, 0, st>>>(
+        ni, ad, ti, I.rec.ptr, nullptr, I.lists.ptr, I.lmax, I.nmax, KsArgs{}, nullptr, fv, nb6_dev_status(),
+        hstatus);
 }
 
 __global__ void ks_scatter_slots(int npair, const int *__restrict__ cm, int *__restrict__ slot) {
@@ -1885,7 +1965,9 @@ void irr_firr_vec_impl(double ti, int ni, const int *addr, double (*acc)[3], dou
     cudaStream_t st = nb6_stream();
     // the pinned staging is reused only after this call's synchronize, so
     // the uploads enqueued here read it intact
-    const int *daddr = irr_flush(st, addr, ni);
+    const bool small = ni <= IRR_INLINE && sizeof(double) * 7 * (size_t)ni <= zero_copy_out_bytes() &&
+                       I.ks_npair <= 0 && !irr_wants_predicted_set(ni);
+    const int *daddr = small ? irr_flush(st) : irr_flush(st, addr, ni);
     // Results in the caller's layout, per chunk of bodies [a, a+m): at
     // double offset 7a, acc[m][3] | jrk[m][3] (doubles) | nnbid[m] | nnb[m]
     // (ints) -- one chunk covering all ni is exactly the caller's three
@@ -1920,9 +2002,11 @@ void irr_firr_vec_impl(double ti, int ni, const int *addr, double (*acc)[3], dou
     auto chunk_lo = [&](int c) { return (int)((long long)ni * c / nch); };
     NB6_CUDA_CHECK(cudaEventRecord(I.ev0, st));
     const Pv *pv = irr_predicted_set(ni, ti, st);
+    int *hstatus = direct ? nb6_status_post() : nullptr;
     for (int c = 0; c < nch; ++c) {
         const int a = chunk_lo(c), m = chunk_lo(c + 1) - a;
-        launch_irr_kernel(m, daddr + a, ti, nullptr, st, out + 7 * (size_t)a, pv);
+        if (small) launch_irr_inline(ni, addr, ti, st, out, hstatus);
+        else launch_irr_kernel(m, daddr + a, ti, nullptr, st, out + 7 * (size_t)a, pv, hstatus);
         NB6_CUDA_CHECK(cudaGetLastError());
         if (!direct) {
             NB6_CUDA_CHECK(cudaEventRecord(I.evk[c], st));
@@ -1933,7 +2017,7 @@ void irr_firr_vec_impl(double ti, int ni, const int *addr, double (*acc)[3], dou
         }
     }
     NB6_CUDA_CHECK(cudaEventRecord(I.ev1, st));
-    nb6_status_fetch(st);
+    if (!direct) nb6_status_fetch(st);
     unsigned long long inter = 0;
     if (pool) pool->arm();
     if (!direct) {

@@ -146,3 +146,41 @@ def test_list_rows_at_register_widths(nb6, orc, cap):
             assert lst[r, 0] == c
             np.testing.assert_array_equal(lst[r, 1:1 + c], np.sort(order[:c]))
             assert np.all(lst[r, 1 + c:] == 0)
+
+
+@pytest.mark.parametrize("mode", [0, 2])
+@pytest.mark.parametrize("ni", [1, 3, 255, 256, 257, 292, 293, 8193])
+def test_irregular_rounds_and_call_sizes(nb6, orc, mode, ni):
+    """Lists on either side of the walk's rounds of 32 and of the row's end,
+    and calls on either side of the sizes that pass their addresses with the
+    launch and write their results in place.  FP64 sums of at most 199 terms:
+    1e-10 relative leaves four digits for cancellation."""
+    n, lmax = 600, 200
+    rng = np.random.default_rng(ni)
+    lens = np.array([0, 1, 2, 31, 32, 33, 63, 64, 65, 95, 96, 97, 127, 128, 129, 160, 191, 192, 193, 199])
+    lists = np.zeros((n, lmax), dtype=np.int32)
+    for i in range(n):
+        k = int(lens[i % len(lens)])
+        lists[i, 0] = k
+        lists[i, 1:1 + k] = np.sort(rng.choice(np.delete(np.arange(1, n + 1), i), k, replace=False))
+    x0, v0, f2, fd6 = (rng.normal(size=(n, 3)) for _ in range(4))
+    m, t0 = rng.uniform(0.5, 1.5, n) / n, -rng.integers(0, 16, n) / 2048.0
+    addr = (rng.permutation(max(n, ni))[:ni] % n + 1).astype(np.int32)
+    nb6.irr_open(n, lmax, 0)
+    try:
+        nb6.lib.nb6_irr_pv_(C.byref(C.c_int(mode)))
+        nb6.irr_set_jp_all(x0, v0, f2, fd6, m, t0)
+        for i in range(n):
+            nb6.irr_set_list(i + 1, lists[i])
+        for _ in range(2):       # the second call has nothing staged before it
+            acc, jrk, nnbid = nb6.irr_firr_vec(1.0 / 2048, addr)
+            oa, oj, oid = orc.firr(1.0 / 2048, addr, x0, v0, f2, fd6, m, t0, lists)
+            ok = lists[addr - 1, 0] > 0
+            np.testing.assert_array_equal(nnbid, oid)
+            assert np.all(acc[~ok] == 0) and np.all(jrk[~ok] == 0)
+            if ok.any():
+                assert rel_err_vec(acc[ok], oa[ok]).max() <= 1e-10
+                assert rel_err_vec(jrk[ok], oj[ok]).max() <= 1e-10
+    finally:
+        nb6.lib.nb6_irr_pv_(C.byref(C.c_int(1)))
+        nb6.irr_close(0)
