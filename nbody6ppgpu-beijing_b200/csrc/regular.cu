@@ -168,12 +168,27 @@ NB6_DEV bool reg_pair(const IPart &ip, const float4 &a, const float4 &b, const f
 // Operation order matches the FP64 rule of regint.f:41-65 with the strict
 // "<" of gpunb.velocity.cu:188,236; no FMA contraction.
 // Returns whether a contribution was added.
+struct IExact {   // the call's FP64 data of one i-particle
+    double h2, dt, x[3], v[3];
+};
+NB6_DEV IExact load_iexact(const RegArgs &a, int i) {
+    IExact e;
+    e.h2 = a.ih2[i];
+    e.dt = a.idtr[i];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        e.x[c] = a.ix[3 * (size_t)i + c];
+        e.v[c] = a.iv[3 * (size_t)i + c];
+    }
+    return e;
+}
+
 template <bool MFLAG>
-NB6_DEV bool reg_exact(const RegArgs &a, int i, int jslot, Sums &s, int joff = 0) {
+NB6_DEV bool reg_exact(const RegArgs &a, const IExact &ie, int i, int jslot, Sums &s, int joff = 0) {
     const int j = a.perm ? a.perm[jslot] : jslot;  // the caller's index of the body in this slot
-    const double xi0 = a.ix[3 * i], xi1 = a.ix[3 * i + 1], xi2 = a.ix[3 * i + 2];
-    const double vi0 = a.iv[3 * i], vi1 = a.iv[3 * i + 1], vi2 = a.iv[3 * i + 2];
-    const double h2 = a.ih2[i], dt = a.idtr[i];
+    const double xi0 = ie.x[0], xi1 = ie.x[1], xi2 = ie.x[2];
+    const double vi0 = ie.v[0], vi1 = ie.v[1], vi2 = ie.v[2];
+    const double h2 = ie.h2, dt = ie.dt;
     {
         const double dx = __dsub_rn(a.jx[3 * j], xi0);
         const double dy = __dsub_rn(a.jx[3 * j + 1], xi1);
@@ -223,7 +238,7 @@ __device__ FLUSH_INLINE Sums reg_flush(const RegArgs &a, const IPart ip, int i, 
         if (!reg_geom<MFLAG>(ip, A[b], B[b], Cv[b]).cand) continue;
         const int j = jbase + b;
         if (j >= a.nj) continue;  // padding slots are never neighbours
-        reg_exact<MFLAG>(a, i, j, s);
+        reg_exact<MFLAG>(a, load_iexact(a, i), i, j, s);
     }
     return s;
 }
@@ -678,7 +693,7 @@ __global__ void __launch_bounds__(NT, X2_MINB / NI) regf_x2_kernel(const RegArgs
         }
         Sums x;
         zero(x);
-        const bool add = lane < c && reg_exact<MFLAG>(a, i, e.x, x);
+        const bool add = lane < c && reg_exact<MFLAG>(a, load_iexact(a, i), i, e.x, x);
         for (unsigned m = __ballot_sync(0xffffffffu, add); m; m &= m - 1) {
             const int src = __ffs(m) - 1;
             const int o = __shfl_sync(0xffffffffu, e.y, src);
@@ -901,7 +916,7 @@ __global__ void __launch_bounds__(NT, X2_MINB / NI) regf_x2_kernel(const RegArgs
 // busy even for ni = 1.  Same pair math, candidate test and exact FP64 rare
 // path as regf_kernel; the per-thread FP32 partials are reduced over the CTA
 // in FP64 and written as (hi, lo) slice partials for regf_finalize.
-constexpr int JPAR_NT = 256;
+constexpr int JPAR_NT = 256, JPAR_CTAS = 512 / JPAR_NT;   // 16 warps per SM
 
 // The i-particles of a j-parallel CTA in shared memory: sip[k] = (xH, yH, zH,
 // 1.01 h2), (xL, yL, zL, dtr), (vx, vy, vz, 0) of particle k, and, for the
@@ -911,6 +926,7 @@ constexpr int JPAR_NT = 256;
 template <int IB> struct JparI {
     static constexpr int V = 7 * IB;           // sums of a CTA's i-particles
     static constexpr int CH = V < 28 ? V : 28; // of which this many are transposed at a time
+    IExact ie[2][IB];   // the call's own data of the particles (segmented kernel: and of the next item's)
     float4 sip[IB][3];
     IP2 sip2[IB > 1 ? IB / 2 : 1];
     // each warp's queue of neighbour candidates (j << 3 | k) awaiting the
@@ -921,19 +937,37 @@ template <int IB> struct JparI {
     double red[JPAR_NT / 32][V];
 };
 
+// Bring the FP64 data of i-particles i0 .. i0 + nvalid - 1 into S.ie[buf],
+// asynchronously: it may still sit in the caller's pinned block, a trip over
+// the bus away.  (8 IB threads, one word each: h2, dtr, x, v of a particle.)
+template <int IB>
+NB6_DEV void jpar_fetch_i(const RegArgs &a, JparI<IB> &S, int buf, int i0, int nvalid) {
+    const int k = threadIdx.x >> 3, c = threadIdx.x & 7;
+    if (k < IB && k < nvalid) {
+        const size_t i = (size_t)(i0 + k);
+        const double *src = c == 0 ? a.ih2 + i : c == 1 ? a.idtr + i : c < 5 ? a.ix + 3 * i + (c - 2)
+                                                                             : a.iv + 3 * i + (c - 5);
+        double *dst = reinterpret_cast<double *>(&S.ie[buf][k]) + c;
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+}
+
+// The fetched particles as the pair loops take them.  The caller's barriers
+// stand before (every thread's words have landed) and after.
 template <int IB, bool X2>
-NB6_DEV void jpar_stage_i(const RegArgs &a, JparI<IB> &S, int i0, int nvalid) {
+NB6_DEV void jpar_stage_i(JparI<IB> &S, int buf, int nvalid) {
     const int k = threadIdx.x;
     if (k >= IB) return;
     float4 p = make_float4(0.f, 0.f, 0.f, 0.f), q = p, r = p;
     if (k < nvalid) {
-        const int i = i0 + k;
-        split_hl(a.ix[3 * i], p.x, q.x);
-        split_hl(a.ix[3 * i + 1], p.y, q.y);
-        split_hl(a.ix[3 * i + 2], p.z, q.z);
-        p.w = (float)a.ih2[i] * CAND_SLACK;
-        q.w = (float)a.idtr[i];
-        r = make_float4((float)a.iv[3 * i], (float)a.iv[3 * i + 1], (float)a.iv[3 * i + 2], 0.f);
+        const IExact &e = S.ie[buf][k];
+        split_hl(e.x[0], p.x, q.x);
+        split_hl(e.x[1], p.y, q.y);
+        split_hl(e.x[2], p.z, q.z);
+        p.w = (float)e.h2 * CAND_SLACK;
+        q.w = (float)e.dt;
+        r = make_float4((float)e.v[0], (float)e.v[1], (float)e.v[2], 0.f);
     }
     S.sip[k][0] = p;
     S.sip[k][1] = q;
@@ -945,6 +979,10 @@ NB6_DEV void jpar_stage_i(const RegArgs &a, JparI<IB> &S, int i0, int nvalid) {
 #pragma unroll
         for (int c = 0; c < 11; ++c) l[2 * c] = v[c];
     }
+}
+NB6_DEV void jpar_fetch_wait() {
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
 }
 
 // The j-parallel inner loop: this thread's j's of [j_begin, j_end) against
@@ -966,7 +1004,7 @@ NB6_DEV void jpar_stage_i(const RegArgs &a, JparI<IB> &S, int i0, int nvalid) {
 // reduction (jpar_reduce): 37 i of 500,009 bodies 70 -> 56 us, 531 of 16,384
 // 41 -> 32 us, the 64-cluster work list of regf_seg_kernel 299 -> 245 us.
 template <int IB, bool MFLAG, bool X2>
-NB6_DEV void jpar_loop(const RegArgs &a, JparI<IB> &S, int j_begin, int j_end, int i0, int nvalid,
+NB6_DEV void jpar_loop(const RegArgs &a, JparI<IB> &S, int buf, int j_begin, int j_end, int i0, int nvalid,
                        int jbase, Sums *s) {
     if constexpr (X2 || IB == 1) {
         constexpr int NP = IB > 1 ? IB / 2 : 1;
@@ -995,7 +1033,7 @@ NB6_DEV void jpar_loop(const RegArgs &a, JparI<IB> &S, int j_begin, int j_end, i
             const int k = (int)(e & 7u), jj = (int)(e >> 3);
             Sums t;
             zero(t);
-            if (!reg_exact<MFLAG>(a, i0 + k, jj, t, jbase)) return;
+            if (!reg_exact<MFLAG>(a, S.ie[buf][k], i0 + k, jj, t, jbase)) return;
             if constexpr (IB == 1) {
                 s[0].ax += t.ax; s[0].ay += t.ay; s[0].az += t.az;
                 s[0].jx += t.jx; s[0].jy += t.jy; s[0].jz += t.jz; s[0].po += t.po;
@@ -1093,20 +1131,21 @@ NB6_DEV void jpar_loop(const RegArgs &a, JparI<IB> &S, int j_begin, int j_end, i
                     ip.xh = p.x; ip.yh = p.y; ip.zh = p.z; ip.h2c = p.w;
                     ip.xl = q.x; ip.yl = q.y; ip.zl = q.z; ip.dt = q.w;
                     ip.vx = r.x; ip.vy = r.y; ip.vz = r.z;
-                    if (reg_geom<MFLAG>(ip, pa, pb, pc).cand) reg_exact<MFLAG>(a, i0 + k, j, s[k], jbase);
+                    if (reg_geom<MFLAG>(ip, pa, pb, pc).cand)
+                        reg_exact<MFLAG>(a, S.ie[buf][k], i0 + k, j, s[k], jbase);
                 }
             }
         }
     }
 }
 
-// The CTA's sums of its IB i-particles in FP64, as (hi, lo) pairs into the
-// partial rows part[4 row(k)] of its first nvalid particles.  Each warp
-// transposes its lanes' sums through shared memory, so that a lane adds up
-// one sum's 32 terms: a shuffle tree for each of the 28 sums of IB = 4 took
-// 420 instructions, a fifth of a 4,600-pair work item.
-template <int IB, class Row>
-NB6_DEV void jpar_reduce(JparI<IB> &S, const Sums *s, float4 *__restrict__ part, int nvalid, Row row) {
+// The CTA's sums of its IB i-particles in FP64: S.red[warp][7 k + c], summed
+// over the warps by jpar_total (after the barrier here).  Each warp transposes
+// its lanes' sums through shared memory, so that a lane adds up one sum's 32
+// terms: a shuffle tree for each of the 28 sums of IB = 4 took 420
+// instructions, a fifth of a 4,600-pair work item.
+template <int IB>
+NB6_DEV void jpar_reduce(JparI<IB> &S, const Sums *s) {
     constexpr int V = JparI<IB>::V, CH = JparI<IB>::CH;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
 #pragma unroll
@@ -1127,32 +1166,29 @@ NB6_DEV void jpar_reduce(JparI<IB> &S, const Sums *s, float4 *__restrict__ part,
         __syncwarp();
     }
     __syncthreads();
-    if (tid < V && tid / 7 < nvalid) {
-        double w = 0.0;
-#pragma unroll
-        for (int q = 0; q < JPAR_NT / 32; ++q) w += S.red[q][tid];
-        const float hi = (float)w;
-        reinterpret_cast<float2 *>(part + 4 * row(tid / 7))[tid % 7] = make_float2(hi, (float)(w - (double)hi));
-    }
 }
-
-// (IB = 8 keeps 56 sums: one CTA per SM.)
-template <int IB, bool MFLAG, bool X2 = false>
-__global__ void __launch_bounds__(JPAR_NT, IB <= 4 ? 2 : 1) regf_jpar_kernel(const RegArgs a) {
-    __shared__ __align__(16) JparI<IB> S;
-    const int i0 = blockIdx.x * IB;
-    jpar_stage_i<IB, X2>(a, S, i0, a.ni - i0);
-    __syncthreads();
-    const int j_begin = (int)(((long long)blockIdx.y * a.nj) / a.nslices);
-    const int j_end = (int)(((long long)(blockIdx.y + 1) * a.nj) / a.nslices);
-    Sums s[IB];
-    jpar_loop<IB, MFLAG, X2>(a, S, j_begin, j_end, i0, a.ni - i0, 0, s);
-    jpar_reduce<IB>(S, s, a.part, a.ni - i0, [&](int k) { return (size_t)blockIdx.y * a.ni_pad + i0 + k; });
+template <int IB>
+NB6_DEV double jpar_total(const JparI<IB> &S, int t) {
+    double w = 0.0;
+#pragma unroll
+    for (int q = 0; q < JPAR_NT / 32; ++q) w += S.red[q][t];
+    return w;
+}
+// They as (hi, lo) pairs into the partial rows part[4 row(k)] of the first
+// nvalid particles.
+template <int IB, class Row>
+NB6_DEV void jpar_partials(const JparI<IB> &S, float4 *__restrict__ part, int nvalid, Row row) {
+    const int t = threadIdx.x;
+    if (t < JparI<IB>::V && t / 7 < nvalid) {
+        const double w = jpar_total(S, t);
+        const float hi = (float)w;
+        reinterpret_cast<float2 *>(part + 4 * row(t / 7))[t % 7] = make_float2(hi, (float)(w - (double)hi));
+    }
 }
 
 // Accumulate one (hi, lo) slice partial into FP64 sums.
 NB6_DEV void add_partial(const float4 *p, double *v) {
-    const float4 q0 = p[0], q1 = p[1], q2 = p[2], q3 = p[3];
+    const float4 q0 = __ldcg(p), q1 = __ldcg(p + 1), q2 = __ldcg(p + 2), q3 = __ldcg(p + 3);
     v[0] += (double)q0.x + (double)q0.y;
     v[1] += (double)q0.z + (double)q0.w;
     v[2] += (double)q1.x + (double)q1.y;
@@ -1170,10 +1206,10 @@ NB6_DEV void add_partial(const float4 *p, double *v) {
 // 531 rows of up to 400 ids 184 us, now 150).
 constexpr int ROW_REGS = 16;
 template <int R>
-NB6_DEV void write_sorted_row(int *__restrict__ row, const int *__restrict__ src, int n, int lane) {
+NB6_DEV void write_sorted_row(int *__restrict__ row, const int *src, int n, int lane) {
     int key[R];
 #pragma unroll
-    for (int r = 0; r < R; ++r) key[r] = r * 32 + lane < n ? src[r * 32 + lane] : INT_MAX;
+    for (int r = 0; r < R; ++r) key[r] = r * 32 + lane < n ? __ldcg(src + r * 32 + lane) : INT_MAX;
 #pragma unroll
     for (int kk = 2; kk <= 32 * R; kk <<= 1) {
 #pragma unroll
@@ -1209,38 +1245,11 @@ NB6_DEV void write_sorted_row(int *__restrict__ row, const int *__restrict__ src
     if (n == 32 * R && lane == 0) row[n] = before;
 }
 
-// Second half of a finalize row (one warp, one i): reduce the lanes' FP64
-// sums, write outf, reset the neighbour counter, and write the list row
-// sorted ascending (sb: shared memory for rows beyond 32 ROW_REGS ids) or
-// -nnb on overflow.
-// Host calls have the rows written straight into pinned host memory, where a
-// store costs a bus transaction of its own unless the warp's lanes write one
-// run: the eight doubles leave as one 64-byte store and the list row (its
-// stride ls a multiple of 32 ints there) as whole 128-byte lines, count
-// included (a call of 531 bodies 217 -> 198 us, one of 7 bodies 61 -> 52 us).
-NB6_DEV void finalize_row(int i, int lane, double *v, int *__restrict__ nbcnt,
-                          const int *__restrict__ nbbuf, int lcap, int cap, int ls, int *sb,
-                          double *__restrict__ outf, int *__restrict__ outl, const MlpArgs &mlp,
-                          const __nv_bfloat16 *sw) {
-#pragma unroll
-    for (int c = 0; c < 7; ++c) v[c] = warp_sum_d(v[c]);
-    const int n = nbcnt[i];
-    __syncwarp();
-    if (lane == 0) nbcnt[i] = 0;
-    double o = 0.0;   // lane c < 8 holds value c of the row
-    if (mlp.on) {
-        // learned radius proposal from this call's own results (out slot 7)
-        float fe[MLP_IN];
-        const double ax = v[0] * 0.125, ay = v[1] * 0.125, az = v[2] * 0.125;
-        mlp_features((double)n, mlp.h2[i], ax * ax + ay * ay + az * az, mlp.dtr[i], fe);
-        MlpAct act;
-        const float out = mlp_forward_warp(sw, mlp.norm, fe, lane, act);
-        o = (double)(out * mlp.norm[2 * MLP_IN + 1] + mlp.norm[2 * MLP_IN]);
-    }
-#pragma unroll
-    for (int c = 0; c < 7; ++c)
-        if (lane == c) o = v[c] * (c < 6 ? 0.125 : 0.5);
-    if (lane < 8) outf[(size_t)i * 8 + lane] = o;
+// The list row of i (one warp): the n recorded ids sorted ascending (sb:
+// shared memory for rows beyond 32 ROW_REGS ids), or -nnb on overflow.  The
+// ids are read through L2: the launch that recorded them may still be running.
+NB6_DEV void write_list_row(int i, int lane, int n, const int *nbbuf, int lcap, int cap, int ls, int *sb,
+                            int *__restrict__ outl) {
     int *row = outl + (size_t)i * ls;
     if (n > cap) {
         if (lane == 0) row[0] = -n;
@@ -1255,7 +1264,7 @@ NB6_DEV void finalize_row(int i, int lane, double *v, int *__restrict__ nbcnt,
     else {
         int P = 32;
         while (P < n) P <<= 1;
-        for (int k = lane; k < P; k += 32) sb[k] = (k < n) ? src[k] : INT_MAX;
+        for (int k = lane; k < P; k += 32) sb[k] = (k < n) ? __ldcg(src + k) : INT_MAX;
         __syncwarp();
         for (int kk = 2; kk <= P; kk <<= 1) {
             for (int jj = kk >> 1; jj > 0; jj >>= 1) {
@@ -1277,10 +1286,68 @@ NB6_DEV void finalize_row(int i, int lane, double *v, int *__restrict__ nbcnt,
     }
 }
 
+// Second half of a finalize row (one warp, one i): reduce the lanes' FP64
+// sums, write outf, reset the neighbour counter, and write the list row.
+// Host calls have the rows written straight into pinned host memory, where a
+// store costs a bus transaction of its own unless the warp's lanes write one
+// run: the eight doubles leave as one 64-byte store and the list row (its
+// stride ls a multiple of 32 ints there) as whole 128-byte lines, count
+// included (a call of 531 bodies 217 -> 198 us, one of 7 bodies 61 -> 52 us).
+NB6_DEV void finalize_row(int i, int lane, double *v, int *nbcnt,
+                          const int *nbbuf, int lcap, int cap, int ls, int *sb,
+                          double *__restrict__ outf, int *__restrict__ outl, const MlpArgs &mlp,
+                          const __nv_bfloat16 *sw) {
+#pragma unroll
+    for (int c = 0; c < 7; ++c) v[c] = warp_sum_d(v[c]);
+    const int n = __ldcg(nbcnt + i);
+    __syncwarp();
+    if (lane == 0) nbcnt[i] = 0;
+    double o = 0.0;   // lane c < 8 holds value c of the row
+    if (mlp.on) {
+        // learned radius proposal from this call's own results (out slot 7)
+        float fe[MLP_IN];
+        const double ax = v[0] * 0.125, ay = v[1] * 0.125, az = v[2] * 0.125;
+        mlp_features((double)n, mlp.h2[i], ax * ax + ay * ay + az * az, mlp.dtr[i], fe);
+        MlpAct act;
+        const float out = mlp_forward_warp(sw, mlp.norm, fe, lane, act);
+        o = (double)(out * mlp.norm[2 * MLP_IN + 1] + mlp.norm[2 * MLP_IN]);
+    }
+#pragma unroll
+    for (int c = 0; c < 7; ++c)
+        if (lane == c) o = v[c] * (c < 6 ? 0.125 : 0.5);
+    if (lane < 8) outf[(size_t)i * 8 + lane] = o;
+    write_list_row(i, lane, n, nbbuf, lcap, cap, ls, sb, outl);
+}
+
 // The device status word into the pinned copy the host reads after the
 // call's synchronize (hstatus null: the caller fetches it itself).
 NB6_DEV void post_status(const int *status, int *hstatus) {
     if (hstatus && blockIdx.x == 0 && threadIdx.x == 0) *hstatus = *status;
+}
+
+// Where the segmented kernel writes the rows it finishes itself.
+struct RowOut {
+    double *outf = nullptr;   // [ni][8]; null: every row is left to the finalize kernel
+    int *outl = nullptr;      // [ni][ls]
+    int ls = 0, cap = 0;
+    int *hstatus = nullptr;
+};
+
+// (IB = 8 keeps 56 sums: half the warps per SM.)
+template <int IB, bool MFLAG, bool X2 = false>
+__global__ void __launch_bounds__(JPAR_NT, IB <= 4 ? JPAR_CTAS : JPAR_CTAS / 2) regf_jpar_kernel(const RegArgs a) {
+    __shared__ __align__(16) JparI<IB> S;
+    const int i0 = blockIdx.x * IB, nvalid = min(IB, a.ni - i0);
+    jpar_fetch_i<IB>(a, S, 0, i0, nvalid);
+    jpar_fetch_wait();
+    jpar_stage_i<IB, X2>(S, 0, nvalid);
+    __syncthreads();
+    const int j_begin = (int)(((long long)blockIdx.y * a.nj) / a.nslices);
+    const int j_end = (int)(((long long)(blockIdx.y + 1) * a.nj) / a.nslices);
+    Sums s[IB];
+    jpar_loop<IB, MFLAG, X2>(a, S, 0, j_begin, j_end, i0, nvalid, 0, s);
+    jpar_reduce<IB>(S, s);
+    jpar_partials<IB>(S, a.part, nvalid, [&](int k) { return (size_t)blockIdx.y * a.ni_pad + i0 + k; });
 }
 
 // One warp per i: FP64 sum over slices in a fixed order, then the neighbour
@@ -1323,29 +1390,61 @@ __global__ void __launch_bounds__(FIN_WARPS * 32)
 // i writes its (hi, lo) partial to slot pinfo[i].x + q; regf_finalize_seg
 // sums the pinfo[i].y slots of each i in order.
 // ----------------------------------------------------------------------------
+//
+// A group whose j range is one item (Q = 1, nearly all groups of an ensemble)
+// is finished by its CTA: sums, list rows and their way over the bus then
+// overlap the other items.  As a launch of its own after this one the rows of
+// 19,046 bodies (6 MB of pinned memory) took a quarter of the call.  The next
+// item and its i data, which are read from the caller's staging over the bus,
+// are fetched during this one.
 struct SegItem {
-    int i0, ni, j0, j1, jbase, q, pad0, pad1;
+    int i0, ni, j0, j1, jbase, q, Q, slot;   // slot: of the group's first particle
 };
 
 template <int IB, bool MFLAG, bool X2 = false>
-__global__ void __launch_bounds__(JPAR_NT, 2)
-    regf_seg_kernel(const RegArgs a, const SegItem *__restrict__ items, const int *__restrict__ nitems_p,
-                    const int2 *__restrict__ pinfo) {
+__global__ void __launch_bounds__(JPAR_NT, JPAR_CTAS)
+    regf_seg_kernel(const RegArgs a, const SegItem *__restrict__ items, int nitems, const RowOut ro) {
     __shared__ __align__(16) JparI<IB> S;
-    const int nitems = *nitems_p;
-    for (int w = blockIdx.x; w < nitems; w += gridDim.x) {
-        const SegItem it = items[w];
-        __syncthreads();  // the previous item is done with the staged i and red
-        jpar_stage_i<IB, X2>(a, S, it.i0, it.ni);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    int w = blockIdx.x;
+    SegItem it = items[w];   // (the grid is no larger than the list)
+    jpar_fetch_i<IB>(a, S, 0, it.i0, it.ni);
+    for (int buf = 0;; buf ^= 1) {
+        const int wn = w + gridDim.x;
+        SegItem nx = it;
+        if (wn < nitems) nx = items[wn];
+        jpar_fetch_wait();   // (and the previous item is done with the staged i and red)
+        jpar_stage_i<IB, X2>(S, buf, it.ni);
+        if (wn < nitems) jpar_fetch_i<IB>(a, S, buf ^ 1, nx.i0, nx.ni);
         __syncthreads();
         Sums s[IB];
-        jpar_loop<IB, MFLAG, X2>(a, S, it.j0, it.j1, it.i0, it.ni, it.jbase, s);
-        jpar_reduce<IB>(S, s, a.part, it.ni, [&](int k) { return (size_t)pinfo[it.i0 + k].x + it.q; });
+        jpar_loop<IB, MFLAG, X2>(a, S, buf, it.j0, it.j1, it.i0, it.ni, it.jbase, s);
+        jpar_reduce<IB>(S, s);
+        if (ro.outf && it.Q == 1) {
+            if (tid < 8 * IB && (tid >> 3) < it.ni) {
+                const int k = tid >> 3, c = tid & 7;
+                const double v = c < 7 ? jpar_total(S, 7 * k + c) : 0.0;
+                ro.outf[(size_t)(it.i0 + k) * 8 + c] = v * (c < 6 ? 0.125 : 0.5);
+            }
+            for (int k = warp; k < it.ni; k += JPAR_NT / 32) {
+                const int i = it.i0 + k, n = __ldcg(a.nbcnt + i);
+                __syncwarp();
+                if (lane == 0) a.nbcnt[i] = 0;
+                write_list_row(i, lane, n, a.nbbuf, a.lcap, ro.cap, ro.ls, nullptr, ro.outl);
+            }
+        } else {
+            jpar_partials<IB>(S, a.part, it.ni, [&](int k) { return (size_t)it.slot + (size_t)k * it.Q + it.q; });
+        }
+        if (wn >= nitems) break;
+        w = wn;
+        it = nx;
     }
+    if (ro.hstatus && blockIdx.x == 0 && tid == 0) *ro.hstatus = *a.status;
 }
 
 __global__ void __launch_bounds__(FIN_WARPS * 32)
-    regf_finalize_seg(const float4 *__restrict__ part, const int2 *__restrict__ pinfo, int ni,
+    regf_finalize_seg(const float4 *__restrict__ part, const int2 *__restrict__ pinfo, bool all_one, bool one_done,
+                      int ni,
                       int *__restrict__ nbcnt, const int *__restrict__ nbbuf, int lcap, int cap, int ls,
                       int pmax, double *__restrict__ outf, int *__restrict__ outl, const int *status,
                       int *hstatus, const MlpArgs mlp) {
@@ -1360,7 +1459,10 @@ __global__ void __launch_bounds__(FIN_WARPS * 32)
     const int lane = threadIdx.x & 31;
     const int i = blockIdx.x * FIN_WARPS + warp;
     if (i >= ni) return;
-    const int2 pi = pinfo[i];
+    // all_one: one partial per particle, slots in order; one_done: rows of one
+    // partial were finished by the force kernel
+    const int2 pi = all_one ? make_int2(i, 1) : pinfo[i];
+    if (one_done && pi.y == 1) return;
     double v[7] = {0, 0, 0, 0, 0, 0, 0};
     for (int q = lane; q < pi.y; q += 32) add_partial(part + ((size_t)pi.x + q) * 4, v);
     finalize_row(i, lane, v, nbcnt, nbbuf, lcap, cap, ls, sbuf + warp * pmax, outf, outl, mlp, sw);
@@ -2009,16 +2111,19 @@ struct FinArgs {
 
 // The neighbour counters of ni rows.  A new buffer is cleared over its
 // whole capacity: the kernels count into rows [0, ni) of every call and
-// regf_finalize resets the rows it reads, so rows beyond the calls so far
-// must start at zero too (a later, larger call reads them without a
-// clear).  Returns whether the buffer was replaced.
-static bool nbcnt_reserve(int ni, cudaStream_t st) {
+// reset the rows they have read, so rows beyond the calls so far must start
+// at zero too (a later, larger call reads them without a clear).
+static void nbcnt_reserve(int ni, cudaStream_t st) {
     const int *before = R.nbcnt.ptr;
     const size_t cap_before = R.nbcnt.cap;
     R.nbcnt.reserve(ni);
-    if (R.nbcnt.ptr == before && R.nbcnt.cap == cap_before) return false;
+    if (R.nbcnt.ptr == before && R.nbcnt.cap == cap_before) return;
     NB6_CUDA_CHECK(cudaMemsetAsync(R.nbcnt.ptr, 0, sizeof(int) * R.nbcnt.cap, st));
-    return true;
+}
+
+// Clear them all, after a call that may have left some counted.
+static void nbcnt_clear(cudaStream_t st) {
+    NB6_CUDA_CHECK(cudaMemsetAsync(R.nbcnt.ptr, 0, sizeof(int) * R.nbcnt.cap, st));
 }
 
 // Arguments of regf_stage, addressable for a kernel node.
@@ -2270,7 +2375,7 @@ static void regf_copy_out(const RegLaunch &L, cudaStream_t st) {
 
 static void regf_eager(const RegLaunch &L, cudaStream_t st) {
     regf_stage_launch(L, st);
-    NB6_CUDA_CHECK(cudaMemsetAsync(R.nbcnt.ptr, 0, sizeof(int) * (R.nbcnt_dirty ? R.nbcnt.cap : (size_t)L.ni), st));
+    if (R.nbcnt_dirty) nbcnt_clear(st);
     // kernel-only timing of the main force kernel (read by
     // nb6_regf_last_kernel_ms_ after the stream has drained)
     NB6_CUDA_CHECK(cudaEventRecord(R.ev0, st));
@@ -2351,8 +2456,7 @@ static bool graph_build(RegState::Graph &G, const RegLaunch &L) {
 }
 
 static bool graph_update(RegState::Graph &G, const RegLaunch &L) {
-    const bool io = L.hin != nullptr;
-    if (io) {
+    if (L.hin) {
         StageArgs g(L);
         const cudaKernelNodeParams ks = stage_node(g);
         NB6_GRAPH_TRY(cudaGraphExecKernelNodeSetParams(G.x, G.kstage, &ks));
@@ -2396,7 +2500,7 @@ static void regf_submit(const RegLaunch &L, cudaStream_t st) {
     if (ok) {
         // (a call that failed or the tuner's trials may have left any row
         // counted: clear them all)
-        if (R.nbcnt_dirty) NB6_CUDA_CHECK(cudaMemsetAsync(R.nbcnt.ptr, 0, sizeof(int) * R.nbcnt.cap, st));
+        if (R.nbcnt_dirty) nbcnt_clear(st);
         ok = cudaGraphLaunch(G.x, st) == cudaSuccess;
     }
     if (!ok) {
@@ -2712,21 +2816,21 @@ static int seg_occupancy(int ib, bool mf) {
 }
 
 template <int IB, bool MF>
-static void launch_seg_t(int grid, const RegArgs &a, const SegItem *items, const int *nit,
-                         const int2 *pinfo, cudaStream_t st) {
-    if (IB > 1 && jpar_x2()) regf_seg_kernel<IB, MF, true><<<grid, JPAR_NT, 0, st>>>(a, items, nit, pinfo);
-    else regf_seg_kernel<IB, MF><<<grid, JPAR_NT, 0, st>>>(a, items, nit, pinfo);
+static void launch_seg_t(int grid, const RegArgs &a, const SegItem *items, int nitems, const RowOut &ro,
+                         cudaStream_t st) {
+    if (IB > 1 && jpar_x2()) regf_seg_kernel<IB, MF, true><<<grid, JPAR_NT, 0, st>>>(a, items, nitems, ro);
+    else regf_seg_kernel<IB, MF><<<grid, JPAR_NT, 0, st>>>(a, items, nitems, ro);
 }
 
-static void launch_seg(int ib, bool mf, int grid, const RegArgs &a, const SegItem *items, const int *nit,
-                       const int2 *pinfo, cudaStream_t st) {
+static void launch_seg(int ib, bool mf, int grid, const RegArgs &a, const SegItem *items, int nitems,
+                       const RowOut &ro, cudaStream_t st) {
     switch (ib * 2 + (mf ? 1 : 0)) {
-        case 2: launch_seg_t<1, false>(grid, a, items, nit, pinfo, st); break;
-        case 3: launch_seg_t<1, true>(grid, a, items, nit, pinfo, st); break;
-        case 4: launch_seg_t<2, false>(grid, a, items, nit, pinfo, st); break;
-        case 5: launch_seg_t<2, true>(grid, a, items, nit, pinfo, st); break;
-        case 8: launch_seg_t<4, false>(grid, a, items, nit, pinfo, st); break;
-        default: launch_seg_t<4, true>(grid, a, items, nit, pinfo, st); break;
+        case 2: launch_seg_t<1, false>(grid, a, items, nitems, ro, st); break;
+        case 3: launch_seg_t<1, true>(grid, a, items, nitems, ro, st); break;
+        case 4: launch_seg_t<2, false>(grid, a, items, nitems, ro, st); break;
+        case 5: launch_seg_t<2, true>(grid, a, items, nitems, ro, st); break;
+        case 8: launch_seg_t<4, false>(grid, a, items, nitems, ro, st); break;
+        default: launch_seg_t<4, true>(grid, a, items, nitems, ro, st); break;
     }
 }
 
@@ -2892,55 +2996,59 @@ void nb6_regf_seg_(int *ni_, int *iseg, double *h2, double *dtr, double (*xi)[3]
         work += (double)(run_k0[r + 1] - run_k0[r]) * (seg_j0[run_c[r] + 1] - seg_j0[run_c[r]]);
     R.numInter += (long long)work;
     // items of about a quarter wave's share of the work each, at least 4 j
-    // per thread
+    // per thread, the runs whose items are longest first
     const double wt = std::max(work / (4.0 * grid_max), (double)ib * JPAR_NT * 4);
-    std::vector<SegItem> items;
-    std::vector<int2> pinfo(ni);
+    struct Run {
+        int k0, k1, j0, nc, Q, slot;
+        long long cost;
+    };
+    std::vector<Run> runs(nrun);
     long long slots = 0;
+    size_t nitems_z = 0;
+    bool all_one = true;   // every group's j range is one item
     for (int r = 0; r < nrun; ++r) {
-        const int c = run_c[r], k0 = run_k0[r], k1 = run_k0[r + 1];
-        const int j0 = seg_j0[c], nc = seg_j0[c + 1] - seg_j0[c];
-        const int g = std::min(ib, k1 - k0);
-        int Q = 0;
-        if (nc > 0) {
-            const int qmax = (nc + JPAR_NT * 4 - 1) / (JPAR_NT * 4);
-            Q = std::max(1, std::min(qmax, (int)std::ceil((double)g * nc / wt)));
+        Run &u = runs[r];
+        u.k0 = run_k0[r];
+        u.k1 = run_k0[r + 1];
+        u.j0 = seg_j0[run_c[r]];
+        u.nc = seg_j0[run_c[r] + 1] - u.j0;
+        const int g = std::min(ib, u.k1 - u.k0);
+        u.Q = 0;
+        if (u.nc > 0) {
+            const int qmax = (u.nc + JPAR_NT * 4 - 1) / (JPAR_NT * 4);
+            u.Q = std::max(1, std::min(qmax, (int)std::ceil((double)g * u.nc / wt)));
         }
-        for (int k = k0; k < k1; ++k) pinfo[k] = make_int2((int)(slots + (long long)(k - k0) * Q), Q);
-        slots += (long long)(k1 - k0) * Q;
-        for (int i0 = k0; i0 < k1; i0 += ib)
-            for (int q = 0; q < Q; ++q) {
-                SegItem it;
-                it.i0 = i0;
-                it.ni = std::min(ib, k1 - i0);
-                it.j0 = j0 + (int)((long long)nc * q / Q);
-                it.j1 = j0 + (int)((long long)nc * (q + 1) / Q);
-                it.jbase = j0;
-                it.q = q;
-                it.pad0 = it.pad1 = 0;
-                items.push_back(it);
-            }
+        u.slot = (int)slots;
+        u.cost = u.Q ? (long long)g * u.nc / u.Q : 0;
+        slots += (long long)(u.k1 - u.k0) * u.Q;
+        nitems_z += (size_t)((u.k1 - u.k0 + ib - 1) / ib) * u.Q;
+        all_one &= u.Q == 1;
+        if (slots > INT_MAX / 4) {
+            fprintf(stderr, "nb6_regf_seg: too many partial slots (%lld)\n", slots);
+            nb6_fatal(NB6_ERR_TOO_LARGE);
+            return;
+        }
     }
-    std::stable_sort(items.begin(), items.end(), [](const SegItem &x, const SegItem &y) {
-        return (long long)x.ni * (x.j1 - x.j0) > (long long)y.ni * (y.j1 - y.j0);
-    });
-    const int nitems = (int)items.size();
-    if (slots > INT_MAX / 4) {
-        fprintf(stderr, "nb6_regf_seg: too many partial slots (%lld)\n", slots);
-        nb6_fatal(NB6_ERR_TOO_LARGE);
-        return;
+    std::stable_sort(runs.begin(), runs.end(), [](const Run &x, const Run &y) { return x.cost > y.cost; });
+    const int nitems = (int)nitems_z;
+    // int staging: [items (8 ints each) | pinfo (2 ints per particle: first
+    // slot and number of partials, for regf_finalize_seg)]
+    const size_t nint = (size_t)8 * nitems + (all_one ? 0 : (size_t)2 * ni);
+    R.hseg.reserve(std::max<size_t>(nint, 8));
+    R.dseg.reserve(std::max<size_t>(nint, 8));
+    SegItem *hit = reinterpret_cast<SegItem *>(R.hseg.ptr);
+    int2 *hpi = reinterpret_cast<int2 *>(R.hseg.ptr + (size_t)8 * nitems);
+    for (const Run &u : runs) {
+        for (int i0 = u.k0; i0 < u.k1; i0 += ib)
+            for (int q = 0; q < u.Q; ++q)
+                *hit++ = SegItem{i0, std::min(ib, u.k1 - i0), u.j0 + (int)((long long)u.nc * q / u.Q),
+                                 u.j0 + (int)((long long)u.nc * (q + 1) / u.Q), u.j0, q, u.Q,
+                                 u.slot + (i0 - u.k0) * u.Q};
+        if (!all_one)
+            for (int k = u.k0; k < u.k1; ++k) hpi[k] = make_int2(u.slot + (k - u.k0) * u.Q, u.Q);
     }
-    // int staging: [nitems, 0, 0, 0 | items (8 ints each) | pinfo (2 ints each)]
-    const size_t nint = 4 + (size_t)8 * nitems + (size_t)2 * ni;
-    R.hseg.reserve(nint);
-    R.dseg.reserve(nint);
-    int *hs = R.hseg.ptr;
-    hs[0] = nitems;
-    hs[1] = hs[2] = hs[3] = 0;
-    if (nitems) memcpy(hs + 4, items.data(), sizeof(SegItem) * nitems);
-    memcpy(hs + 4 + (size_t)8 * nitems, pinfo.data(), sizeof(int2) * ni);
-    const SegItem *d_items = reinterpret_cast<const SegItem *>(R.dseg.ptr + 4);
-    const int2 *d_pinfo = reinterpret_cast<const int2 *>(R.dseg.ptr + 4 + (size_t)8 * nitems);
+    const SegItem *d_items = reinterpret_cast<const SegItem *>(R.dseg.ptr);
+    const int2 *d_pinfo = reinterpret_cast<const int2 *>(R.dseg.ptr + (size_t)8 * nitems);
 
     R.part.reserve((size_t)std::max<long long>(slots, 1) * 4);
     nbcnt_reserve(ni, st);
@@ -2966,7 +3074,9 @@ void nb6_regf_seg_(int *ni_, int *iseg, double *h2, double *dtr, double (*xi)[3]
     a.nj = R.nj;
     a.ntile = R.ntile;
     a.nslices = 1;
-    const double *d = R.iin.ptr;
+    // the items fetch their i data from the staging itself, each word once or
+    // (Q > 1) a few times
+    const double *d = nb6_uva() ? h : R.iin.ptr;
     a.ih2 = d;
     a.idtr = d + ni;
     a.ix = d + 2 * (size_t)ni;
@@ -2984,32 +3094,47 @@ void nb6_regf_seg_(int *ni_, int *iseg, double *h2, double *dtr, double (*xi)[3]
     const double t_prep = nb6_wtime();
     R.time_out += t_prep - t_start;
     R.time_grav -= t_prep;
-    NB6_CUDA_CHECK(cudaMemcpyAsync(R.iin.ptr, h, sizeof(double) * nin, cudaMemcpyHostToDevice, st));
-    NB6_CUDA_CHECK(cudaMemcpyAsync(R.dseg.ptr, hs, sizeof(int) * nint, cudaMemcpyHostToDevice, st));
-    NB6_CUDA_CHECK(cudaMemsetAsync(R.nbcnt.ptr, 0, sizeof(int) * ni, st));
+    if (!nb6_uva())
+        NB6_CUDA_CHECK(cudaMemcpyAsync(R.iin.ptr, h, sizeof(double) * nin, cudaMemcpyHostToDevice, st));
+    if (nint) NB6_CUDA_CHECK(cudaMemcpyAsync(R.dseg.ptr, R.hseg.ptr, sizeof(int) * nint, cudaMemcpyHostToDevice, st));
+    if (R.nbcnt_dirty) nbcnt_clear(st);
+    // rows go to the pinned host staging in place, unless a device kernel
+    // consumes the results (regular_seg_on_device)
+    const bool direct = nb6_uva() && !g_seg_keep_device;
+    const int ls = direct ? host_row_stride(W) : W;
+    double *outf = direct ? R.houtf.ptr : R.outf.ptr;
+    int *outl = direct ? R.houtl.ptr : R.outl.ptr;
+    int *hstatus = direct ? nb6_status_post() : nullptr;
+    const MlpArgs mlp = nb6_mlp_args(a.ih2, a.idtr);
+    // groups of one item finish their rows in the kernel (no rows longer than
+    // it sorts in registers, no proposals); the finalize launch takes the others
+    RowOut ro;
+    if (cap <= 32 * ROW_REGS && !mlp.on) {
+        ro.outf = outf;
+        ro.outl = outl;
+        ro.ls = ls;
+        ro.cap = cap;
+        ro.hstatus = hstatus;
+    }
     NB6_CUDA_CHECK(cudaEventRecord(R.ev0, st));
-    if (nitems > 0)
-        launch_seg(ib, mf, std::min(nitems, grid_max), a, d_items, R.dseg.ptr, d_pinfo, st);
+    if (nitems > 0) launch_seg(ib, mf, std::min(nitems, grid_max), a, d_items, nitems, ro, st);
     NB6_CUDA_CHECK(cudaGetLastError());
     NB6_CUDA_CHECK(cudaEventRecord(R.ev1, st));
     R.last_geometry[0] = -ib;
     R.last_geometry[1] = std::min(nitems, grid_max);
     R.last_geometry[2] = nitems;
-    const int pmax = sort_words(cap);
-    const MlpArgs mlp = nb6_mlp_args(a.ih2, a.idtr);
-    const size_t smem = (size_t)FIN_WARPS * pmax * sizeof(int) + (mlp.on ? MLP_SMEM_BYTES : 0);
-    if (smem > 48 * 1024)
-        NB6_CUDA_CHECK(cudaFuncSetAttribute(regf_finalize_seg, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                            (int)smem));
-    // finalize writes the pinned host staging in place, unless a device
-    // kernel consumes the results (regular_seg_on_device)
-    const bool direct = nb6_uva() && !g_seg_keep_device;
-    const int ls = direct ? host_row_stride(W) : W;
-    regf_finalize_seg<<<(ni + FIN_WARPS - 1) / FIN_WARPS, FIN_WARPS * 32, smem, st>>>(
-        R.part.ptr, d_pinfo, ni, R.nbcnt.ptr, R.nbbuf.ptr, a.lcap, cap, ls, pmax,
-        direct ? R.houtf.ptr : R.outf.ptr, direct ? R.houtl.ptr : R.outl.ptr, a.status,
-        direct ? nb6_status_post() : nullptr, mlp);
-    NB6_CUDA_CHECK(cudaGetLastError());
+    if (!(all_one && ro.outf)) {
+        const int pmax = sort_words(cap);
+        const size_t smem = (size_t)FIN_WARPS * pmax * sizeof(int) + (mlp.on ? MLP_SMEM_BYTES : 0);
+        if (smem > 48 * 1024)
+            NB6_CUDA_CHECK(cudaFuncSetAttribute(regf_finalize_seg, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                (int)smem));
+        regf_finalize_seg<<<(ni + FIN_WARPS - 1) / FIN_WARPS, FIN_WARPS * 32, smem, st>>>(
+            R.part.ptr, d_pinfo, all_one, ro.outf != nullptr, ni, R.nbcnt.ptr, R.nbbuf.ptr, a.lcap, cap, ls, pmax,
+            outf, outl, a.status, hstatus, mlp);
+        NB6_CUDA_CHECK(cudaGetLastError());
+    }
+    R.nbcnt_dirty = false;
     if (g_seg_keep_device) {
         R.time_grav += nb6_wtime();
         return;
@@ -3216,7 +3341,7 @@ constexpr size_t NB6_NOALLOC_SCRATCH_BYTES = 12u << 20;
 constexpr int NA_NIMAX = 1024;
 constexpr int NA_CAPMAX = 511;
 constexpr int NA_SLICES_MAX = 128;
-constexpr int NA_IB = 4;  // i-particles per CTA of the j-parallel kernel
+constexpr int NA_IB = 4, NA_NT = 256;  // i-particles and threads per CTA of the j-parallel kernel
 
 // Layout inside the array: neighbour counters [NA_NIMAX], neighbour ids
 // [NA_NIMAX][NA_CAPMAX], slice partials [NA_SLICES_MAX][NA_NIMAX][4] float4.
@@ -3241,9 +3366,9 @@ __global__ void na_clear_counts(int *cnt, int ni) {
 // (hi/lo split on the fly); pair math, candidate test and exact FP64
 // re-decision are those of the other regular kernels.
 template <bool MFLAG>
-__global__ void __launch_bounds__(JPAR_NT) regf_na_kernel(const RegArgs a) {
+__global__ void __launch_bounds__(NA_NT) regf_na_kernel(const RegArgs a) {
     __shared__ float4 sip[NA_IB][3];
-    __shared__ double red[JPAR_NT / 32][NA_IB][7];
+    __shared__ double red[NA_NT / 32][NA_IB][7];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int i0 = blockIdx.x * NA_IB;
     if (tid < NA_IB) {
@@ -3267,7 +3392,7 @@ __global__ void __launch_bounds__(JPAR_NT) regf_na_kernel(const RegArgs a) {
     Sums s[NA_IB];
 #pragma unroll
     for (int k = 0; k < NA_IB; ++k) zero(s[k]);
-    for (int j = j_begin + tid; j < j_end; j += JPAR_NT) {
+    for (int j = j_begin + tid; j < j_end; j += NA_NT) {
         float4 pa, pb;
         split_hl(a.jx[3 * (size_t)j], pa.x, pb.x);
         split_hl(a.jx[3 * (size_t)j + 1], pa.y, pb.y);
@@ -3289,7 +3414,8 @@ __global__ void __launch_bounds__(JPAR_NT) regf_na_kernel(const RegArgs a) {
         }
         if (any) {
             for (int k = 0; k < NA_IB; ++k)
-                if (reg_geom<MFLAG>(ips[k], pa, pb, pc).cand) reg_exact<MFLAG>(a, i0 + k, j, s[k]);
+                if (reg_geom<MFLAG>(ips[k], pa, pb, pc).cand)
+                    reg_exact<MFLAG>(a, load_iexact(a, i0 + k), i0 + k, j, s[k]);
         }
     }
 #pragma unroll
@@ -3306,7 +3432,7 @@ __global__ void __launch_bounds__(JPAR_NT) regf_na_kernel(const RegArgs a) {
         const int k = tid / 7, c = tid % 7;
         double w = 0.0;
 #pragma unroll
-        for (int q = 0; q < JPAR_NT / 32; ++q) w += red[q][k][c];
+        for (int q = 0; q < NA_NT / 32; ++q) w += red[q][k][c];
         const int i = i0 + k;
         if (i < a.ni) {
             float *p = reinterpret_cast<float *>(a.part + ((size_t)blockIdx.y * a.ni_pad + i) * 4);
@@ -3460,14 +3586,14 @@ void nb6_regf_noalloc_(int *nj_, const double *d_mj, const double *d_xj, const d
     // Two waves of CTAs, and at most 64 j per thread and slice: each
     // thread's FP32 sums then cover as few pairs as a tile of the other
     // kernels before they reach FP64 (up to 2M j within NA_SLICES_MAX).
-    const int by_waves = std::min(2 * sms / igroups, nj / (JPAR_NT * 4));
-    const int by_sums = (int)(((long long)nj + JPAR_NT * 64 - 1) / (JPAR_NT * 64));
+    const int by_waves = std::min(2 * sms / igroups, nj / (NA_NT * 4));
+    const int by_sums = (int)(((long long)nj + NA_NT * 64 - 1) / (NA_NT * 64));
     a.nslices = std::max(1, std::min(std::max(by_waves, by_sums), NA_SLICES_MAX));
 
     na_clear_counts<<<(ni + 255) / 256, 256, 0, st>>>(a.nbcnt, ni);
     dim3 grid(igroups, a.nslices);
-    if (*m_flag) regf_na_kernel<true><<<grid, JPAR_NT, 0, st>>>(a);
-    else regf_na_kernel<false><<<grid, JPAR_NT, 0, st>>>(a);
+    if (*m_flag) regf_na_kernel<true><<<grid, NA_NT, 0, st>>>(a);
+    else regf_na_kernel<false><<<grid, NA_NT, 0, st>>>(a);
     regf_na_finalize<<<(ni + FIN_WARPS - 1) / FIN_WARPS, FIN_WARPS * 32, 0, st>>>(
         a.part, a.nslices, ni, a.nbcnt, a.nbbuf, a.lcap, cap, lmax, d_acc, d_jrk, d_pot, d_list);
     const cudaError_t e = cudaGetLastError();
