@@ -916,7 +916,9 @@ __global__ void __launch_bounds__(NT, X2_MINB / NI) regf_x2_kernel(const RegArgs
 // busy even for ni = 1.  Same pair math, candidate test and exact FP64 rare
 // path as regf_kernel; the per-thread FP32 partials are reduced over the CTA
 // in FP64 and written as (hi, lo) slice partials for regf_finalize.
-constexpr int JPAR_NT = 256, JPAR_CTAS = 512 / JPAR_NT;   // 16 warps per SM
+// (Four warps per CTA: with eight the segmented kernel's warps waited at its
+// barriers for a fifth of their time, 308 us against 278 for 64 clusters.)
+constexpr int JPAR_NT = 128, JPAR_CTAS = 512 / JPAR_NT;   // 16 warps per SM
 
 // The i-particles of a j-parallel CTA in shared memory: sip[k] = (xH, yH, zH,
 // 1.01 h2), (xL, yL, zL, dtr), (vx, vy, vz, 0) of particle k, and, for the
