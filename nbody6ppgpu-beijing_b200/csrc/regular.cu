@@ -1333,6 +1333,12 @@ struct RowOut {
     int *outl = nullptr;      // [ni][ls]
     int ls = 0, cap = 0;
     int *hstatus = nullptr;
+    // Progress for a host that unpacks the rows meanwhile: a CTA's items are
+    // rounds 0, 1, ... of the launch, stage_rounds of them a stage; the last CTA
+    // to finish stage s resets stage_done[s] and sets stage_flag[s] (pinned).
+    // stage_rounds = 0: none.
+    int stage_rounds = 0;
+    int *stage_done = nullptr, *stage_flag = nullptr;
 };
 
 // (IB = 8 keeps 56 sums: half the warps per SM.)
@@ -1398,7 +1404,8 @@ __global__ void __launch_bounds__(FIN_WARPS * 32)
 // overlap the other items.  As a launch of its own after this one the rows of
 // 19,046 bodies (6 MB of pinned memory) took a quarter of the call.  The next
 // item and its i data, which are read from the caller's staging over the bus,
-// are fetched during this one.
+// are fetched during this one.  The host copies the finished rows of a stage
+// into the caller's arrays while the next one computes.
 struct SegItem {
     int i0, ni, j0, j1, jbase, q, Q, slot;   // slot: of the group's first particle
 };
@@ -1408,14 +1415,26 @@ __global__ void __launch_bounds__(JPAR_NT, JPAR_CTAS)
     regf_seg_kernel(const RegArgs a, const SegItem *__restrict__ items, int nitems, const RowOut ro) {
     __shared__ __align__(16) JparI<IB> S;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    int w = blockIdx.x;
+    int w = blockIdx.x, round = 0;
     SegItem it = items[w];   // (the grid is no larger than the list)
     jpar_fetch_i<IB>(a, S, 0, it.i0, it.ni);
-    for (int buf = 0;; buf ^= 1) {
+    int ready = -1;          // the stage whose last item this CTA has just finished
+    auto post_stage = [&]() {   // (thread 0, after a barrier behind the rows' stores)
+        if (ready < 0) return;
+        const int ctas = min((int)gridDim.x, nitems - ready * ro.stage_rounds * (int)gridDim.x);
+        __threadfence_system();
+        if (atomicAdd(ro.stage_done + ready, 1) == ctas - 1) {
+            ro.stage_done[ready] = 0;
+            __threadfence_system();
+            *(volatile int *)(ro.stage_flag + ready) = 1;
+        }
+    };
+    for (int buf = 0;; buf ^= 1, ++round) {
         const int wn = w + gridDim.x;
         SegItem nx = it;
         if (wn < nitems) nx = items[wn];
         jpar_fetch_wait();   // (and the previous item is done with the staged i and red)
+        if (tid == 0) post_stage();
         jpar_stage_i<IB, X2>(S, buf, it.ni);
         if (wn < nitems) jpar_fetch_i<IB>(a, S, buf ^ 1, nx.i0, nx.ni);
         __syncthreads();
@@ -1437,9 +1456,16 @@ __global__ void __launch_bounds__(JPAR_NT, JPAR_CTAS)
         } else {
             jpar_partials<IB>(S, a.part, it.ni, [&](int k) { return (size_t)it.slot + (size_t)k * it.Q + it.q; });
         }
+        ready = ro.stage_rounds > 0 && ((round + 1) % ro.stage_rounds == 0 || wn >= nitems)
+                    ? round / ro.stage_rounds
+                    : -1;
         if (wn >= nitems) break;
         w = wn;
         it = nx;
+    }
+    if (ro.stage_rounds > 0) {
+        __syncthreads();
+        if (tid == 0) post_stage();
     }
     if (ro.hstatus && blockIdx.x == 0 && tid == 0) *ro.hstatus = *a.status;
 }
@@ -1516,6 +1542,10 @@ struct TuneKey {
     }
 };
 
+// Stages of a segmented host call: rows of one are copied to the caller while
+// the next computes.
+constexpr int SEG_STAGES = 8;
+
 struct RegState {
     bool open = false;
     int nbodymax = 0;
@@ -1561,6 +1591,8 @@ struct RegState {
     // segmented calls: work list and per-i partial slots, staged as ints
     HostBuf<int> hseg;
     DevBuf<int> dseg;
+    DevBuf<int> stage_done;    // see RowOut
+    HostBuf<int> stage_flag;
     // spatially ordered copy of the j set (see jset_keys)
     int use_jsort = -1;                // -1 = read NB6_JSORT on first use
     long long jver = 0, sorted_ver = -1;
@@ -2126,6 +2158,7 @@ static void nbcnt_reserve(int ni, cudaStream_t st) {
 // Clear them all, after a call that may have left some counted.
 static void nbcnt_clear(cudaStream_t st) {
     NB6_CUDA_CHECK(cudaMemsetAsync(R.nbcnt.ptr, 0, sizeof(int) * R.nbcnt.cap, st));
+    if (R.stage_done.ptr) NB6_CUDA_CHECK(cudaMemsetAsync(R.stage_done.ptr, 0, sizeof(int) * SEG_STAGES, st));
 }
 
 // Arguments of regf_stage, addressable for a kernel node.
@@ -2583,6 +2616,8 @@ void gpunb_close_() {
     R.outf.release();
     R.outl.release();
     R.hin.release();
+    R.stage_done.release();
+    R.stage_flag.release();
     R.houtf.release();
     R.houtl.release();
     R.nbodymax = 0;
@@ -2795,6 +2830,21 @@ static void selfcheck_rows(int ni, const double *h2, const double *dtr, const do
 // Set while regular_seg_on_device runs nb6_regf_seg_: results stay in the
 // device buffers and nothing is synchronised or unpacked.
 static bool g_seg_keep_device = false;
+
+// Wait until the running work of `st` sets *flag; false when the stream has
+// drained (or failed) without it.
+static bool wait_flag(const int *flag, cudaStream_t st) {
+    const volatile int *f = flag;
+    for (unsigned spin = 1; *f == 0; ++spin) {
+        NB6_CPU_PAUSE();
+        if ((spin & 2047u) == 0 && cudaStreamQuery(st) != cudaErrorNotReady) {
+            std::atomic_thread_fence(std::memory_order_acquire);
+            return *f != 0;
+        }
+    }
+    std::atomic_thread_fence(std::memory_order_acquire);
+    return true;
+}
 
 template <bool MF> static const void *seg_kernel_of(int ib) {
     switch (ib) {
@@ -3118,12 +3168,25 @@ void nb6_regf_seg_(int *ni_, int *iseg, double *h2, double *dtr, double (*xi)[3]
         ro.cap = cap;
         ro.hstatus = hstatus;
     }
+    // a host call of many rounds in stages (every row finished by the kernel)
+    const int grid = std::min(nitems, grid_max), rounds = grid ? (nitems + grid - 1) / grid : 0;
+    if (ro.outf && all_one && direct && rounds >= SEG_STAGES) {
+        ro.stage_rounds = (rounds + SEG_STAGES - 1) / SEG_STAGES;
+        if (!R.stage_done.ptr) {
+            R.stage_done.reserve(SEG_STAGES);
+            NB6_CUDA_CHECK(cudaMemsetAsync(R.stage_done.ptr, 0, sizeof(int) * SEG_STAGES, st));
+            R.stage_flag.reserve(SEG_STAGES);
+        }
+        for (int k = 0; k < SEG_STAGES; ++k) R.stage_flag.ptr[k] = 0;
+        ro.stage_done = R.stage_done.ptr;
+        ro.stage_flag = R.stage_flag.ptr;
+    }
     NB6_CUDA_CHECK(cudaEventRecord(R.ev0, st));
-    if (nitems > 0) launch_seg(ib, mf, std::min(nitems, grid_max), a, d_items, nitems, ro, st);
+    if (nitems > 0) launch_seg(ib, mf, grid, a, d_items, nitems, ro, st);
     NB6_CUDA_CHECK(cudaGetLastError());
     NB6_CUDA_CHECK(cudaEventRecord(R.ev1, st));
     R.last_geometry[0] = -ib;
-    R.last_geometry[1] = std::min(nitems, grid_max);
+    R.last_geometry[1] = grid;
     R.last_geometry[2] = nitems;
     if (!(all_one && ro.outf)) {
         const int pmax = sort_words(cap);
@@ -3148,15 +3211,34 @@ void nb6_regf_seg_(int *ni_, int *iseg, double *h2, double *dtr, double (*xi)[3]
                                        cudaMemcpyDeviceToHost, st));
         nb6_status_fetch(st);
     }
+    bool unpacked = false;
+    if (ro.stage_rounds > 0) {
+        CopyPool &pool = nb6_copy_pool();
+        pool.arm();
+        const SegItem *items = reinterpret_cast<const SegItem *>(R.hseg.ptr);
+        const int per = ro.stage_rounds * grid;   // items per stage
+        unpacked = true;
+        for (int lo = 0, sg = 0; lo < nitems && unpacked; lo += per, ++sg) {
+            const int hi = std::min(lo + per, nitems);
+            unpacked = wait_flag(R.stage_flag.ptr + sg, st);
+            if (!unpacked) break;
+            const int np = pool.parts();
+            pool.run([&](int p) {
+                const int b = lo + (int)((long long)(hi - lo) * (p + 1) / np);
+                for (int q = lo + (int)((long long)(hi - lo) * p / np); q < b; ++q)
+                    unpack_rows(items[q].i0, items[q].i0 + items[q].ni, ls, lmax, acc, jrk, pot, list);
+            });
+        }
+    }
     NB6_CUDA_CHECK(cudaStreamSynchronize(st));
     const double wt2 = nb6_wtime();
     R.time_grav += wt2;
     R.time_reduce -= wt2;
-    if (nb6_check_dev_status() != 0) {
+    if (nb6_check_dev_status() != 0) {   // (the caller's arrays may hold part of the results)
         R.nbcnt_dirty = true;
         return;
     }
-    unpack_results(ni, ls, lmax, acc, jrk, pot, list);
+    if (!unpacked) unpack_results(ni, ls, lmax, acc, jrk, pot, list);
     R.time_reduce += nb6_wtime();
 }
 

@@ -184,3 +184,39 @@ def test_irregular_rounds_and_call_sizes(nb6, orc, mode, ni):
     finally:
         nb6.lib.nb6_irr_pv_(C.byref(C.c_int(1)))
         nb6.irr_close(0)
+
+
+@pytest.mark.parametrize("cap", [20, 60, 600])
+def test_segmented_many_items(nb6, orc, cap):
+    """A segmented call of many work items per CTA, whose rows reach the
+    caller in stages while later ones compute: ragged segments, groups of
+    one to four, a lone body, an empty segment in between, rows that
+    overflow (cap 20), rows longer than the kernel sorts itself (cap 600);
+    every row against the oracle of its segment."""
+    rng = np.random.default_rng(cap)
+    ns = np.concatenate([rng.integers(250, 420, 66), [0, 1, 2, 3]])
+    rng.shuffle(ns)
+    j0 = np.concatenate([[0], np.cumsum(ns)]).astype(np.int32)
+    n = int(j0[-1])
+    x, v = rng.normal(size=(n, 3)), 0.3 * rng.normal(size=(n, 3))
+    m = rng.uniform(0.5, 1.5, n) / n
+    iseg = np.repeat(np.arange(len(ns)), ns).astype(np.int32)
+    h2 = rng.uniform(0.2, 0.8, n) ** 2
+    dtr = np.full(n, 2.0 ** -6)
+    nb6.gpunb_open(n, 0)
+    try:
+        nb6.gpunb_send(m, x, v)
+        for _ in range(2):
+            acc, jrk, pot, lst = nb6.regf_seg(h2, dtr, x, v, iseg, j0, cap + 1, cap, 0)
+            for c in range(len(ns)):
+                s = slice(j0[c], j0[c + 1])
+                if ns[c] == 0:
+                    continue
+                oa, oj, op, ol = orc.regf(m[s], x[s], v[s], h2[s], dtr[s], x[s], v[s], cap + 1, cap, 0)
+                np.testing.assert_array_equal(lst[s], ol)
+                ok = (np.abs(oa).sum(1) > 0) & (ol[:, 0] >= 0)
+                if ok.any():
+                    assert rel_err_vec(acc[s][ok], oa[ok]).max() <= 1e-5
+                    assert rel_err_vec(pot[s][ok], op[ok]).max() <= 1e-6
+    finally:
+        nb6.gpunb_close()
