@@ -44,21 +44,13 @@ NB6_DEV void split_hl(double x, float &hi, float &lo) {
     lo = __double2float_rn(x - (double)hi);
 }
 
-// Regular-force j set in HBM, written by the send/predict pack kernels.
-// Two layouts of the same data:
-//   posH/posL/vel  float4 per j: (xH,yH,zH,m), (xL,yL,zL,0), (vx,vy,vz,0) --
-//                  read per j by the j-parallel kernel;
-//   comp           10 float arrays of npad entries, component-major
-//                  (xH,yH,zH,m,xL,yL,zL,vx,vy,vz) -- tiles of it are bulk-copied
-//                  to shared memory so that one LDS.128 yields 4 consecutive j
-//                  of one component, the operand shape of packed f32x2 math.
+// Regular-force j set in HBM, written by the send/predict pack kernels: per j
+// (xH,yH,zH,m), (xL,yL,zL,0), (vx,vy,vz,0), beside the FP64 arrays.  The tile
+// kernels' own layout is made from the FP64 arrays when one of them is to run
+// (jset_tiles), so sets that only the j-parallel kernels see never pay for it.
 // Padding slots (j >= n) are massless and far away: never neighbours.
-constexpr int NB6_NCOMP = 10;
-
 struct JSetOut {
     float4 *posH, *posL, *vel;
-    float *comp;
-    double *compd;  // FP64 positions, component-major (x, y, z) x npad
     size_t npad;
 };
 
@@ -80,22 +72,6 @@ NB6_DEV void write_j(const JSetOut &o, size_t j, bool real, double x0, double x1
     o.posH[j] = h;
     o.posL[j] = l;
     o.vel[j] = v;
-    float *c = o.comp + j;
-    const size_t s = o.npad;
-    c[0] = h.x;
-    c[s] = h.y;
-    c[2 * s] = h.z;
-    c[3 * s] = h.w;
-    c[4 * s] = l.x;
-    c[5 * s] = l.y;
-    c[6 * s] = l.z;
-    c[7 * s] = v.x;
-    c[8 * s] = v.y;
-    c[9 * s] = v.z;
-    double *d = o.compd + j;
-    d[0] = real ? x0 : 1.0e15;
-    d[s] = real ? x1 : 1.0e15;
-    d[2 * s] = real ? x2 : 1.0e15;
 }
 
 // Error-free sum (Knuth TwoSum): s + e == a + b exactly.

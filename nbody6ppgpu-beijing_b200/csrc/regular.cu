@@ -26,8 +26,7 @@
 #include "nb6_common.cuh"
 #include "copy_pool.h"
 #include "mlp.cuh"
-
-#include <cub/device/device_radix_sort.cuh>
+#include "spatial.cuh"
 
 #include <algorithm>
 #include <climits>
@@ -69,9 +68,13 @@ struct RegArgs {
     const float4 *__restrict__ posH;  // (xH, yH, zH, m)
     const float4 *__restrict__ posL;  // (xL, yL, zL, 0)
     const float4 *__restrict__ vel;   // (vx, vy, vz, 0)
-    const float *__restrict__ comp;   // component-major copy (NB6_NCOMP x npad)
-    const double *__restrict__ compd; // FP64 positions, component-major (3 x npad)
-    size_t npad;
+    // tile kernels: [ntile][trows][JT], rows xH, yH, zH, m, xL, yL, zL, vx,
+    // vy, vz and, of an ordered set, xr, yr, zr: positions relative to the
+    // tile's box centre, fl32(x - c), the far-tile operands
+    const float *__restrict__ tiles = nullptr;
+    int trows = 0;
+    // their FP64 form: rows 0-5 x, y, z as doubles, then m, vx, vy, vz
+    const float *__restrict__ tilesd = nullptr;
     const double *__restrict__ jm;    // FP64 copies for the exact recheck
     const double *__restrict__ jx;
     const double *__restrict__ jv;
@@ -95,9 +98,6 @@ struct RegArgs {
     // in the same spatial order, so a warp covers a compact region); null =
     // slot order.  Every index into i data and outputs stays the caller's.
     const int *__restrict__ iperm = nullptr;
-    // ordered j set only: positions relative to their tile's box centre,
-    // fl32(x - c), component-major (3 x npad) -- the far-tile operands
-    const float *__restrict__ comprel = nullptr;
 };
 
 struct IPart {
@@ -388,7 +388,7 @@ __global__ void __launch_bounds__(NT) regf_kernel(const RegArgs a) {
 // Packed variant: two j per instruction in the f32x2 lanes (fma/add/mul.f32x2
 // of sm_100).  Each FP32 add/mul/fma of the pair math processes two pairs per
 // issue slot, which moves the kernel from issue-bound to FMA-pipe-bound.  The
-// j tile sits in shared memory component-major (NB6_NCOMP rows of JT floats),
+// j tile sits in shared memory component-major (ROWS_J rows of JT floats),
 // so one LDS.128 brings four consecutive j of one component.  The arithmetic
 // is the scalar reg_pair's, operation for operation (negated i operands turn
 // subtractions into adds; sums are kept negated), so candidates and results
@@ -555,38 +555,25 @@ NB6_DEV unsigned pair_x2d(const IP2 &ip, double xi, double yi, double zi, double
     return (c0 ? 1u : 0u) | (c1 ? 2u : 0u);
 }
 
-// One tile into a stage of NB6_NCOMP float rows.  FP32 layout: the ten float
-// components.  FP64 layout: x, y, z as doubles in row pairs (0,1) (2,3) (4,5),
-// then m, vx, vy, vz in rows 6..9 -- the same 10*JT*4 bytes.
+// Rows of a tile: of every set, and with the relative positions of an ordered
+// one.  The FP64 layout keeps x, y, z as doubles in row pairs (0,1) (2,3)
+// (4,5), then m, vx, vy, vz in rows 6..9.
+constexpr int ROWS_J = 10, ROWS_ORD = 13;
+
+// One tile, a contiguous block, into a stage by one bulk copy.  (Component
+// rows of the whole set took a copy each, 13 per tile and CTA, issued by a
+// thread of the first warp.)
 template <bool F64DX>
 NB6_DEV void issue_tile_soa(const RegArgs &a, float (*stage)[JT], uint64_t *bar, int tile) {
-    const size_t off = (size_t)tile * JT;
-    // rows 10..12: the tile-relative positions of an ordered j set
-    const bool rel = !F64DX && a.comprel != nullptr;
-    mbar_arrive_expect_tx(bar, (uint32_t)((NB6_NCOMP + (rel ? 3 : 0)) * JT * sizeof(float)));
-    if constexpr (F64DX) {
-#pragma unroll
-        for (int c = 0; c < 3; ++c)
-            bulk_g2s(stage[2 * c], a.compd + (size_t)c * a.npad + off, JT * sizeof(double), bar);
-        bulk_g2s(stage[6], a.comp + (size_t)3 * a.npad + off, JT * sizeof(float), bar);
-#pragma unroll
-        for (int c = 7; c < 10; ++c)
-            bulk_g2s(stage[c], a.comp + (size_t)c * a.npad + off, JT * sizeof(float), bar);
-    } else {
-#pragma unroll
-        for (int c = 0; c < NB6_NCOMP; ++c)
-            bulk_g2s(stage[c], a.comp + (size_t)c * a.npad + off, JT * sizeof(float), bar);
-        if (rel) {
-#pragma unroll
-            for (int c = 0; c < 3; ++c)
-                bulk_g2s(stage[NB6_NCOMP + c], a.comprel + (size_t)c * a.npad + off, JT * sizeof(float), bar);
-        }
-    }
+    const int rows = F64DX ? ROWS_J : a.trows;
+    const uint32_t bytes = (uint32_t)(rows * JT * sizeof(float));
+    mbar_arrive_expect_tx(bar, bytes);
+    bulk_g2s(stage[0], (F64DX ? a.tilesd : a.tiles) + (size_t)tile * (rows * JT), bytes, bar);
 }
 
 template <int NI, bool MFLAG, bool F64DX = false>
 __global__ void __launch_bounds__(NT, X2_MINB / NI) regf_x2_kernel(const RegArgs a) {
-    __shared__ __align__(128) float sj[NSTAGE][NB6_NCOMP + 3][JT];
+    __shared__ __align__(128) float sj[NSTAGE][ROWS_ORD][JT];
     __shared__ __align__(8) uint64_t bar[NSTAGE];
     __shared__ __align__(8) uint64_t ebar[NSTAGE];
     // double-single accumulators, touched once per tile: kept in shared
@@ -733,7 +720,7 @@ __global__ void __launch_bounds__(NT, X2_MINB / NI) regf_x2_kernel(const RegArgs
         bool far = false;
         float2 nxr[NI], nyr[NI], nzr[NI];  // -fl32(x_i - c) of this tile (far path)
         if constexpr (!F64DX && NI == 1) {  // (two i per thread: no registers left for it)
-            if (a.comprel) {
+            if (a.tbox) {
                 const float4 bc = __ldg(&a.tbox[2 * tile]);
                 const float4 bh = __ldg(&a.tbox[2 * tile + 1]);
                 bool f = true;
@@ -761,9 +748,9 @@ __global__ void __launch_bounds__(NT, X2_MINB / NI) regf_x2_kernel(const RegArgs
                     const float4 VX = *reinterpret_cast<const float4 *>(&S[7][q]);
                     const float4 VY = *reinterpret_cast<const float4 *>(&S[8][q]);
                     const float4 VZ = *reinterpret_cast<const float4 *>(&S[9][q]);
-                    const float4 XR = *reinterpret_cast<const float4 *>(&S[NB6_NCOMP][q]);
-                    const float4 YR = *reinterpret_cast<const float4 *>(&S[NB6_NCOMP + 1][q]);
-                    const float4 ZR = *reinterpret_cast<const float4 *>(&S[NB6_NCOMP + 2][q]);
+                    const float4 XR = *reinterpret_cast<const float4 *>(&S[ROWS_J][q]);
+                    const float4 YR = *reinterpret_cast<const float4 *>(&S[ROWS_J + 1][q]);
+                    const float4 ZR = *reinterpret_cast<const float4 *>(&S[ROWS_J + 2][q]);
 #pragma unroll
                     for (int k = 0; k < NI; ++k) {
                         pair_x2_rel<MFLAG>(ip[k], nxr[k], nyr[k], nzr[k], make_float2(XR.x, XR.y),
@@ -1552,8 +1539,6 @@ struct RegState {
     int nj = 0;
     int ntile = 0;
     DevBuf<float4> posH, posL, vel;
-    DevBuf<float> comp;              // NB6_NCOMP x npad, component-major
-    DevBuf<double> compd;            // 3 x npad FP64 positions, component-major
     size_t npad = 0;
     DevBuf<double> jall;             // the bodies in FP64: m, x, v back to back, npad apart
     double *jm = nullptr, *jx = nullptr, *jv = nullptr;
@@ -1593,15 +1578,15 @@ struct RegState {
     DevBuf<int> dseg;
     DevBuf<int> stage_done;    // see RowOut
     HostBuf<int> stage_flag;
-    // spatially ordered copy of the j set (see jset_keys)
+    // the tile kernels' layout (see ensure_tiles), of version tiles_ver of the
+    // set; with its FP64 form once that was asked for
     int use_jsort = -1;                // -1 = read NB6_JSORT on first use
-    long long jver = 0, sorted_ver = -1;
-    DevBuf<float4> posH_s, posL_s, vel_s, tbox;
-    DevBuf<float> comp_s, comprel;  // ordered layout; tile-relative positions (3 x npad)
-    DevBuf<double> compd_s;
-    DevBuf<int> perm, vals_in, iperm;
-    DevBuf<unsigned> keys_in, keys_out, ext;
-    DevBuf<unsigned char> sort_tmp;
+    long long jver = 0, tiles_ver = -1, tilesd_ver = -1;
+    bool tiles_ordered = false;
+    DevBuf<float> tiles, tilesd;
+    DevBuf<float4> tbox;
+    SpatialOrder order;
+    DevBuf<int> iperm;
     // NB6_SELFCHECK=1: host copy of the last send, to re-derive sample rows
     int selfcheck = -1;
     std::vector<double> chk_m, chk_x, chk_v;
@@ -1778,120 +1763,86 @@ int ilog2(int v) {
 // neighbour ids are the caller's.
 // ----------------------------------------------------------------------------
 
-// ext[0..2] = min x, y, z and ext[3..5] = max (order-preserving uints).
-__global__ void jset_extent(int nj, const double *__restrict__ jx, unsigned *__restrict__ ext) {
-    unsigned mn[3] = {0xffffffffu, 0xffffffffu, 0xffffffffu}, mx[3] = {0u, 0u, 0u};
-    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < nj; j += gridDim.x * blockDim.x)
+// One CTA per tile: its rows of the tile layout (RegArgs::tiles, tilesd) from
+// the FP64 bodies, in the sent order or (ORD) in Morton order, then with the
+// tile's box: centre rounded to nearest, half extents, largest speed and mass
+// rounded up, over the hi positions of its real bodies.  Padding slots are
+// massless and far away.  (As a permutation of float layouts, boxes and relative
+// positions in launches of their own: 124 us for 996,147 bodies, now 40.)
+template <bool ORD>
+__global__ void __launch_bounds__(JT) jset_tiles(int nj, const int *__restrict__ perm, const double *__restrict__ m,
+                                                 const double *__restrict__ x, const double *__restrict__ v,
+                                                 float *__restrict__ tiles, float *__restrict__ tilesd,
+                                                 float4 *__restrict__ tbox) {
+    constexpr int ROWS = ORD ? ROWS_ORD : ROWS_J;
+    const int t = threadIdx.x, s = blockIdx.x * JT + t;
+    const bool real = s < nj;
+    double c[3] = {1.0e15, 1.0e15, 1.0e15};
+    float mj = 0.f, w[3] = {0.f, 0.f, 0.f}, h[3];
+    if (real) {
+        const size_t j = ORD ? perm[s] : s;
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
-            const unsigned o = f2ord((float)jx[3 * (size_t)j + k]);
-            mn[k] = min(mn[k], o);
-            mx[k] = max(mx[k], o);
+            c[k] = x[3 * j + k];
+            w[k] = (float)v[3 * j + k];
         }
-#pragma unroll
-    for (int k = 0; k < 3; ++k)
-        for (int o = 16; o > 0; o >>= 1) {
-            mn[k] = min(mn[k], __shfl_xor_sync(0xffffffffu, mn[k], o));
-            mx[k] = max(mx[k], __shfl_xor_sync(0xffffffffu, mx[k], o));
-        }
-    if ((threadIdx.x & 31) == 0)
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            atomicMin(&ext[k], mn[k]);
-            atomicMax(&ext[3 + k], mx[k]);
-        }
-}
-
-
-// 30-bit Morton key of each body on a 1024^3 grid over the extent.
-__global__ void jset_keys(int nj, const double *__restrict__ jx, const unsigned *__restrict__ ext,
-                          unsigned *__restrict__ keys, int *__restrict__ vals) {
-    float lo[3], sc[3];
+        mj = (float)m[j];
+    }
+    float *o = tiles + (size_t)blockIdx.x * (ROWS * JT) + t;
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-        lo[k] = ord2f(ext[k]);
-        const float w = ord2f(ext[3 + k]) - lo[k];
-        sc[k] = w > 0.f ? 1023.99f / w : 0.f;
+        float l;
+        split_hl(c[k], h[k], l);
+        o[k * JT] = h[k];
+        o[(4 + k) * JT] = l;
+        o[(7 + k) * JT] = w[k];
     }
-    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < nj; j += gridDim.x * blockDim.x) {
-        unsigned key = 0;
+    o[3 * JT] = mj;
+    if (tilesd) {
+        float *d = tilesd + (size_t)blockIdx.x * (ROWS_J * JT);
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
-            const float q = ((float)jx[3 * (size_t)j + k] - lo[k]) * sc[k];
-            const unsigned c = q <= 0.f ? 0u : (q >= 1023.f ? 1023u : (unsigned)q);
-            key |= spread10(c) << k;
+            reinterpret_cast<double *>(d)[k * JT + t] = c[k];
+            d[(7 + k) * JT + t] = w[k];
         }
-        keys[j] = key;
-        vals[j] = j;
+        d[6 * JT + t] = mj;
     }
-}
-
-// Ordered copies of the float layouts (slot k <- body perm[k]; padding slots
-// k >= nj are copied in place).
-__global__ void jset_permute(int nj, JSetOut src, JSetOut dst, const int *__restrict__ perm) {
-    const size_t np = src.npad;
-    for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < np; k += (size_t)gridDim.x * blockDim.x) {
-        const size_t o = k < (size_t)nj ? (size_t)perm[k] : k;
-        dst.posH[k] = src.posH[o];
-        dst.posL[k] = src.posL[o];
-        dst.vel[k] = src.vel[o];
+    if constexpr (ORD) {
+        __shared__ unsigned red[JT / 32][8];   // min x, y, z, max x, y, z, speed, mass (order-preserving)
+        __shared__ float sc[3];
+        const float sp = real ? __double2float_ru(sqrt((double)w[0] * w[0] + (double)w[1] * w[1] + (double)w[2] * w[2]))
+                              : 0.f;
+        unsigned u[8];
 #pragma unroll
-        for (int c = 0; c < NB6_NCOMP; ++c) dst.comp[c * np + k] = src.comp[c * np + o];
-#pragma unroll
-        for (int c = 0; c < 3; ++c) dst.compd[c * np + k] = src.compd[c * np + o];
-    }
-}
-
-// One warp per tile: bounding box of the hi positions of its real bodies
-// (centre rounded to nearest, half extent, speeds and masses rounded up).
-__global__ void jset_tile_boxes(int nj, int ntile, const float4 *__restrict__ posH, const float4 *__restrict__ vel,
-                                float4 *__restrict__ tbox) {
-    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    if (warp >= ntile) return;
-    double mn[3] = {1e300, 1e300, 1e300}, mx[3] = {-1e300, -1e300, -1e300}, vm = 0.0, mm = 0.0;
-    for (int q = lane; q < JT; q += 32) {
-        const int k = warp * JT + q;
-        if (k >= nj) break;
-        const float4 p = posH[k], v = vel[k];
-        const double c[3] = {p.x, p.y, p.z};
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-            mn[d] = fmin(mn[d], c[d]);
-            mx[d] = fmax(mx[d], c[d]);
+        for (int k = 0; k < 3; ++k) {
+            u[k] = __reduce_min_sync(0xffffffffu, real ? f2ord(h[k]) : 0xffffffffu);
+            u[3 + k] = __reduce_max_sync(0xffffffffu, real ? f2ord(h[k]) : 0u);
         }
-        vm = fmax(vm, sqrt((double)v.x * v.x + (double)v.y * v.y + (double)v.z * v.z));
-        mm = fmax(mm, (double)p.w);
-    }
+        u[6] = __reduce_max_sync(0xffffffffu, f2ord(sp));
+        u[7] = __reduce_max_sync(0xffffffffu, f2ord(fmaxf(mj, 0.f)));
+        if ((t & 31) == 0)
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-            mn[d] = fmin(mn[d], __shfl_xor_sync(0xffffffffu, mn[d], o));
-            mx[d] = fmax(mx[d], __shfl_xor_sync(0xffffffffu, mx[d], o));
+            for (int k = 0; k < 8; ++k) red[t >> 5][k] = u[k];
+        __syncthreads();
+        if (t < 3) {
+            unsigned a = red[0][t], b = red[0][3 + t];
+            for (int q = 1; q < JT / 32; ++q) {
+                a = min(a, red[q][t]);
+                b = max(b, red[q][3 + t]);
+            }
+            const double lo = ord2f(a), hi = ord2f(b);
+            float *bx = reinterpret_cast<float *>(tbox + 2 * blockIdx.x);
+            sc[t] = __double2float_rn(0.5 * (lo + hi));
+            bx[t] = sc[t];
+            bx[4 + t] = __double2float_ru(0.5 * (hi - lo));
+        } else if (t < 5) {   // bx[3] = largest speed, bx[7] = largest mass
+            unsigned a = red[0][t + 3];
+            for (int q = 1; q < JT / 32; ++q) a = max(a, red[q][t + 3]);
+            reinterpret_cast<float *>(tbox + 2 * blockIdx.x)[t == 3 ? 3 : 7] = ord2f(a);
         }
-        vm = fmax(vm, __shfl_xor_sync(0xffffffffu, vm, o));
-        mm = fmax(mm, __shfl_xor_sync(0xffffffffu, mm, o));
-    }
-    if (lane == 0) {
-        tbox[2 * warp] = make_float4(__double2float_rn(0.5 * (mn[0] + mx[0])), __double2float_rn(0.5 * (mn[1] + mx[1])),
-                                     __double2float_rn(0.5 * (mn[2] + mx[2])), __double2float_ru(vm));
-        tbox[2 * warp + 1] = make_float4(__double2float_ru(0.5 * (mx[0] - mn[0])), __double2float_ru(0.5 * (mx[1] - mn[1])),
-                                         __double2float_ru(0.5 * (mx[2] - mn[2])), __double2float_ru(mm));
-    }
-}
-
-// Tile-relative positions of the ordered j set: xr = fl32(x - c) with c the
-// box centre of the body's tile (an FP32 number, so x - c is formed exactly
-// in FP64 up to one rounding).  Padding slots keep their far-away marker.
-__global__ void jset_rel(int npad, int ntile, const double *__restrict__ compd, const float4 *__restrict__ tbox,
-                         float *__restrict__ comprel) {
-    for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < (size_t)npad;
-         q += (size_t)gridDim.x * blockDim.x) {
-        const int t = (int)(q / JT);
-        const float4 c = t < ntile ? tbox[2 * t] : make_float4(0.f, 0.f, 0.f, 0.f);
-        comprel[q] = __double2float_rn(compd[q] - (double)c.x);
-        comprel[(size_t)npad + q] = __double2float_rn(compd[(size_t)npad + q] - (double)c.y);
-        comprel[2 * (size_t)npad + q] = __double2float_rn(compd[2 * (size_t)npad + q] - (double)c.z);
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < 3; ++k) o[(ROWS_J + k) * JT] = __double2float_rn(c[k] - (double)sc[k]);
     }
 }
 
@@ -1904,13 +1855,7 @@ constexpr int ISORT_MAX = 4096, STAGE_NT = 1024;
 template <int E>
 NB6_DEV void order_active(int ni, const double *__restrict__ ix, const unsigned *__restrict__ ext,
                           int *__restrict__ iperm, unsigned long long *kv) {
-    float lo[3], sc[3];
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        lo[k] = ord2f(ext[k]);
-        const float w = ord2f(ext[3 + k]) - lo[k];
-        sc[k] = w > 0.f ? 1023.99f / w : 0.f;
-    }
+    const KeyGrid grid = key_grid(ext);
     const int tid = threadIdx.x;
     unsigned long long v[E];
 #pragma unroll
@@ -1918,13 +1863,7 @@ NB6_DEV void order_active(int ni, const double *__restrict__ ix, const unsigned 
         const int s = r * STAGE_NT + tid;
         v[r] = ~0ull;  // padding sorts last
         if (s < ni) {
-            unsigned key = 0;
-#pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                const float q = ((float)ix[3 * (size_t)s + k] - lo[k]) * sc[k];
-                const unsigned c = q <= 0.f ? 0u : (q >= 1023.f ? 1023u : (unsigned)q);
-                key |= spread10(c) << k;
-            }
+            const unsigned key = key_of(grid, ix + 3 * (size_t)s);
             v[r] = ((unsigned long long)key << 32) | (unsigned)s;
         }
     }
@@ -2007,8 +1946,6 @@ static JSetOut size_j_buffers(int n) {
     R.posH.reserve(R.npad);
     R.posL.reserve(R.npad);
     R.vel.reserve(R.npad);
-    R.comp.reserve((size_t)NB6_NCOMP * R.npad);
-    R.compd.reserve((size_t)3 * R.npad);
     R.jall.reserve(7 * R.npad);
     R.jm = R.jall.ptr;
     R.jx = R.jm + R.npad;
@@ -2017,62 +1954,42 @@ static JSetOut size_j_buffers(int n) {
     o.posH = R.posH.ptr;
     o.posL = R.posL.ptr;
     o.vel = R.vel.ptr;
-    o.comp = R.comp.ptr;
-    o.compd = R.compd.ptr;
     o.npad = R.npad;
     return o;
 }
 
-// Build (once per j set) the spatially ordered copy used by the tile and
-// j-parallel kernels.  Stream-ordered after the producer's kernels.
-static bool ensure_sorted(cudaStream_t st) {
+// Make (once per j set) the layout the packed tile kernels read, and its FP64
+// form if asked for.  Returns whether it is spatially ordered.
+// Stream-ordered after the producer's kernels.
+static bool ensure_tiles(bool want_d, cudaStream_t st) {
     if (R.use_jsort < 0) {
         const char *e = getenv("NB6_JSORT");
         R.use_jsort = (e && atoi(e) == 0) ? 0 : 1;
     }
-    // small sets: the j-parallel kernel serves them and tiles span the whole
-    // system, so the order would only cost the sort (NB6_JSORT_MIN overrides)
+    // small sets: tiles span the whole system, so the order would only cost
+    // the sort (NB6_JSORT_MIN overrides)
     static const int jsort_min = [] {
         const char *e = getenv("NB6_JSORT_MIN");
         return e ? atoi(e) : 32768;
     }();
-    if (!R.use_jsort || R.nj < 1 || R.nj < jsort_min) return false;
-    if (R.sorted_ver == R.jver) return true;
-    const int nj = R.nj;
-    const size_t np = R.npad;
-    R.posH_s.reserve(np);
-    R.posL_s.reserve(np);
-    R.vel_s.reserve(np);
-    R.comp_s.reserve((size_t)NB6_NCOMP * np);
-    R.compd_s.reserve((size_t)3 * np);
-    R.perm.reserve(nj);
-    R.vals_in.reserve(nj);
-    R.keys_in.reserve(nj);
-    R.keys_out.reserve(nj);
-    R.ext.reserve(6);
-    R.tbox.reserve((size_t)2 * R.ntile);
-    const unsigned init[6] = {0xffffffffu, 0xffffffffu, 0xffffffffu, 0u, 0u, 0u};
-    NB6_CUDA_CHECK(cudaMemcpyAsync(R.ext.ptr, init, sizeof(init), cudaMemcpyHostToDevice, st));
-    const int blocks = std::max(1, std::min((nj + 255) / 256, nb6_num_sms() * 8));
-    jset_extent<<<blocks, 256, 0, st>>>(nj, R.jx, R.ext.ptr);
-    jset_keys<<<blocks, 256, 0, st>>>(nj, R.jx, R.ext.ptr, R.keys_in.ptr, R.vals_in.ptr);
+    const bool ord = R.use_jsort && R.nj >= 1 && R.nj >= jsort_min;
+    if (R.tiles_ver == R.jver && R.tiles_ordered == ord && (!want_d || R.tilesd_ver == R.jver)) return ord;
+    R.tiles.reserve((size_t)R.ntile * (ord ? ROWS_ORD : ROWS_J) * JT);
+    if (want_d) R.tilesd.reserve((size_t)R.ntile * ROWS_J * JT);
+    float *d = want_d ? R.tilesd.ptr : nullptr;
+    if (ord) {
+        if (R.tiles_ver != R.jver || !R.tiles_ordered) R.order.build(R.nj, R.jx, st);
+        R.tbox.reserve((size_t)2 * R.ntile);
+        jset_tiles<true><<<R.ntile, JT, 0, st>>>(R.nj, R.order.perm.ptr, R.jm, R.jx, R.jv, R.tiles.ptr, d,
+                                                 R.tbox.ptr);
+    } else {
+        jset_tiles<false><<<R.ntile, JT, 0, st>>>(R.nj, nullptr, R.jm, R.jx, R.jv, R.tiles.ptr, d, nullptr);
+    }
     NB6_CUDA_CHECK(cudaGetLastError());
-    size_t tmp = 0;
-    NB6_CUDA_CHECK(cub::DeviceRadixSort::SortPairs(nullptr, tmp, R.keys_in.ptr, R.keys_out.ptr, R.vals_in.ptr,
-                                                   R.perm.ptr, nj, 0, 30, st));
-    R.sort_tmp.reserve(tmp + 16);
-    NB6_CUDA_CHECK(cub::DeviceRadixSort::SortPairs(R.sort_tmp.ptr, tmp, R.keys_in.ptr, R.keys_out.ptr,
-                                                   R.vals_in.ptr, R.perm.ptr, nj, 0, 30, st));
-    JSetOut src{R.posH.ptr, R.posL.ptr, R.vel.ptr, R.comp.ptr, R.compd.ptr, np};
-    JSetOut dst{R.posH_s.ptr, R.posL_s.ptr, R.vel_s.ptr, R.comp_s.ptr, R.compd_s.ptr, np};
-    const int pblocks = (int)std::min<size_t>((np + 255) / 256, (size_t)nb6_num_sms() * 8);
-    jset_permute<<<pblocks, 256, 0, st>>>(nj, src, dst, R.perm.ptr);
-    jset_tile_boxes<<<(R.ntile * 32 + 255) / 256, 256, 0, st>>>(nj, R.ntile, R.posH_s.ptr, R.vel_s.ptr, R.tbox.ptr);
-    R.comprel.reserve((size_t)3 * np);
-    jset_rel<<<pblocks, 256, 0, st>>>((int)np, R.ntile, R.compd_s.ptr, R.tbox.ptr, R.comprel.ptr);
-    NB6_CUDA_CHECK(cudaGetLastError());
-    R.sorted_ver = R.jver;
-    return true;
+    R.tiles_ver = R.jver;
+    R.tilesd_ver = want_d ? R.jver : -1;
+    R.tiles_ordered = ord;
+    return ord;
 }
 
 // ----------------------------------------------------------------------------
@@ -2171,7 +2088,7 @@ struct StageArgs {
     int *iperm, grid;
     void *p[7];
     explicit StageArgs(const RegLaunch &L)
-        : ni(L.ni), order(L.order), src(L.direct ? L.hin : nullptr), dst(R.iin.ptr), ix(L.ix), ext(R.ext.ptr),
+        : ni(L.ni), order(L.order), src(L.direct ? L.hin : nullptr), dst(R.iin.ptr), ix(L.ix), ext(R.order.ext.ptr),
           iperm(R.iperm.ptr), grid(order + (src ? (int)std::min<size_t>((4 * (size_t)ni + STAGE_NT - 1) / STAGE_NT, 64) : 0)) {
         void *q[7] = {&ni, &order, &src, &dst, &ix, &ext, &iperm};
         memcpy(p, q, sizeof(q));
@@ -2188,20 +2105,17 @@ static void regf_stage_launch(const RegLaunch &L, cudaStream_t st) {
     NB6_CUDA_CHECK(cudaLaunchKernel((const void *)regf_stage, dim3(g.grid), dim3(STAGE_NT), g.p, 0, st));
 }
 
-// The j set in its sent order, for the j-parallel kernel: the same variant
-// then always sums in the same order, whether or not other calls made the
-// spatial order, and one CTA's j's do not hold a whole neighbourhood.
+// The j set in its sent order, for every kernel but the packed tile kernels:
+// the same variant then always sums in the same order, whether or not other
+// calls made the spatial order, and one CTA's j's do not hold a whole
+// neighbourhood.
 static void unordered(RegArgs &a) {
-    a.posH = R.posH.ptr;
-    a.posL = R.posL.ptr;
-    a.vel = R.vel.ptr;
-    a.comp = R.comp.ptr;
-    a.compd = R.compd.ptr;
     a.perm = nullptr;
     a.tbox = nullptr;
     a.iperm = nullptr;
-    a.comprel = nullptr;
 }
+// Whether a variant reads the tile layout.
+static bool takes_tiles(int v) { return v > 10; }
 
 static void regf_prepare(int ni, const double *d_h2, const double *d_dtr, const double *d_x,
                          const double *d_v, int lmax, int nnbmax, int mflag, cudaStream_t st,
@@ -2234,13 +2148,10 @@ static void regf_prepare(int ni, const double *d_h2, const double *d_dtr, const 
     int cands[12], ncand = 0;
     if (tune_now) {
         if (ni >= NT / 2) {
-            cands[ncand++] = 1;
+            // (the scalar kernels and the FP64 differences are for callers
+            // that force them: they were never the fastest)
             cands[ncand++] = 11;
-            cands[ncand++] = 13;
-            if (ni >= NT * 2) {
-                cands[ncand++] = 2;
-                cands[ncand++] = 12;
-            }
+            if (ni >= NT * 2) cands[ncand++] = 12;
         }
         if (ni <= 2048)
             for (int ib : {1, 2, 4, 8})
@@ -2258,22 +2169,25 @@ static void regf_prepare(int ni, const double *d_h2, const double *d_dtr, const 
     R.outf.reserve((size_t)ni * 8);
     R.outl.reserve((size_t)ni * W);
 
-    // the spatial order serves the packed tile kernels (far tiles); a call
-    // that runs the j-parallel kernel does not wait for it
-    const bool sorted = (tune_now || variant > 0) && ensure_sorted(st);
+    // the tile layout, spatially ordered for large sets, serves the packed tile
+    // kernels; a call that runs another kernel does not wait for it
+    const bool tiles = tune_now || takes_tiles(variant);
+    const bool sorted = tiles && ensure_tiles(variant == 13, st);
     RegArgs a;
-    a.posH = sorted ? R.posH_s.ptr : R.posH.ptr;
-    a.posL = sorted ? R.posL_s.ptr : R.posL.ptr;
-    a.vel = sorted ? R.vel_s.ptr : R.vel.ptr;
-    a.comp = sorted ? R.comp_s.ptr : R.comp.ptr;
-    a.compd = sorted ? R.compd_s.ptr : R.compd.ptr;
-    a.perm = sorted ? R.perm.ptr : nullptr;
+    a.posH = R.posH.ptr;
+    a.posL = R.posL.ptr;
+    a.vel = R.vel.ptr;
+    if (tiles) {
+        a.tiles = R.tiles.ptr;
+        a.trows = sorted ? ROWS_ORD : ROWS_J;
+        a.tilesd = R.tilesd.ptr;
+    }
+    a.perm = sorted ? R.order.perm.ptr : nullptr;
     static const int far_path = [] {
         const char *e = getenv("NB6_FARPATH");
         return (e && atoi(e) == 0) ? 0 : 1;
     }();
     a.tbox = (sorted && far_path) ? R.tbox.ptr : nullptr;
-    a.comprel = (sorted && far_path) ? R.comprel.ptr : nullptr;
     static const int i_order = [] {
         const char *e = getenv("NB6_IORDER");
         return (e && atoi(e) == 0) ? 0 : 1;
@@ -2286,7 +2200,6 @@ static void regf_prepare(int ni, const double *d_h2, const double *d_dtr, const 
     L.ix = d_x;
     L.ni = ni;
     L.direct = L.hin != nullptr && nb6_uva();
-    a.npad = R.npad;
     a.jm = R.jm;
     a.jx = R.jx;
     a.jv = R.jv;
@@ -2328,7 +2241,7 @@ static void regf_prepare(int ni, const double *d_h2, const double *d_dtr, const 
             const int v = cands[c < 0 ? 0 : c];
             Plan p = make_plan(v, nt, R.nj, R.ntile, mf, 0);
             RegArgs t = a;
-            if (v < 0) unordered(t);   // as the call itself would run
+            if (!takes_tiles(v)) unordered(t);   // as the call itself would run
             t.nslices = p.nslices;
             t.ni = t.ni_pad = nt;
             float vbest = 1e30f;
@@ -2367,7 +2280,7 @@ static void regf_prepare(int ni, const double *d_h2, const double *d_dtr, const 
             fprintf(stderr, "# nb6 autotune: ni~2^%d nj~2^%d mflag %d -> variant %d (%.3f ms)\n",
                     key.li, key.lj, key.mf, bestv, best);
     }
-    if (plan.variant < 0) {
+    if (!takes_tiles(plan.variant)) {
         unordered(a);
         L.order = 0;
     }
@@ -2605,8 +2518,6 @@ void gpunb_close_() {
     R.posH.release();
     R.posL.release();
     R.vel.release();
-    R.comp.release();
-    R.compd.release();
     R.jall.release();
     R.jm = R.jx = R.jv = nullptr;
     R.iin.release();
@@ -3117,9 +3028,6 @@ void nb6_regf_seg_(int *ni_, int *iseg, double *h2, double *dtr, double (*xi)[3]
     a.posH = R.posH.ptr;
     a.posL = R.posL.ptr;
     a.vel = R.vel.ptr;
-    a.comp = R.comp.ptr;
-    a.compd = R.compd.ptr;
-    a.npad = R.npad;
     a.jm = R.jm;
     a.jx = R.jx;
     a.jv = R.jv;
@@ -3363,7 +3271,7 @@ int nb6_regf_jsort_(int *flag) {
     }
     if (flag && (*flag == 0 || *flag == 1)) {
         R.use_jsort = *flag;
-        R.sorted_ver = -1;  // rebuild on the next call if turned on
+        R.tiles_ver = -1;  // rebuild on the next call
     }
     return R.use_jsort;
 }
