@@ -7,10 +7,11 @@
 // NNBOPT neighbours at its next regular step (estimated from the count that
 // step found, nnb ~ RS^3).  Loss: mean squared error in standardised units.
 //
-//   mlp_grad_kernel   32 samples per CTA and round, one warp each: bf16-weight
-//                     forward pass, FP32 backward pass to the layers' inputs;
-//                     then every thread sums its own parameters' gradients
-//                     over the samples, in a fixed order;
+//   mlp_grad_kernel   eight samples per CTA and round, one warp each:
+//                     bf16-weight forward pass, FP32 backward pass to the
+//                     layers' inputs; then every thread sums its own
+//                     parameters' gradients over the samples, in a fixed
+//                     order;
 //   mlp_reduce        CTA partials summed in block order (deterministic), and
 //                     in training the Adam step on the FP32 master copy and
 //                     the bf16 copy that every forward pass reads.
@@ -27,17 +28,19 @@
 
 namespace {
 
-// Gradient kernel: GW sample streams per CTA, GK samples of each per round,
-// a warp for each of the GW * GK samples.
-constexpr int GW = 4, GK = 8, GS = GW * GK;
+// Gradient kernel: GW sample streams per block of samples, a CTA each, GK
+// samples of a stream per round, a warp each.
+constexpr int GW = 4, GK = 8, GS = GW * GK, GRAD_NT = GK * 32;
 constexpr int W2S = MLP_H + 8;  // row stride of W2 in shared memory (bf16): 16-byte reads of 8 lanes miss no bank
+constexpr int MLP_NSMALL = MLP_NPARAM - MLP_H * MLP_H;   // W1, B1, B2, W3, B3 back to back
+// The bf16 copy: the flat parameters, then W2 transposed ([r][k]).
+constexpr int W16_T = MLP_SMEM_BYTES / 2;
 // What one sample hands from its warp to the gradient sums.
 struct MlpSample {
     float h1[MLP_H], dz1[MLP_H], h2[MLP_H], dz2[MLP_H];
     float xn[MLP_IN], d, err2, pad;
 };
 static_assert(sizeof(MlpSample) % 16 == 0, "float4 reads of the sample rows");
-constexpr size_t GRAD_SMEM = (size_t)MLP_SMEM_BYTES + 2 * (size_t)MLP_H * W2S * 2 + GS * sizeof(MlpSample);
 
 struct MlpState {
     bool have = false;      // parameters set or trained
@@ -50,10 +53,26 @@ struct MlpState {
 };
 MlpState M;
 
+// Parameter k into the bf16 copies.
+NB6_DEV void store_bf16(__nv_bfloat16 *w16, int k, float w) {
+    const __nv_bfloat16 v = __float2bfloat16_rn(w);
+    w16[k] = v;
+    const int q = k - MLP_OFF_W2;
+    if (q >= 0 && q < MLP_H * MLP_H) w16[W16_T + (q % MLP_H) * MLP_H + q / MLP_H] = v;
+}
+
 __global__ void mlp_to_bf16(const float *__restrict__ w32, __nv_bfloat16 *__restrict__ w16) {
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < MLP_SMEM_BYTES / 2; k += gridDim.x * blockDim.x)
-        w16[k] = __float2bfloat16_rn(k < MLP_NPARAM ? w32[k] : 0.0f);
+        store_bf16(w16, k, k < MLP_NPARAM ? w32[k] : 0.0f);
 }
+
+// The kernels of a training run are launched back to back, each allowed on
+// the SMs while the one before drains (programmatic dependent launch): it
+// waits here before it touches what that one wrote.
+NB6_DEV void wait_for_previous() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+NB6_DEV void let_next_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // Eight bf16 weights (one 16-byte read) times eight inputs, in index order.
 NB6_DEV float fma8(const __nv_bfloat16 *w, const float *in, float z) {
@@ -75,50 +94,61 @@ NB6_DEV float fma8(const __nv_bfloat16 *w, const float *in, float z) {
 //
 // Sample q = (block GW + w) + k (blocks GW) is the k-th of stream w of its
 // block.  A parameter's gradient is summed over k within a stream, then over
-// the streams, so the sums do not depend on how many samples run at a time.
-// Eight samples of each stream are in flight (a warp each): with one warp per
-// stream the kernel was a chain of eight samples' forward and backward passes
-// and of 8,192 read-modify-writes each of a gradient buffer in shared memory
-// (45 us for 1,024 samples; an epoch of 32,768 samples in batches of 1,024
-// 2,070 us, now 1,037 us).  The layers read eight weights per 16-byte load,
-// W2 along its rows (backward) and, from a transposed copy, along its columns
-// (forward).
-__global__ void __launch_bounds__(GS * 32)
+// the streams, then over the blocks, so the sums do not depend on how many
+// samples run at a time.  Eight samples of a stream are in flight (a warp
+// each), the four streams of a block on different SMs: with one warp per stream
+// the kernel was a chain of eight samples' forward and backward passes and of
+// 8,192 read-modify-writes each of a gradient buffer in shared memory (45 us
+// for 1,024 samples); with the block's 32 warps in one CTA the shared-memory
+// reads of 32 SMs bounded it (16 us, now 11).  The layers read eight weights per
+// 16-byte load, W2 along its rows (backward) and, from the transposed copy,
+// along its columns (forward).
+__global__ void __launch_bounds__(GRAD_NT)
     mlp_grad_kernel(int cnt, int off, float inv_n, const float *__restrict__ x, const float *__restrict__ y,
-                    const int *__restrict__ perm, const __nv_bfloat16 *__restrict__ w16,
-                    const float *__restrict__ norm, float *__restrict__ part, float *__restrict__ part_loss) {
-    extern __shared__ __align__(16) unsigned char smem[];
-    __nv_bfloat16 *sw = reinterpret_cast<__nv_bfloat16 *>(smem);
-    __nv_bfloat16 *w2 = sw + MLP_SMEM_BYTES / 2;   // w2[k][r] = W2[k][r]
-    __nv_bfloat16 *w2t = w2 + MLP_H * W2S;         // w2t[r][k] = W2[k][r]
-    MlpSample *smp = reinterpret_cast<MlpSample *>(w2t + MLP_H * W2S);
+                    const int *__restrict__ perm, const __nv_bfloat16 *w16, const float *__restrict__ norm,
+                    float *part, float *part_loss) {
+    __shared__ __align__(16) __nv_bfloat16 sw[(MLP_NSMALL + 7) / 8 * 8];   // W1, B1 | B2, W3, B3
+    __shared__ __align__(16) __nv_bfloat16 w2[MLP_H * W2S], w2t[MLP_H * W2S];
+    __shared__ __align__(16) MlpSample smp[GK];
+    constexpr int B2 = MLP_OFF_W2, W3 = B2 + MLP_H, B3 = W3 + MLP_H;   // places in sw
+    let_next_start();
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    mlp_load(sw, w16);
-    for (int q = tid; q < MLP_H * MLP_H; q += GS * 32) {
-        const int k = q / MLP_H, r = q % MLP_H;
-        const __nv_bfloat16 v = w16[MLP_OFF_W2 + q];
-        w2[k * W2S + r] = v;
-        w2t[r * W2S + k] = v;
-    }
-    __syncthreads();
-    // this thread's parameters: W2[gk][gr .. gr+3], and one of the others
-    const int gk = tid >> 4, gr = (tid & 15) * 4;
-    float g2[GW][4], g1[GW];
-#pragma unroll
-    for (int w = 0; w < GW; ++w) g1[w] = g2[w][0] = g2[w][1] = g2[w][2] = g2[w][3] = 0.0f;
-    float lsum[GW] = {0.0f, 0.0f, 0.0f, 0.0f};
+    const int stride = gridDim.x * GW, first = blockIdx.x * GW + blockIdx.y;
     const float ymean = norm[2 * MLP_IN], yinv = 1.0f / norm[2 * MLP_IN + 1];
-    const int sw_w = warp % GW, sw_k = warp / GW;
+    // this warp's sample of a round: its standardised inputs and target
+    float xn[MLP_IN], target = 0.0f;
+    auto fetch = [&](int base) {
+        const int q = base + warp * stride + first;
+        if (q >= cnt) return false;
+        const int s = perm ? perm[off + q] : off + q;
+#pragma unroll
+        for (int k = 0; k < MLP_IN; ++k) xn[k] = (x[(size_t)s * MLP_IN + k] - norm[k]) * norm[MLP_IN + k];
+        target = y[s];
+        return true;
+    };
+    bool have = fetch(0);
+    wait_for_previous();   // the weights
+    const uint4 *src = reinterpret_cast<const uint4 *>(w16);
+    for (int q = tid; q < MLP_H * MLP_H / 8; q += GRAD_NT) {
+        const int r = q / (MLP_H / 8), c = q % (MLP_H / 8);
+        reinterpret_cast<uint4 *>(w2 + r * W2S)[c] = __ldcg(src + MLP_OFF_W2 / 8 + q);
+        reinterpret_cast<uint4 *>(w2t + r * W2S)[c] = __ldcg(src + W16_T / 8 + q);
+    }
+    for (int q = tid; q < (MLP_NSMALL + 7) / 8; q += GRAD_NT)
+        reinterpret_cast<uint4 *>(sw)[q] = __ldcg(src + (q < MLP_OFF_W2 / 8 ? q : q + MLP_H * MLP_H / 8));
+    __syncthreads();
+    // this thread's parameters: W2[gk][gr .. gr+15], and others
+    const int gk = tid >> 2, gr = (tid & 3) * 16;
+    constexpr int NO = (MLP_NSMALL + GRAD_NT - 1) / GRAD_NT;
+    float g2[16], g1[NO], lsum = 0.0f;
+#pragma unroll
+    for (int c = 0; c < 16; ++c) g2[c] = 0.0f;
+#pragma unroll
+    for (int c = 0; c < NO; ++c) g1[c] = 0.0f;
     MlpSample &S = smp[warp];
-    const int stride = gridDim.x * GW;
     for (int base = 0; base < cnt; base += GK * stride) {
         // forward and backward pass of this warp's sample
-        const int q = base + sw_k * stride + blockIdx.x * GW + sw_w;
-        if (q < cnt) {
-            const int s = perm ? perm[off + q] : off + q;
-            float xn[MLP_IN];
-#pragma unroll
-            for (int k = 0; k < MLP_IN; ++k) xn[k] = (x[(size_t)s * MLP_IN + k] - norm[k]) * norm[MLP_IN + k];
+        if (have) {
             float z1[2], z2[2];
 #pragma unroll
             for (int u = 0; u < 2; ++u) {
@@ -131,23 +161,23 @@ __global__ void __launch_bounds__(GS * 32)
             }
             __syncwarp();
 #pragma unroll
-            for (int u = 0; u < 2; ++u) z2[u] = bf(sw, MLP_OFF_B2 + lane + 32 * u);
+            for (int u = 0; u < 2; ++u) z2[u] = bf(sw, B2 + lane + 32 * u);
 #pragma unroll
             for (int k = 0; k < MLP_H; k += 8)
 #pragma unroll
                 for (int u = 0; u < 2; ++u) z2[u] = fma8(w2t + (lane + 32 * u) * W2S + k, S.h1 + k, z2[u]);
             const float h2[2] = {mlp_silu(z2[0]), mlp_silu(z2[1])};
-            float o = bf(sw, MLP_OFF_W3 + lane) * h2[0] + bf(sw, MLP_OFF_W3 + lane + 32) * h2[1];
+            float o = bf(sw, W3 + lane) * h2[0] + bf(sw, W3 + lane + 32) * h2[1];
 #pragma unroll
             for (int t = 16; t > 0; t >>= 1) o += __shfl_xor_sync(0xffffffffu, o, t);
-            const float out = o + bf(sw, MLP_OFF_B3);
-            const float err = out - (y[s] - ymean) * yinv;
+            const float out = o + bf(sw, B3);
+            const float err = out - (target - ymean) * yinv;
             const float d = 2.0f * err * inv_n;
 #pragma unroll
             for (int u = 0; u < 2; ++u) {
                 const int r = lane + 32 * u;
                 S.h2[r] = h2[u];
-                S.dz2[r] = d * bf(sw, MLP_OFF_W3 + r) * mlp_dsilu(z2[u]);
+                S.dz2[r] = d * bf(sw, W3 + r) * mlp_dsilu(z2[u]);
             }
             __syncwarp();
             float dh1[2] = {0.0f, 0.0f};
@@ -166,52 +196,48 @@ __global__ void __launch_bounds__(GS * 32)
         } else {   // no sample: every product below is zero
             for (int k = lane; k < (int)(sizeof(MlpSample) / 4); k += 32) reinterpret_cast<float *>(&S)[k] = 0.0f;
         }
+        have = fetch(base + GK * stride);
         __syncthreads();
 #pragma unroll
-        for (int w = 0; w < GW; ++w)
-#pragma unroll 4
-            for (int k = 0; k < GK; ++k) {
-                const MlpSample &T = smp[k * GW + w];
-                const float h = T.h1[gk];
-                const float4 z = *reinterpret_cast<const float4 *>(&T.dz2[gr]);
-                g2[w][0] = fmaf(z.x, h, g2[w][0]);
-                g2[w][1] = fmaf(z.y, h, g2[w][1]);
-                g2[w][2] = fmaf(z.z, h, g2[w][2]);
-                g2[w][3] = fmaf(z.w, h, g2[w][3]);
-            }
-        // the other parameters, by thread: W1, B1, B2, W3, B3 and the loss
+        for (int k = 0; k < GK; ++k) {
+            const MlpSample &T = smp[k];
+            const float h = T.h1[gk];
 #pragma unroll
-        for (int w = 0; w < GW; ++w)
+            for (int c = 0; c < 16; c += 4) {
+                const float4 z = *reinterpret_cast<const float4 *>(&T.dz2[gr + c]);
+                g2[c] = fmaf(z.x, h, g2[c]);
+                g2[c + 1] = fmaf(z.y, h, g2[c + 1]);
+                g2[c + 2] = fmaf(z.z, h, g2[c + 2]);
+                g2[c + 3] = fmaf(z.w, h, g2[c + 3]);
+            }
+        }
+        // the other parameters: W1, B1, B2, W3, B3 and the loss
+#pragma unroll
+        for (int c = 0; c < NO; ++c) {
+            const int p = tid + c * GRAD_NT, r = p % MLP_H;
+#pragma unroll
             for (int k = 0; k < GK; ++k) {
-                const MlpSample &T = smp[k * GW + w];
-                if (tid < MLP_IN * MLP_H) g1[w] = fmaf(T.dz1[tid % MLP_H], T.xn[tid / MLP_H], g1[w]);
-                else if (tid < MLP_OFF_W2) g1[w] += T.dz1[tid % MLP_H];
-                else if (tid < MLP_OFF_W2 + MLP_H) g1[w] += T.dz2[tid % MLP_H];
-                else if (tid < MLP_OFF_W2 + 2 * MLP_H) g1[w] = fmaf(T.d, T.h2[tid % MLP_H], g1[w]);
-                else if (tid == MLP_OFF_W2 + 2 * MLP_H) {
-                    g1[w] += T.d;
-                    lsum[w] = fmaf(T.err2, T.err2, lsum[w]);
+                const MlpSample &T = smp[k];
+                if (p < MLP_OFF_B1) g1[c] = fmaf(T.dz1[r], T.xn[p / MLP_H], g1[c]);
+                else if (p < B2) g1[c] += T.dz1[r];
+                else if (p < W3) g1[c] += T.dz2[r];
+                else if (p < B3) g1[c] = fmaf(T.d, T.h2[r], g1[c]);
+                else if (p == B3) {
+                    g1[c] += T.d;
+                    lsum = fmaf(T.err2, T.err2, lsum);
                 }
             }
+        }
         __syncthreads();
     }
-    float *p = part + (size_t)blockIdx.x * MLP_NPARAM;
+    float *o = part + (size_t)first * MLP_NPARAM;
 #pragma unroll
-    for (int c = 0; c < 4; ++c) {
-        float acc = 0.0f;
+    for (int c = 0; c < 16; ++c) o[MLP_OFF_W2 + gk * MLP_H + gr + c] = g2[c];
 #pragma unroll
-        for (int w = 0; w < GW; ++w) acc += g2[w][c];
-        p[MLP_OFF_W2 + gk * MLP_H + gr + c] = acc;
-    }
-    if (tid <= MLP_OFF_W2 + 2 * MLP_H) {
-        float acc = 0.0f, l = 0.0f;
-#pragma unroll
-        for (int w = 0; w < GW; ++w) {
-            acc += g1[w];
-            l += lsum[w];
-        }
-        p[tid < MLP_OFF_W2 ? tid : tid + MLP_H * MLP_H] = acc;
-        if (tid == MLP_OFF_W2 + 2 * MLP_H) part_loss[blockIdx.x] = l;
+    for (int c = 0; c < NO; ++c) {
+        const int p = tid + c * GRAD_NT;
+        if (p < MLP_NSMALL) o[p < MLP_OFF_W2 ? p : p + MLP_H * MLP_H] = g1[c];
+        if (p == B3) part_loss[first] = lsum;
     }
 }
 
@@ -222,35 +248,62 @@ struct AdamArgs {
     float lr, b1, b2, eps, bc1, bc2;
 };
 
-// grad[k] = sum over blocks in block order; loss[0] += sum of squared errors.
-// ADAM: then the step on parameter k and its bf16 copy, which the next
-// batch's forward pass reads, in the same launch.
-constexpr int RED_NT = 64;
+// grad[k] = sum over blocks, in order, of the sum over a block's streams;
+// loss[0] += sum of squared errors, likewise (as parameter MLP_NPARAM).  ADAM:
+// then the step on parameter k and its bf16 copies, which the next batch's
+// forward pass reads, in the same launch.  A CTA takes RED_P parameters; its
+// threads sum the streams of 32 blocks side by side (one memory round trip; a
+// thread per parameter walked 128 partials, 10 us for a batch of 1,024), then
+// one warp adds the blocks in order.
+constexpr int RED_P = 32, RED_NT = 256;
+static_assert(GW == 4, "mlp_reduce adds four streams");
 template <bool ADAM>
 __global__ void __launch_bounds__(RED_NT)
-    mlp_reduce(int nb, const float *__restrict__ part, const float *__restrict__ part_loss,
-               float *__restrict__ grad, float *__restrict__ loss, const AdamArgs ad) {
-    const int k = blockIdx.x * RED_NT + threadIdx.x;
-    if (k < MLP_NPARAM) {
-        float g = 0.0f;
-#pragma unroll 16
-        for (int b = 0; b < nb; ++b) g += __ldg(part + (size_t)b * MLP_NPARAM + k);
+    mlp_reduce(int nb, const float *part, const float *part_loss, float *__restrict__ grad, float *loss,
+               const AdamArgs ad) {
+    __shared__ float acc[32][RED_P];
+    let_next_start();
+    wait_for_previous();
+    const int p = threadIdx.x % RED_P, row = threadIdx.x / RED_P, k = blockIdx.x * RED_P + p;
+    const float *src = k < MLP_NPARAM ? part + k : part_loss;
+    const size_t step = k < MLP_NPARAM ? MLP_NPARAM : 1;
+    const bool mine = row == 0 && k < MLP_NPARAM;
+    float m1 = 0.f, m2 = 0.f, w = 0.f, g = 0.f;
+    if (ADAM && mine) {
+        m1 = ad.m1[k];
+        m2 = ad.m2[k];
+        w = ad.w[k];
+    }
+    for (int b0 = 0; b0 < nb; b0 += 32) {
+#pragma unroll
+        for (int r = row; r < 32; r += RED_NT / RED_P) {
+            if (b0 + r < nb && k <= MLP_NPARAM) {
+                const float *q = src + (size_t)(b0 + r) * GW * step;
+                acc[r][p] = ((__ldcg(q) + __ldcg(q + step)) + __ldcg(q + 2 * step)) + __ldcg(q + 3 * step);
+            }
+        }
+        __syncthreads();
+        if (row == 0 && k <= MLP_NPARAM) {
+            const int n = min(32, nb - b0);
+#pragma unroll 8
+            for (int r = 0; r < n; ++r) g += acc[r][p];
+        }
+        __syncthreads();
+    }
+    if (mine) {
         if (ADAM) {
-            const float a = ad.b1 * ad.m1[k] + (1.0f - ad.b1) * g;
-            const float b = ad.b2 * ad.m2[k] + (1.0f - ad.b2) * g * g;
+            const float a = ad.b1 * m1 + (1.0f - ad.b1) * g;
+            const float b = ad.b2 * m2 + (1.0f - ad.b2) * g * g;
             ad.m1[k] = a;
             ad.m2[k] = b;
-            const float w = ad.w[k] - ad.lr * (a / ad.bc1) / (sqrtf(b / ad.bc2) + ad.eps);
+            w -= ad.lr * (a / ad.bc1) / (sqrtf(b / ad.bc2) + ad.eps);
             ad.w[k] = w;
-            ad.w16[k] = __float2bfloat16_rn(w);
+            store_bf16(ad.w16, k, w);
         } else {
             grad[k] = g;
         }
-    } else if (k == MLP_NPARAM) {
-        float l = 0.0f;
-#pragma unroll 16
-        for (int b = 0; b < nb; ++b) l += __ldg(part_loss + b);
-        loss[0] += l;
+    } else if (row == 0 && k == MLP_NPARAM) {
+        loss[0] += g;
     }
 }
 
@@ -280,10 +333,8 @@ void mlp_alloc() {
     M.grad.reserve(MLP_NPARAM);
     M.norm.reserve(MLP_NNORM);
     M.loss.reserve(1);
-    M.w16.reserve(MLP_SMEM_BYTES / 2);
+    M.w16.reserve(W16_T + MLP_H * MLP_H);
     M.host.assign(MLP_NPARAM + MLP_NNORM, 0.0f);
-    NB6_CUDA_CHECK(cudaFuncSetAttribute(mlp_grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)GRAD_SMEM));
 }
 
 // Host copy -> device FP32 master, moments and the bf16 copy; resets Adam.
@@ -308,11 +359,14 @@ void mlp_download() {
 }
 
 void mlp_upload_samples(int n, const float *x, const float *y) {
+    cudaStream_t st = nb6_stream();
     M.dx.reserve((size_t)n * MLP_IN);
-    NB6_CUDA_CHECK(cudaMemcpy(M.dx.ptr, x, sizeof(float) * MLP_IN * (size_t)n, cudaMemcpyHostToDevice));
+    const Nb6Seg sx{0, x, sizeof(float) * MLP_IN * (size_t)n};
+    nb6_upload(M.dx.ptr, &sx, 1, sx.len, st);
     if (y) {
         M.dy.reserve(n);
-        NB6_CUDA_CHECK(cudaMemcpy(M.dy.ptr, y, sizeof(float) * (size_t)n, cudaMemcpyHostToDevice));
+        const Nb6Seg sy{0, y, sizeof(float) * (size_t)n};
+        nb6_upload(M.dy.ptr, &sy, 1, sy.len, st);
     }
 }
 
@@ -322,15 +376,25 @@ int grad_blocks(int cnt) { return std::max(1, std::min((cnt + GS - 1) / GS, nb6_
 // or through the Adam step `adam` into the parameters.
 void mlp_grad_launch(int cnt, int off, const int *perm, const AdamArgs *adam, cudaStream_t st) {
     const int nb = grad_blocks(cnt);
-    M.part.reserve((size_t)nb * (MLP_NPARAM + 1));
-    float *part_loss = M.part.ptr + (size_t)nb * MLP_NPARAM;
-    mlp_grad_kernel<<<nb, GS * 32, GRAD_SMEM, st>>>(cnt, off, 1.0f / (float)cnt, M.dx.ptr, M.dy.ptr, perm,
-                                                    M.w16.ptr, M.norm.ptr, M.part.ptr, part_loss);
-    NB6_CUDA_CHECK(cudaGetLastError());
-    constexpr int rb = MLP_NPARAM / RED_NT + 1;   // every parameter, and the loss
-    if (adam) mlp_reduce<true><<<rb, RED_NT, 0, st>>>(nb, M.part.ptr, part_loss, nullptr, M.loss.ptr, *adam);
-    else mlp_reduce<false><<<rb, RED_NT, 0, st>>>(nb, M.part.ptr, part_loss, M.grad.ptr, M.loss.ptr, AdamArgs{});
-    NB6_CUDA_CHECK(cudaGetLastError());
+    M.part.reserve((size_t)nb * GW * (MLP_NPARAM + 1));
+    float *part = M.part.ptr, *part_loss = part + (size_t)nb * GW * MLP_NPARAM;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t c{};
+    c.stream = st;
+    c.attrs = &at;
+    c.numAttrs = 1;
+    c.gridDim = dim3(nb, GW);
+    c.blockDim = dim3(GRAD_NT);
+    NB6_CUDA_CHECK(cudaLaunchKernelEx(&c, mlp_grad_kernel, cnt, off, 1.0f / (float)cnt, (const float *)M.dx.ptr,
+                                      (const float *)M.dy.ptr, perm, (const __nv_bfloat16 *)M.w16.ptr,
+                                      (const float *)M.norm.ptr, part, part_loss));
+    c.gridDim = dim3(MLP_NPARAM / RED_P + 1);   // every parameter, and the loss
+    c.blockDim = dim3(RED_NT);
+    const AdamArgs ad = adam ? *adam : AdamArgs{};
+    NB6_CUDA_CHECK(cudaLaunchKernelEx(&c, adam ? mlp_reduce<true> : mlp_reduce<false>, nb, (const float *)part,
+                                      (const float *)part_loss, M.grad.ptr, M.loss.ptr, ad));
 }
 
 bool check_n(int n) {
