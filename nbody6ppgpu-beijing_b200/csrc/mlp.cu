@@ -444,7 +444,7 @@ void mlp_grad_launch(int cnt, int off, const int *perm, const AdamArgs *adam, cu
     NB6_CUDA_CHECK(cudaLaunchKernelEx(&c, mlp_grad_kernel, cnt, off, 1.0f / (float)cnt, (const float *)M.dx.ptr,
                                       (const float *)M.dy.ptr, perm, (const __nv_bfloat16 *)M.w16.ptr,
                                       (const float *)M.norm.ptr, part, part_loss));
-    c.gridDim = dim3(MLP_NPARAM / RED_NT + 1);   // every parameter, and the loss
+    c.gridDim = dim3(MLP_NPARAM / RED_P + 1);   // every parameter, and the loss
     c.blockDim = dim3(RED_NT);
     const AdamArgs ad = adam ? *adam : AdamArgs{};
     NB6_CUDA_CHECK(cudaLaunchKernelEx(&c, adam ? mlp_reduce<true> : mlp_reduce<false>, nb, (const float *)part,
