@@ -14,7 +14,8 @@
 //                     order;
 //   mlp_reduce        CTA partials summed in block order (deterministic), and
 //                     in training the Adam step on the FP32 master copy and
-//                     the bf16 copy that every forward pass reads.
+//                     the bf16 copy that every forward pass reads;
+//   mlp_steps         both for all the steps of an epoch in one launch.
 //
 // The model is small (4,609 parameters, ~4.5 kFLOP per sample), so the
 // passes run on the FP32 pipes: a batch of 1024 samples is ~10 MFLOP, far
@@ -42,14 +43,23 @@ struct MlpSample {
 };
 static_assert(sizeof(MlpSample) % 16 == 0, "float4 reads of the sample rows");
 
+// What the CTAs of mlp_steps wait on, each word in a line of its own, and what
+// a training run reports.
+struct TrainSync {
+    unsigned done_grad, pad0[31], done_red, pad1[31];
+    float loss;
+    unsigned err;   // a wait ran out
+};
+
 struct MlpState {
     bool have = false;      // parameters set or trained
     int enabled = 0;        // proposals in regular-force calls
     std::vector<float> host;  // FP32 parameters + moments
-    DevBuf<float> w32, m1, m2, grad, part, norm, dx, dy, loss;
+    DevBuf<float> w32, m1, m2, grad, part, norm, dx, dy;
     DevBuf<__nv_bfloat16> w16;
-    DevBuf<int> perm;
+    DevBuf<int> perm;          // one epoch's order, then its bias corrections (float2 per step)
     DevBuf<double> mom;
+    DevBuf<TrainSync> sync;
     long long adam_t = 0;
 };
 MlpState M;
@@ -67,8 +77,8 @@ __global__ void mlp_to_bf16(const float *__restrict__ w32, __nv_bfloat16 *__rest
         store_bf16(w16, k, k < MLP_NPARAM ? w32[k] : 0.0f);
 }
 
-// The kernels of a training run are launched back to back, each allowed on
-// the SMs while the one before drains (programmatic dependent launch): it
+// The kernels of a gradient, and of training steps too large for mlp_steps, are
+// launched back to back, each allowed on the SMs while the one before drains (programmatic dependent launch): it
 // waits here before it touches what that one wrote.
 NB6_DEV void wait_for_previous() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -104,39 +114,53 @@ NB6_DEV float fma8(const __nv_bfloat16 *w, const float *in, float z) {
 // reads of 32 SMs bounded it (16 us, now 11).  The layers read eight weights per
 // 16-byte load, W2 along its rows (backward) and, from the transposed copy,
 // along its columns (forward).
-__global__ void __launch_bounds__(GRAD_NT)
-    mlp_grad_kernel(int cnt, int off, float inv_n, const float *__restrict__ x, const float *__restrict__ y,
-                    const int *__restrict__ perm, const __nv_bfloat16 *w16, const float *__restrict__ norm,
-                    float *part, float *part_loss) {
-    __shared__ __align__(16) __nv_bfloat16 sw[(MLP_NSMALL + 7) / 8 * 8];   // W1, B1 | B2, W3, B3
-    __shared__ __align__(16) __nv_bfloat16 w2[MLP_H * W2S], w2t[MLP_H * W2S];
-    __shared__ __align__(16) MlpSample smp[GK];
-    constexpr int B2 = MLP_OFF_W2, W3 = B2 + MLP_H, B3 = W3 + MLP_H;   // places in sw
-    let_next_start();
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int stride = gridDim.x * GW, first = blockIdx.x * GW + blockIdx.y;
-    const float ymean = norm[2 * MLP_IN], yinv = 1.0f / norm[2 * MLP_IN + 1];
-    // this warp's sample of a round: its standardised inputs and target
-    float xn[MLP_IN], target = 0.0f;
-    auto fetch = [&](int base) {
-        const int q = base + warp * stride + first;
-        if (q >= cnt) return false;
-        const int s = perm ? perm[off + q] : off + q;
+struct GradSmem {
+    __align__(16) __nv_bfloat16 sw[(MLP_NSMALL + 7) / 8 * 8];   // W1, B1 | B2, W3, B3
+    __align__(16) __nv_bfloat16 w2[MLP_H * W2S], w2t[MLP_H * W2S];
+    __align__(16) MlpSample smp[GK];
+};
+struct GradArgs {
+    int cnt;        // samples of the batch
+    float inv_n;
+    const float *x, *y;
+    const int *perm;
+    const __nv_bfloat16 *w16;
+    const float *norm;
+    float *part, *part_loss;
+};
+// A warp's sample of a round: its standardised inputs and target.
+struct SampleIn {
+    float xn[MLP_IN], target;
+    bool have;
+};
+// The sample of stream `first` at `base` samples into the batch at `off`.
+NB6_DEV void fetch_sample(const GradArgs &g, int off, int base, int first, int stride, SampleIn &in) {
+    const int q = base + (int)(threadIdx.x >> 5) * stride + first;
+    in.have = q < g.cnt;
+    if (!in.have) return;
+    const int s = g.perm ? g.perm[off + q] : off + q;
 #pragma unroll
-        for (int k = 0; k < MLP_IN; ++k) xn[k] = (x[(size_t)s * MLP_IN + k] - norm[k]) * norm[MLP_IN + k];
-        target = y[s];
-        return true;
-    };
-    bool have = fetch(0);
-    wait_for_previous();   // the weights
-    const uint4 *src = reinterpret_cast<const uint4 *>(w16);
+    for (int k = 0; k < MLP_IN; ++k) in.xn[k] = (g.x[(size_t)s * MLP_IN + k] - g.norm[k]) * g.norm[MLP_IN + k];
+    in.target = g.y[s];
+}
+
+// The gradient sums of stream `first`, whose first sample is in `in`.
+NB6_DEV void grad_pass(GradSmem &sm, const GradArgs &g, int off, int first, int stride, SampleIn &in) {
+    constexpr int B2 = MLP_OFF_W2, W3 = B2 + MLP_H, B3 = W3 + MLP_H;   // places in sw
+    const __nv_bfloat16 *sw = sm.sw, *w2 = sm.w2, *w2t = sm.w2t;
+    MlpSample *smp = sm.smp;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int cnt = g.cnt;
+    const float inv_n = g.inv_n, ymean = g.norm[2 * MLP_IN], yinv = 1.0f / g.norm[2 * MLP_IN + 1];
+    const float (&xn)[MLP_IN] = in.xn;
+    const uint4 *src = reinterpret_cast<const uint4 *>(g.w16);
     for (int q = tid; q < MLP_H * MLP_H / 8; q += GRAD_NT) {
         const int r = q / (MLP_H / 8), c = q % (MLP_H / 8);
-        reinterpret_cast<uint4 *>(w2 + r * W2S)[c] = __ldcg(src + MLP_OFF_W2 / 8 + q);
-        reinterpret_cast<uint4 *>(w2t + r * W2S)[c] = __ldcg(src + W16_T / 8 + q);
+        reinterpret_cast<uint4 *>(sm.w2 + r * W2S)[c] = __ldcg(src + MLP_OFF_W2 / 8 + q);
+        reinterpret_cast<uint4 *>(sm.w2t + r * W2S)[c] = __ldcg(src + W16_T / 8 + q);
     }
     for (int q = tid; q < (MLP_NSMALL + 7) / 8; q += GRAD_NT)
-        reinterpret_cast<uint4 *>(sw)[q] = __ldcg(src + (q < MLP_OFF_W2 / 8 ? q : q + MLP_H * MLP_H / 8));
+        reinterpret_cast<uint4 *>(sm.sw)[q] = __ldcg(src + (q < MLP_OFF_W2 / 8 ? q : q + MLP_H * MLP_H / 8));
     __syncthreads();
     // this thread's parameters: W2[gk][gr .. gr+15], and others
     const int gk = tid >> 2, gr = (tid & 3) * 16;
@@ -149,7 +173,7 @@ __global__ void __launch_bounds__(GRAD_NT)
     MlpSample &S = smp[warp];
     for (int base = 0; base < cnt; base += GK * stride) {
         // forward and backward pass of this warp's sample
-        if (have) {
+        if (in.have) {
             float z1[2], z2[2];
 #pragma unroll
             for (int u = 0; u < 2; ++u) {
@@ -172,7 +196,7 @@ __global__ void __launch_bounds__(GRAD_NT)
 #pragma unroll
             for (int t = 16; t > 0; t >>= 1) o += __shfl_xor_sync(0xffffffffu, o, t);
             const float out = o + bf(sw, B3);
-            const float err = out - (target - ymean) * yinv;
+            const float err = out - (in.target - ymean) * yinv;
             const float d = 2.0f * err * inv_n;
 #pragma unroll
             for (int u = 0; u < 2; ++u) {
@@ -197,7 +221,7 @@ __global__ void __launch_bounds__(GRAD_NT)
         } else {   // no sample: every product below is zero
             for (int k = lane; k < (int)(sizeof(MlpSample) / 4); k += 32) reinterpret_cast<float *>(&S)[k] = 0.0f;
         }
-        have = fetch(base + GK * stride);
+        fetch_sample(g, off, base + GK * stride, first, stride, in);
         __syncthreads();
 #pragma unroll
         for (int k = 0; k < GK; ++k) {
@@ -231,15 +255,25 @@ __global__ void __launch_bounds__(GRAD_NT)
         }
         __syncthreads();
     }
-    float *o = part + (size_t)first * MLP_NPARAM;
+    float *o = g.part + (size_t)first * MLP_NPARAM;
 #pragma unroll
     for (int c = 0; c < 16; ++c) o[MLP_OFF_W2 + gk * MLP_H + gr + c] = g2[c];
 #pragma unroll
     for (int c = 0; c < NO; ++c) {
         const int p = tid + c * GRAD_NT;
         if (p < MLP_NSMALL) o[p < MLP_OFF_W2 ? p : p + MLP_H * MLP_H] = g1[c];
-        if (p == B3) part_loss[first] = lsum;
+        if (p == B3) g.part_loss[first] = lsum;
     }
+}
+
+__global__ void __launch_bounds__(GRAD_NT) mlp_grad_kernel(const GradArgs g, int off) {
+    __shared__ GradSmem sm;
+    let_next_start();
+    const int stride = gridDim.x * GW, first = blockIdx.x * GW + blockIdx.y;
+    SampleIn in;
+    fetch_sample(g, off, 0, first, stride, in);
+    wait_for_previous();   // the weights
+    grad_pass(sm, g, off, first, stride, in);
 }
 
 // The Adam step of one training batch.
@@ -259,13 +293,9 @@ struct AdamArgs {
 constexpr int RED_P = 32, RED_NT = 256;
 static_assert(GW == 4, "mlp_reduce adds four streams");
 template <bool ADAM>
-__global__ void __launch_bounds__(RED_NT)
-    mlp_reduce(int nb, const float *part, const float *part_loss, float *__restrict__ grad, float *loss,
-               const AdamArgs ad) {
-    __shared__ float acc[32][RED_P];
-    let_next_start();
-    wait_for_previous();
-    const int p = threadIdx.x % RED_P, row = threadIdx.x / RED_P, k = blockIdx.x * RED_P + p;
+NB6_DEV void reduce_slice(int slice, int nb, const float *part, const float *part_loss, float *grad, float *loss,
+                          const AdamArgs &ad, float (*acc)[RED_P]) {
+    const int p = threadIdx.x % RED_P, row = threadIdx.x / RED_P, k = slice * RED_P + p;
     const float *src = k < MLP_NPARAM ? part + k : part_loss;
     const size_t step = k < MLP_NPARAM ? MLP_NPARAM : 1;
     const bool mine = row == 0 && k < MLP_NPARAM;
@@ -305,6 +335,75 @@ __global__ void __launch_bounds__(RED_NT)
         }
     } else if (row == 0 && k == MLP_NPARAM) {
         loss[0] += g;
+    }
+}
+
+template <bool ADAM>
+__global__ void __launch_bounds__(RED_NT)
+    mlp_reduce(int nb, const float *part, const float *part_loss, float *grad, float *loss, const AdamArgs ad) {
+    __shared__ float acc[32][RED_P];
+    let_next_start();
+    wait_for_previous();
+    reduce_slice<ADAM>(blockIdx.x, nb, part, part_loss, grad, loss, ad, acc);
+}
+
+// Wait until *count has reached `target`; false (and *err set) after WAIT_MAX
+// polls, about a second.
+constexpr int WAIT_MAX = 1 << 21;
+NB6_DEV bool wait_count(const unsigned *count, unsigned target, unsigned *err) {
+    int bad = 0;
+    if (threadIdx.x == 0) {
+        bad = 1;
+        for (int t = 0; t < WAIT_MAX && bad; ++t) {
+            unsigned c;
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(c) : "l"(count) : "memory");
+            bad = (int)(c - target) < 0;
+        }
+        if (bad) *err = 1u;
+    }
+    return !__syncthreads_or(bad);
+}
+NB6_DEV void add_count(unsigned *count) {
+    __syncthreads();
+    if (threadIdx.x == 0) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(count) : "memory");
+}
+
+// A run of training steps in one cooperative launch: CTA c < ngrad is stream
+// c of a batch, CTA c < nred sums and steps slices of the parameters, and two
+// counters in global memory (partials written, parameters written) order the
+// phases.  Same sums in the same order as mlp_grad_kernel and mlp_reduce.  A
+// step is a chain of short phases, so what a launch costs (its start, the
+// drain before it) was a third of it: 32 steps of 1,024 samples 845 us as 64
+// launches, with the upload and the host's shuffle (some 350 us), now 670.  The
+// next batch's samples are fetched before the wait for the parameters.
+constexpr int NSLICE = MLP_NPARAM / RED_P + 1;   // every parameter, and the loss
+__global__ void __launch_bounds__(GRAD_NT)
+    mlp_steps(const GradArgs g, int nb, int step0, int steps, const float2 *__restrict__ bc, AdamArgs ad,
+              TrainSync *sync) {
+    __shared__ GradSmem sm;
+    __shared__ float acc[32][RED_P];
+    const int stride = nb * GW, first = blockIdx.x, nred = min((int)gridDim.x, NSLICE);
+    const bool grads = first < stride;
+    SampleIn in;
+    if (grads) fetch_sample(g, step0 * g.cnt, 0, first, stride, in);
+    for (int s = step0; s < step0 + steps; ++s) {
+        if (grads) {
+            grad_pass(sm, g, s * g.cnt, first, stride, in);
+            add_count(&sync->done_grad);
+            if (s + 1 < step0 + steps) fetch_sample(g, (s + 1) * g.cnt, 0, first, stride, in);
+        }
+        if (first < nred) {
+            if (!wait_count(&sync->done_grad, (unsigned)(s + 1) * stride, &sync->err)) return;
+            const float2 b = bc[s];
+            ad.bc1 = b.x;
+            ad.bc2 = b.y;
+            for (int k = first; k < NSLICE; k += nred)
+                reduce_slice<true>(k, nb, g.part, g.part_loss, nullptr, &sync->loss, ad, acc);
+            add_count(&sync->done_red);
+        }
+        if (grads && s + 1 < step0 + steps &&
+            !wait_count(&sync->done_red, (unsigned)(s + 1) * nred, &sync->err))
+            return;
     }
 }
 
@@ -382,7 +481,7 @@ void mlp_alloc() {
     M.m2.reserve(MLP_NPARAM);
     M.grad.reserve(MLP_NPARAM);
     M.norm.reserve(MLP_NNORM);
-    M.loss.reserve(1);
+    M.sync.reserve(1);
     M.mom.reserve(MOM_CTAS * MOM_N);
     M.w16.reserve(W16_T + MLP_H * MLP_H);
     M.host.assign(MLP_NPARAM + MLP_NNORM, 0.0f);
@@ -426,12 +525,17 @@ void mlp_upload_samples(int n, const float *x, const float *y) {
 
 int grad_blocks(int cnt) { return std::max(1, std::min((cnt + GS - 1) / GS, nb6_num_sms() * 2)); }
 
+GradArgs grad_args(int cnt, int nb, const int *perm) {
+    M.part.reserve((size_t)nb * GW * (MLP_NPARAM + 1));
+    return GradArgs{cnt,        1.0f / (float)cnt, M.dx.ptr,   M.dy.ptr,   perm,
+                    M.w16.ptr,  M.norm.ptr,        M.part.ptr, M.part.ptr + (size_t)nb * GW * MLP_NPARAM};
+}
+
 // One gradient over samples [off, off+cnt) of the uploaded set: into M.grad,
 // or through the Adam step `adam` into the parameters.
 void mlp_grad_launch(int cnt, int off, const int *perm, const AdamArgs *adam, cudaStream_t st) {
     const int nb = grad_blocks(cnt);
-    M.part.reserve((size_t)nb * GW * (MLP_NPARAM + 1));
-    float *part = M.part.ptr, *part_loss = part + (size_t)nb * GW * MLP_NPARAM;
+    const GradArgs g = grad_args(cnt, nb, perm);
     cudaLaunchAttribute at{};
     at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at.val.programmaticStreamSerializationAllowed = 1;
@@ -441,14 +545,49 @@ void mlp_grad_launch(int cnt, int off, const int *perm, const AdamArgs *adam, cu
     c.numAttrs = 1;
     c.gridDim = dim3(nb, GW);
     c.blockDim = dim3(GRAD_NT);
-    NB6_CUDA_CHECK(cudaLaunchKernelEx(&c, mlp_grad_kernel, cnt, off, 1.0f / (float)cnt, (const float *)M.dx.ptr,
-                                      (const float *)M.dy.ptr, perm, (const __nv_bfloat16 *)M.w16.ptr,
-                                      (const float *)M.norm.ptr, part, part_loss));
-    c.gridDim = dim3(MLP_NPARAM / RED_P + 1);   // every parameter, and the loss
+    NB6_CUDA_CHECK(cudaLaunchKernelEx(&c, mlp_grad_kernel, g, off));
+    c.gridDim = dim3(NSLICE);
     c.blockDim = dim3(RED_NT);
     const AdamArgs ad = adam ? *adam : AdamArgs{};
-    NB6_CUDA_CHECK(cudaLaunchKernelEx(&c, adam ? mlp_reduce<true> : mlp_reduce<false>, nb, (const float *)part,
-                                      (const float *)part_loss, M.grad.ptr, M.loss.ptr, ad));
+    NB6_CUDA_CHECK(cudaLaunchKernelEx(&c, adam ? mlp_reduce<true> : mlp_reduce<false>, nb, (const float *)g.part,
+                                      (const float *)g.part_loss, M.grad.ptr, &M.sync.ptr->loss, ad));
+}
+
+// CTAs of mlp_steps that the device holds at a time; 0 without cooperative
+// launches.
+int steps_capacity() {
+    static const int cap = [] {
+        int dev = 0, coop = 0, occ = 0;
+        NB6_CUDA_CHECK(cudaGetDevice(&dev));
+        NB6_CUDA_CHECK(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
+        NB6_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, mlp_steps, GRAD_NT, 0));
+        return coop ? occ * nb6_num_sms() : 0;
+    }();
+    return cap;
+}
+
+// The training steps of one epoch; bc[s] are the bias corrections of step s.
+// One launch of mlp_steps per STEPS_MAX of them when a batch's CTAs are all on
+// the device at once and its step is short, else two launches a step.
+void mlp_train_steps(int B, int steps, const float2 *bc, const float2 *dbc, AdamArgs ad, cudaStream_t st) {
+    constexpr int STEPS_MAX = 1024, BATCH_MAX = 1 << 20;   // (a step within a millisecond or so)
+    const int nb = grad_blocks(B), ctas = std::max(nb * GW, std::min(NSLICE, nb6_num_sms()));
+    if (ctas > steps_capacity() || B > BATCH_MAX) {
+        for (int s = 0; s < steps; ++s) {
+            ad.bc1 = bc[s].x;
+            ad.bc2 = bc[s].y;
+            mlp_grad_launch(B, s * B, M.perm.ptr, &ad, st);
+        }
+        return;
+    }
+    GradArgs g = grad_args(B, nb, M.perm.ptr);
+    TrainSync *sync = M.sync.ptr;
+    for (int s0 = 0; s0 < steps; s0 += STEPS_MAX) {
+        int n = std::min(STEPS_MAX, steps - s0), b = nb;
+        void *arg[] = {&g, &b, &s0, &n, &dbc, &ad, &sync};
+        NB6_CUDA_CHECK(
+            cudaLaunchCooperativeKernel((const void *)mlp_steps, dim3(ctas), dim3(GRAD_NT), arg, 0, st));
+    }
 }
 
 bool check_n(int n) {
@@ -522,12 +661,12 @@ void nb6_mlp_grad_(int *n, const float *x, const float *y, float *grad, float *l
     if (!check_n(*n)) return;
     mlp_upload_samples(*n, x, y);
     cudaStream_t st = nb6_stream();
-    NB6_CUDA_CHECK(cudaMemsetAsync(M.loss.ptr, 0, sizeof(float), st));
+    NB6_CUDA_CHECK(cudaMemsetAsync(M.sync.ptr, 0, sizeof(TrainSync), st));
     mlp_grad_launch(*n, 0, nullptr, nullptr, st);
     NB6_CUDA_CHECK(cudaStreamSynchronize(st));
     NB6_CUDA_CHECK(cudaMemcpy(grad, M.grad.ptr, sizeof(float) * MLP_NPARAM, cudaMemcpyDeviceToHost));
     float l = 0.0f;
-    NB6_CUDA_CHECK(cudaMemcpy(&l, M.loss.ptr, sizeof(float), cudaMemcpyDeviceToHost));
+    NB6_CUDA_CHECK(cudaMemcpy(&l, &M.sync.ptr->loss, sizeof(float), cudaMemcpyDeviceToHost));
     *loss = l / (float)*n;
 }
 
@@ -554,29 +693,40 @@ void nb6_mlp_train_(int *n_, const float *x, const float *y, int *epochs, int *b
     NB6_CUDA_CHECK(cudaMemsetAsync(M.m1.ptr, 0, sizeof(float) * MLP_NPARAM, st));
     NB6_CUDA_CHECK(cudaMemsetAsync(M.m2.ptr, 0, sizeof(float) * MLP_NPARAM, st));
     M.adam_t = 0;
-    M.perm.reserve(n);
+    const int steps = n / B;
+    const size_t bc_at = ((size_t)n + 1) / 2 * 2;   // in ints, 8-byte aligned
+    M.perm.reserve(bc_at + 2 * (size_t)steps);
     std::vector<int> perm(n);
+    std::vector<float2> bc(steps);
     for (int q = 0; q < n; ++q) perm[q] = q;
     std::mt19937 gen((unsigned)*seed);
     const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
+    const AdamArgs ad{M.w32.ptr, M.m1.ptr, M.m2.ptr, M.w16.ptr, *lr, b1, b2, eps, 1.0f, 1.0f};
     if (*epochs > 0) std::shuffle(perm.begin(), perm.end(), gen);
     for (int e = 0; e < *epochs; ++e) {
-        const Nb6Seg sp{0, perm.data(), sizeof(int) * (size_t)n};
-        nb6_upload(M.perm.ptr, &sp, 1, sp.len, st);
-        NB6_CUDA_CHECK(cudaMemsetAsync(M.loss.ptr, 0, sizeof(float), st));
-        for (int off = 0; off + B <= n; off += B) {
+        for (float2 &c : bc) {
             M.adam_t++;
-            const float bc1 = 1.0f - std::pow(b1, (float)M.adam_t);
-            const float bc2 = 1.0f - std::pow(b2, (float)M.adam_t);
-            const AdamArgs ad{M.w32.ptr, M.m1.ptr, M.m2.ptr, M.w16.ptr, *lr, b1, b2, eps, bc1, bc2};
-            mlp_grad_launch(B, off, M.perm.ptr, &ad, st);
+            c = make_float2(1.0f - std::pow(b1, (float)M.adam_t), 1.0f - std::pow(b2, (float)M.adam_t));
         }
+        const Nb6Seg sp[2] = {{0, perm.data(), sizeof(int) * (size_t)n},
+                              {sizeof(int) * bc_at, bc.data(), sizeof(float2) * (size_t)steps}};
+        nb6_upload(M.perm.ptr, sp, 2, sp[1].off + sp[1].len, st);
+        NB6_CUDA_CHECK(cudaMemsetAsync(M.sync.ptr, 0, sizeof(TrainSync), st));
+        mlp_train_steps(B, steps, bc.data(), reinterpret_cast<const float2 *>(M.perm.ptr + bc_at), ad, st);
         // (the next epoch's order, while the GPU works on this one's)
         if (e + 1 < *epochs) std::shuffle(perm.begin(), perm.end(), gen);
-        float l = 0.0f;
         NB6_CUDA_CHECK(cudaStreamSynchronize(st));
-        NB6_CUDA_CHECK(cudaMemcpy(&l, M.loss.ptr, sizeof(float), cudaMemcpyDeviceToHost));
-        if (loss_hist) loss_hist[e] = l / (float)((n / B) * B);
+        struct {
+            float loss;
+            unsigned err;
+        } res{};
+        static_assert(offsetof(TrainSync, err) == offsetof(TrainSync, loss) + sizeof(float), "read together");
+        NB6_CUDA_CHECK(cudaMemcpy(&res, &M.sync.ptr->loss, sizeof(res), cudaMemcpyDeviceToHost));
+        if (res.err) {
+            nb6_fatal(NB6_ERR_WAIT_TIMEOUT);
+            return;
+        }
+        if (loss_hist) loss_hist[e] = res.loss / (float)(steps * B);
     }
     mlp_download();
 }

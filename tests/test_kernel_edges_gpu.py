@@ -4,6 +4,7 @@ other parity tests (acceleration and potential 1e-6, jerk 1e-5 relative), which
 the FP32 pair math on hi/lo differences with double-single sums meets at any
 size; neighbour lists identical."""
 import ctypes as C
+import subprocess
 
 import numpy as np
 import pytest
@@ -50,6 +51,77 @@ def test_mlp_gradient_sample_counts(n):
     gr, lr = M.grad(model, x, y)
     assert abs(loss - lr) <= 1e-5 * lr
     assert np.linalg.norm(g - gr) <= 2e-5 * np.linalg.norm(gr)
+
+
+@pytest.fixture(scope="module")
+def shuffled(tmp_path_factory):
+    """The order std::shuffle gives 0..n-1 with a std::mt19937 of `seed`."""
+    d = tmp_path_factory.mktemp("shuffle")
+    (d / "s.cpp").write_text("""#include <algorithm>
+#include <numeric>
+#include <random>
+extern "C" void order(int n, unsigned seed, int *p) {
+    std::iota(p, p + n, 0);
+    std::mt19937 gen(seed);
+    std::shuffle(p, p + n, gen);
+}""")
+    subprocess.run(["g++", "-O1", "-shared", "-fPIC", "-o", str(d / "s.so"), str(d / "s.cpp")], check=True)
+    lib = C.CDLL(str(d / "s.so"))
+
+    def order(n, seed):
+        p = np.empty(n, dtype=np.int32)
+        lib.order(n, seed, p.ctypes.data_as(C.c_void_p))
+        return p
+    return order
+
+
+# 32 samples per four CTAs, one round; 145 CTAs sum the parameters, more CTAs
+# hold the samples from a batch of 1,153; 1,024 steps per launch; two launches
+# a step once the CTAs no longer fit (4,736 here at the latest: 4 per SM)
+@pytest.mark.parametrize("n,batch", [(1, 1), (1030, 1), (700, 33), (3000, 256), (4100, 1000), (4000, 1152),
+                                     (4000, 1184), (20011, 2500), (11000, 3552), (15000, 4737)])
+def test_mlp_training_steps(shuffled, n, batch):
+    """One epoch against Adam on the FP64 oracle's gradients.  A gradient
+    within 2e-5 of its norm turns the sign of about that share of its elements,
+    which moves a parameter by two learning rates: 1% of the parameters' change
+    (bound 2%).  The mean loss follows to 1e-3; a second run gives the same
+    bits."""
+    import mlp_oracle as M
+    from nb6b200 import mlp
+    rng = np.random.default_rng(n + batch)
+    model = np.zeros(M.NPARAM + M.NNORM, dtype=np.float32)
+    model[:M.NPARAM] = rng.normal(size=M.NPARAM) * 0.15
+    model[M.NPARAM + M.IN:M.NPARAM + 2 * M.IN] = 1.0
+    model[-1] = 1.0
+    x = rng.normal(size=(n, 5)).astype(np.float32)
+    y = (x[:, 0] - 0.3 * x[:, 1] * x[:, 2] + 0.1 * rng.normal(size=n)).astype(np.float32)
+    lr = 1e-5 if n // batch > 100 else 1e-4
+    runs = []
+    for _ in range(2):
+        mlp.set_model(model)
+        hist = mlp.train(x, y, epochs=1, batch=batch, lr=lr, seed=5)
+        runs.append((mlp.get_model(), hist))
+    np.testing.assert_array_equal(runs[0][0], runs[1][0])
+    np.testing.assert_array_equal(runs[0][1], runs[1][1])
+    got, hist = runs[0]
+    nm = got[M.NPARAM:].astype(np.float64)
+    xs = x.astype(np.float64)
+    std = np.sqrt(np.maximum(xs.var(0), 1e-12))
+    np.testing.assert_allclose(nm[:5], xs.mean(0), atol=1e-6)
+    np.testing.assert_allclose(nm[5:10], 1 / std, rtol=1e-6)
+    order = shuffled(n, 5)
+    w = model[:M.NPARAM].astype(np.float64)
+    b1, b2, one = np.float32(0.9), np.float32(0.999), np.float32(1)
+    m1, m2, losses = np.zeros(M.NPARAM), np.zeros(M.NPARAM), []
+    for t in range(1, n // batch + 1):
+        s = order[(t - 1) * batch:t * batch]
+        g, loss = M.grad64(M.bf16_round(w).astype(np.float64), nm, x[s], y[s])
+        losses.append(loss)
+        m1 = b1 * m1 + (one - b1) * g
+        m2 = b2 * m2 + (one - b2) * g * g
+        w = w - lr * (m1 / (1 - float(b1) ** t)) / (np.sqrt(m2 / (1 - float(b2) ** t)) + 1e-8)
+    assert abs(hist[0] - np.mean(losses)) <= 1e-3 * np.mean(losses) + 1e-12
+    assert np.linalg.norm(got[:M.NPARAM] - w) <= 0.02 * np.linalg.norm(w - model[:M.NPARAM])
 
 
 def _shells(n, seed):
