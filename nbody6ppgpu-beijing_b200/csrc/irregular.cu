@@ -443,11 +443,12 @@ template <bool KS, bool PV, int NA>
 __global__ void __launch_bounds__(IRR_WARPS * 32)
     irr_kernel(int ni, const __grid_constant__ ActiveAddr<NA> addr, double ti, const Rec *__restrict__ rec,
                const Pv *__restrict__ pv, const int *__restrict__ lists, int ls, int nmax, KsArgs ks,
-               double *__restrict__ out, double *__restrict__ fv, const int *status, int *hstatus) {
+               double *__restrict__ out, double *__restrict__ fv, const int *status, int *hstatus, DevSpan *span) {
     static_assert(!(KS && PV), "the predicted-set walk has no pair table");
     __shared__ __align__(128) double2 sm[KS ? 1 : IRR_WARPS][KS ? 1 : 64 * (PV ? 4 : 8)];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int k = blockIdx.x * IRR_WARPS + warp;
+    if (NA > 0 && k == 0 && lane == 0) span_begin(span);
     if (hstatus && k == 0 && lane == 0) *hstatus = *status;
     if (k >= ni) return;
     const int i = addr[k] - 1;
@@ -475,6 +476,7 @@ __global__ void __launch_bounds__(IRR_WARPS * 32)
         else if (lane == 6) oi[k] = id;
         else if (lane == 7) oi[ni + k] = nnb;
     }
+    if (NA > 0 && lane == 0) span_end(span);
 }
 
 // ----------------------------------------------------------------------------
@@ -1523,7 +1525,9 @@ struct IrrState {
     size_t list_words = 0;
     double time_grav = 0;
     unsigned long long num_inter = 0, num_fcall = 0, num_steps = 0;
-    cudaEvent_t ev0 = nullptr, ev1 = nullptr;  // irr_kernel of the last call
+    cudaEvent_t ev0 = nullptr, ev1 = nullptr;  // irr_kernel of the last call; a small one stamps its own time
+    DevBuf<DevSpan> span;
+    bool stamped = false;
     cudaStream_t cst = nullptr;                // downloads of the chunks' results
     cudaEvent_t evk[IRR_CHUNKS] = {}, evc[IRR_CHUNKS] = {};   // chunk kernel / download done
     int chunks_max = IRR_CHUNKS;               // nb6_irr_tune_
@@ -1636,13 +1640,13 @@ void launch_irr_kernel(int ni, const int *daddr, double ti, double *out, cudaStr
     const ActiveAddr<0> ad{daddr};
     if (ks.slot)
         irr_kernel<true, false, 0><<<grid, block, 0, st>>>(ni, ad, ti, rec, nullptr, lists, I.lmax, I.nmax, ks, out,
-                                                           fv, status, hstatus);
+                                                           fv, status, hstatus, nullptr);
     else if (pv)
         irr_kernel<false, true, 0><<<grid, block, 0, st>>>(ni, ad, ti, rec, pv, lists, I.lmax, I.nmax, ks, out, fv,
-                                                           status, hstatus);
+                                                           status, hstatus, nullptr);
     else
         irr_kernel<false, false, 0><<<grid, block, 0, st>>>(ni, ad, ti, rec, nullptr, lists, I.lmax, I.nmax, ks, out,
-                                                            fv, status, hstatus);
+                                                            fv, status, hstatus, nullptr);
 }
 
 // The record walk of ni <= IRR_INLINE bodies, their addresses (host memory)
@@ -1652,7 +1656,7 @@ void launch_irr_inline(int ni, const int *addr, double ti, cudaStream_t st, doub
     memcpy(ad.v, addr, sizeof(int) * ni);
     irr_kernel<false, false, IRR_INLINE><<<(ni + IRR_WARPS - 1) / IRR_WARPS, IRR_WARPS * 32, 0, st>>>(
         ni, ad, ti, I.rec.ptr, nullptr, I.lists.ptr, I.lmax, I.nmax, KsArgs{}, nullptr, fv, nb6_dev_status(),
-        hstatus);
+        hstatus, I.span.ptr);
 }
 
 __global__ void ks_scatter_slots(int npair, const int *__restrict__ cm, int *__restrict__ slot) {
@@ -2000,7 +2004,12 @@ void irr_firr_vec_impl(double ti, int ni, const int *addr, double (*acc)[3], dou
     }
     CopyPool *pool = direct ? nullptr : &nb6_copy_pool();
     auto chunk_lo = [&](int c) { return (int)((long long)ni * c / nch); };
-    NB6_CUDA_CHECK(cudaEventRecord(I.ev0, st));
+    if (small && !I.span.ptr) {
+        I.span.reserve(1);
+        NB6_CUDA_CHECK(cudaMemsetAsync(I.span.ptr, 0, sizeof(DevSpan), st));
+    }
+    I.stamped = small;
+    if (!small) NB6_CUDA_CHECK(cudaEventRecord(I.ev0, st));
     const Pv *pv = irr_predicted_set(ni, ti, st);
     int *hstatus = direct ? nb6_status_post() : nullptr;
     for (int c = 0; c < nch; ++c) {
@@ -2016,7 +2025,7 @@ void irr_firr_vec_impl(double ti, int ni, const int *addr, double (*acc)[3], dou
             NB6_CUDA_CHECK(cudaEventRecord(I.evc[c], I.cst));
         }
     }
-    NB6_CUDA_CHECK(cudaEventRecord(I.ev1, st));
+    if (!small) NB6_CUDA_CHECK(cudaEventRecord(I.ev1, st));
     if (!direct) nb6_status_fetch(st);
     unsigned long long inter = 0;
     if (pool) pool->arm();
@@ -2145,6 +2154,7 @@ void irr_correct_impl(double time, int ni, const int *addr, double *out) {
         NB6_CUDA_CHECK(cudaEventCreate(&I.ev0));
         NB6_CUDA_CHECK(cudaEventCreate(&I.ev1));
     }
+    I.stamped = false;
     NB6_CUDA_CHECK(cudaEventRecord(I.ev0, st));
     launch_irr_kernel(ni, daddr, time, force, st, nullptr, irr_predicted_set(ni, time, st));
     NB6_CUDA_CHECK(cudaGetLastError());
@@ -2929,6 +2939,7 @@ void nb6_regf_correct_(double *time, int *ni, int *addr, int *iseg, int *nseg, i
 // kernel of the last irr_simd_firr_vec_ call.
 float nb6_irr_last_kernel_ms_() {
     if (!I.ev1) return 0.f;
+    if (I.stamped) return nb6_span_ms(I.span.ptr, nb6_stream());
     float ms = 0.f;
     NB6_CUDA_CHECK(cudaEventSynchronize(I.ev1));
     NB6_CUDA_CHECK(cudaEventElapsedTime(&ms, I.ev0, I.ev1));

@@ -258,7 +258,7 @@ __global__ void __launch_bounds__(NT, NI == 2 ? 5 : 8) pot_kernel(const PotArgs 
 // index) or out[k].  hstatus: see nb6_status_post.
 __global__ void pot_finalize(const float2 *__restrict__ part, int nslices, int i0, int ni,
                              const int *__restrict__ idx, double *__restrict__ out, const int *status,
-                             int *hstatus) {
+                             int *hstatus, DevSpan *span) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (hstatus && k == 0) *hstatus = *status;
     if (k >= ni) return;
@@ -269,6 +269,7 @@ __global__ void pot_finalize(const float2 *__restrict__ part, int nslices, int i
         v += (double)p.x + (double)p.y;
     }
     out[idx ? idx[k] - i0 : k] = v;
+    if (span && threadIdx.x == 0) span_end(span);
 }
 
 // One CTA per tile: its rows of the tile layout, from the bodies in the
@@ -280,9 +281,11 @@ __global__ void pot_finalize(const float2 *__restrict__ part, int nslices, int i
 template <bool ORD>
 __global__ void __launch_bounds__(JT) pot_tiles(int n, const int *__restrict__ perm, const double *__restrict__ m,
                                                 const double *__restrict__ x, double *__restrict__ keep,
-                                                float *__restrict__ tiles, float4 *__restrict__ tbox, int *status) {
+                                                float *__restrict__ tiles, float4 *__restrict__ tbox, int *status,
+                                                DevSpan *span) {
     constexpr int ROWS = ORD ? ROWS_ORD : ROWS_HL;
     const int t = threadIdx.x, s = blockIdx.x * JT + t;
+    if (span && s == 0) span_begin(span);
     double c[3] = {1.0e15, 1.0e15, 1.0e15}, mj = 0.0;
     if (s < n) {
         const size_t j = ORD ? perm[s] : s;
@@ -382,7 +385,9 @@ struct PotState {
     int n = 0, ntile = 0;
     const double *dm = nullptr, *dx = nullptr;  // the m, x of the call, readable by kernels
     double *keep = nullptr;                     // where to keep x when dx is pinned host memory
-    cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+    cudaEvent_t ev0 = nullptr, ev1 = nullptr;   // an ordered call's time; an unordered one stamps its own
+    DevBuf<DevSpan> span;
+    bool stamped = false;
     float last_ms = 0.f;
 };
 PotState P;
@@ -438,7 +443,7 @@ bool pot_compute(int i0, int ni, double *hout, cudaStream_t st) {
         P.order.build(n, P.dx, st);
         P.tbox.reserve(2 * (size_t)P.ntile);
         pot_tiles<true><<<P.ntile, JT, 0, st>>>(n, P.order.perm.ptr, P.dm, P.dx, nullptr, P.tiles.ptr, P.tbox.ptr,
-                                                a.status);
+                                                a.status, nullptr);
         NB6_CUDA_CHECK(cudaGetLastError());
         a.tbox = P.tbox.ptr;
         a.idx = P.order.perm.ptr;
@@ -452,7 +457,8 @@ bool pot_compute(int i0, int ni, double *hout, cudaStream_t st) {
             a.idx = P.idx.ptr;
         }
     } else {
-        pot_tiles<false><<<P.ntile, JT, 0, st>>>(n, nullptr, P.dm, P.dx, P.keep, P.tiles.ptr, nullptr, a.status);
+        pot_tiles<false><<<P.ntile, JT, 0, st>>>(n, nullptr, P.dm, P.dx, P.keep, P.tiles.ptr, nullptr, a.status,
+                                                 P.span.ptr);
         NB6_CUDA_CHECK(cudaGetLastError());
     }
     // two i per thread once that still leaves a tile of i for every SM
@@ -464,9 +470,17 @@ bool pot_compute(int i0, int ni, double *hout, cudaStream_t st) {
     P.out.reserve(ni);
     pot_finalize<<<(ni + 127) / 128, 128, 0, st>>>(P.part.ptr, a.nslices, i0, ni, a.idx,
                                                    direct ? hout : P.out.ptr, a.status,
-                                                   direct ? nb6_status_post() : nullptr);
+                                                   direct ? nb6_status_post() : nullptr, ord ? nullptr : P.span.ptr);
     NB6_CUDA_CHECK(cudaGetLastError());
     return direct;
+}
+
+void pot_timing_init(cudaStream_t st) {
+    if (P.ev0) return;
+    NB6_CUDA_CHECK(cudaEventCreate(&P.ev0));
+    NB6_CUDA_CHECK(cudaEventCreate(&P.ev1));
+    P.span.reserve(1);
+    NB6_CUDA_CHECK(cudaMemsetAsync(P.span.ptr, 0, sizeof(DevSpan), st));
 }
 
 // The bodies of a call where kernels read them: on the device, or (a small
@@ -506,15 +520,13 @@ void gpupot_(int *irank, int *istart, int *ni_, int *n_, double *m, double (*x)[
     }
     const double t0 = nb6_wtime();
     cudaStream_t st = nb6_stream();
-    if (!P.ev0) {
-        NB6_CUDA_CHECK(cudaEventCreate(&P.ev0));
-        NB6_CUDA_CHECK(cudaEventCreate(&P.ev1));
-    }
+    pot_timing_init(st);
     P.hout.reserve(ni);
     pot_upload(n, m, &x[0][0], st, true);
-    NB6_CUDA_CHECK(cudaEventRecord(P.ev0, st));
+    P.stamped = !pot_ordered(ni);
+    if (!P.stamped) NB6_CUDA_CHECK(cudaEventRecord(P.ev0, st));
     const bool direct = pot_compute(i0, ni, nb6_uva() ? P.hout.ptr : nullptr, st);
-    NB6_CUDA_CHECK(cudaEventRecord(P.ev1, st));
+    if (!P.stamped) NB6_CUDA_CHECK(cudaEventRecord(P.ev1, st));
     if (!direct) {
         NB6_CUDA_CHECK(cudaMemcpyAsync(P.hout.ptr, P.out.ptr, sizeof(double) * ni, cudaMemcpyDeviceToHost, st));
         nb6_status_fetch(st);
@@ -534,20 +546,19 @@ void nb6_pot_device_(int *istart, int *ni, int *n, const double *d_m, const doub
                      double **d_out) {
     nb6_devinit_once(0);
     cudaStream_t st = nb6_stream();
-    if (!P.ev0) {
-        NB6_CUDA_CHECK(cudaEventCreate(&P.ev0));
-        NB6_CUDA_CHECK(cudaEventCreate(&P.ev1));
-    }
+    pot_timing_init(st);
     pot_upload(*n, d_m, d_x, st, false);
-    NB6_CUDA_CHECK(cudaEventRecord(P.ev0, st));
+    P.stamped = !pot_ordered(*ni);
+    if (!P.stamped) NB6_CUDA_CHECK(cudaEventRecord(P.ev0, st));
     pot_compute(*istart - 1, *ni, nullptr, st);
-    NB6_CUDA_CHECK(cudaEventRecord(P.ev1, st));
+    if (!P.stamped) NB6_CUDA_CHECK(cudaEventRecord(P.ev1, st));
     *d_out = P.out.ptr;
 }
 
 // Device time (ms) of the last potential call after its upload: packing,
 // spatial order, kernel and sums (after a sync).
 float nb6_pot_last_kernel_ms_() {
+    if (P.stamped) return P.last_ms = nb6_span_ms(P.span.ptr, nb6_stream());
     NB6_CUDA_CHECK(cudaEventSynchronize(P.ev1));
     NB6_CUDA_CHECK(cudaEventElapsedTime(&P.last_ms, P.ev0, P.ev1));
     return P.last_ms;

@@ -187,6 +187,13 @@ int *nb6_status_post() {
     return g_status_host;
 }
 
+float nb6_span_ms(const DevSpan *s, cudaStream_t st) {
+    DevSpan h{};
+    NB6_CUDA_CHECK(cudaStreamSynchronize(st));
+    NB6_CUDA_CHECK(cudaMemcpy(&h, s, sizeof(h), cudaMemcpyDeviceToHost));
+    return h.t1 > h.t0 ? 1e-6f * (float)(h.t1 - h.t0) : 0.0f;
+}
+
 // Read (and clear) the device status word; call after a stream sync.
 int nb6_check_dev_status() {
     int st = 0;

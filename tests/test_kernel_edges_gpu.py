@@ -292,3 +292,44 @@ def test_segmented_many_items(nb6, orc, cap):
                     assert rel_err_vec(pot[s][ok], op[ok]).max() <= 1e-6
     finally:
         nb6.gpunb_close()
+
+
+def test_kernel_times_of_small_and_large_calls(nb6):
+    """The kernel time of a call that stamps its own (small) and of one timed
+    by events (large), alternating: more than zero, within the call's wall
+    time, and the large one's not left over from the small one."""
+    import time
+
+    from nb6b200 import ics
+    lib = nb6.lib
+
+    def timed(call, ms):
+        t = time.perf_counter()
+        call()
+        wall = 1e3 * (time.perf_counter() - t)
+        got = float(ms())
+        assert 0.0 < got <= wall
+        return got
+
+    big, small = ics.plummer(40960, seed=3), ics.plummer(300, seed=4)
+    nb6.gpupot(big.mass, big.pos)
+    for _ in range(2):
+        a = timed(lambda: nb6.gpupot(small.mass, small.pos), lib.nb6_pot_last_kernel_ms_)
+        b = timed(lambda: nb6.gpupot(big.mass, big.pos), lib.nb6_pot_last_kernel_ms_)
+        assert b > a
+    n, zero = 20000, np.zeros((20000, 3))
+    cl = ics.plummer(n, seed=5)
+    rng = np.random.default_rng(6)
+    nb6.irr_open(n, 64, 0)
+    try:
+        nb6.irr_set_jp_all(cl.pos, cl.vel, zero, zero, cl.mass, np.zeros(n))
+        for i in range(n):
+            nb6.irr_set_list(i + 1, np.concatenate([[40], rng.integers(1, n + 1, 40)]).astype(np.int32))
+        few, many = np.arange(1, 101, dtype=np.int32), np.arange(1, n + 1, dtype=np.int32)
+        nb6.irr_firr_vec(0.0, many)
+        for _ in range(2):
+            a = timed(lambda: nb6.irr_firr_vec(0.0, few), lib.nb6_irr_last_kernel_ms_)
+            b = timed(lambda: nb6.irr_firr_vec(0.0, many), lib.nb6_irr_last_kernel_ms_)
+            assert b > a
+    finally:
+        nb6.irr_close(0)
