@@ -52,9 +52,10 @@ METRIC = "Regular force+jerk+nbr pair interactions/s at N=1M"
 FLOPS_PER_PAIR = 60          # gpunb.velocity.cu:895, reg.avx.cpp:343
 # DRAM bytes (read + write) per launch of the headline force kernel,
 # regf_x2_kernel<1> with 1024 i x 996,147 j over the Morton-ordered j set
-# (tile-relative far operands included), from one ncu capture of that
-# launch: dram__bytes_read.sum 69.58 MB + dram__bytes_write.sum 3.45 MB.
-NCU_TRAFFIC_PER_LAUNCH = 69.58e6 + 3.45e6
+# (tile-relative far operands included), from an ncu capture of two such
+# launches (means): dram__bytes_read.sum 69.52 MB + dram__bytes_write.sum
+# 6.88 MB.
+NCU_TRAFFIC_PER_LAUNCH = 69.52e6 + 6.88e6
 
 
 def parse():
