@@ -1662,6 +1662,7 @@ int occupancy(int variant, bool mf) {
 // end (1,024 of 996,147 King bodies: one wave 1,131 us, three 1,069, six
 // 1,062, twelve 1,076).
 constexpr int X2_WAVES = 6, X2_MIN_TILES = 8;
+constexpr int GRID_Y_MAX = 65535;   // slices are the grid's y
 Plan make_plan(int variant, int ni, int nj, int ntile, bool mf, int forced_slices) {
     Plan p;
     p.variant = variant;
@@ -1690,8 +1691,9 @@ Plan make_plan(int variant, int ni, int nj, int ntile, bool mf, int forced_slice
             }
         }
     }
-    if (forced_slices > 0) p.nslices = variant > 0 ? std::min(forced_slices, ntile) : forced_slices;
-    p.nslices = std::max(p.nslices, 1);
+    // (slices beyond the tiles, or the bodies, would be empty)
+    if (forced_slices > 0) p.nslices = std::min(forced_slices, variant > 0 ? ntile : std::max(nj, 1));
+    p.nslices = std::min(std::max(p.nslices, 1), GRID_Y_MAX);
     return p;
 }
 
@@ -2159,10 +2161,16 @@ static void regf_prepare(int ni, const double *d_h2, const double *d_dtr, const 
         if (ncand == 0) tune_now = false;
     }
     Plan plan = make_plan(variant, ni, R.nj, R.ntile, mf, R.forced_slices);
+    // room for the partials of the default, of every trial, and of the call
+    // itself whichever variant the trials choose
     size_t part_need = (size_t)plan.nslices * ni_pad;
     if (tune_now)
-        for (int c = 0; c < ncand; ++c)
-            part_need = std::max<size_t>(part_need, (size_t)make_plan(cands[c], nt, R.nj, R.ntile, mf, 0).nslices * nt);
+        for (int c = 0; c < ncand; ++c) {
+            const size_t trial = (size_t)make_plan(cands[c], nt, R.nj, R.ntile, mf, 0).nslices * nt;
+            const size_t call =
+                (size_t)make_plan(cands[c], ni, R.nj, R.ntile, mf, R.forced_slices).nslices * ni_pad;
+            part_need = std::max(part_need, std::max(trial, call));
+        }
     R.part.reserve(part_need * 4);
     nbcnt_reserve(ni, st);
     R.nbbuf.reserve((size_t)ni * std::max(cap, 1));

@@ -186,6 +186,42 @@ def test_candidate_queue_band_and_overflow(nb6, orc, variant, n):
         nb6.gpunb_close()
 
 
+@pytest.mark.parametrize("ni,nj,slices", [(200, 1024, 500), (5, 1024, 500), (1500, 2050, 77), (9000, 9000, 3),
+                                          (3, 1025, 70000)])
+def test_forced_slices_on_the_tuning_call(nb6, orc, ni, nj, slices):
+    """A forced slice count with the variant left to the tuner, on the first
+    call of its bucket: the partials have room for the variant that wins, more
+    slices than bodies (or than a grid holds) are accepted, and a second call,
+    which no longer tunes, gives the same bits."""
+    from nb6b200 import ics
+    cl = ics.plummer(nj, seed=nj, imf=True)
+    h2 = cl.h2(0)[:ni]
+    raw, geom = nb6.lib, (C.c_int * 3)()
+    raw.nb6_regf_tune_(C.byref(C.c_int(0)), C.byref(C.c_int(slices)))
+    raw.nb6_regf_autotune_(C.byref(C.c_int(-1)))
+    try:
+        nb6.gpunb_open(nj, 0)
+        nb6.gpunb_send(cl.mass, cl.pos, cl.vel)
+        runs = []
+        for _ in range(2):
+            runs.append(nb6.gpunb_regf(h2, cl.dtr[:ni], cl.pos[:ni], cl.vel[:ni], 512, 400, 0))
+            raw.nb6_regf_last_geometry_(geom)
+            most = -(-nj // 128) if geom[0] > 0 else nj
+            assert geom[2] == min(slices, most, 65535)
+    finally:
+        raw.nb6_regf_tune_(C.byref(C.c_int(0)), C.byref(C.c_int(0)))
+        raw.nb6_regf_autotune_(C.byref(C.c_int(-1)))
+        nb6.gpunb_close()
+    for a, b in zip(*runs):
+        np.testing.assert_array_equal(a, b)
+    acc, jrk, pot, lst = runs[0]
+    oa, oj, op, ol = orc.regf(cl.mass, cl.pos, cl.vel, h2, cl.dtr[:ni], cl.pos[:ni], cl.vel[:ni], 512, 400, 0)
+    np.testing.assert_array_equal(lst, ol)
+    assert rel_err_vec(acc, oa).max() <= 1e-6
+    assert rel_err_vec(jrk, oj).max() <= 1e-5
+    assert rel_err_vec(pot, op).max() <= 1e-6
+
+
 @pytest.mark.parametrize("cap", [31, 400, 512, 700])
 def test_list_rows_at_register_widths(nb6, orc, cap):
     """List rows whose count falls on either side of the widths the sort
