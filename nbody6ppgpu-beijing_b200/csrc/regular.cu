@@ -1402,6 +1402,9 @@ __global__ void __launch_bounds__(JPAR_NT, JPAR_CTAS)
     regf_seg_kernel(const RegArgs a, const SegItem *__restrict__ items, int nitems, const RowOut ro) {
     __shared__ __align__(16) JparI<IB> S;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    // at the head (nothing here sets it): the host reads it behind the first
+    // stage's flag, before it touches the caller's arrays
+    post_status(a.status, ro.hstatus);
     int w = blockIdx.x, round = 0;
     SegItem it = items[w];   // (the grid is no larger than the list)
     jpar_fetch_i<IB>(a, S, 0, it.i0, it.ni);
@@ -1454,7 +1457,6 @@ __global__ void __launch_bounds__(JPAR_NT, JPAR_CTAS)
         __syncthreads();
         if (tid == 0) post_stage();
     }
-    if (ro.hstatus && blockIdx.x == 0 && tid == 0) *ro.hstatus = *a.status;
 }
 
 __global__ void __launch_bounds__(FIN_WARPS * 32)
@@ -3136,7 +3138,8 @@ void nb6_regf_seg_(int *ni_, int *iseg, double *h2, double *dtr, double (*xi)[3]
         unpacked = true;
         for (int lo = 0, sg = 0; lo < nitems && unpacked; lo += per, ++sg) {
             const int hi = std::min(lo + per, nitems);
-            unpacked = wait_flag(R.stage_flag.ptr + sg, st);
+            // (with an error from the launches before, none is unpacked)
+            unpacked = wait_flag(R.stage_flag.ptr + sg, st) && *(volatile const int *)hstatus == NB6_OK;
             if (!unpacked) break;
             const int np = pool.parts();
             pool.run([&](int p) {
@@ -3150,7 +3153,7 @@ void nb6_regf_seg_(int *ni_, int *iseg, double *h2, double *dtr, double (*xi)[3]
     const double wt2 = nb6_wtime();
     R.time_grav += wt2;
     R.time_reduce -= wt2;
-    if (nb6_check_dev_status() != 0) {   // (the caller's arrays may hold part of the results)
+    if (nb6_check_dev_status() != 0) {
         R.nbcnt_dirty = true;
         return;
     }

@@ -294,6 +294,44 @@ def test_irregular_rounds_and_call_sizes(nb6, orc, mode, ni):
         nb6.irr_close(0)
 
 
+def test_failed_segmented_call_leaves_the_callers_arrays(nb6, orc):
+    """A segmented call in stages against a j set with a NaN in its last
+    segment: the status is reported and no row of the caller's arrays is
+    touched; a good set sent afterwards gives the oracle's rows."""
+    import nb6b200
+    rng = np.random.default_rng(8)
+    nc, nseg = 300, 70
+    n, cap = nc * nseg, 60
+    x, v = rng.normal(size=(n, 3)), 0.3 * rng.normal(size=(n, 3))
+    m = rng.uniform(0.5, 1.5, n) / n
+    j0 = (nc * np.arange(nseg + 1)).astype(np.int32)
+    iseg = np.repeat(np.arange(nseg), nc).astype(np.int32)
+    h2, dtr = np.full(n, 0.2), np.full(n, 2.0 ** -6)
+    bad = x.copy()
+    bad[n - 1, 1] = np.nan
+    nb6b200.set_abort_on_error(False)
+    nb6.gpunb_open(n, 0)
+    try:
+        nb6b200.last_status()
+        nb6.gpunb_send(m, bad, v)
+        for o in nb6.regf_seg(h2, dtr, x, v, iseg, j0, cap + 1, cap, 0):
+            assert not o.any()
+        assert nb6b200.last_status() == 3
+        geom = (C.c_int * 3)()
+        nb6.lib.nb6_regf_last_geometry_(geom)
+        assert geom[2] >= 8 * geom[1]      # rounds enough for stages
+        nb6.gpunb_send(m, x, v)
+        out = nb6.regf_seg(h2, dtr, x, v, iseg, j0, cap + 1, cap, 0)
+        assert nb6b200.last_status() == 0
+    finally:
+        nb6b200.set_abort_on_error(True)
+        nb6.gpunb_close()
+    for c in (0, 34, nseg - 1):
+        s = slice(j0[c], j0[c + 1])
+        ol = orc.regf(m[s], x[s], v[s], h2[s], dtr[s], x[s], v[s], cap + 1, cap, 0)[3]
+        np.testing.assert_array_equal(out[3][s], ol)
+
+
 @pytest.mark.parametrize("cap", [20, 60, 600])
 def test_segmented_many_items(nb6, orc, cap):
     """A segmented call of many work items per CTA, whose rows reach the
