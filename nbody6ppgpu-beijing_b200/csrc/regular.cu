@@ -906,6 +906,17 @@ __global__ void __launch_bounds__(NT, X2_MINB / NI) regf_x2_kernel(const RegArgs
 // (Four warps per CTA: with eight the segmented kernel's warps waited at its
 // barriers for a fifth of their time, 308 us against 278 for 64 clusters.)
 constexpr int JPAR_NT = 128, JPAR_CTAS = 512 / JPAR_NT;   // 16 warps per SM
+// How many terms a thread's FP32 sums take before they join the FP64 ones:
+// the segmented kernel folds them every SEG_FOLD j's, and half way through an
+// item that is all of its group's j range (Q = 1; its chains were half as long
+// with 256 threads).  The j-parallel launches get enough slices for JPAR_CHAIN.
+// With a chain per item, 2 segments of 262,144 bodies (2,048 terms a thread)
+// were up to 2.8e-5 off where all terms are alike, now 1.1e-7; 2 Plummer clusters
+// of about 60,000, a fifth active, 6.5e-8 (acceleration, root mean square), now
+// 4.6e-8, and 64 of 512-8,192, a tenth active, 5.8e-8, now 5.6e-8.  A fold costs
+// three quarters of a j's work: the kernel takes 308 -> 315 us on those 64 and
+// 3.29 -> 3.46 ms on those two.
+constexpr int SEG_FOLD = 32, SEG_FOLD_MIN = 4, JPAR_CHAIN = 128;
 
 // The i-particles of a j-parallel CTA in shared memory: sip[k] = (xH, yH, zH,
 // 1.01 h2), (xL, yL, zL, dtr), (vx, vy, vz, 0) of particle k, and, for the
@@ -990,7 +1001,7 @@ NB6_DEV void jpar_fetch_wait() {
 // Each thread loads its next j before the arithmetic of the current one: at
 // 16 warps per SM (the sums of four i take 100 registers) the L2 round trip
 // was the top stall.  With the ballot-ranked pushes and the transposing
-// reduction (jpar_reduce): 37 i of 500,009 bodies 70 -> 56 us, 531 of 16,384
+// reduction (jpar_fold): 37 i of 500,009 bodies 70 -> 56 us, 531 of 16,384
 // 41 -> 32 us, the 64-cluster work list of regf_seg_kernel 299 -> 245 us.
 template <int IB, bool MFLAG, bool X2>
 NB6_DEV void jpar_loop(const RegArgs &a, JparI<IB> &S, int buf, int j_begin, int j_end, int i0, int nvalid,
@@ -1128,13 +1139,13 @@ NB6_DEV void jpar_loop(const RegArgs &a, JparI<IB> &S, int buf, int j_begin, int
     }
 }
 
-// The CTA's sums of its IB i-particles in FP64: S.red[warp][7 k + c], summed
-// over the warps by jpar_total (after the barrier here).  Each warp transposes
-// its lanes' sums through shared memory, so that a lane adds up one sum's 32
-// terms: a shuffle tree for each of the 28 sums of IB = 4 took 420
-// instructions, a fifth of a 4,600-pair work item.
+// A warp's FP32 sums of the IB i-particles into its FP64 ones, S.red[warp][7 k
+// + c] (add: there are some already), which jpar_total sums over the warps
+// (after a barrier).  The warp transposes its lanes' sums through shared memory,
+// so that a lane adds up one sum's 32 terms: a shuffle tree for each of the 28
+// sums of IB = 4 took 420 instructions, a fifth of a 4,600-pair work item.
 template <int IB>
-NB6_DEV void jpar_reduce(JparI<IB> &S, const Sums *s) {
+NB6_DEV void jpar_fold(JparI<IB> &S, const Sums *s, bool add = false) {
     constexpr int V = JparI<IB>::V, CH = JparI<IB>::CH;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
 #pragma unroll
@@ -1150,11 +1161,12 @@ NB6_DEV void jpar_reduce(JparI<IB> &S, const Sums *s) {
             double w[4] = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll
             for (int l = 0; l < 32; ++l) w[l & 3] += (double)S.tr[warp][lane][l];
-            S.red[warp][base + lane] = (w[0] + w[1]) + (w[2] + w[3]);
+            double &red = S.red[warp][base + lane];
+            const double sum = (w[0] + w[1]) + (w[2] + w[3]);
+            red = add ? red + sum : sum;
         }
         __syncwarp();
     }
-    __syncthreads();
 }
 template <int IB>
 NB6_DEV double jpar_total(const JparI<IB> &S, int t) {
@@ -1341,7 +1353,8 @@ __global__ void __launch_bounds__(JPAR_NT, IB <= 4 ? JPAR_CTAS : JPAR_CTAS / 2) 
     const int j_end = (int)(((long long)(blockIdx.y + 1) * a.nj) / a.nslices);
     Sums s[IB];
     jpar_loop<IB, MFLAG, X2>(a, S, 0, j_begin, j_end, i0, nvalid, 0, s);
-    jpar_reduce<IB>(S, s);
+    jpar_fold<IB>(S, s);
+    __syncthreads();
     jpar_partials<IB>(S, a.part, nvalid, [&](int k) { return (size_t)blockIdx.y * a.ni_pad + i0 + k; });
 }
 
@@ -1428,9 +1441,14 @@ __global__ void __launch_bounds__(JPAR_NT, JPAR_CTAS)
         jpar_stage_i<IB, X2>(S, buf, it.ni);
         if (wn < nitems) jpar_fetch_i<IB>(a, S, buf ^ 1, nx.i0, nx.ni);
         __syncthreads();
-        Sums s[IB];
-        jpar_loop<IB, MFLAG, X2>(a, S, buf, it.j0, it.j1, it.i0, it.ni, it.jbase, s);
-        jpar_reduce<IB>(S, s);
+        const int half = (it.j1 - it.j0 + 2 * JPAR_NT - 1) / (2 * JPAR_NT);
+        const int len = JPAR_NT * (it.Q > 1 ? SEG_FOLD : max(SEG_FOLD_MIN, min(half, SEG_FOLD)));
+        for (int j0 = it.j0; j0 < it.j1; j0 += len) {
+            Sums s[IB];
+            jpar_loop<IB, MFLAG, X2>(a, S, buf, j0, min(j0 + len, it.j1), it.i0, it.ni, it.jbase, s);
+            jpar_fold<IB>(S, s, j0 != it.j0);
+        }
+        __syncthreads();
         if (ro.outf && it.Q == 1) {
             if (tid < 8 * IB && (tid >> 3) < it.ni) {
                 const int k = tid >> 3, c = tid & 7;
@@ -1683,8 +1701,9 @@ Plan make_plan(int variant, int ni, int nj, int ntile, bool mf, int forced_slice
         p.igrid = (ni + ib - 1) / ib;
         const double steps = std::max(1.0, (double)nj / JPAR_NT);
         double best = 1e300;
+        const double least = std::ceil(steps / JPAR_CHAIN);   // (its FP32 sums stay short)
         for (int w = 1; w <= 8; ++w) {
-            const int sl = (int)std::max(1.0, std::min((double)((long long)w * target / p.igrid), steps));
+            const int sl = (int)std::max(least, std::min((double)((long long)w * target / p.igrid), steps));
             const int waves = (int)(((long long)p.igrid * sl + target - 1) / target);
             const double cost = waves * (std::ceil(steps / sl) + 4.0);
             if (cost < best) {

@@ -407,3 +407,45 @@ def test_kernel_times_of_small_and_large_calls(nb6):
             assert b > a
     finally:
         nb6.irr_close(0)
+
+
+@pytest.mark.parametrize("kind", ["segments", "j-parallel"])
+def test_long_sums(nb6, kind):
+    """Active bodies far outside a compact clump of bodies of one mass: every
+    thread adds nearly the same term again and again, and its FP32 sum drifts
+    the same way in all of them.  A sum of N equal terms is off by at most N / 2
+    half-ulps of its value: 32 terms in a segmented call, 128 in a j-parallel
+    one, and six more half-ulps for the terms."""
+    seg = kind == "segments"
+    nseg, nc, na = (2, 65536, 6000) if seg else (1, 262144, 6000)
+    rng = np.random.default_rng(7)
+    n, ni = nseg * nc, nseg * na
+    x, v, m = 1e-6 * rng.normal(size=(n, 3)), 1e-6 * rng.normal(size=(n, 3)), np.full(n, 1.0 / nc)
+    xi = np.zeros((ni, 3))
+    xi[:, 0] = np.tile(1.0 + np.arange(na) / na, nseg)
+    xi[:, 1] = 0.3 * xi[:, 0]
+    vi = np.tile([0.0, 0.7, 0.0], (ni, 1))
+    h2, dtr = np.full(ni, 1e-4), np.full(ni, 2.0 ** -10)
+    nb6.gpunb_open(n, 0)
+    try:
+        nb6.gpunb_send(m, x, v)
+        if seg:
+            out = nb6.regf_seg(h2, dtr, xi, vi, np.repeat(np.arange(nseg), na), np.arange(nseg + 1) * nc, 64, 50, 0)
+        else:
+            nb6.lib.nb6_regf_tune_(C.byref(C.c_int(-1)), C.byref(C.c_int(0)))
+            out = nb6.gpunb_regf(h2, dtr, xi, vi, 64, 50, 0)
+    finally:
+        nb6.lib.nb6_regf_tune_(C.byref(C.c_int(0)), C.byref(C.c_int(0)))
+        nb6.gpunb_close()
+    bound = ((32 if seg else 128) / 2 + 6) * 2.0 ** -24
+    for k in range(0, ni, 250):
+        s = slice(k // na * nc, (k // na + 1) * nc)
+        dx, dv = x[s] - xi[k], v[s] - vi[k]
+        r2 = (dx * dx).sum(1)
+        mr3 = m[s] / (r2 * np.sqrt(r2))
+        al = -3.0 * (dx * dv).sum(1) / r2
+        for got, ref in ((out[0][k], (mr3[:, None] * dx).sum(0)),
+                         (out[1][k], (mr3[:, None] * (dv + al[:, None] * dx)).sum(0)),
+                         (out[2][k:k + 1], (m[s] / np.sqrt(r2)).sum(keepdims=True))):
+            assert np.linalg.norm(got - ref) <= bound * np.linalg.norm(ref)
+        assert out[3][k, 0] == 0
