@@ -13,8 +13,12 @@
 //
 // NB6_COPY_THREADS sets the number of parts (1 = the calling thread alone);
 // the default is min(4, hardware threads / 2).  One pool serves the whole
-// library (nb6_copy_pool); its threads start with the first large call and
-// stop when the last of the regular and irregular libraries is closed.
+// library (nb6_copy_pool); its threads start with the first large copy of any
+// call and stop when the last of the regular and irregular libraries is closed.
+// Calls that need neither open (gpupot_, the radius model) may start them with
+// none open: asleep between calls, they then stop with the next such close or
+// at exit.  A forked child has none of them: it copies on the calling thread and
+// leaves what belongs to them alone.
 #pragma once
 
 #include <atomic>
@@ -37,7 +41,14 @@
 
 class CopyPool {
   public:
-    ~CopyPool() { stop(); }
+    CopyPool() = default;
+    CopyPool(const CopyPool &) = delete;
+    ~CopyPool() {
+        stop();
+        // (helpers left: a forked child, which cannot join them, nor end the
+        // condition variable that they waited on)
+        if (th_.empty()) delete sh_;
+    }
 
     static int default_parts() {
         if (const char *e = getenv("NB6_COPY_THREADS")) {
@@ -139,9 +150,14 @@ class CopyPool {
         }
     }
 
-    std::vector<std::thread> th_;
+    struct Shared {
+        std::vector<std::thread> th;
+        std::condition_variable cv;
+    };
+    Shared *sh_ = new Shared;
+    std::vector<std::thread> &th_ = sh_->th;
+    std::condition_variable &cv_ = sh_->cv;
     std::mutex mu_;
-    std::condition_variable cv_;
     std::atomic<unsigned> gen_{0};
     std::atomic<int> left_{0};
     std::atomic<bool> quit_{false};

@@ -73,3 +73,48 @@ def test_copy_pool_default_parts_from_environment(tmp_path):
     env = {k: v for k, v in os.environ.items() if k != "NB6_COPY_THREADS"}
     r = subprocess.run([str(exe)], capture_output=True, text=True, env=env)
     assert 1 <= int(r.stdout) <= 4
+
+
+FORK_PROGRAM = textwrap.dedent(r"""
+    #include "copy_pool.h"
+    #include <cstdio>
+    #include <sys/wait.h>
+    static CopyPool pool;
+    int main() {
+        pool.start(4);
+        int hits[4] = {};
+        pool.run([&](int p) { ++hits[p]; });
+        std::this_thread::sleep_for(std::chrono::milliseconds(20));   // helpers asleep
+        const pid_t child = fork();
+        int rc = 0;
+        if (child == 0) {
+            pool.run([&](int p) { ++hits[p]; });   // every part on the calling thread
+            for (int h : hits) rc |= h != 2;
+            return rc;                             // through the static destructors
+        }
+        for (int t = 0, st = 0; t < 500; ++t) {
+            if (waitpid(child, &st, WNOHANG) == child) {
+                printf("child %s\n", WIFEXITED(st) && WEXITSTATUS(st) == 0 ? "ok" : "failed");
+                return 0;
+            }
+            std::this_thread::sleep_for(std::chrono::milliseconds(10));
+        }
+        kill(child, SIGKILL);
+        printf("child hangs\n");
+        return 0;
+    }
+""")
+
+
+def test_copy_pool_in_a_forked_child(tmp_path):
+    """A child forked while helpers exist has none of them: its jobs run on the
+    calling thread, and it exits by itself."""
+    gxx = shutil.which("g++")
+    if gxx is None:
+        pytest.skip("no g++")
+    src = tmp_path / "pool_fork.cpp"
+    src.write_text("#include <csignal>\n" + FORK_PROGRAM)
+    exe = tmp_path / "pool_fork"
+    subprocess.run([gxx, "-O2", "-std=c++17", "-pthread", "-I", CSRC, str(src), "-o", str(exe)], check=True)
+    r = subprocess.run([str(exe)], capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0 and r.stdout.strip() == "child ok", r.stdout + r.stderr
