@@ -2555,6 +2555,14 @@ void gpunb_close_() {
     R.nbbuf.release();
     R.outf.release();
     R.outl.release();
+    R.tiles.release();
+    R.tilesd.release();
+    R.tiles_ver = R.tilesd_ver = -1;
+    R.tbox.release();
+    R.order.release();
+    R.iperm.release();
+    R.hseg.release();
+    R.dseg.release();
     R.hin.release();
     R.stage_done.release();
     R.stage_flag.release();

@@ -90,6 +90,15 @@ struct SpatialOrder {
     DevBuf<int> vals_in, perm;
     DevBuf<unsigned char> tmp;
 
+    void release() {
+        keys_in.release();
+        keys_out.release();
+        ext.release();
+        vals_in.release();
+        perm.release();
+        tmp.release();
+    }
+
     void build(int n, const double *x, cudaStream_t st) {
         keys_in.reserve(n);
         keys_out.reserve(n);

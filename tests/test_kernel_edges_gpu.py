@@ -449,3 +449,39 @@ def test_long_sums(nb6, kind):
                          (out[2][k:k + 1], (m[s] / np.sqrt(r2)).sum(keepdims=True))):
             assert np.linalg.norm(got - ref) <= bound * np.linalg.norm(ref)
         assert out[3][k, 0] == 0
+
+
+def test_close_gives_the_device_memory_back(nb6):
+    """A session over a set larger than any before it, through every layout and
+    kernel form of the regular force: what it took on the device is free again
+    after the close (but for what the context keeps for its kernels: a first,
+    small session loads those; allocations come in units of 2 MB)."""
+    import torch
+    rng = np.random.default_rng(3)
+
+    def session(n):
+        x, v, m = rng.normal(size=(n, 3)), 0.1 * rng.normal(size=(n, 3)), np.full(n, 1.0 / n)
+        ni = 300
+        h2, dtr = np.full(ni, 1e-4), np.full(ni, 2.0 ** -8)
+        nb6.gpunb_open(n, 0)
+        try:
+            nb6.gpunb_send(m, x, v)
+            for variant in (11, 13, 12, -4, 1, 11):
+                nb6.lib.nb6_regf_tune_(C.byref(C.c_int(variant)), C.byref(C.c_int(0)))
+                last = nb6.gpunb_regf(h2, dtr, x[:ni], v[:ni], 512, 400, 0)
+            iseg, j0 = np.repeat([0, 1], ni // 2), np.array([0, n // 2, n])
+            nb6.regf_seg(h2, dtr, x[:ni], v[:ni], iseg, j0, 512, 400, 0)
+        finally:
+            nb6.lib.nb6_regf_tune_(C.byref(C.c_int(0)), C.byref(C.c_int(0)))
+            nb6.gpunb_close()
+        return last
+
+    session(40000)
+    free = torch.cuda.mem_get_info()[0]
+    n = 1500000
+    state = rng.bit_generator.state
+    first = session(n)
+    assert free - torch.cuda.mem_get_info()[0] <= 8 << 20
+    rng.bit_generator.state = state
+    for a, b in zip(first, session(n)):     # and a session after it starts afresh
+        np.testing.assert_array_equal(a, b)
