@@ -463,7 +463,8 @@ __global__ void __launch_bounds__(32) mlp_moments(int n, const double *__restric
         s1 += part[b * MOM_N + 2 * k];
         s2 += part[b * MOM_N + 2 * k + 1];
     }
-    const double mean = s1 / n, var = fmax(s2 / n - mean * mean, 1e-12);
+    const double mean = s1 / n, v = s2 / n - mean * mean;
+    const double var = v < 1e-12 ? 1e-12 : v;   // (a NaN stays one, as the mean does; fmax would drop it)
     if (k < MLP_IN) {
         norm[k] = (float)mean;
         norm[MLP_IN + k] = (float)(1.0 / sqrt(var));

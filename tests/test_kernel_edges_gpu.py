@@ -124,6 +124,30 @@ def test_mlp_training_steps(shuffled, n, batch):
     assert np.linalg.norm(got[:M.NPARAM] - w) <= 0.02 * np.linalg.norm(w - model[:M.NPARAM])
 
 
+def test_mlp_moments_of_unusable_columns():
+    """A NaN or an infinity among the samples shows in the stored moments of its
+    column, mean and scale (the variance is a NaN), and in no other; a constant
+    column has the least variance, 1e-12."""
+    import mlp_oracle as M
+    from nb6b200 import mlp
+    rng = np.random.default_rng(4)
+    n = 2500
+    x, y = rng.normal(size=(n, 5)).astype(np.float32), rng.normal(size=n).astype(np.float32)
+    x[1700, 1], x[3, 2], x[:, 3] = np.nan, np.inf, 2.0
+    model = np.zeros(M.NPARAM + M.NNORM, dtype=np.float32)
+    model[M.NPARAM + M.IN:M.NPARAM + 2 * M.IN] = 1.0
+    model[-1] = 1.0
+    mlp.set_model(model)
+    mlp.train(x, y, epochs=0, batch=100, lr=1e-3, seed=1)
+    mean, scale = np.split(mlp.get_model()[M.NPARAM:M.NPARAM + 10], 2)
+    assert np.isnan(mean[1]) and np.isnan(scale[1])
+    assert np.isposinf(mean[2]) and np.isnan(scale[2])
+    assert mean[3] == 2.0 and scale[3] == np.float32(1e6)
+    ok = x[:, [0, 4]].astype(np.float64)
+    np.testing.assert_allclose(mean[[0, 4]], ok.mean(0), atol=1e-6)
+    np.testing.assert_allclose(scale[[0, 4]], 1 / ok.std(0), rtol=1e-6)
+
+
 def _shells(n, seed):
     """n bodies, of which the first 40 sit at the centre of dense shells: most
     pairs of theirs lie within 1% of their radius, inside and outside."""
