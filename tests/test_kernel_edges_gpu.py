@@ -1,8 +1,9 @@
 """The force kernels at the sizes where their tiles, ranges and queues can go
 wrong, against the FP64 oracle.  Tolerances: the per-particle bounds of the
-other parity tests (acceleration and potential 1e-6, jerk 1e-5 relative), which
-the FP32 pair math on hi/lo differences with double-single sums meets at any
-size; neighbour lists identical."""
+other parity tests (acceleration and potential 1e-6, jerk 1e-5), which the FP32
+pair math on hi/lo differences with double-single or FP64 sums meets at any size:
+relative to the value where its terms mostly add up, to the sum of the terms'
+sizes (_sizes) where they may cancel; neighbour lists identical."""
 import ctypes as C
 import subprocess
 
@@ -148,6 +149,17 @@ def test_mlp_moments_of_unusable_columns():
     np.testing.assert_allclose(scale[[0, 4]], 1 / ok.std(0), rtol=1e-6)
 
 
+def _sizes(m, x, v, xi, vi, near):
+    """Sums of the sizes of one body's acceleration and jerk terms over the
+    bodies that are not its neighbours."""
+    d, w = x - xi, v - vi
+    r2 = (d * d).sum(1)
+    use = (r2 > 0) & ~np.isin(np.arange(len(m)), near)
+    d, w, r2, m = d[use], w[use], r2[use], m[use]
+    r = np.sqrt(r2)
+    return (m / r2).sum(), (m / (r * r2) * (np.sqrt((w * w).sum(1)) + 3 * np.abs((d * w).sum(1)) / r)).sum()
+
+
 def _shells(n, seed):
     """n bodies, of which the first 40 sit at the centre of dense shells: most
     pairs of theirs lie within 1% of their radius, inside and outside."""
@@ -192,18 +204,15 @@ def test_candidate_queue_band_and_overflow(nb6, orc, variant, n):
                 k = max(int(ol[r, 0]), 0)
                 np.testing.assert_array_equal(lst[r, 1:1 + k], ol[r, 1:1 + k])
             # FP32 sums of n terms against the sum of their sizes
-            j = np.arange(n)
             for r in range(ni):
-                d = x - x[r]
-                r2 = (d * d).sum(1)
-                use = (r2 > 0) & ~np.isin(j, ol[r, 1:1 + max(int(ol[r, 0]), 0)])
                 if ol[r, 0] < 0:
                     continue
                 if np.isnan(oa[r]).any():   # radius zero: the body acts on itself
                     assert h2[r] == 0.0 and np.isnan(acc[r]).any()
                     continue
-                size = (m[use] / r2[use]).sum()
-                assert np.abs(acc[r] - oa[r]).max() <= 1e-6 * size
+                sa, sj = _sizes(m, x, v, x[r], v[r], ol[r, 1:1 + max(int(ol[r, 0]), 0)])
+                assert np.abs(acc[r] - oa[r]).max() <= 1e-6 * sa
+                assert np.abs(jrk[r] - oj[r]).max() <= 1e-5 * sj
                 assert abs(pot[r] - op[r]) <= 1e-6 * abs(op[r]) + 1e-300
     finally:
         raw.nb6_regf_tune_(C.byref(C.c_int(0)), C.byref(C.c_int(0)))
@@ -356,13 +365,14 @@ def test_failed_segmented_call_leaves_the_callers_arrays(nb6, orc):
         np.testing.assert_array_equal(out[3][s], ol)
 
 
-@pytest.mark.parametrize("cap", [20, 60, 600])
-def test_segmented_many_items(nb6, orc, cap):
+@pytest.mark.parametrize("cap,mf", [(20, 0), (60, 0), (60, 1), (600, 0)])
+def test_segmented_many_items(nb6, orc, cap, mf):
     """A segmented call of many work items per CTA, whose rows reach the
-    caller in stages while later ones compute: ragged segments, groups of
-    one to four, a lone body, an empty segment in between, rows that
-    overflow (cap 20), rows longer than the kernel sorts itself (cap 600);
-    every row against the oracle of its segment."""
+    caller in stages while later ones compute (cap 20 and 60): ragged segments,
+    groups of one to four, a lone body, an empty segment in between, rows that
+    overflow (cap 20), rows longer than the kernel sorts itself (cap 600),
+    radii that scale with the bodies' masses (mf 1); every row against the
+    oracle of its segment."""
     rng = np.random.default_rng(cap)
     ns = np.concatenate([rng.integers(250, 420, 66), [0, 1, 2, 3]])
     rng.shuffle(ns)
@@ -371,23 +381,31 @@ def test_segmented_many_items(nb6, orc, cap):
     x, v = rng.normal(size=(n, 3)), 0.3 * rng.normal(size=(n, 3))
     m = rng.uniform(0.5, 1.5, n) / n
     iseg = np.repeat(np.arange(len(ns)), ns).astype(np.int32)
-    h2 = rng.uniform(0.2, 0.8, n) ** 2
+    h2 = rng.uniform(0.2, 0.8, n) ** 2 * (n if mf else 1)
     dtr = np.full(n, 2.0 ** -6)
     nb6.gpunb_open(n, 0)
     try:
         nb6.gpunb_send(m, x, v)
         for _ in range(2):
-            acc, jrk, pot, lst = nb6.regf_seg(h2, dtr, x, v, iseg, j0, cap + 1, cap, 0)
+            acc, jrk, pot, lst = nb6.regf_seg(h2, dtr, x, v, iseg, j0, cap + 1, cap, mf)
+            geom = (C.c_int * 3)()
+            nb6.lib.nb6_regf_last_geometry_(geom)
+            if cap <= 512:                # eight rounds of items: in stages
+                assert geom[2] > 7 * geom[1]
             for c in range(len(ns)):
                 s = slice(j0[c], j0[c + 1])
                 if ns[c] == 0:
                     continue
-                oa, oj, op, ol = orc.regf(m[s], x[s], v[s], h2[s], dtr[s], x[s], v[s], cap + 1, cap, 0)
+                oa, oj, op, ol = orc.regf(m[s], x[s], v[s], h2[s], dtr[s], x[s], v[s], cap + 1, cap, mf)
                 np.testing.assert_array_equal(lst[s], ol)
                 ok = (np.abs(oa).sum(1) > 0) & (ol[:, 0] >= 0)
                 if ok.any():
                     assert rel_err_vec(acc[s][ok], oa[ok]).max() <= 1e-5
                     assert rel_err_vec(pot[s][ok], op[ok]).max() <= 1e-6
+                for r in np.flatnonzero(ok)[::5]:
+                    sa, sj = _sizes(m[s], x[s], v[s], x[s][r], v[s][r], ol[r, 1:1 + ol[r, 0]])
+                    assert np.abs(acc[s][r] - oa[r]).max() <= 1e-6 * sa
+                    assert np.abs(jrk[s][r] - oj[r]).max() <= 1e-5 * sj
     finally:
         nb6.gpunb_close()
 
