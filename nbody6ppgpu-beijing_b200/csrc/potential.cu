@@ -34,7 +34,12 @@ constexpr int ROWS_HL = 7, ROWS_ORD = 10;
 // least POT_ORDER_MIN bodies, orders the set: the order costs about 80 us at
 // 131,071 bodies, and a far pair takes half the time of a near one.  (32,767 of
 // 131,071 bodies, 4.3e9 pairs: 3,017 us as a scalar loop over the unordered
-// set, 1,480 us ordered and packed, the order included.)
+// set, 1,480 us ordered and packed, the order included.)  A far pair has one
+// FP32 difference and no Newton step, yet the sums are no further off than the
+// scalar loop's over hi/lo differences, which folded 128 terms at a time: on
+// ranges of 1/8 to 1/2 of 45,000 to 239,999 bodies 0.8-1.3e-8 of the potential
+// (2-norm) against 1.5-1.8e-8, on sets with heavy bodies, two clumps, a distant
+// origin or one shell 0.8-12e-8 against 1.5-33e-8.
 constexpr int POT_ORDER_MIN = 32768;
 constexpr double POT_ORDER_PAIRS = 1.0e9;
 
@@ -461,7 +466,12 @@ bool pot_compute(int i0, int ni, double *hout, cudaStream_t st) {
                                                  P.span.ptr);
         NB6_CUDA_CHECK(cudaGetLastError());
     }
-    // two i per thread once that still leaves a tile of i for every SM
+    // two i per thread from a tile of 256 i per eight SMs (the slices fill the
+    // rest).  The line matters little: 33.8 us with one and 34.4 with two for a
+    // set of 5,000, 108.7 and 106.0 for 12,000, 251 and 245 for 20,000; 4,500 i of
+    // 131,071 ordered bodies 368 and 358, 7,000 539 and 559, all of 100,000 3,144
+    // and 3,091, of 249,036 18.0 and 17.3 ms; below it 3,000 of 131,071 259 and
+    // 272, of 249,036 463 and 450
     const bool two = ni >= 2 * NT * nb6_num_sms() / 8;
     if (ord) two ? pot_launch<2, true>(a, st) : pot_launch<1, true>(a, st);
     else two ? pot_launch<2, false>(a, st) : pot_launch<1, false>(a, st);

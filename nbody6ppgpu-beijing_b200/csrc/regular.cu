@@ -17,7 +17,8 @@
 //                   loop, so the list equals the FP64 rule's list.
 //   regf_finalize   one warp per i: deterministic FP64 sum of the slice
 //                   partials, and the neighbour ids sorted ascending (warp
-//                   bitonic sort in shared memory), overflow -> -nnb.
+//                   bitonic sort, of up to 512 ids in registers, of more in
+//                   shared memory), overflow -> -nnb.
 //
 // Semantics kept from the reference: acc/jrk/pot exclude neighbours, pot is
 // positive, jrk is adot, list ids are 0-based j relative to the first particle
@@ -1394,10 +1395,10 @@ __global__ void __launch_bounds__(FIN_WARPS * 32)
 // consecutive i of that segment, j chunk), built on the host with the costly
 // items first; one persistent launch of SMs x occupancy CTAs walks the list
 // (grid-stride), each item running the j-parallel inner loop of
-// regf_jpar_kernel (threads over j, the IB i in shared memory).  Item q of an
-// i writes its (hi, lo) partial to slot pinfo[i].x + q; regf_finalize_seg
-// sums the pinfo[i].y slots of each i in order.
-// ----------------------------------------------------------------------------
+// regf_jpar_kernel (threads over j, the IB i in shared memory).  Where a
+// group's j range is cut into several items, item q writes each i's (hi, lo)
+// partial to slot pinfo[i].x + q, and regf_finalize_seg sums the pinfo[i].y slots
+// of the i in order.
 //
 // A group whose j range is one item (Q = 1, nearly all groups of an ensemble)
 // is finished by its CTA: sums, list rows and their way over the bus then
@@ -1406,6 +1407,7 @@ __global__ void __launch_bounds__(FIN_WARPS * 32)
 // item and its i data, which are read from the caller's staging over the bus,
 // are fetched during this one.  The host copies the finished rows of a stage
 // into the caller's arrays while the next one computes.
+// ----------------------------------------------------------------------------
 struct SegItem {
     int i0, ni, j0, j1, jbase, q, Q, slot;   // slot: of the group's first particle
 };
@@ -1641,7 +1643,8 @@ int i_per_thread(int v) { return v == 13 ? 1 : v > 10 ? v - 10 : v; }
 
 // The j-parallel and segmented kernels with two or more i per CTA run the
 // packed (f32x2) inner loop; NB6_JPAR_X2=0 in the environment selects the
-// scalar loop (the same bits, for comparison).
+// scalar loop, for comparison: the same lists and pair terms, whose sums take
+// the candidates' shares in another order (equal within the FP32 rounding).
 bool jpar_x2() {
     static const bool on = [] {
         const char *e = getenv("NB6_JPAR_X2");
@@ -1695,7 +1698,7 @@ Plan make_plan(int variant, int ni, int nj, int ntile, bool mf, int forced_slice
         p.nslices = std::max(p.nslices, 1);
     } else {
         // the j range of each i-group cut so that the launch is short: w
-        // waves of CTAs, each of nj / (256 slices) steps and about four
+        // waves of CTAs, each of nj / (JPAR_NT slices) steps and about four
         // steps' worth of set-up and reduction
         const int ib = -variant;
         p.igrid = (ni + ib - 1) / ib;
@@ -1777,10 +1780,11 @@ int ilog2(int v) {
 }
 
 // ----------------------------------------------------------------------------
-// Spatial order of the j set.  After every send the bodies are put in Morton
-// (Z-curve) order of their positions, so that the 128 bodies of a tile are
-// close together, and each tile gets a bounding box.  The packed kernel then
-// skips the neighbour-candidate arithmetic for every (warp, tile) whose box is
+// Tile layout and spatial order of the j set.  When a packed tile kernel is to
+// run on a new set (ensure_tiles), its layout is made from the FP64 bodies; those
+// of a large set are put in Morton (Z-curve) order of their positions for it, so
+// that the 128 bodies of a tile are close together, and each tile gets a
+// bounding box.  The packed kernel then skips the neighbour-candidate arithmetic for every (warp, tile) whose box is
 // provably out of reach of all the warp's i-particles.  Slot k of the ordered
 // set holds the caller's body perm[k]; the exact FP64 path maps slots back, so
 // neighbour ids are the caller's.
@@ -2171,8 +2175,11 @@ static void regf_prepare(int ni, const double *d_h2, const double *d_dtr, const 
     int cands[12], ncand = 0;
     if (tune_now) {
         if (ni >= NT / 2) {
-            // (the scalar kernels and the FP64 differences are for callers
-            // that force them: they were never the fastest)
+            // (the scalar kernels and the FP64 differences are for callers that
+            // force them.  Kernel times of variants 1, 2, 4, 13 against 11: 1,024
+            // i on 65,536 bodies 344, 510, 984, 131 and 121 us; 1,024 on 990,000
+            // 2,127, 2,251, 3,213, 1,608 and 1,076; 531 on 16,384 108, 256, 880, 31
+            // and 31; 300 on 250,000 321, 500, 692, 172 and 135)
             cands[ncand++] = 11;
             if (ni >= NT * 2) cands[ncand++] = 12;
         }
@@ -2985,9 +2992,10 @@ void nb6_regf_seg_(int *ni_, int *iseg, double *h2, double *dtr, double (*xi)[3]
         }
     const int nrun = (int)run_k0.size();
     run_k0.push_back(ni);
-    // at most 4: the IB = 8 form needs 184 registers (one CTA of 8 warps per
-    // SM) against 112 for IB = 4 (two CTAs), and ran 15-17% slower on
-    // ensembles of 2-100% active bodies
+    // at most 4: built with eight i the kernel takes 207 registers, two CTAs of
+    // four warps per SM against four, and ran slower at every active share of 64
+    // clusters of 512-8,192 bodies (2, 10, 30, 100%: 98, 354, 973, 3,154 us against
+    // 81, 305, 841, 2,693; with two i 100, 386, 1,077, 3,466)
     int ib = 1;
     while (ib < 4 && ib * nrun < ni) ib <<= 1;
     const int grid_max = nb6_num_sms() * seg_occupancy(ib, mf);
