@@ -1600,10 +1600,13 @@ KsArgs ks_args() {
 // the record walk serves the call: with a pair table, or when the call's
 // list entries (ni x the mean list length) number fewer than 4 per body
 // set.  The prediction pass reads every record set so far and writes its
-// 64-byte body (192 bytes per body) and saves 64 bytes per list entry; on
-// a B200 (lists of 64 in a Plummer N = 262,144) the call took 7% less time
-// at 4 entries per body set, 16% less at 16, the same at 2 and 9% more at
-// 1.
+// 64-byte body (192 bytes per body) and saves 64 bytes per list entry.  The
+// line was drawn while each lane gathered its own record: the call (lists of
+// 64 in a Plummer N = 262,144) took 7% less time at 4 entries per body set, 16%
+// less at 16, the same at 2 and 9% more at 1.  With the warp's gathers both
+// walks are faster and the sets cost as much as they save: at 1, 2, 4, 8 and 16
+// entries 59, 72, 87, 129 and 200 us by the set, 54, 65, 83, 123 and 200 by the
+// records.
 bool irr_wants_predicted_set(int ni) {
     if (I.pv_mode < 0) {
         const char *e = getenv("NB6_IRR_PV");
